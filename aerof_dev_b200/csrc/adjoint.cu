@@ -1374,7 +1374,7 @@ void dRdX_T_dev(aerof_gpu_ctx* c, const double* dU, const double* dlam, double* 
   const size_t n5 = 5 * (size_t)m.N;
   c->s.k2.ensure(n5);
   double* R = c->s.k2.p;
-  residual_dev(c, dU, R);
+  residual_dev(c, dU, R, kCountSum);
   // node records P in the caller's numbering for the node and face passes
   prim_dev(c, dU);
   a.lam.ensure(n5);

@@ -124,9 +124,13 @@ extern "C" int aerof_gpu_create(const aerof_gpu_config* cfg, aerof_gpu_ctx** out
   aerof_gpu_ctx* c = new aerof_gpu_ctx();
   c->cfg = *cfg;
   c->dev = cfg->device;
+  auto& hc = c->s.host_count;
   if (cudaSetDevice(c->dev) != cudaSuccess ||
-      cudaStreamCreateWithFlags(&c->own_stream, cudaStreamNonBlocking) != cudaSuccess) {
+      cudaStreamCreateWithFlags(&c->own_stream, cudaStreamNonBlocking) != cudaSuccess ||
+      cudaHostAlloc((void**)&hc.host, sizeof(int), cudaHostAllocMapped) != cudaSuccess ||
+      cudaHostGetDevicePointer((void**)&hc.dev, hc.host, 0) != cudaSuccess) {
     cudaGetLastError();
+    if (c->own_stream) cudaStreamDestroy(c->own_stream);
     delete c;
     return AEROF_ECUDA;
   }

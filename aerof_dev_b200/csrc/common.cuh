@@ -154,6 +154,7 @@ struct DeviceMesh {
   // ---- blocked residual: Morton-renumbered copy of the node data ----
   int NB = 256;            // nodes per block
   int nblk = 0, maxE = 0, nX = 0, maxH = 0, maxL = 0, maxHf = 0, maxLp = 0;
+  int grad_grid = 0;       // resident CTAs of the persistent gradient kernel (0: not asked yet)
   DBuf<int> n2o, o2n;      // [N] new -> old and old -> new node ids
   DBuf<double> P2;         // [N][8] node records in new numbering
   DBuf<double> W2;         // [6][N] LSQ constants, new numbering
@@ -235,6 +236,17 @@ struct Scratch {
   DBuf<double> dt, k1, k2, U0;
   DBuf<int> tag;           // [N] failsafe tags
   DBuf<int> counters;      // [8] device counters
+  // page-locked word that the node assembly writes the unphysical count to,
+  // and whether the device counter is known to be zero
+  struct HostWord {
+    int* host = nullptr;
+    int* dev = nullptr;
+    ~HostWord() {
+      if (host) cudaFreeHost(host);
+    }
+  } host_count;
+  bool count_clear = false;
+  DBuf<double> gsplit;     // [3][N][5] staging of aerof_gpu_gradients' host outputs
   DBuf<double> red;        // reduction partials
   DBuf<double> tetc;       // [4T][4] Galerkin shares of each (tet, vertex)
   DBuf<double> viscq;      // [N][8] node records of the Galerkin term
@@ -478,9 +490,14 @@ __device__ __forceinline__ void prefetch_pairs_l2(const double2* h2, size_t E, i
   if (k < npair && e1 > e0) prefetch_l2_bulk(h2 + (size_t)k * E + e0, 16u * (unsigned)(e1 - e0));
 }
 
-// implemented in residual.cu (used by implicit.cu and adjoint.cu).  With
-// sync == false the unphysical count is left on the device (counters[2]).
-int residual_dev(aerof_gpu_ctx* c, const double* dU, double* dR, bool sync = true);
+// Residual of device state dU into device dR (both [N][5]), implemented in
+// residual.cu.  kCountSync: waits and returns the number of non-positive
+// reconstructed states of the first pass.  Otherwise nothing waits and that
+// number is added to the device counter of the mode's index (returns 0);
+// with the failsafe on every mode is kCountSync.  kCountAsync: the counter
+// of aerof_gpu_status; kCountSum: one that the caller zeroes and reads.
+constexpr int kCountSync = 0, kCountAsync = 2, kCountSum = 3;
+int residual_dev(aerof_gpu_ctx* c, const double* dU, double* dR, int mode = kCountSync);
 void prim_dev(aerof_gpu_ctx* c, const double* dU);
 void prim_grad_blocked_dev(aerof_gpu_ctx* c, const double* dU, const int* tag);
 void grad_records_blocked_dev(aerof_gpu_ctx* c, const double* P2src, double* G2dst);

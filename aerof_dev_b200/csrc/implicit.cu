@@ -2216,7 +2216,7 @@ double matvec_fd_dev(aerof_gpu_ctx* c, const double* dU, const double* dF, const
   J.fdFm.ensure(n);
   k_fd_shift<<<gv, kIB, 0, s>>>(n, eps, dU, dp, J.fdQ.p);
   AEROF_LAUNCH_CHECK();
-  residual_dev(c, J.fdQ.p, J.fdFp.p, true);
+  residual_dev(c, J.fdQ.p, J.fdFp.p, kCountSum);
   if (ddt) {
     k_fd_time<<<gv, kIB, 0, s>>>(n, J.fdQ.p, dU, ddt, J.fdFp.p);
     AEROF_LAUNCH_CHECK();
@@ -2224,7 +2224,7 @@ double matvec_fd_dev(aerof_gpu_ctx* c, const double* dU, const double* dF, const
   if (fd_order == 2) {
     k_fd_shift<<<gv, kIB, 0, s>>>(n, -eps, dU, dp, J.fdQ.p);
     AEROF_LAUNCH_CHECK();
-    residual_dev(c, J.fdQ.p, J.fdFm.p, true);
+    residual_dev(c, J.fdQ.p, J.fdFm.p, kCountSum);
     if (ddt) {
       k_fd_time<<<gv, kIB, 0, s>>>(n, J.fdQ.p, dU, ddt, J.fdFm.p);
       AEROF_LAUNCH_CHECK();
@@ -2233,7 +2233,7 @@ double matvec_fd_dev(aerof_gpu_ctx* c, const double* dU, const double* dF, const
   } else {
     const double* Fm = dF;
     if (!Fm) {
-      residual_dev(c, dU, J.fdFm.p, true);
+      residual_dev(c, dU, J.fdFm.p, kCountSum);
       Fm = J.fdFm.p;
     }
     k_fd_diff<<<gv, kIB, 0, s>>>(n, 1.0 / eps, J.fdFp.p, Fm, dy);
@@ -2431,10 +2431,12 @@ extern "C" int aerof_gpu_newton(aerof_gpu_ctx* c, double* U, const aerof_newton_
     AEROF_CUDA(cudaEventRecord(e0, s));
     double res0 = 0.0, rel = 1.0, rel_prev = 1.0, cfl = p->cfl0;
     int k = 0, lits = 0, bad = 0, redos = 0;
+    int* bad_d = c->s.counters.p + kCountSum;
+    AEROF_CUDA(cudaMemsetAsync(bad_d, 0, sizeof(int), s));
     bool redo = false;
     while (k <= p->max_steps) {
       if (!redo) {
-        bad += residual_dev(c, dU, R);
+        bad += residual_dev(c, dU, R, kCountSum);
         double res = norm2_dev(c, R, n);
         // a NaN initial residual would make res0 > 0 false and look converged
         if (!std::isfinite(res)) throw ApiError{AEROF_EINVAL, "non-finite residual in Newton step " + std::to_string(k)};
@@ -2501,7 +2503,10 @@ extern "C" int aerof_gpu_newton(aerof_gpu_ctx* c, double* U, const aerof_newton_
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     if (dU != U) AEROF_CUDA(cudaMemcpyAsync(U, dU, n * sizeof(double), cudaMemcpyDeviceToHost, s));
+    int bad_sum = 0;
+    AEROF_CUDA(cudaMemcpyAsync(&bad_sum, bad_d, sizeof(int), cudaMemcpyDeviceToHost, s));
     AEROF_CUDA(cudaStreamSynchronize(s));
+    bad += bad_sum;
     if (out) {
       out->steps = k;
       out->linear_its = lits;

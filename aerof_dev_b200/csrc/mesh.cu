@@ -482,6 +482,7 @@ extern "C" int aerof_gpu_set_mesh(aerof_gpu_ctx* c, int N, int T, int F, const d
     DeviceMesh& m = c->mesh;
     cudaStream_t s = c->stream;
     m.N = N; m.T = T; m.F = F; m.E = E;
+    m.grad_grid = 0;
     for (int k = 0; k < 5; ++k) m.Ub[k] = Ub[k];
     m.Ubd.upload(Ub, 5, s);
     m.X.upload(X, 3 * (size_t)N, s);

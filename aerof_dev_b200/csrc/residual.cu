@@ -32,12 +32,30 @@ __global__ void k_prim(int N, Gas g, const double* __restrict__ U, double* __res
   for (int k = 0; k < 5; ++k) P[8 * (size_t)i + k] = v[k];
 }
 
-// V[N][5] primitive (caller layout) copied into the node records.
-__global__ void k_setV(int N, const double* __restrict__ V, double* __restrict__ P) {
+// V[N][5] primitive (caller layout) copied into the node records: row n of P
+// from row n2o[n] of V (n2o null: the caller's numbering).
+__global__ void k_setV(int N, const int* __restrict__ n2o, const double* __restrict__ V, double* __restrict__ P) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= N) return;
+  const size_t o = (size_t)(n2o ? n2o[i] : i);
 #pragma unroll
-  for (int k = 0; k < 5; ++k) P[8 * (size_t)i + k] = V[5 * (size_t)i + k];
+  for (int k = 0; k < 5; ++k) P[8 * (size_t)i + k] = V[5 * o + k];
+}
+
+// Gradient records G[N][16] split into the three [N][5] arrays of
+// aerof_gpu_gradients, row n to row n2o[n] (n2o null: row n).  16 threads
+// per node, so that a warp reads whole records.  Bound by HBM (248 bytes per
+// node); the records used to be split on the host: 8.3 ms per call at 61^3,
+// 0.08 ms with this.
+__global__ void k_split_grad(int N, const int* __restrict__ n2o, const double* __restrict__ G, double* __restrict__ dx,
+                             double* __restrict__ dy, double* __restrict__ dz) {
+  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= 16 * (long long)N) return;
+  const int i = (int)(t >> 4), e = (int)(t & 15);
+  if (e == 15) return;
+  const size_t o = (size_t)(n2o ? n2o[i] : i);
+  double* const d = e < 5 ? dx : (e < 10 ? dy : dz);
+  d[5 * o + e % 5] = G[t];
 }
 
 // Least-squares gradients, ddV_i = sum_j W_i(X_j - X_i) (V_j - V_i), with
@@ -588,8 +606,15 @@ __global__ void k_fv_nodes_b(int N, Gas g, const int* __restrict__ n2o, const do
                              const double* __restrict__ fbuf, int F, const double* __restrict__ Ub0,
                              const int* __restrict__ fcode, const double* __restrict__ fn,
                              const double* __restrict__ P2, const double* __restrict__ vol2, double* __restrict__ R,
-                             const int* __restrict__ blist, int nlist, int NB) {
+                             const int* __restrict__ blist, int nlist, int NB, int* __restrict__ cnt,
+                             volatile int* __restrict__ pub) {
   int n = blockIdx.x * blockDim.x + threadIdx.x;
+  // the edge fluxes are complete: their unphysical count goes to the host's
+  // page-locked word, and the counter back to zero for the next call
+  if (pub && n == 0) {
+    *pub = *cnt;
+    *cnt = 0;
+  }
   if (blist) {
     // the nodes of blocks blist[0, nlist)
     const int i = n / NB;
@@ -918,9 +943,6 @@ static int* counters(aerof_gpu_ctx* c) {
   return c->s.counters.p;
 }
 
-// Residual of device state dU into device dR (both [N][5]).  Returns the
-// number of non-positive reconstructed states of the first pass (sync), or
-// 0 with the count accumulated in counters[2] (no sync, failsafe off).
 constexpr size_t kMaxStagedSmem = 160 * 1024;
 
 static int grad_kernel_choice() {
@@ -959,11 +981,17 @@ static void prim_to_P2(const DeviceMesh& m, const Gas& g, const double* dU, cuda
   AEROF_LAUNCH_CHECK();
 }
 
+// whether the persistent gradient kernel can stage this mesh's blocks
+// (AEROF_GRAD_KERNEL selects another organisation)
+static bool grad_piped(const DeviceMesh& m) {
+  return grad_kernel_choice() == 3 && m.maxH <= 512 && 2 * grad_stage(m).size * sizeof(double) <= kMaxStagedSmem;
+}
+
 // persistent pipelined gradients of the records P2src (with dU,
 // k_prim_blocked writes the mesh's P2 first and P2src is that)
 static void launch_grad_pipe(aerof_gpu_ctx* c, const Gas& g, const double* dU, const int* tag, double* G2,
                              cudaStream_t s, const double* P2src = nullptr) {
-  const DeviceMesh& m = c->mesh;
+  DeviceMesh& m = c->mesh;
   if (dU) {
     prim_to_P2(m, g, dU, s);
   }
@@ -973,11 +1001,13 @@ static void launch_grad_pipe(aerof_gpu_ctx* c, const Gas& g, const double* dU, c
   const int L = kBlock / m.NB;
   auto go = [&](auto kern) {
     AEROF_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    int per_sm = 0;
-    AEROF_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kBlock, smem));
-    int sms = 0;
-    AEROF_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->cfg.device));
-    const int grid = std::max(1, std::min(m.nblk, std::max(per_sm, 1) * sms));
+    if (!m.grad_grid) {  // resident CTAs of this mesh's staging size
+      int per_sm = 0, sms = 0;
+      AEROF_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kBlock, smem));
+      AEROF_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->cfg.device));
+      m.grad_grid = std::max(per_sm, 1) * sms;
+    }
+    const int grid = std::max(1, std::min(m.nblk, m.grad_grid));
     kern<<<grid, kBlock, smem, s>>>(m.N, m.NB, m.nblk, m.maxH, m.maxLp, st, P2src, m.W2.p, m.nb2_ptr.p, m.lpad.p,
                                     m.hpad.p, tag, G2, nullptr);
     AEROF_LAUNCH_CHECK();
@@ -1029,8 +1059,7 @@ void prim_grad_blocked_dev(aerof_gpu_ctx* c, const double* dU, const int* tag) {
   // 3 (default) staged, persistent and software pipelined
   const int gk = grad_kernel_choice();
   const bool staged = gsmem <= kMaxStagedSmem && gk != 2;
-  const bool piped = gk == 3 && m.maxH <= 512 && 2 * grad_stage(m).size * sizeof(double) <= kMaxStagedSmem;
-  if (piped) {
+  if (grad_piped(m)) {
     launch_grad_pipe(c, g, dU, tag, c->s.G2.p, s);
   } else if (staged) {
     launch_grad_staged(m, g, dU, tag, c->s.G2.p, gsmem, gk == 1, s);
@@ -1049,8 +1078,7 @@ void grad_records_blocked_dev(aerof_gpu_ctx* c, const double* P2src, double* G2d
   const DeviceMesh& m = c->mesh;
   const Gas g = make_gas(c->cfg.gamma);
   cudaStream_t s = c->stream;
-  const bool piped = grad_kernel_choice() == 3 && m.maxH <= 512 && 2 * grad_stage(m).size * sizeof(double) <= kMaxStagedSmem;
-  if (piped) {
+  if (grad_piped(m)) {
     launch_grad_pipe(c, g, nullptr, nullptr, G2dst, s, P2src);
   } else {
     k_grad<<<grid_for(4 * (size_t)m.N, kBlock), kBlock, 0, s>>>(m.N, P2src, m.W2.p, m.nb2_ptr.p, m.nb2_node.p, nullptr,
@@ -1060,19 +1088,26 @@ void grad_records_blocked_dev(aerof_gpu_ctx* c, const double* P2src, double* G2d
 }
 
 // BLOCKED organisation of residual_dev (see k_fv_blocked).
-static int residual_blocked_dev(aerof_gpu_ctx* c, const double* dU, double* dR, bool sync) {
+static int residual_blocked_dev(aerof_gpu_ctx* c, const double* dU, double* dR, int mode) {
   DeviceMesh& m = c->mesh;
   const Gas g = make_gas(c->cfg.gamma);
   const int rec = c->cfg.reconstruction;
   cudaStream_t s = c->stream;
   int* cnt = counters(c);
-  if (sync) AEROF_CUDA(cudaMemsetAsync(cnt, 0, sizeof(int) * 2, s));
-  int* ecnt = sync ? cnt : cnt + 2;
+  const bool failsafe = c->cfg.failsafe != 0;
+  // the synchronous count starts at zero: the node assembly leaves it so
+  // after publishing it, otherwise (first call, failsafe, a call that
+  // threw) it is cleared here
+  if (mode == kCountSync) {
+    if (failsafe || !c->s.count_clear) AEROF_CUDA(cudaMemsetAsync(cnt, 0, sizeof(int) * 2, s));
+    c->s.count_clear = false;
+  }
+  int* ecnt = mode == kCountSync ? cnt : cnt + mode;
   c->s.G2.ensure(16 * (size_t)m.N);
   c->s.part.ensure(5 * (size_t)m.N);
   c->s.spill.ensure(5 * (size_t)std::max(m.nX, 1));
   c->s.fbuf.ensure(15 * (size_t)std::max(m.F, 1));
-  if (c->cfg.failsafe) {
+  if (failsafe) {
     c->s.tag.ensure(m.N);
     c->s.tag.zero(s);
   }
@@ -1107,11 +1142,18 @@ static int residual_blocked_dev(aerof_gpu_ctx* c, const double* dU, double* dR, 
     TimerScope t(c, AEROF_T_FV_EDGES);
     fv(c->cfg.failsafe, ecnt);
   }
+  // only the failsafe needs the count before the assembly (it re-runs the
+  // edges); otherwise the whole residual is queued and waited for once, its
+  // count written to the host by the assembly.  Copying the count back and
+  // waiting for it before the assembly left the GPU idle for 12 us per call
+  // (641 -> 629 us per call at 101^3, 121 -> 103 us at 47^3; ten RK2 steps
+  // of 21^3, which now wait once: 1.32 -> 1.00 ms)
   int bad = 0;
-  if (sync) {
+  if (mode == kCountSync && failsafe) {
     AEROF_CUDA(cudaMemcpyAsync(&bad, cnt, sizeof(int), cudaMemcpyDeviceToHost, s));
     AEROF_CUDA(cudaStreamSynchronize(s));
   }
+  int* pub = mode == kCountSync && !failsafe ? c->s.host_count.dev : nullptr;
   c->s.p2g2_valid = true;
   if (bad && c->cfg.failsafe && rec != AEROF_REC_CONSTANT) {
     TimerScope t(c, AEROF_T_FV_TERM);
@@ -1130,7 +1172,7 @@ static int residual_blocked_dev(aerof_gpu_ctx* c, const double* dU, double* dR, 
     if (faces_in_nodes) {
       k_fv_nodes_b<true><<<grid_for(m.N, kBlock), kBlock, 0, s>>>(
           m.N, g, m.n2o.p, c->s.part.p, m.xin_ptr.p, c->s.spill.p, m.bnf_ptr.p, m.bnf_ent.p, nullptr, m.F, m.Ubd.p,
-          m.fcode.p, m.fnrm.p, m.P2.p, m.vol2.p, dR, nullptr, 0, m.NB);
+          m.fcode.p, m.fnrm.p, m.P2.p, m.vol2.p, dR, nullptr, 0, m.NB, cnt, pub);
     } else {
       if (m.F) {
         k_face_flux<<<grid_for(m.F, kBlock), kBlock, 0, s>>>(m.F, g, m.Ubd.p, m.faces.p, m.fcode.p, m.fnrm.p,
@@ -1139,24 +1181,35 @@ static int residual_blocked_dev(aerof_gpu_ctx* c, const double* dU, double* dR, 
       }
       k_fv_nodes_b<false><<<grid_for(m.N, kBlock), kBlock, 0, s>>>(
           m.N, g, m.n2o.p, c->s.part.p, m.xin_ptr.p, c->s.spill.p, m.bnf_ptr.p, m.bnf_ent.p, c->s.fbuf.p, m.F,
-          m.Ubd.p, m.fcode.p, m.fnrm.p, m.P2.p, m.vol2.p, dR, nullptr, 0, m.NB);
+          m.Ubd.p, m.fcode.p, m.fnrm.p, m.P2.p, m.vol2.p, dR, nullptr, 0, m.NB, cnt, pub);
     }
     AEROF_LAUNCH_CHECK();
+    if (pub) c->s.count_clear = true;
     galerkin_add(c, dU, dR);
+  }
+  if (pub) {
+    AEROF_CUDA(cudaStreamSynchronize(s));
+    bad = *c->s.host_count.host;
   }
   return bad;
 }
 
-int residual_dev(aerof_gpu_ctx* c, const double* dU, double* dR, bool sync) {
+int residual_dev(aerof_gpu_ctx* c, const double* dU, double* dR, int mode) {
   DeviceMesh& m = c->mesh;
   c->s.p2g2_valid = false;
+  // the failsafe decides on the host: its calls always wait
+  if (c->cfg.failsafe) mode = kCountSync;
   if (c->cfg.residual_kernel == AEROF_KERNEL_BLOCKED && fv_blocked_smem(m) <= 200 * 1024)
-    return residual_blocked_dev(c, dU, dR, sync);
+    return residual_blocked_dev(c, dU, dR, mode);
+  const bool sync = mode == kCountSync;
   const Gas g = make_gas(c->cfg.gamma);
   const int rec = c->cfg.reconstruction;
   int* cnt = counters(c);
-  if (sync) AEROF_CUDA(cudaMemsetAsync(cnt, 0, sizeof(int) * 2, c->stream));
-  int* ecnt = sync ? cnt : cnt + 2;
+  if (sync) {
+    AEROF_CUDA(cudaMemsetAsync(cnt, 0, sizeof(int) * 2, c->stream));
+    c->s.count_clear = false;
+  }
+  int* ecnt = sync ? cnt : cnt + mode;
   c->s.flux.ensure(5 * (size_t)m.E);
   c->s.G.ensure(16 * (size_t)m.N);
   if (c->cfg.failsafe) {
@@ -1393,7 +1446,7 @@ static void stage_kernels(aerof_gpu_ctx* c, ResidualPipe& p, int st, cudaStream_
     // small face kernel per stage)
     k_fv_nodes_b<true><<<grid_for((size_t)nl * m.NB, kBlock), kBlock, 0, s>>>(
         m.N, g, m.n2o.p, c->s.part.p, m.xin_ptr.p, c->s.spill.p, m.bnf_ptr.p, m.bnf_ent.p, nullptr, m.F, m.Ubd.p,
-        m.fcode.p, m.fnrm.p, m.P2.p, m.vol2.p, dR, lp, nl, m.NB);
+        m.fcode.p, m.fnrm.p, m.P2.p, m.vol2.p, dR, lp, nl, m.NB, nullptr, nullptr);
     AEROF_LAUNCH_CHECK();
   }
 }
@@ -1470,6 +1523,7 @@ static void pipelined_enqueue(aerof_gpu_ctx* c, ResidualPipe& p, const double* U
   double* dU = c->s.Ustage.p;
   double* dR = c->s.Rstage.p;
   AEROF_CUDA(cudaMemsetAsync(cnt, 0, sizeof(int) * 2, s));
+  c->s.count_clear = false;
   // the copy streams start after the work already queued on s (which may
   // still read Ustage or write Rstage)
   AEROF_CUDA(cudaEventRecord(p.ev_go, s));
@@ -1525,8 +1579,7 @@ static bool residual_host_pipelined(aerof_gpu_ctx* c, const double* U, double* R
   const bool grad = rec != AEROF_REC_CONSTANT;
   if (m.N < kPipeMinNodes || c->cfg.failsafe || c->visc.model != 0 || c->timers.on) return false;
   if (c->cfg.residual_kernel != AEROF_KERNEL_BLOCKED || fv_blocked_smem(m) > 200 * 1024) return false;
-  if (grad && grad_kernel_choice() != 3) return false;
-  if (grad && !(m.maxH <= 512 && 2 * grad_stage(m).size * sizeof(double) <= kMaxStagedSmem)) return false;
+  if (grad && !grad_piped(m)) return false;
   void* Rdev = nullptr;
   if (!pinned_host(U) || !pinned_host(R, &Rdev)) return false;
   ResidualPipe& p = pipe_for(c);
@@ -1614,7 +1667,7 @@ extern "C" int aerof_gpu_residual_async(aerof_gpu_ctx* c, const double* U, doubl
       counters(c);
       AEROF_CUDA(cudaMemsetAsync(c->s.counters.p, 0, sizeof(int) * 8, c->stream));
     }
-    residual_dev(c, U, R, false);
+    residual_dev(c, U, R, kCountAsync);
     return AEROF_OK;
   });
 }
@@ -1637,29 +1690,39 @@ extern "C" int aerof_gpu_gradients(aerof_gpu_ctx* c, const double* V, double* dd
     if (!V || !ddx || !ddy || !ddz) return AEROF_EINVAL;
     DeviceMesh& m = c->mesh;
     const size_t n5 = 5 * (size_t)m.N;
+    cudaStream_t s = c->stream;
     const double* dV = in_dev(c, V, n5, c->s.Vstage);
-    k_setV<<<grid_for(m.N, kBlock), kBlock, 0, c->stream>>>(m.N, dV, m.P.p);
-    AEROF_LAUNCH_CHECK();
-    gradients_dev(c);
-    std::vector<double> G(16 * (size_t)m.N);
-    AEROF_CUDA(cudaMemcpyAsync(G.data(), c->s.G.p, G.size() * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-    AEROF_CUDA(cudaStreamSynchronize(c->stream));
-    std::vector<double> hx(n5), hy(n5), hz(n5);
-    for (int i = 0; i < m.N; ++i)
-      for (int k = 0; k < 5; ++k) {
-        hx[5 * (size_t)i + k] = G[16 * (size_t)i + k];
-        hy[5 * (size_t)i + k] = G[16 * (size_t)i + 5 + k];
-        hz[5 * (size_t)i + k] = G[16 * (size_t)i + 10 + k];
-      }
-    double* outs[3] = {ddx, ddy, ddz};
-    std::vector<double>* src[3] = {&hx, &hy, &hz};
-    for (int a = 0; a < 3; ++a) {
-      if (is_device_ptr(outs[a]))
-        AEROF_CUDA(cudaMemcpyAsync(outs[a], src[a]->data(), n5 * sizeof(double), cudaMemcpyHostToDevice, c->stream));
-      else
-        std::copy(src[a]->begin(), src[a]->end(), outs[a]);
+    // in the blocked numbering where the persistent gradient kernel runs
+    // (the residual's own), else node by node in the caller's; the records
+    // are split into the three arrays on the device
+    const bool piped = c->cfg.residual_kernel == AEROF_KERNEL_BLOCKED && grad_piped(m);
+    const int* n2o = piped ? m.n2o.p : nullptr;
+    const double* G;
+    if (piped) {
+      c->s.p2g2_valid = false;
+      c->s.G2.ensure(16 * (size_t)m.N);
+      k_setV<<<grid_for(m.N, kBlock), kBlock, 0, s>>>(m.N, n2o, dV, m.P2.p);
+      AEROF_LAUNCH_CHECK();
+      launch_grad_pipe(c, make_gas(c->cfg.gamma), nullptr, nullptr, c->s.G2.p, s);
+      G = c->s.G2.p;
+    } else {
+      k_setV<<<grid_for(m.N, kBlock), kBlock, 0, s>>>(m.N, nullptr, dV, m.P.p);
+      AEROF_LAUNCH_CHECK();
+      gradients_dev(c);
+      G = c->s.G.p;
     }
-    AEROF_CUDA(cudaStreamSynchronize(c->stream));
+    double* const outs[3] = {ddx, ddy, ddz};
+    double* d[3];
+    bool host = false;
+    for (int a = 0; a < 3; ++a) host = host || !is_device_ptr(outs[a]);
+    if (host) c->s.gsplit.ensure(3 * n5);
+    for (int a = 0; a < 3; ++a) d[a] = is_device_ptr(outs[a]) ? outs[a] : c->s.gsplit.p + a * n5;
+    k_split_grad<<<grid_for(16 * (size_t)m.N, kBlock), kBlock, 0, s>>>(m.N, n2o, G, d[0], d[1], d[2]);
+    AEROF_LAUNCH_CHECK();
+    for (int a = 0; a < 3; ++a)
+      if (d[a] != outs[a])
+        AEROF_CUDA(cudaMemcpyAsync(outs[a], d[a], n5 * sizeof(double), cudaMemcpyDeviceToHost, s));
+    AEROF_CUDA(cudaStreamSynchronize(s));
     return AEROF_OK;
   });
 }
@@ -1692,21 +1755,27 @@ extern "C" int aerof_gpu_rk2(aerof_gpu_ctx* c, double* U, double cfl, int nsteps
       dU = c->s.Ustage.p;
     }
     c->s.dt.ensure(m.N); c->s.k1.ensure(n5); c->s.k2.ensure(n5); c->s.U0.ensure(n5);
+    // the unphysical counts of all steps add up on the device (the failsafe
+    // counts on the host, per call): one wait at the end
     int bad = 0;
+    int* nbad = counters(c) + kCountSum;
+    AEROF_CUDA(cudaMemsetAsync(nbad, 0, sizeof(int), c->stream));
     const int gb = grid_for(n5, kBlock);
     for (int s = 0; s < nsteps; ++s) {
       timestep_dev(c, dU, cfl, c->s.dt.p);
-      bad += residual_dev(c, dU, c->s.k1.p);
+      bad += residual_dev(c, dU, c->s.k1.p, kCountSum);
       k_rk_stage1<<<gb, kBlock, 0, c->stream>>>(m.N, c->s.dt.p, dU, c->s.k1.p, c->s.U0.p);
       AEROF_LAUNCH_CHECK();
-      bad += residual_dev(c, c->s.U0.p, c->s.k2.p);
+      bad += residual_dev(c, c->s.U0.p, c->s.k2.p, kCountSum);
       k_rk_stage2<<<gb, kBlock, 0, c->stream>>>(m.N, c->s.dt.p, c->s.k1.p, c->s.k2.p, dU);
       AEROF_LAUNCH_CHECK();
     }
     if (dU != U)
       AEROF_CUDA(cudaMemcpyAsync(U, dU, n5 * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+    int sum = 0;
+    AEROF_CUDA(cudaMemcpyAsync(&sum, nbad, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
     AEROF_CUDA(cudaStreamSynchronize(c->stream));
-    return bad;
+    return bad + sum;
   });
 }
 
