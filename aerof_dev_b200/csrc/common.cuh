@@ -256,6 +256,18 @@ struct Scratch {
   DBuf<double> redout;     // reduction results
 };
 
+// State of a device-driven Krylov method (krylov.cuh): per-system doubles
+// and integers, reduction partials, and the page-locked words its kernels
+// report to the host.
+struct KrylovWork {
+  DBuf<double> d, part;
+  DBuf<int> i;
+  void *pub = nullptr, *dpub = nullptr;   // GsPub [kMaxSys], host and device address
+  ~KrylovWork() {
+    if (pub) cudaFreeHost(pub);
+  }
+};
+
 // Implicit operator: BSR-by-rows of the H1 Jacobian.
 struct Implicit {
   int precision = 0;       // 32 or 64, 0 = not assembled
@@ -267,20 +279,7 @@ struct Implicit {
   DBuf<double> basis;      // [(m+1)][5N]
   DBuf<double> w, r, x, b, t;
   DBuf<double> hcol;       // device scratch for one Hessenberg column
-  // device-driven GMRES: Hessenberg matrix, rotations, g, y, estimate and
-  // target, per-CTA partials; counters and barrier arrivals
-  DBuf<double> gst;
-  DBuf<int> gsti;
-  // pinned copy of its done flag and the event that marks it current, for
-  // the host's non-blocking polls inside a cycle
-  struct Poll {
-    int* done = nullptr;
-    cudaEvent_t ev = nullptr;
-    ~Poll() {
-      if (done) cudaFreeHost(done);
-      if (ev) cudaEventDestroy(ev);
-    }
-  } poll;
+  KrylovWork kin, kout;    // GMRES on H1, and the flexible method around it
   DBuf<unsigned> ticket;   // grid-reduction ticket of the fused Gram-Schmidt kernels
   DBuf<double> fsum;       // [nbrow][25] boundary-face blocks of the boundary rows
   // preconditioner: AEROF_PC_JACOBI or AEROF_PC_ILU0 (block ILU(0) in the
@@ -292,17 +291,12 @@ struct Implicit {
   int ilu_tr = 0;
   DBuf<double> ilu64, iluw;
   DBuf<float> ilu32;
-  // flexible GMRES on the exact linearisation (outer FP64 vectors)
-  DBuf<double> fV, fZ, fw, fr, fh;
   // finite-difference products (MatVecProdFD): perturbed states and
   // residuals, staged inputs, reduction partials
   DBuf<double> fdQ, fdFp, fdFm, fdIn, fdRed;
-  // lockstep solves of several right-hand sides: outer (FP64) and inner
-  // (FP32) bases and work vectors, Hessenberg columns, pointer arrays of the
-  // batched kernels
-  DBuf<double> bV, bZ, bw, br, bh, ih, bB, bX;
-  DBuf<float> iV, iw, ir, iz;
-  DBuf<unsigned long long> bptr, iptr;
+  // flexible GMRES (outer FP64 vectors of every system that runs together)
+  // and the staged right-hand sides and solutions of a batch
+  DBuf<double> bV, bZ, bw, bB, bX;
 };
 
 // Dual-number work arrays of the forward-mode linearisation.
@@ -474,6 +468,11 @@ __device__ __forceinline__ void cp_async16(void* sdst, const void* gsrc) {
 __device__ __forceinline__ void cp_async8(void* sdst, const void* gsrc) {
   const unsigned s = (unsigned)__cvta_generic_to_shared(sdst);
   asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(s), "l"(gsrc) : "memory");
+}
+// 4-byte variant
+__device__ __forceinline__ void cp_async4(void* sdst, const void* gsrc) {
+  const unsigned s = (unsigned)__cvta_generic_to_shared(sdst);
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(s), "l"(gsrc) : "memory");
 }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }

@@ -16,6 +16,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "krylov.cuh"
 #include "physics.cuh"
 
 namespace aerof {
@@ -355,30 +356,36 @@ __global__ void __launch_bounds__(256) k_spmv(int N, const int* __restrict__ nbr
   for (int k = 0; k < 5; ++k) y[5 * (size_t)r + k] = (TO)acc[k];
 }
 
-// y_q = A p_q (or A^T p_q) for the R vectors of a batch (pointer arrays):
-// every block is read once per group of RB vectors and applied to each in
-// k_spmv's per-row order (diagonal block, then the neighbours ascending).
+// y_q = A p_q (or A^T p_q) for the R vectors of a batch (vector q at p + q ps,
+// y + q ys): every block is read once per group of RB vectors and applied to
+// each in k_spmv's per-row order (diagonal block, then the neighbours
+// ascending).  skip: flags, one per 8 ints; flagged vectors are left out.
 template <class S, bool TRANS, class TV, int RB>
 __global__ void __launch_bounds__(256) k_spmv_batch(int N, int R, const int* __restrict__ nbr_ptr,
                                                     const int* __restrict__ nbr_tpos, const int* __restrict__ sptr,
                                                     const int* __restrict__ scol, const S* __restrict__ diag,
-                                                    const S* __restrict__ off, const TV* const* __restrict__ P,
-                                                    TV* const* __restrict__ Y) {
+                                                    const S* __restrict__ off, const TV* __restrict__ p, size_t ps,
+                                                    TV* __restrict__ y, size_t ys, const int* __restrict__ skip) {
   const int r = blockIdx.x * blockDim.x + threadIdx.x;
   if (r >= N) return;
   const int p0 = nbr_ptr[r], cnt = nbr_ptr[r + 1] - p0;
   const size_t cb = (size_t)sptr[r >> 5] * 32 + (r & 31);
   for (int q0 = 0; q0 < R; q0 += RB) {
+    bool on[RB], any = false;
     double acc[RB][5];
 #pragma unroll
-    for (int q = 0; q < RB; ++q)
+    for (int q = 0; q < RB; ++q) {
+      on[q] = q0 + q < R && !(skip && skip[8 * (q0 + q)]);
+      any = any || on[q];
 #pragma unroll
       for (int k = 0; k < 5; ++k) acc[q][k] = 0.0;
+    }
+    if (!any) continue;
     auto apply = [&](const double* av, int col, bool tr) {
 #pragma unroll
       for (int q = 0; q < RB; ++q) {
-        if (q0 + q >= R) break;
-        const TV* x = P[q0 + q] + 5 * (size_t)col;
+        if (!on[q]) continue;
+        const TV* x = p + (size_t)(q0 + q) * ps + 5 * (size_t)col;
         double xv[5];
 #pragma unroll
         for (int k = 0; k < 5; ++k) xv[k] = (double)x[k];
@@ -407,10 +414,10 @@ __global__ void __launch_bounds__(256) k_spmv_batch(int N, int R, const int* __r
     }
 #pragma unroll
     for (int q = 0; q < RB; ++q) {
-      if (q0 + q >= R) break;
-      TV* y = Y[q0 + q] + 5 * (size_t)r;
+      if (!on[q]) continue;
+      TV* yr = y + (size_t)(q0 + q) * ys + 5 * (size_t)r;
 #pragma unroll
-      for (int k = 0; k < 5; ++k) y[k] = (TV)acc[q][k];
+      for (int k = 0; k < 5; ++k) yr[k] = (TV)acc[q][k];
     }
   }
 }
@@ -446,16 +453,18 @@ __global__ void k_bj_invert(int N, int n_owned, const S* __restrict__ diag, S* _
   store_block_vec<S>(dinv, b, i & 31, a);
 }
 
-// z = D^-1 x (or D^-T x): JacobiPrec::apply/applyT (KspPrec.C:86-111)
+// z = D^-1 x (or D^-T x): JacobiPrec::apply/applyT (KspPrec.C:86-111), for
+// the vectors x + q xs (q = blockIdx.y) whose flag skip[8 q] is clear
 template <class S, class TI, class TO>
-__global__ void k_bj_apply(int N, const S* __restrict__ dinv, const TI* __restrict__ x, TO* __restrict__ z,
-                           int trans, const int* __restrict__ skip) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= N || (skip && *skip)) return;
+__global__ void k_bj_apply(int N, const S* __restrict__ dinv, const TI* __restrict__ x, size_t xs, TO* __restrict__ z,
+                           size_t zs, int trans, const int* __restrict__ skip) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x, q = blockIdx.y;
+  if (i >= N || (skip && skip[8 * q])) return;
   double acc[5] = {0, 0, 0, 0, 0};
-  gemv_sl(dinv, sl_dblk(i), i & 31, x + 5 * (size_t)i, acc, trans != 0);
+  gemv_sl(dinv, sl_dblk(i), i & 31, x + (size_t)q * xs + 5 * (size_t)i, acc, trans != 0);
+  TO* zi = z + (size_t)q * zs + 5 * (size_t)i;
 #pragma unroll
-  for (int k = 0; k < 5; ++k) z[5 * (size_t)i + k] = (TO)acc[k];
+  for (int k = 0; k < 5; ++k) zi[k] = (TO)acc[k];
 }
 
 // ------------------------------------------------------------ vector ops
@@ -510,10 +519,6 @@ __device__ __forceinline__ void grid_sum_last_block(double v, double* __restrict
     *ticket = 0u;
   }
 }
-
-template <class TV> struct Vec16;
-template <> struct Vec16<float> { using T = float4; static constexpr int W = 4; };
-template <> struct Vec16<double> { using T = double2; static constexpr int W = 2; };
 
 // Modified Gram-Schmidt step with the projection of the previous step fused
 // in, 16-byte loads, and the reduction finished in the same launch:
@@ -572,228 +577,6 @@ __global__ void k_combine(size_t n, int k, const double* __restrict__ y, const T
   for (int m = 0; m < k; ++m) s += y[m] * (double)V[(size_t)m * ld + q];
   out[q] = (TV)s;
 }
-// ---------------------------------------------------------------------
-// Device-driven GMRES iteration (GmresSolver::solve, KspSolver.C:396-449,
-// with applyPreviousRotations / applyNewRotation / backwardSolve,
-// KspSolver.C:917-982): the modified Gram-Schmidt steps of one iteration,
-// the Givens update of the Hessenberg column and the next basis vector in
-// one cooperative launch.  Every CTA owns a fixed slice of the vectors; the
-// projections run in the reference's MGS order, one grid-wide sum per step
-// (partials in CTA order, identical in every CTA); the grid barriers are
-// bounded spins that record a timeout in ist[3] and never hang.  The
-// rotation arithmetic is written with explicitly rounded operations (no
-// contraction), so it is the host loop's arithmetic.  Once ist[1] (done)
-// is set, the rest of the cycle's kernels return at once, so the host
-// waits for the GPU only once per restart cycle.
-constexpr int kMaxKrylov = 64;
-constexpr int kCoopThreads = 256;
-struct GmresState {
-  double* H;        // [(m+1) * m], h(i, j) = H[i m + j]
-  double* cs;       // [2 m] rotations
-  double* g;        // [m + 1] right-hand side of the least-squares problem
-  double* y;        // [m] its solution
-  double* scal;     // [0] estimated residual norm, [1] target
-  int* ist;         // [0] iterations, [1] done, [2] last column, [3] barrier timeout, [4] maxits, [5] breakdown
-  double* part;     // [2][grid] per-CTA partial sums
-  unsigned* bar;    // grid barrier arrivals (zeroed per cycle)
-};
-
-// bounded grid barrier: every CTA adds one arrival and waits until the
-// count reaches target (co-residency is guaranteed by the cooperative
-// launch); after about a second a timeout is recorded and the CTA goes on
-__device__ __forceinline__ void grid_barrier(unsigned* bar, unsigned target, int* timeout) {
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    __threadfence();
-    atomicAdd(bar, 1u);
-    unsigned spins = 0;
-    while (*(volatile unsigned*)bar < target) {
-      if (++spins > (1u << 23)) {
-        atomicExch(timeout, 1);
-        break;
-      }
-      __nanosleep(128);
-    }
-    __threadfence();
-  }
-  __syncthreads();
-}
-
-template <class TV>
-__global__ void __launch_bounds__(kCoopThreads, 4) k_gmres_iter(size_t n, int j, int m, TV* __restrict__ V,
-                                                               size_t ld, TV* __restrict__ w, GmresState st,
-                                                               unsigned base) {
-  if (*(volatile int*)(st.ist + 1)) return;
-  __shared__ double ws[32];
-  __shared__ double hsh[kMaxKrylov + 2];
-  __shared__ double css[2 * kMaxKrylov];
-  __shared__ double sprev[3];  // g[j], estimated residual, target
-  __shared__ int iprev[2];     // iterations, maxits
-  __shared__ double sinv;
-  __shared__ int sdone;
-  // the previous state is read before the first barrier: CTA 0 overwrites
-  // it only after the last one
-  for (int k = threadIdx.x; k < 2 * j; k += blockDim.x) css[k] = st.cs[k];
-  if (threadIdx.x == 0) {
-    sprev[0] = st.g[j];
-    sprev[1] = st.scal[0];
-    sprev[2] = st.scal[1];
-    iprev[0] = st.ist[0];
-    iprev[1] = st.ist[4];
-  }
-  using VT = typename Vec16<TV>::T;
-  constexpr int W = Vec16<TV>::W;
-  const size_t nv = n / W;
-  const size_t per = (nv + gridDim.x - 1) / gridDim.x;
-  const size_t lo = min(nv, (size_t)blockIdx.x * per), hi = min(nv, lo + per);
-  const bool tail = blockIdx.x == gridDim.x - 1;
-  unsigned target = base;
-  for (int i = 0; i <= j + 1; ++i) {
-    const bool norm = i == j + 1;
-    const bool proj = i > 0;
-    const double h = proj ? hsh[i - 1] : 0.0;
-    const TV* Vp = proj ? V + (size_t)(i - 1) * ld : nullptr;
-    const TV* Vc = norm ? nullptr : V + (size_t)i * ld;
-    double s = 0.0;
-    // two vectors of each array per thread and trip, loads issued first
-    constexpr int U = 2;
-    for (size_t q0 = lo + threadIdx.x; q0 < hi; q0 += (size_t)U * blockDim.x) {
-      VT wv[U], pv[U], cv[U];
-#pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const size_t q = q0 + (size_t)u * blockDim.x;
-        if (q < hi) {
-          wv[u] = reinterpret_cast<const VT*>(w)[q];
-          if (proj) pv[u] = reinterpret_cast<const VT*>(Vp)[q];
-          if (!norm) cv[u] = reinterpret_cast<const VT*>(Vc)[q];
-        }
-      }
-#pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const size_t q = q0 + (size_t)u * blockDim.x;
-        if (q >= hi) break;
-        TV* wp = reinterpret_cast<TV*>(&wv[u]);
-        if (proj) {
-          const TV* pp = reinterpret_cast<const TV*>(&pv[u]);
-#pragma unroll
-          for (int k = 0; k < W; ++k) wp[k] = (TV)((double)wp[k] - h * (double)pp[k]);
-          reinterpret_cast<VT*>(w)[q] = wv[u];
-        }
-        if (norm) {
-#pragma unroll
-          for (int k = 0; k < W; ++k) s += (double)wp[k] * (double)wp[k];
-        } else {
-          const TV* cp = reinterpret_cast<const TV*>(&cv[u]);
-#pragma unroll
-          for (int k = 0; k < W; ++k) s += (double)wp[k] * (double)cp[k];
-        }
-      }
-    }
-    if (tail)
-      for (size_t q = nv * W + threadIdx.x; q < n; q += blockDim.x) {
-        double wq = (double)w[q];
-        if (proj) {
-          w[q] = (TV)(wq - h * (double)Vp[q]);
-          wq = (double)w[q];
-        }
-        s += wq * (norm ? wq : (double)Vc[q]);
-      }
-    const double b = block_sum(s, ws);
-    double* part = st.part + (size_t)(i & 1) * gridDim.x;
-    if (threadIdx.x == 0) part[blockIdx.x] = b;
-    target += gridDim.x;
-    grid_barrier(st.bar, target, st.ist + 3);
-    double t = 0.0;
-    for (int k = threadIdx.x; k < (int)gridDim.x; k += blockDim.x) t += __ldcg(part + k);
-    t = block_sum(t, ws);
-    if (threadIdx.x == 0) hsh[i] = t;
-    __syncthreads();
-  }
-  // Givens update of column j (every CTA computes it; CTA 0 stores it)
-  if (threadIdx.x == 0) {
-    double hc[kMaxKrylov + 1];
-    for (int i = 0; i <= j; ++i) hc[i] = hsh[i];
-    const double hj1 = __dsqrt_rn(hsh[j + 1]);
-    const bool breakdown = hj1 == 0.0;
-    for (int i = 0; i < j; ++i) {
-      const double c0 = css[2 * i], c1 = css[2 * i + 1];
-      const double a = hc[i], bb = hc[i + 1];
-      hc[i] = __dadd_rn(__dmul_rn(c1, a), __dmul_rn(c0, bb));
-      hc[i + 1] = __dadd_rn(__dmul_rn(-c0, a), __dmul_rn(c1, bb));
-    }
-    double c0, c1;
-    const double hjj = hc[j];
-    if (__dmul_rn(hjj, hjj) == 0.0) {
-      c1 = 0.0;
-      c0 = 1.0;
-    } else {
-      const double coef = __ddiv_rn(1.0, __dsqrt_rn(__dadd_rn(__dmul_rn(hjj, hjj), __dmul_rn(hj1, hj1))));
-      c1 = __dmul_rn(__dsqrt_rn(__dmul_rn(hjj, hjj)), coef);
-      c0 = __ddiv_rn(__dmul_rn(c1, hj1), hjj);
-    }
-    hc[j] = __dadd_rn(__dmul_rn(c1, hjj), __dmul_rn(c0, hj1));
-    const double gj = sprev[0];
-    const double gj1 = __dmul_rn(-c0, gj);
-    const int iter = iprev[0] + 1;
-    double l2res = sprev[1];
-    bool done = breakdown;
-    if (!breakdown) {
-      l2res = fabs(gj1);
-      done = l2res <= sprev[2] || iter >= iprev[1];
-    }
-    sdone = done;
-    sinv = breakdown ? 0.0 : 1. / hj1;
-    if (blockIdx.x == 0) {
-      for (int i = 0; i <= j; ++i) st.H[(size_t)i * m + j] = hc[i];
-      st.H[(size_t)(j + 1) * m + j] = 0.0;
-      st.cs[2 * j] = c0;
-      st.cs[2 * j + 1] = c1;
-      st.g[j + 1] = gj1;
-      st.g[j] = __dmul_rn(c1, gj);
-      st.scal[0] = l2res;
-      st.ist[0] = iter;
-      st.ist[2] = j;
-      st.ist[5] = breakdown;
-    }
-  }
-  __syncthreads();
-  // every CTA has read what it needs of the previous state; CTA 0's done
-  // flag is written after the grid's last barrier, so no CTA of this launch
-  // reads it again
-  if (sdone) {
-    if (blockIdx.x == 0 && threadIdx.x == 0) st.ist[1] = 1;
-    return;
-  }
-  const double a = sinv;
-  TV* Vn = V + (size_t)(j + 1) * ld;
-  for (size_t q = lo * W + threadIdx.x; q < hi * W; q += blockDim.x) Vn[q] = (TV)(a * (double)w[q]);
-  if (tail)
-    for (size_t q = nv * W + threadIdx.x; q < n; q += blockDim.x) Vn[q] = (TV)(a * (double)w[q]);
-}
-
-// back substitution (KspSolver.C:966-982) of the last cycle, one thread:
-// y[0..jl] from the rotated Hessenberg matrix and g
-__global__ void k_gmres_backsolve(int m, GmresState st) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  const int j = st.ist[2];
-  for (int i = j; i >= 0; --i) {
-    double yi = st.g[i];
-    for (int k = j; k >= i + 1; --k) yi = __dsub_rn(yi, __dmul_rn(st.H[(size_t)i * m + k], st.y[k]));
-    st.y[i] = __ddiv_rn(yi, st.H[(size_t)i * m + i]);
-  }
-}
-// out = sum_{m <= last column} y_m V_m
-template <class TV>
-__global__ void k_combine_dev(size_t n, const int* __restrict__ jl, const double* __restrict__ y,
-                              const TV* __restrict__ V, size_t ld, TV* __restrict__ out) {
-  size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= n) return;
-  const int k = *jl + 1;
-  double s = 0.0;
-  for (int mm = 0; mm < k; ++mm) s += y[mm] * (double)V[(size_t)mm * ld + q];
-  out[q] = (TV)s;
-}
-
 template <class TA>
 __global__ void k_add(size_t n, const TA* __restrict__ a, double* __restrict__ x) {
   size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -1104,13 +887,14 @@ __global__ void k_ilu_bwd(int i0, int cnt, int s0, const int* __restrict__ cperm
   }
 }
 
-// The same sweeps for R vectors at once (pointer arrays X, Z; work vectors
-// W + q * ldw): every factor block is read once per group of RB vectors.
+// The same sweeps for R vectors at once (vector q at x + q xs, z + q zs, work
+// vector W + q ldw): every factor block is read once per group of RB
+// vectors.  skip: flags, one per 8 ints; flagged vectors are left out.
 template <int L, int RB, class S, class TI>
 __global__ void k_ilu_fwd_b(int i0, int cnt, int s0, int R, const int* __restrict__ cperm,
                             const int* __restrict__ rju, const int* __restrict__ isp, const int* __restrict__ jc,
-                            const S* __restrict__ lu, const TI* const* __restrict__ X, double* __restrict__ W,
-                            size_t ldw) {
+                            const S* __restrict__ lu, const TI* __restrict__ x, size_t xs, double* __restrict__ W,
+                            size_t ldw, const int* __restrict__ skip) {
   const int g = blockIdx.x * blockDim.x + threadIdx.x;
   const int t = g / L, sub = g % L;
   const bool act = t < cnt;
@@ -1118,18 +902,23 @@ __global__ void k_ilu_fwd_b(int i0, int cnt, int s0, int R, const int* __restric
   const size_t base = act ? (size_t)isp[s0 + (t >> 5)] : 0;
   const int d = act ? rju[i0 + t] : 0;
   for (int q0 = 0; q0 < R; q0 += RB) {
+    bool on[RB], any = false;
     double acc[RB][5];
 #pragma unroll
-    for (int q = 0; q < RB; ++q)
+    for (int q = 0; q < RB; ++q) {
+      on[q] = q0 + q < R && !(skip && skip[8 * (q0 + q)]);
+      any = any || on[q];
 #pragma unroll
       for (int c = 0; c < 5; ++c) acc[q][c] = 0.0;
+    }
+    if (!any) continue;
     for (int k = sub; k < d; k += L) {
       double a[25];
       load_block<S>(lu, (base + k) * 800, lane, a);
       const size_t col = 5 * (size_t)jc[(base + k) * 32 + lane];
 #pragma unroll
       for (int q = 0; q < RB; ++q) {
-        if (q0 + q >= R) break;
+        if (!on[q]) continue;
         const double* wk = W + (size_t)(q0 + q) * ldw + col;
         double v[5];
 #pragma unroll
@@ -1151,10 +940,11 @@ __global__ void k_ilu_fwd_b(int i0, int cnt, int s0, int R, const int* __restric
       const size_t r = (size_t)cperm[i];
 #pragma unroll
       for (int q = 0; q < RB; ++q) {
-        if (q0 + q >= R) break;
+        if (!on[q]) continue;
         double* wi = W + (size_t)(q0 + q) * ldw + 5 * (size_t)i;
+        const TI* xi = x + (size_t)(q0 + q) * xs + 5 * r;
 #pragma unroll
-        for (int c = 0; c < 5; ++c) wi[c] = (double)X[q0 + q][5 * r + c] + acc[q][c];
+        for (int c = 0; c < 5; ++c) wi[c] = (double)xi[c] + acc[q][c];
       }
     }
   }
@@ -1163,7 +953,7 @@ template <int L, int RB, class S, class TO>
 __global__ void k_ilu_bwd_b(int i0, int cnt, int s0, int R, const int* __restrict__ cperm,
                             const int* __restrict__ rlen, const int* __restrict__ rju, const int* __restrict__ isp,
                             const int* __restrict__ jc, const S* __restrict__ lu, double* __restrict__ W, size_t ldw,
-                            TO* const* __restrict__ Z) {
+                            TO* __restrict__ z, size_t zs, const int* __restrict__ skip) {
   const int g = blockIdx.x * blockDim.x + threadIdx.x;
   const int t = g / L, sub = g % L;
   const bool act = t < cnt;
@@ -1171,18 +961,23 @@ __global__ void k_ilu_bwd_b(int i0, int cnt, int s0, int R, const int* __restric
   const size_t base = act ? (size_t)isp[s0 + (t >> 5)] : 0;
   const int d = act ? rju[i0 + t] : 0, len = act ? rlen[i0 + t] : 0;
   for (int q0 = 0; q0 < R; q0 += RB) {
+    bool on[RB], any = false;
     double acc[RB][5];
 #pragma unroll
-    for (int q = 0; q < RB; ++q)
+    for (int q = 0; q < RB; ++q) {
+      on[q] = q0 + q < R && !(skip && skip[8 * (q0 + q)]);
+      any = any || on[q];
 #pragma unroll
       for (int c = 0; c < 5; ++c) acc[q][c] = 0.0;
+    }
+    if (!any) continue;
     for (int k = d + 1 + sub; k < len; k += L) {
       double a[25];
       load_block<S>(lu, (base + k) * 800, lane, a);
       const size_t col = 5 * (size_t)jc[(base + k) * 32 + lane];
 #pragma unroll
       for (int q = 0; q < RB; ++q) {
-        if (q0 + q >= R) break;
+        if (!on[q]) continue;
         const double* wk = W + (size_t)(q0 + q) * ldw + col;
         double v[5];
 #pragma unroll
@@ -1206,18 +1001,19 @@ __global__ void k_ilu_bwd_b(int i0, int cnt, int s0, int R, const int* __restric
       load_block<S>(lu, (base + d) * 800, lane, dg);
 #pragma unroll
       for (int q = 0; q < RB; ++q) {
-        if (q0 + q >= R) break;
+        if (!on[q]) continue;
         double* wi = W + (size_t)(q0 + q) * ldw + 5 * (size_t)i;
+        TO* zi = z + (size_t)(q0 + q) * zs + 5 * r;
         double v[5];
 #pragma unroll
         for (int c = 0; c < 5; ++c) v[c] = acc[q][c] + wi[c];
 #pragma unroll
         for (int rr = 0; rr < 5; ++rr) {
-          double x = 0.0;
+          double t2 = 0.0;
 #pragma unroll
-          for (int c = 0; c < 5; ++c) x += dg[5 * rr + c] * v[c];
-          wi[rr] = x;
-          Z[q0 + q][5 * r + rr] = (TO)x;
+          for (int c = 0; c < 5; ++c) t2 += dg[5 * rr + c] * v[c];
+          wi[rr] = t2;
+          zi[rr] = (TO)t2;
         }
       }
     }
@@ -1292,24 +1088,14 @@ static void ilu_apply(aerof_gpu_ctx* c, const TI* x, TO* z, const int* skip = nu
   else run((const double*)J.ilu64.p);
 }
 
-// z_q = (LU)^-1 x_q for R vectors (device pointer arrays on the host)
+// z_q = (LU)^-1 x_q for the R vectors x + q xs, z + q zs
 template <class TI, class TO>
-static void ilu_apply_batch(aerof_gpu_ctx* c, int R, const TI* const* x, TO* const* z) {
+static void ilu_apply_batch(aerof_gpu_ctx* c, int R, const TI* x, size_t xs, TO* z, size_t zs, const int* skip) {
   DeviceMesh& m = c->mesh;
   Implicit& J = c->imp;
   cudaStream_t s = c->stream;
   const size_t ldw = 5 * (size_t)m.N;
   J.iluw.ensure((size_t)R * ldw);
-  J.iptr.ensure(2 * (size_t)R);
-  std::vector<unsigned long long> p(2 * (size_t)R);
-  for (int q = 0; q < R; ++q) {
-    p[q] = (unsigned long long)x[q];
-    p[R + q] = (unsigned long long)z[q];
-  }
-  AEROF_CUDA(cudaMemcpyAsync(J.iptr.p, p.data(), sizeof(unsigned long long) * 2 * (size_t)R, cudaMemcpyHostToDevice,
-                             s));
-  const TI* const* X = reinterpret_cast<const TI* const*>(J.iptr.p);
-  TO* const* Z = reinterpret_cast<TO* const*>(J.iptr.p + R);
   double* w = J.iluw.p;
   auto run = [&](const auto* lu) {
     using S = std::remove_const_t<std::remove_pointer_t<decltype(lu)>>;
@@ -1317,13 +1103,13 @@ static void ilu_apply_batch(aerof_gpu_ctx* c, int R, const TI* const* x, TO* con
     for (int col = 0; col < m.ncolor; ++col) {
       const int i0 = m.h_cptr[col], cnt = m.h_cptr[col + 1] - i0;
       k_ilu_fwd_b<L, RB, S, TI><<<grid_for((size_t)L * cnt, kIB), kIB, 0, s>>>(
-          i0, cnt, m.h_cslice[col], R, m.cperm.p, m.rju.p, m.isp.p, m.jc.p, lu, X, w, ldw);
+          i0, cnt, m.h_cslice[col], R, m.cperm.p, m.rju.p, m.isp.p, m.jc.p, lu, x, xs, w, ldw, skip);
       AEROF_LAUNCH_CHECK();
     }
     for (int col = m.ncolor - 1; col >= 0; --col) {
       const int i0 = m.h_cptr[col], cnt = m.h_cptr[col + 1] - i0;
       k_ilu_bwd_b<L, RB, S, TO><<<grid_for((size_t)L * cnt, kIB), kIB, 0, s>>>(
-          i0, cnt, m.h_cslice[col], R, m.cperm.p, m.rlen.p, m.rju.p, m.isp.p, m.jc.p, lu, w, ldw, Z);
+          i0, cnt, m.h_cslice[col], R, m.cperm.p, m.rlen.p, m.rju.p, m.isp.p, m.jc.p, lu, w, ldw, z, zs, skip);
       AEROF_LAUNCH_CHECK();
     }
   };
@@ -1360,13 +1146,16 @@ int prec_setup_dev(aerof_gpu_ctx* c, int trans = 0) {
 }
 
 // z = D^-1 x or D^-T x; with transposed storage the inverted blocks are
-// those of D^T, so the roles swap
+// those of D^T, so the roles swap.  R vectors at strides xs, zs; skip:
+// device flags, one per 8 ints (the device-driven GMRES leaves converged
+// systems idle)
 template <class TI, class TO>
-void prec_apply_t(aerof_gpu_ctx* c, const TI* x, TO* z, int trans, const int* skip = nullptr) {
+void prec_apply_t(aerof_gpu_ctx* c, const TI* x, TO* z, int trans, int R = 1, size_t xs = 0, size_t zs = 0,
+                  const int* skip = nullptr) {
   DeviceMesh& m = c->mesh;
   TimerScope tp(c, AEROF_T_KSP_OTHER);
   Implicit& J = c->imp;
-  const int gn = grid_for(m.N, kIB);
+  const dim3 gn(grid_for(m.N, kIB), R);
   const int tr = ((trans != 0) != J.transposed) ? 1 : 0;
   if (J.pc == AEROF_PC_ILU0) {
     // factored for the other orientation (or not yet): factor this one
@@ -1374,24 +1163,21 @@ void prec_apply_t(aerof_gpu_ctx* c, const TI* x, TO* z, int trans, const int* sk
       if (int nb = ilu_setup(c, tr))
         throw ApiError{AEROF_ESINGULAR, std::to_string(nb) + " singular diagonal block(s) in the ILU(0) factors"};
     }
-    ilu_apply(c, x, z, skip);
+    if (R == 1) ilu_apply(c, x, z, skip);
+    else ilu_apply_batch(c, R, x, xs, z, zs, skip);
     return;
   }
   if (J.precision == AEROF_PREC_FP32)
-    k_bj_apply<float, TI, TO><<<gn, kIB, 0, c->stream>>>(m.N, J.dinv32.p, x, z, tr, skip);
+    k_bj_apply<float, TI, TO><<<gn, kIB, 0, c->stream>>>(m.N, J.dinv32.p, x, xs, z, zs, tr, skip);
   else
-    k_bj_apply<double, TI, TO><<<gn, kIB, 0, c->stream>>>(m.N, J.dinv64.p, x, z, tr, skip);
+    k_bj_apply<double, TI, TO><<<gn, kIB, 0, c->stream>>>(m.N, J.dinv64.p, x, xs, z, zs, tr, skip);
   AEROF_LAUNCH_CHECK();
 }
 void prec_apply_dev(aerof_gpu_ctx* c, const double* x, double* z, int trans) {
   prec_apply_t<double, double>(c, x, z, trans);
 }
 
-// Device-driven form of gmres_t for the assembled operator (block-Jacobi or
-// block ILU(0)): per iteration the preconditioner, the product and
-// k_gmres_iter, no host synchronisation inside a restart cycle;
-// the host reads the cycle's status once at its end (AEROF_GMRES_DEVICE=0
-// selects the host-driven loop).
+// AEROF_GMRES_DEVICE=0 selects the host-driven loop of gmres_t
 static bool gmres_device_loop_enabled() {
   static const int v = [] {
     const char* e = std::getenv("AEROF_GMRES_DEVICE");
@@ -1400,148 +1186,255 @@ static bool gmres_device_loop_enabled() {
   return v != 0;
 }
 
+// y_q = H1 x_q (or H1^T x_q) of the R vectors x + q xs, y + q ys
 template <class TV>
-static int gmres_devloop(aerof_gpu_ctx* c, const double* b, double* x, int numVec, int maxits, double eps, int trans,
-                         double* final_res) {
+static void h1_product(aerof_gpu_ctx* c, int R, const TV* x, size_t xs, TV* y, size_t ys, int trans,
+                       const int* skip) {
+  if (R == 1) {
+    matvec_t<TV, TV>(c, x, y, trans, skip);
+    return;
+  }
   DeviceMesh& m = c->mesh;
   Implicit& J = c->imp;
-  const size_t n = 5 * (size_t)m.N;
-  const int gv = grid_for(n, kIB);
-  cudaStream_t s = c->stream;
-  const size_t ld = (n + 63) / 64 * 64;
-  J.basis.ensure(((size_t)(numVec + 1) * ld * sizeof(TV) + 7) / 8);
-  J.w.ensure((n * sizeof(TV) + 7) / 8);
-  J.r.ensure((n * sizeof(TV) + 7) / 8);
-  J.ticket.ensure(1);
-  AEROF_CUDA(cudaMemsetAsync(J.ticket.p, 0, sizeof(unsigned), s));
-  c->s.red.ensure(kGB);
-  J.hcol.ensure(1);
-  TV* Vb = reinterpret_cast<TV*>(J.basis.p);
-  TV* w = reinterpret_cast<TV*>(J.w.p);
-  TV* r = reinterpret_cast<TV*>(J.r.p);
-  // cooperative grid: every CTA resident at once
-  static int coop_grid = 0;
-  if (!coop_grid) {
-    int per_sm = 0, sms = 0;
-    AEROF_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_gmres_iter<TV>, kCoopThreads, 0));
-    AEROF_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->cfg.device));
-    coop_grid = std::max(1, std::min(per_sm, 4)) * sms;
-  }
-  const int grid = coop_grid;
-  // device state: H, cs, g, y, scal | ist, part, bar
-  const size_t nH = (size_t)(numVec + 1) * numVec;
-  J.gst.ensure(nH + 2 * (size_t)numVec + (numVec + 1) + numVec + 2 + 2 * (size_t)grid);
-  J.gsti.ensure(8 + 1);
-  GmresState st;
-  st.H = J.gst.p;
-  st.cs = st.H + nH;
-  st.g = st.cs + 2 * numVec;
-  st.y = st.g + numVec + 1;
-  st.scal = st.y + numVec;
-  st.part = st.scal + 2;
-  st.ist = J.gsti.p;
-  st.bar = reinterpret_cast<unsigned*>(J.gsti.p + 8);
-  double* part = c->s.red.p;
-  unsigned* ticket = J.ticket.p;
-  double* hd = J.hcol.p;
-  auto norm2 = [&](TV* v) -> double {
-    k_mgs<TV, true><<<kGB, kIB, 0, s>>>(n, nullptr, nullptr, nullptr, v, part, ticket, hd);
+  TimerScope t(c, AEROF_T_KSP_MATVEC);
+  const bool tr = (trans != 0) != J.transposed;
+  auto go = [&](auto kern, auto* diag, auto* off) {
+    kern<<<grid_for(m.N, kIB), kIB, 0, c->stream>>>(m.N, R, m.nbr_ptr.p, m.nbr_tpos.p, m.sptr.p, m.scol.p, diag, off,
+                                                    x, xs, y, ys, skip);
     AEROF_LAUNCH_CHECK();
-    double h = 0.0;
-    AEROF_CUDA(cudaMemcpyAsync(&h, hd, sizeof(double), cudaMemcpyDeviceToHost, s));
-    AEROF_CUDA(cudaStreamSynchronize(s));
-    return std::sqrt(h);
   };
-  AEROF_CUDA(cudaMemsetAsync(x, 0, n * sizeof(double), s));
-  int iter = 0;
-  double target = 0.0, l2res = 0.0;
-  const double bnorm = norm2_dev(c, b, n);
-  std::vector<double> ginit(numVec + 1 + numVec + 2);
-  for (;;) {
-    if (iter == 0) {
-      k_scale<double, TV><<<gv, kIB, 0, s>>>(n, 1.0, b, r);
-      AEROF_LAUNCH_CHECK();
-    } else {
-      k_scale<double, TV><<<gv, kIB, 0, s>>>(n, 1.0, x, r);
-      AEROF_LAUNCH_CHECK();
-      matvec_t<TV, TV>(c, r, w, trans);
-      k_sub<TV, TV><<<gv, kIB, 0, s>>>(n, b, w, r);
-      AEROF_LAUNCH_CHECK();
-    }
-    const double beta = norm2(r);
-    if (iter == 0) target = eps * bnorm;
-    if (beta == 0.0) {
-      if (final_res) *final_res = 0.0;
-      return iter;
-    }
-    k_scale<TV, TV><<<gv, kIB, 0, s>>>(n, 1.0 / beta, r, Vb);
-    AEROF_LAUNCH_CHECK();
-    // this cycle's state: g = (beta, 0, ...), the estimate, the target,
-    // the counters, zero barrier arrivals
-    std::fill(ginit.begin(), ginit.end(), 0.0);
-    ginit[0] = beta;
-    ginit[2 * (size_t)numVec + 1] = l2res;
-    ginit[2 * (size_t)numVec + 2] = target;
-    AEROF_CUDA(cudaMemcpyAsync(st.g, ginit.data(), ginit.size() * sizeof(double), cudaMemcpyHostToDevice, s));
-    const int iinit[9] = {iter, 0, -1, 0, maxits, 0, 0, 0, 0};
-    AEROF_CUDA(cudaMemcpyAsync(st.ist, iinit, sizeof(iinit), cudaMemcpyHostToDevice, s));
-    unsigned base = 0;
-    const int* done = st.ist + 1;
-    // every four iterations the done flag is copied to pinned memory behind
-    // an event; the host looks at the previous copy without waiting and
-    // stops issuing the cycle once it shows convergence (the kernels issued
-    // after convergence return at once anyway)
-    if (!J.poll.done) {
-      AEROF_CUDA(cudaMallocHost((void**)&J.poll.done, sizeof(int)));
-      AEROF_CUDA(cudaEventCreateWithFlags(&J.poll.ev, cudaEventDisableTiming));
-    }
-    bool polled = false;
-    for (int j = 0; j < numVec; ++j) {
-      if (polled) {
-        const cudaError_t q = cudaEventQuery(J.poll.ev);
-        if (q == cudaSuccess) {
-          polled = false;
-          if (*J.poll.done) break;
-        } else if (q != cudaErrorNotReady) {
-          AEROF_CUDA(q);
-        } else if (cudaPeekAtLastError() == cudaErrorNotReady) {
-          cudaGetLastError();  // "not ready" is a state, not an error for the next launch check
-        }
-      }
-      prec_apply_t<TV, TV>(c, Vb + (size_t)j * ld, r, trans, done);
-      matvec_t<TV, TV>(c, r, w, trans, done);
-      {
-        TimerScope t(c, AEROF_T_KSP_OTHER);
-        void* args[] = {(void*)&n, (void*)&j, (void*)&numVec, (void*)&Vb, (void*)&ld, (void*)&w, (void*)&st,
-                        (void*)&base};
-        AEROF_CUDA(cudaLaunchCooperativeKernel((const void*)k_gmres_iter<TV>, grid, kCoopThreads, args, 0, s));
-        AEROF_LAUNCH_CHECK();
-        base += (unsigned)(j + 2) * (unsigned)grid;
-      }
-      if ((j & 3) == 3 && !polled && j + 1 < numVec) {
-        AEROF_CUDA(cudaMemcpyAsync(J.poll.done, done, sizeof(int), cudaMemcpyDeviceToHost, s));
-        AEROF_CUDA(cudaEventRecord(J.poll.ev, s));
-        polled = true;
-      }
-    }
-    if (polled) AEROF_CUDA(cudaEventSynchronize(J.poll.ev));
-    k_gmres_backsolve<<<1, 32, 0, s>>>(numVec, st);
-    AEROF_LAUNCH_CHECK();
-    k_combine_dev<TV><<<gv, kIB, 0, s>>>(n, st.ist + 2, st.y, Vb, ld, w);
-    AEROF_LAUNCH_CHECK();
-    prec_apply_t<TV, TV>(c, w, r, trans);
-    k_add<TV><<<gv, kIB, 0, s>>>(n, r, x);
-    AEROF_LAUNCH_CHECK();
-    int ist[6];
-    AEROF_CUDA(cudaMemcpyAsync(ist, st.ist, sizeof(ist), cudaMemcpyDeviceToHost, s));
-    AEROF_CUDA(cudaMemcpyAsync(&l2res, st.scal, sizeof(double), cudaMemcpyDeviceToHost, s));
-    AEROF_CUDA(cudaStreamSynchronize(s));
-    if (ist[3]) throw ApiError{AEROF_ETIMEDOUT, "GMRES grid barrier timed out"};
-    iter = ist[0];
-    if (ist[1]) break;  // converged, saturated or broke down
+  if (J.precision == AEROF_PREC_FP32) {
+    if (tr) go(k_spmv_batch<float, true, TV, 4>, J.diag32.p, J.off32.p);
+    else go(k_spmv_batch<float, false, TV, 4>, J.diag32.p, J.off32.p);
+  } else {
+    if (tr) go(k_spmv_batch<double, true, TV, 4>, J.diag64.p, J.off64.p);
+    else go(k_spmv_batch<double, false, TV, 4>, J.diag64.p, J.off64.p);
   }
-  if (final_res) *final_res = l2res;
-  return iter;
+}
+
+// Device state of R systems with restart length m over vectors of n
+// elements (E per 16 bytes): one CTA of the sweeps per SM and system, fewer
+// for short vectors.
+static GsDev gs_state(aerof_gpu_ctx* c, KrylovWork& k, int R, int m, size_t n, int E) {
+  GsDev st;
+  int sms = 0;
+  AEROF_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->cfg.device));
+  const size_t need = (n / E + kGsT - 1) / kGsT;
+  st.m = m;
+  st.G = (int)std::max<size_t>(1, std::min<size_t>(need, (size_t)sms));
+  st.sd = (st.size() + 1) / 2 * 2;
+  k.d.ensure((size_t)R * st.sd);
+  k.part.ensure((size_t)R * 2 * (m + 1) * st.G);
+  if (k.i.n < (size_t)8 * R) {
+    k.i.alloc((size_t)8 * R);
+    k.i.zero(c->stream);   // the tickets start at zero and re-arm themselves
+  }
+  if (!k.pub) {
+    AEROF_CUDA(cudaHostAlloc((void**)&k.pub, sizeof(GsPub) * kMaxSys, cudaHostAllocMapped));
+    AEROF_CUDA(cudaHostGetDevicePointer((void**)&k.dpub, k.pub, 0));
+  }
+  st.d = k.d.p;
+  st.i = k.i.p;
+  st.part = k.part.p;
+  st.pub = (GsPub*)k.dpub;
+  return st;
+}
+// dynamic shared memory of the two sweeps
+static size_t gs_smem(int m) { return sizeof(double) * ((size_t)3 * (m + 1) + kGsL); }
+
+// Gram-Schmidt step j of the R systems and the Givens update.  Measured with
+// everything around it (stored products): a pseudo-time step of 81^3 with 20
+// FP32 iterations 7.21 -> 6.28 ms against one cooperative launch per
+// iteration with a grid barrier per dot product; five Newton steps of 61^3
+// (8 to 20 iterations each) 28.7 -> 21.5 ms, where also the idle launches
+// after convergence went (kGsAhead); four sensitivities of 41^3 in one batch
+// 171 -> 102 ms, where every system took j + 2 launches per iteration and
+// the host a wait.
+template <class TV>
+static void gs_iteration(aerof_gpu_ctx* c, const GsDev& st, int R, size_t n, int j, TV* V, size_t vs, size_t ld,
+                         const TV* W, size_t ws) {
+  TimerScope t(c, AEROF_T_KSP_OTHER);
+  const size_t smem = gs_smem(st.m);
+  if (smem > 44 * 1024)
+    AEROF_CUDA(cudaFuncSetAttribute(k_gs_dots<TV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  const dim3 grid(st.G, R);
+  k_gs_dots<TV><<<grid, kGsT, smem, c->stream>>>(n, j, V, vs, ld, W, ws, st);
+  AEROF_LAUNCH_CHECK();
+  k_gs_update<TV><<<grid, kGsT, sizeof(double) * (st.m + 1), c->stream>>>(n, j, V, vs, ld, W, ws, st);
+  AEROF_LAUNCH_CHECK();
+}
+
+// The host's side of a running cycle: before the cycle, and until every
+// system has finished `need` iterations of it or is done.  The words are
+// written by the step kernels into page-locked memory, so the host follows
+// the cycle without stopping the stream; an error on the stream, or a
+// stream that has run dry, ends the wait.
+static void gs_reset(KrylovWork& k, int R) {
+  GsPub* p = (GsPub*)k.pub;
+  for (int q = 0; q < R; ++q) p[q] = GsPub{};
+}
+static bool gs_wait(aerof_gpu_ctx* c, KrylovWork& k, int R, int need) {
+  const volatile GsPub* p = (const GsPub*)k.pub;
+  for (unsigned spin = 1;; ++spin) {
+    bool all = true, done = true;
+    for (int q = 0; q < R; ++q) {
+      const bool ready = p[q].seq >= need, dn = p[q].done != 0;
+      all = all && (ready || dn);
+      done = done && dn;
+    }
+    if (all) return done;
+    if (spin % 512 == 0) {
+      const cudaError_t e = cudaStreamQuery(c->stream);
+      if (e == cudaSuccess) {
+        done = true;
+        for (int q = 0; q < R; ++q) done = done && p[q].done != 0;
+        return done;
+      }
+      if (e != cudaErrorNotReady) AEROF_CUDA(e);
+      cudaGetLastError();  // "not ready" is a state, not an error for the next launch check
+    }
+  }
+}
+// iterations that may be queued beyond the last one known to have finished:
+// enough to keep the stream fed, few enough that a converged cycle leaves
+// little idle work behind
+constexpr int kGsAhead = 2;
+
+// Device-driven GMRES(numVec) on the assembled operator for R systems that
+// run together (GmresSolver::solve): per iteration the preconditioner, the
+// product and the two Gram-Schmidt sweeps; a converged system's kernels
+// return at once, and the host waits for the stream once per restart cycle.
+// B[q], X[q]: right-hand sides and solutions (device, [N][5]); X is zeroed
+// first.  TV: storage type of the Krylov vectors.
+template <class TV>
+static void gmres_device(aerof_gpu_ctx* c, int R, const double* const* B, double* const* X, int numVec, int maxits,
+                         double eps, int trans, int* its, double* res) {
+  DeviceMesh& m = c->mesh;
+  Implicit& J = c->imp;
+  cudaStream_t s = c->stream;
+  const size_t n = 5 * (size_t)m.N, ld = (n + 63) / 64 * 64, vs = (size_t)(numVec + 1) * ld;
+  auto bytes = [](size_t count) { return (count * sizeof(TV) + 7) / 8; };
+  J.basis.ensure(bytes((size_t)R * vs));
+  J.w.ensure(bytes((size_t)R * ld));
+  J.r.ensure(bytes((size_t)R * ld));
+  TV *V = reinterpret_cast<TV*>(J.basis.p), *W = reinterpret_cast<TV*>(J.w.p), *Z = reinterpret_cast<TV*>(J.r.p);
+  KrylovWork& kw = J.kin;
+  const GsDev st = gs_state(c, kw, R, numVec, n, Vec16<TV>::W);
+  VecIn b{};
+  VecOut x{};
+  for (int q = 0; q < R; ++q) { b.p[q] = B[q]; x.p[q] = X[q]; }
+  const dim3 gs(st.G, R), gv(grid_for(n, kIB), R);
+  const int* done = st.i + 1;
+  for (bool first = true;; first = false) {
+    gs_reset(kw, R);
+    if (first) {
+      k_gs_start<TV, true><<<gs, kGsT, 0, s>>>(n, b, x, nullptr, 0, V, vs, st, eps, maxits);
+    } else {
+      for (int q = 0; q < R; ++q) {
+        k_scale<double, TV><<<grid_for(n, kIB), kIB, 0, s>>>(n, 1.0, X[q], Z + (size_t)q * ld);
+        AEROF_LAUNCH_CHECK();
+      }
+      h1_product<TV>(c, R, Z, ld, W, ld, trans, done);
+      k_gs_start<TV, false><<<gs, kGsT, 0, s>>>(n, b, x, W, ld, V, vs, st, eps, maxits);
+    }
+    AEROF_LAUNCH_CHECK();
+    for (int j = 0; j < numVec; ++j) {
+      if (gs_wait(c, kw, R, j - kGsAhead)) break;
+      prec_apply_t<TV, TV>(c, V + (size_t)j * ld, Z, trans, R, vs, ld, done);
+      h1_product<TV>(c, R, Z, ld, W, ld, trans, done);
+      gs_iteration<TV>(c, st, R, n, j, V, vs, ld, W, ld);
+    }
+    k_gs_backsolve<<<R, 32, 0, s>>>(st);
+    AEROF_LAUNCH_CHECK();
+    k_gs_combine<TV, false><<<gv, kIB, sizeof(double) * (numVec + 1), s>>>(n, V, vs, ld, st, W, ld, x);
+    AEROF_LAUNCH_CHECK();
+    prec_apply_t<TV, TV>(c, W, Z, trans, R, ld, ld);
+    k_gs_add<TV><<<gv, kIB, 0, s>>>(n, Z, ld, st, x);
+    AEROF_LAUNCH_CHECK();
+    AEROF_CUDA(cudaStreamSynchronize(s));
+    const volatile GsPub* p = (const GsPub*)kw.pub;
+    bool all = true;
+    for (int q = 0; q < R; ++q) {
+      if (its) its[q] = p[q].iter;
+      if (res) res[q] = p[q].l2res;
+      all = all && p[q].done;
+    }
+    if (all) break;
+  }
+}
+
+// Device-driven flexible GMRES on the exact linearisation at exactU (J or
+// J^T, FP64 vectors) for R systems that run together; the preconditioner is
+// itself a solve, z_j = (approximately) H1^{-1} v_j by inner_its iterations
+// of the mixed-precision GMRES on the first-order operator of all running
+// systems (FP32 blocks and Krylov vectors).  The corrections are kept (Z)
+// and x = Z y, so the changing inner solve does not spoil the minimisation.
+// A system that converges stops, the others go on.
+static void fgmres_device(aerof_gpu_ctx* c, int R, const double* const* B, double* const* X, int numVec, int maxits,
+                          double eps, int trans, const double* exactU, int inner_m, int inner_its, double inner_eps,
+                          int* its, double* res) {
+  DeviceMesh& m = c->mesh;
+  Implicit& J = c->imp;
+  cudaStream_t s = c->stream;
+  const size_t n = 5 * (size_t)m.N, ld = (n + 63) / 64 * 64;
+  const size_t vs = (size_t)(numVec + 1) * ld, zs = (size_t)numVec * ld;
+  J.bV.ensure((size_t)R * vs);
+  J.bZ.ensure((size_t)R * zs);
+  J.bw.ensure((size_t)R * ld);
+  double *V = J.bV.p, *Z = J.bZ.p, *W = J.bw.p;
+  KrylovWork& kw = J.kout;
+  const GsDev st = gs_state(c, kw, R, numVec, n, Vec16<double>::W);
+  VecIn b{};
+  VecOut x{};
+  for (int q = 0; q < R; ++q) { b.p[q] = B[q]; x.p[q] = X[q]; }
+  std::vector<char> fin(R, 0);   // done in an earlier cycle
+  const dim3 gs(st.G, R), gv(grid_for(n, kIB), R);
+  auto product = [&](const double* p, double* y) {
+    TimerScope t(c, AEROF_T_KSP_MATVEC);
+    exact_product(c, exactU, p, y, trans != 0);
+  };
+  const volatile GsPub* pub = (const GsPub*)kw.pub;
+  for (bool first = true;; first = false) {
+    gs_reset(kw, R);
+    if (first) {
+      k_gs_start<double, true><<<gs, kGsT, 0, s>>>(n, b, x, nullptr, 0, V, vs, st, eps, maxits);
+    } else {
+      for (int q = 0; q < R; ++q)
+        if (!fin[q]) product(X[q], W + (size_t)q * ld);
+      k_gs_start<double, false><<<gs, kGsT, 0, s>>>(n, b, x, W, ld, V, vs, st, eps, maxits);
+    }
+    AEROF_LAUNCH_CHECK();
+    for (int j = 0; j < numVec; ++j) {
+      if (gs_wait(c, kw, R, j)) break;
+      std::vector<int> rl;
+      std::vector<const double*> bi;
+      std::vector<double*> xi;
+      for (int q = 0; q < R; ++q)
+        if (!fin[q] && !pub[q].done) {
+          rl.push_back(q);
+          bi.push_back(V + (size_t)q * vs + (size_t)j * ld);
+          xi.push_back(Z + (size_t)q * zs + (size_t)j * ld);
+        }
+      if (rl.empty()) break;
+      gmres_device<float>(c, (int)rl.size(), bi.data(), xi.data(), inner_m, inner_its, inner_eps, trans, nullptr,
+                          nullptr);
+      for (size_t k = 0; k < rl.size(); ++k) product(xi[k], W + (size_t)rl[k] * ld);
+      gs_iteration<double>(c, st, R, n, j, V, vs, ld, W, ld);
+    }
+    k_gs_backsolve<<<R, 32, 0, s>>>(st);
+    AEROF_LAUNCH_CHECK();
+    k_gs_combine<double, true><<<gv, kIB, sizeof(double) * (numVec + 1), s>>>(n, Z, zs, ld, st, nullptr, 0, x);
+    AEROF_LAUNCH_CHECK();
+    AEROF_CUDA(cudaStreamSynchronize(s));
+    bool all = true;
+    for (int q = 0; q < R; ++q) {
+      if (its) its[q] = pub[q].iter;
+      if (res) res[q] = pub[q].l2res;
+      fin[q] = pub[q].done != 0;
+      all = all && fin[q];
+    }
+    if (all) break;
+  }
 }
 
 // GmresSolver::solve (KspSolver.C:351-492), typePrec = 2 (right
@@ -1554,8 +1447,11 @@ static int gmres_devloop(aerof_gpu_ctx* c, const double* b, double* x, int numVe
 template <class TV>
 static int gmres_t(aerof_gpu_ctx* c, const double* b, double* x, int numVec, int maxits, double eps, int trans,
                    double* final_res, const double* exactU) {
-  if (!exactU && numVec <= kMaxKrylov && gmres_device_loop_enabled())
-    return gmres_devloop<TV>(c, b, x, numVec, maxits, eps, trans, final_res);
+  if (!exactU && gmres_device_loop_enabled()) {
+    int it = 0;
+    gmres_device<TV>(c, 1, &b, &x, numVec, maxits, eps, trans, &it, final_res);
+    return it;
+  }
   DeviceMesh& m = c->mesh;
   Implicit& J = c->imp;
   const size_t n = 5 * (size_t)m.N;
@@ -1678,379 +1574,6 @@ static int gmres_t(aerof_gpu_ctx* c, const double* b, double* x, int numVec, int
   AEROF_CUDA(cudaStreamSynchronize(s));
   if (final_res) *final_res = l2res;
   return iter;
-}
-
-// Flexible GMRES(m) on the exact linearisation at exactU (J or J^T by
-// forward or reverse mode, FP64 vectors) whose preconditioner is itself a
-// solve: z_j = (approximately) H1^{-1} v_j by inner_its iterations of the
-// mixed-precision GMRES on the assembled first-order operator (FP32 blocks
-// and Krylov vectors, block-Jacobi).  The corrections are kept (Z) and
-// x = Z y, so the changing inner solve does not spoil the minimisation.
-// x = 0 on entry.  Returns outer iterations.
-static int fgmres_exact(aerof_gpu_ctx* c, const double* b, double* x, int numVec, int maxits, double eps, int trans,
-                        double* final_res, const double* exactU, int inner_m, int inner_its, double inner_eps) {
-  DeviceMesh& m = c->mesh;
-  Implicit& J = c->imp;
-  const size_t n = 5 * (size_t)m.N;
-  const size_t ld = (n + 63) / 64 * 64;
-  const int gv = grid_for(n, kIB);
-  cudaStream_t s = c->stream;
-  J.fV.ensure((size_t)(numVec + 1) * ld);
-  J.fZ.ensure((size_t)numVec * ld);
-  J.fw.ensure(ld);
-  J.fr.ensure(ld);
-  J.fh.ensure((size_t)numVec + 2 + (size_t)numVec + 1);
-  J.ticket.ensure(1);
-  c->s.red.ensure(kGB);
-  double* V = J.fV.p;
-  double* Z = J.fZ.p;
-  double* w = J.fw.p;
-  double* r = J.fr.p;
-  double* hd = J.fh.p;
-  double* yd = J.fh.p + numVec + 2;
-  double* part = c->s.red.p;
-  unsigned* ticket = J.ticket.p;
-  AEROF_CUDA(cudaMemsetAsync(ticket, 0, sizeof(unsigned), s));
-  auto op = [&](const double* p, double* y) {
-    TimerScope t(c, AEROF_T_KSP_MATVEC);
-    exact_product(c, exactU, p, y, trans);
-  };
-  auto norm2 = [&](double* v) -> double {
-    k_mgs<double, true><<<kGB, kIB, 0, s>>>(n, nullptr, nullptr, nullptr, v, part, ticket, hd);
-    AEROF_LAUNCH_CHECK();
-    double h = 0.0;
-    AEROF_CUDA(cudaMemcpyAsync(&h, hd, sizeof(double), cudaMemcpyDeviceToHost, s));
-    AEROF_CUDA(cudaStreamSynchronize(s));
-    return std::sqrt(h);
-  };
-  AEROF_CUDA(cudaMemsetAsync(x, 0, n * sizeof(double), s));
-  std::vector<double> H((size_t)(numVec + 1) * numVec, 0.0), cs(2 * (size_t)numVec), g(numVec + 1), y(numVec),
-      hcol(numVec + 2);
-  auto h = [&](int i, int j) -> double& { return H[(size_t)i * numVec + j]; };
-  int iter = 0, exitLoop = 0;
-  double target = 0.0, l2res = 0.0;
-  const double bnorm = norm2_dev(c, b, n);
-  do {
-    if (iter == 0) {
-      AEROF_CUDA(cudaMemcpyAsync(r, b, n * sizeof(double), cudaMemcpyDeviceToDevice, s));
-    } else {
-      op(x, w);
-      k_sub<double, double><<<gv, kIB, 0, s>>>(n, b, w, r);
-      AEROF_LAUNCH_CHECK();
-    }
-    const double beta = norm2(r);
-    if (iter == 0) target = eps * bnorm;
-    if (beta == 0.0) { if (final_res) *final_res = 0.0; return iter; }
-    k_scale<double, double><<<gv, kIB, 0, s>>>(n, 1.0 / beta, r, V);
-    AEROF_LAUNCH_CHECK();
-    std::fill(g.begin(), g.end(), 0.0);
-    g[0] = beta;
-    int j;
-    for (j = 0; j < numVec; ++j) {
-      double* zj = Z + (size_t)j * ld;
-      gmres_t<float>(c, V + (size_t)j * ld, zj, inner_m, inner_its, inner_eps, trans, nullptr, nullptr);
-      op(zj, w);
-      TimerScope t(c, AEROF_T_KSP_OTHER);
-      for (int i = 0; i <= j; ++i) {
-        k_mgs<double, false><<<kGB, kIB, 0, s>>>(n, i ? hd + (i - 1) : nullptr, i ? V + (size_t)(i - 1) * ld : nullptr,
-                                                 V + (size_t)i * ld, w, part, ticket, hd + i);
-        AEROF_LAUNCH_CHECK();
-      }
-      k_mgs<double, true><<<kGB, kIB, 0, s>>>(n, hd + j, V + (size_t)j * ld, nullptr, w, part, ticket, hd + j + 1);
-      AEROF_LAUNCH_CHECK();
-      AEROF_CUDA(cudaMemcpyAsync(hcol.data(), hd, sizeof(double) * (j + 2), cudaMemcpyDeviceToHost, s));
-      AEROF_CUDA(cudaStreamSynchronize(s));
-      for (int i = 0; i <= j; ++i) h(i, j) = hcol[i];
-      h(j + 1, j) = std::sqrt(hcol[j + 1]);
-      const bool breakdown = (h(j + 1, j) == 0.0);
-      if (!breakdown) {
-        k_scale<double, double><<<gv, kIB, 0, s>>>(n, 1. / h(j + 1, j), w, V + (size_t)(j + 1) * ld);
-        AEROF_LAUNCH_CHECK();
-      }
-      for (int i = 0; i < j; ++i) {
-        double hj = cs[2 * i + 1] * h(i, j) + cs[2 * i] * h(i + 1, j);
-        double hjp1 = -cs[2 * i] * h(i, j) + cs[2 * i + 1] * h(i + 1, j);
-        h(i, j) = hj; h(i + 1, j) = hjp1;
-      }
-      if (h(j, j) * h(j, j) == 0.0) { cs[2 * j + 1] = 0.0; cs[2 * j] = 1.0; }
-      else {
-        double coef = 1.0 / std::sqrt(h(j, j) * h(j, j) + h(j + 1, j) * h(j + 1, j));
-        cs[2 * j + 1] = std::sqrt(h(j, j) * h(j, j)) * coef;
-        cs[2 * j] = cs[2 * j + 1] * h(j + 1, j) / h(j, j);
-      }
-      h(j, j) = cs[2 * j + 1] * h(j, j) + cs[2 * j] * h(j + 1, j);
-      h(j + 1, j) = 0.0;
-      g[j + 1] = -cs[2 * j] * g[j];
-      g[j] = cs[2 * j + 1] * g[j];
-      ++iter;
-      if (breakdown) { exitLoop = 1; break; }
-      l2res = std::fabs(g[j + 1]);
-      if (l2res <= target || iter >= maxits) { exitLoop = 1; break; }
-    }
-    if (j == numVec) --j;
-    for (int i = j; i >= 0; --i) {
-      y[i] = g[i];
-      for (int k = j; k >= i + 1; --k) y[i] -= h(i, k) * y[k];
-      y[i] /= h(i, i);
-    }
-    AEROF_CUDA(cudaMemcpyAsync(yd, y.data(), sizeof(double) * (j + 1), cudaMemcpyHostToDevice, s));
-    k_combine<double><<<gv, kIB, 0, s>>>(n, j + 1, yd, Z, ld, w);
-    AEROF_LAUNCH_CHECK();
-    k_add<double><<<gv, kIB, 0, s>>>(n, w, x);
-    AEROF_LAUNCH_CHECK();
-  } while (exitLoop == 0);
-  AEROF_CUDA(cudaStreamSynchronize(s));
-  if (final_res) *final_res = l2res;
-  return iter;
-}
-
-// Lockstep GMRES over R right-hand sides (batched sensitivities): every
-// system runs the algorithm of gmres_t (FLEX = false: FP32 Krylov vectors,
-// right-preconditioned, products with H1 batched over the running systems)
-// or of fgmres_exact (FLEX = true: FP64, the preconditioner one inner
-// lockstep solve of all running systems, exact products), the iterations of
-// all systems together; a system that converges stops, the others go on.
-// B[q] / X[q] are the right-hand sides and solutions (device, [N][5]); X is
-// zeroed first.  The inner solve (FLEX = false) runs one cycle: maxits <=
-// numVec.
-template <class TV, bool FLEX>
-static void gmres_lockstep(aerof_gpu_ctx* c, int R, const double* const* B, double* const* X, int numVec, int maxits,
-                           double eps, int trans, const double* exactU, int inner_m, int inner_its, double inner_eps,
-                           int* its, double* res) {
-  DeviceMesh& m = c->mesh;
-  Implicit& J = c->imp;
-  const size_t n = 5 * (size_t)m.N;
-  const size_t ld = (n + 63) / 64 * 64;
-  const int gv = grid_for(n, kIB);
-  cudaStream_t s = c->stream;
-  const int M1 = numVec + 1, HS = numVec + 2;
-  TV *Vb, *Zb = nullptr, *w, *rr, *pz = nullptr;
-  double* hd;
-  if constexpr (FLEX) {
-    J.bV.ensure((size_t)R * M1 * ld);
-    J.bZ.ensure((size_t)R * numVec * ld);
-    J.bw.ensure((size_t)R * ld);
-    J.br.ensure((size_t)R * ld);
-    J.bh.ensure((size_t)R * (HS + M1));
-    Vb = J.bV.p; Zb = J.bZ.p; w = J.bw.p; rr = J.br.p; hd = J.bh.p;
-  } else {
-    J.iV.ensure((size_t)R * M1 * ld);
-    J.iw.ensure((size_t)R * ld);
-    J.ir.ensure((size_t)R * ld);
-    J.iz.ensure((size_t)R * ld);
-    J.ih.ensure((size_t)R * (HS + M1));
-    J.bptr.ensure(2 * (size_t)R);
-    Vb = J.iV.p; w = J.iw.p; rr = J.ir.p; pz = J.iz.p; hd = J.ih.p;
-  }
-  double* yd = hd + (size_t)R * HS;
-  J.ticket.ensure(1);
-  c->s.red.ensure(kGB);
-  double* part = c->s.red.p;
-  unsigned* ticket = J.ticket.p;
-  AEROF_CUDA(cudaMemsetAsync(ticket, 0, sizeof(unsigned), s));
-  auto V = [&](int q, int j) { return Vb + ((size_t)q * M1 + j) * ld; };
-  auto Zv = [&](int q, int j) { return Zb + ((size_t)q * numVec + j) * ld; };
-  auto W = [&](int q) { return w + (size_t)q * ld; };
-  auto Rv = [&](int q) { return rr + (size_t)q * ld; };
-  auto Hq = [&](int q) { return hd + (size_t)q * HS; };
-  // host state per system
-  std::vector<double> H((size_t)R * M1 * numVec, 0.0), cs((size_t)R * 2 * numVec), g((size_t)R * M1), y(numVec),
-      hcol((size_t)R * HS), target(R, 0.0), l2(R, 0.0), bnorm(R);
-  std::vector<int> iter(R, 0), jl(R, -1);
-  std::vector<char> active(R, 1), run(R, 0), fin(R, 0);
-  auto h = [&](int q, int i, int j) -> double& { return H[((size_t)q * M1 + i) * numVec + j]; };
-  auto fetch = [&]() {
-    AEROF_CUDA(cudaMemcpyAsync(hcol.data(), hd, sizeof(double) * (size_t)R * HS, cudaMemcpyDeviceToHost, s));
-    AEROF_CUDA(cudaStreamSynchronize(s));
-  };
-  // the reductions read 16-byte vectors of the right-hand sides
-  for (int q = 0; q < R; ++q)
-    if (reinterpret_cast<uintptr_t>(B[q]) % 16 != 0)
-      throw ApiError{AEROF_EINVAL, "lockstep GMRES: right-hand side not 16-byte aligned"};
-  for (int q = 0; q < R; ++q) {
-    AEROF_CUDA(cudaMemsetAsync(X[q], 0, n * sizeof(double), s));
-    k_mgs<double, true><<<kGB, kIB, 0, s>>>(n, nullptr, nullptr, nullptr, const_cast<double*>(B[q]), part, ticket,
-                                            Hq(q));
-    AEROF_LAUNCH_CHECK();
-  }
-  fetch();
-  for (int q = 0; q < R; ++q) bnorm[q] = std::sqrt(hcol[(size_t)q * HS]);
-  std::vector<unsigned long long> ptrs(2 * (size_t)R);
-  while (true) {
-    // residuals of the active systems
-    for (int q = 0; q < R; ++q) {
-      if (!active[q]) continue;
-      if (iter[q] == 0) {
-        k_scale<double, TV><<<gv, kIB, 0, s>>>(n, 1.0, B[q], Rv(q));
-        AEROF_LAUNCH_CHECK();
-      } else {
-        TimerScope t(c, AEROF_T_KSP_MATVEC);
-        if constexpr (FLEX) {
-          exact_product(c, exactU, X[q], W(q), trans);
-        } else {
-          k_scale<double, TV><<<gv, kIB, 0, s>>>(n, 1.0, X[q], Rv(q));
-          AEROF_LAUNCH_CHECK();
-          matvec_t<TV, TV>(c, Rv(q), W(q), trans);
-        }
-        k_sub<TV, TV><<<gv, kIB, 0, s>>>(n, B[q], W(q), Rv(q));
-        AEROF_LAUNCH_CHECK();
-      }
-      k_mgs<TV, true><<<kGB, kIB, 0, s>>>(n, nullptr, nullptr, nullptr, Rv(q), part, ticket, Hq(q));
-      AEROF_LAUNCH_CHECK();
-    }
-    fetch();
-    bool any = false;
-    for (int q = 0; q < R; ++q) {
-      run[q] = 0;
-      jl[q] = -1;
-      if (!active[q]) continue;
-      const double beta = std::sqrt(hcol[(size_t)q * HS]);
-      if (iter[q] == 0) target[q] = eps * bnorm[q];
-      if (beta == 0.0) {
-        active[q] = 0;
-        l2[q] = 0.0;
-        continue;
-      }
-      k_scale<TV, TV><<<gv, kIB, 0, s>>>(n, 1.0 / beta, Rv(q), V(q, 0));
-      AEROF_LAUNCH_CHECK();
-      std::fill(g.begin() + (size_t)q * M1, g.begin() + (size_t)(q + 1) * M1, 0.0);
-      g[(size_t)q * M1] = beta;
-      run[q] = 1;
-      fin[q] = 0;
-      any = true;
-    }
-    if (!any) break;
-    for (int j = 0; j < numVec; ++j) {
-      std::vector<int> rl;
-      for (int q = 0; q < R; ++q)
-        if (run[q]) rl.push_back(q);
-      if (rl.empty()) break;
-      const int nr = (int)rl.size();
-      // direction and product of every running system
-      if constexpr (FLEX) {
-        std::vector<const double*> bi(nr);
-        std::vector<double*> xi(nr);
-        for (int k = 0; k < nr; ++k) { bi[k] = V(rl[k], j); xi[k] = Zv(rl[k], j); }
-        gmres_lockstep<float, false>(c, nr, bi.data(), xi.data(), inner_m, inner_its, inner_eps, trans, nullptr, 0, 0,
-                                     0.0, nullptr, nullptr);
-        TimerScope t(c, AEROF_T_KSP_MATVEC);
-        for (int k = 0; k < nr; ++k) exact_product(c, exactU, Zv(rl[k], j), W(rl[k]), trans);
-      } else {
-        {
-          TimerScope t(c, AEROF_T_KSP_OTHER);
-          const int tr = ((trans != 0) != J.transposed) ? 1 : 0;
-          if (J.pc == AEROF_PC_ILU0 && J.ilu_ready && J.ilu_tr == tr) {
-            // every factor block read once for the running systems
-            std::vector<const TV*> xs(nr);
-            std::vector<TV*> zs(nr);
-            for (int k = 0; k < nr; ++k) { xs[k] = V(rl[k], j); zs[k] = pz + (size_t)rl[k] * ld; }
-            ilu_apply_batch<TV, TV>(c, nr, xs.data(), zs.data());
-          } else {
-            for (int k = 0; k < nr; ++k) prec_apply_t<TV, TV>(c, V(rl[k], j), pz + (size_t)rl[k] * ld, trans);
-          }
-        }
-        TimerScope t(c, AEROF_T_KSP_MATVEC);
-        for (int k = 0; k < nr; ++k) {
-          ptrs[k] = (unsigned long long)(pz + (size_t)rl[k] * ld);
-          ptrs[R + k] = (unsigned long long)W(rl[k]);
-        }
-        AEROF_CUDA(cudaMemcpyAsync(J.bptr.p, ptrs.data(), sizeof(unsigned long long) * 2 * (size_t)R,
-                                   cudaMemcpyHostToDevice, s));
-        const TV* const* P = reinterpret_cast<const TV* const*>(J.bptr.p);
-        TV* const* Y = reinterpret_cast<TV* const*>(J.bptr.p + R);
-        const bool tr = (trans != 0) != J.transposed;
-        auto go = [&](auto kern, auto* diag, auto* off) {
-          kern<<<grid_for(m.N, kIB), kIB, 0, s>>>(m.N, nr, m.nbr_ptr.p, m.nbr_tpos.p, m.sptr.p, m.scol.p, diag, off,
-                                                 P, Y);
-          AEROF_LAUNCH_CHECK();
-        };
-        if (J.precision == AEROF_PREC_FP32) {
-          if (tr) go(k_spmv_batch<float, true, TV, 4>, J.diag32.p, J.off32.p);
-          else go(k_spmv_batch<float, false, TV, 4>, J.diag32.p, J.off32.p);
-        } else {
-          if (tr) go(k_spmv_batch<double, true, TV, 4>, J.diag64.p, J.off64.p);
-          else go(k_spmv_batch<double, false, TV, 4>, J.diag64.p, J.off64.p);
-        }
-      }
-      TimerScope t(c, AEROF_T_KSP_OTHER);
-      for (int q : rl) {
-        for (int i = 0; i <= j; ++i) {
-          k_mgs<TV, false><<<kGB, kIB, 0, s>>>(n, i ? Hq(q) + (i - 1) : nullptr, i ? V(q, i - 1) : nullptr, V(q, i),
-                                               W(q), part, ticket, Hq(q) + i);
-          AEROF_LAUNCH_CHECK();
-        }
-        k_mgs<TV, true><<<kGB, kIB, 0, s>>>(n, Hq(q) + j, V(q, j), nullptr, W(q), part, ticket, Hq(q) + j + 1);
-        AEROF_LAUNCH_CHECK();
-      }
-      fetch();
-      for (int q : rl) {
-        const double* hc = hcol.data() + (size_t)q * HS;
-        double* csq = cs.data() + (size_t)q * 2 * numVec;
-        double* gq = g.data() + (size_t)q * M1;
-        for (int i = 0; i <= j; ++i) h(q, i, j) = hc[i];
-        h(q, j + 1, j) = std::sqrt(hc[j + 1]);
-        const bool breakdown = (h(q, j + 1, j) == 0.0);
-        if (!breakdown) {
-          k_scale<TV, TV><<<gv, kIB, 0, s>>>(n, 1. / h(q, j + 1, j), W(q), V(q, j + 1));
-          AEROF_LAUNCH_CHECK();
-        }
-        for (int i = 0; i < j; ++i) {
-          double hj = csq[2 * i + 1] * h(q, i, j) + csq[2 * i] * h(q, i + 1, j);
-          double hjp1 = -csq[2 * i] * h(q, i, j) + csq[2 * i + 1] * h(q, i + 1, j);
-          h(q, i, j) = hj; h(q, i + 1, j) = hjp1;
-        }
-        if (h(q, j, j) * h(q, j, j) == 0.0) { csq[2 * j + 1] = 0.0; csq[2 * j] = 1.0; }
-        else {
-          double coef = 1.0 / std::sqrt(h(q, j, j) * h(q, j, j) + h(q, j + 1, j) * h(q, j + 1, j));
-          csq[2 * j + 1] = std::sqrt(h(q, j, j) * h(q, j, j)) * coef;
-          csq[2 * j] = csq[2 * j + 1] * h(q, j + 1, j) / h(q, j, j);
-        }
-        h(q, j, j) = csq[2 * j + 1] * h(q, j, j) + csq[2 * j] * h(q, j + 1, j);
-        h(q, j + 1, j) = 0.0;
-        gq[j + 1] = -csq[2 * j] * gq[j];
-        gq[j] = csq[2 * j + 1] * gq[j];
-        ++iter[q];
-        jl[q] = j;
-        if (breakdown) { run[q] = 0; fin[q] = 1; continue; }
-        l2[q] = std::fabs(gq[j + 1]);
-        if (l2[q] <= target[q] || iter[q] >= maxits) { run[q] = 0; fin[q] = 1; }
-      }
-    }
-    // solution update of every system that ran in this cycle
-    for (int q = 0; q < R; ++q) {
-      if (jl[q] < 0) continue;
-      const int jj = jl[q];
-      const double* gq = g.data() + (size_t)q * M1;
-      for (int i = jj; i >= 0; --i) {
-        y[i] = gq[i];
-        for (int k = jj; k >= i + 1; --k) y[i] -= h(q, i, k) * y[k];
-        y[i] /= h(q, i, i);
-      }
-      double* yq = yd + (size_t)q * M1;
-      AEROF_CUDA(cudaMemcpyAsync(yq, y.data(), sizeof(double) * (jj + 1), cudaMemcpyHostToDevice, s));
-      if constexpr (FLEX) {
-        k_combine<double><<<gv, kIB, 0, s>>>(n, jj + 1, yq, Zv(q, 0), ld, W(q));
-        AEROF_LAUNCH_CHECK();
-        k_add<double><<<gv, kIB, 0, s>>>(n, W(q), X[q]);
-        AEROF_LAUNCH_CHECK();
-      } else {
-        k_combine<TV><<<gv, kIB, 0, s>>>(n, jj + 1, yq, V(q, 0), ld, W(q));
-        AEROF_LAUNCH_CHECK();
-        prec_apply_t<TV, TV>(c, W(q), Rv(q), trans);
-        k_add<TV><<<gv, kIB, 0, s>>>(n, Rv(q), X[q]);
-        AEROF_LAUNCH_CHECK();
-      }
-      if (fin[q]) active[q] = 0;
-    }
-    bool left = false;
-    for (int q = 0; q < R; ++q) left = left || active[q];
-    if (!left) break;
-  }
-  AEROF_CUDA(cudaStreamSynchronize(s));
-  for (int q = 0; q < R; ++q) {
-    if (its) its[q] = iter[q];
-    if (res) res[q] = l2[q];
-  }
 }
 
 int gmres_dev(aerof_gpu_ctx* c, const double* b, double* x, int numVec, int maxits, double eps, int trans,
@@ -2554,9 +2077,12 @@ extern "C" int aerof_gpu_linearized_solve(aerof_gpu_ctx* c, const double* U, con
       return AEROF_ESINGULAR;
     }
     double r = 0.0;
-    const int it = inner_its ? fgmres_exact(c, db, dx, krylov, maxits, eps, transpose, &r, dU, std::min(inner_its, 30),
-                                            inner_its, 1e-3)
-                             : gmres_dev(c, db, dx, krylov, maxits, eps, transpose, &r, dU);
+    int it = 0;
+    if (inner_its)
+      fgmres_device(c, 1, &db, &dx, krylov, maxits, eps, transpose, dU, std::min(inner_its, 30), inner_its, 1e-3, &it,
+                    &r);
+    else
+      it = gmres_dev(c, db, dx, krylov, maxits, eps, transpose, &r, dU);
     out_finish(c, x, dx, n);
     if (its) *its = it;
     if (res) *res = r;
@@ -2604,7 +2130,6 @@ extern "C" int aerof_gpu_linearized_solve_batch(aerof_gpu_ctx* c, const double* 
     const bool lockstep = inner_its > 0 && inner_its <= 30 && (!lv || std::atoi(lv) != 0);
     if (lockstep) {
       // right-hand sides and solutions staged at a 512-byte aligned stride
-      // (the reductions read 16-byte vectors)
       const size_t ld = (n + 63) / 64 * 64;
       const cudaMemcpyKind kb = is_device_ptr(B) ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
       const cudaMemcpyKind kx = is_device_ptr(X) ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost;
@@ -2615,7 +2140,7 @@ extern "C" int aerof_gpu_linearized_solve_batch(aerof_gpu_ctx* c, const double* 
                          ((size_t)inner_its + 5) * ld * sizeof(float);
       size_t freeb = 0, totalb = 0;
       AEROF_CUDA(cudaMemGetInfo(&freeb, &totalb));
-      const int G = (int)std::max<size_t>(1, std::min<size_t>((size_t)nrhs, (size_t)(0.7 * (double)freeb) / per));
+      const int G = (int)std::max<size_t>(1, std::min<size_t>((size_t)std::min(nrhs, kMaxSys), (size_t)(0.7 * (double)freeb) / per));
       c->imp.bB.ensure((size_t)std::min(G, nrhs) * ld);
       c->imp.bX.ensure((size_t)std::min(G, nrhs) * ld);
       for (int k0 = 0; k0 < nrhs; k0 += G) {
@@ -2628,9 +2153,8 @@ extern "C" int aerof_gpu_linearized_solve_batch(aerof_gpu_ctx* c, const double* 
           bq[q] = c->imp.bB.p + (size_t)q * ld;
           xq[q] = c->imp.bX.p + (size_t)q * ld;
         }
-        gmres_lockstep<double, true>(c, g, bq.data(), xq.data(), krylov, maxits, eps, transpose, dU,
-                                     std::min(inner_its, 30), inner_its, 1e-3, its ? its + k0 : nullptr,
-                                     res ? res + k0 : nullptr);
+        fgmres_device(c, g, bq.data(), xq.data(), krylov, maxits, eps, transpose, dU, std::min(inner_its, 30),
+                      inner_its, 1e-3, its ? its + k0 : nullptr, res ? res + k0 : nullptr);
         for (int q = 0; q < g; ++q)
           AEROF_CUDA(cudaMemcpyAsync(X + (size_t)(k0 + q) * n, xq[q], n * sizeof(double), kx, c->stream));
         AEROF_CUDA(cudaStreamSynchronize(c->stream));
@@ -2641,9 +2165,12 @@ extern "C" int aerof_gpu_linearized_solve_batch(aerof_gpu_ctx* c, const double* 
       const double* db = in_dev(c, B + (size_t)k * n, n, c->s.Vstage);
       double* dx = out_dev(c, X + (size_t)k * n, n, c->s.Rstage);
       double r = 0.0;
-      const int it = inner_its ? fgmres_exact(c, db, dx, krylov, maxits, eps, transpose, &r, dU,
-                                              std::min(inner_its, 30), inner_its, 1e-3)
-                               : gmres_dev(c, db, dx, krylov, maxits, eps, transpose, &r, dU);
+      int it = 0;
+      if (inner_its)
+        fgmres_device(c, 1, &db, &dx, krylov, maxits, eps, transpose, dU, std::min(inner_its, 30), inner_its, 1e-3,
+                      &it, &r);
+      else
+        it = gmres_dev(c, db, dx, krylov, maxits, eps, transpose, &r, dU);
       out_finish(c, X + (size_t)k * n, dx, n);
       if (its) its[k] = it;
       if (res) res[k] = r;

@@ -1,0 +1,435 @@
+// krylov.cuh -- Gram-Schmidt kernels of the device-driven GMRES
+// (GmresSolver::solve, KspSolver.C:396-449, with applyPreviousRotations /
+// applyNewRotation / backwardSolve, KspSolver.C:917-982) for R systems that
+// run together (grid.y = system).
+//
+// The coefficients of modified Gram-Schmidt, h_0 = v_0.w, h_1 = v_1.(w -
+// h_0 v_0), ..., satisfy (I + L) h = V^T w with L the strictly lower part of
+// V^T V: one sweep over the basis gives every v_i.w and the new row v_j.v_k
+// of L, a triangular solve gives h, and a second sweep forms w - V h
+// (Swirydowicz, Langou, Ananthan, Yang, Thomas, "Low synchronization
+// Gram-Schmidt and GMRES algorithms", 2021: the same projector as MGS).
+// Two reads of the basis per iteration and two launches, instead of two
+// reads of the basis, j reads and writes of w and j + 1 grid-wide sums
+// (bound: HBM; figures at gs_iteration).
+//
+// The basis vectors are stored as they come out of the projection, with
+// the factor sig_i = 1/norm beside them (v_i = sig_i * stored), so no pass
+// normalises them.  Dots, norms and the Hessenberg system are FP64 for
+// either storage type; the projected vector is rounded to it once.
+// Reductions run over a fixed grid in a fixed order (no atomics on values);
+// the block that finishes last does the scalar work of the step.
+#pragma once
+
+#include "common.cuh"
+
+namespace aerof {
+
+constexpr int kGsT = 512;        // threads of the sweeps
+constexpr int kGsL = 4000;       // doubles of L kept in shared memory by the triangular solve
+constexpr int kMaxSys = 64;      // systems per launch
+
+// what the host reads while the cycle runs (page-locked, mapped)
+struct GsPub {
+  int seq;                       // iterations finished in this cycle
+  int done, iter, pad;
+  double l2res;
+};
+
+// Device state of the systems: system q's block of doubles at d + q sd,
+// its integers at i + 8 q: [0] iterations, [1] done, [2] last column,
+// [3] active in this cycle, [4] maxits, [5] breakdown, [6] [7] tickets.
+struct GsDev {
+  double* d;
+  size_t sd;
+  int* i;
+  double* part;                  // [R][2 (m + 1)][G] partial sums
+  GsPub* pub;
+  int m, G;
+  __host__ __device__ size_t oL() const { return (size_t)(m + 1) * m; }
+  __host__ __device__ size_t oCs() const { return oL() + (size_t)m * m; }
+  __host__ __device__ size_t oG() const { return oCs() + 2 * (size_t)m; }
+  __host__ __device__ size_t oY() const { return oG() + m + 1; }
+  __host__ __device__ size_t oSig() const { return oY() + m; }
+  __host__ __device__ size_t oH() const { return oSig() + m + 1; }
+  __host__ __device__ size_t oScal() const { return oH() + m + 1; }   // l2res, target
+  __host__ __device__ size_t size() const { return oScal() + 2; }
+};
+
+struct VecIn { const double* p[kMaxSys]; };
+struct VecOut { double* p[kMaxSys]; };
+
+template <class TV> struct Vec16;
+template <> struct Vec16<float> { using T = float4; static constexpr int W = 4; };
+template <> struct Vec16<double> { using T = double2; static constexpr int W = 2; };
+
+// sum of C values over the block's warps (xor tree, then the warps in
+// order): result v of the block at out[v * stride] by thread v
+template <int C>
+__device__ __forceinline__ void block_sums(const double* v, int nv, double* red, double* out, size_t stride) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  __syncthreads();
+#pragma unroll
+  for (int c = 0; c < C; ++c) {
+    if (c >= nv) break;
+    double t = v[c];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    if (lane == 0) red[warp * C + c] = t;
+  }
+  __syncthreads();
+  if ((int)threadIdx.x < nv) {
+    double t = 0.0;
+    for (int w = 0; w < nw; ++w) t += red[w * C + threadIdx.x];
+    out[threadIdx.x * stride] = t;
+  }
+}
+
+// true in every thread of the block that arrives last; the partial sums of
+// the others are then visible (the ticket re-arms itself)
+__device__ __forceinline__ bool last_block(int* ticket) {
+  __shared__ bool last;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    last = atomicAdd(ticket, 1) == (int)gridDim.x - 1;
+    if (last) *ticket = 0;
+  }
+  __syncthreads();
+  if (last) __threadfence();
+  return last;
+}
+
+// vals[v] = sum of part[v][0, G) for v < nv, one warp per value
+__device__ __forceinline__ void sum_partials(const double* part, int G, int nv, double* vals) {
+  const int lane = threadIdx.x & 31;
+  for (int v = threadIdx.x >> 5; v < nv; v += blockDim.x >> 5) {
+    double t = 0.0;
+    for (int k = lane; k < G; k += 32) t += __ldcg(part + (size_t)v * G + k);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    if (lane == 0) vals[v] = t;
+  }
+  __syncthreads();
+}
+
+__device__ __forceinline__ void publish(GsPub* pub, int seq, int done, int iter, double l2res) {
+  volatile GsPub* p = pub;
+  p->done = done;
+  p->iter = iter;
+  p->l2res = l2res;
+  __threadfence_system();
+  p->seq = seq;
+}
+
+// First vector of a cycle: v_0 = b (FIRST, which also zeroes x) or b - w,
+// stored unnormalised, with its norm (and b's, for the target) and the
+// cycle's state.
+template <class TV, bool FIRST>
+__global__ void __launch_bounds__(kGsT) k_gs_start(size_t n, VecIn B, VecOut X, const TV* __restrict__ Wv, size_t ws,
+                                                   TV* __restrict__ V, size_t vs, GsDev st, double eps, int maxits) {
+  __shared__ double red[(kGsT / 32) * 2];
+  __shared__ double vals[2];
+  const int q = blockIdx.y;
+  int* ist = st.i + 8 * q;
+  if (!FIRST && ist[1]) {
+    // done in an earlier cycle: its words stand
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+      ist[3] = 0;
+      publish(st.pub + q, 0, 1, ist[0], st.d[(size_t)q * st.sd + st.oScal()]);
+    }
+    return;
+  }
+  const double* __restrict__ b = B.p[q];
+  const TV* __restrict__ w = Wv + (size_t)q * ws;
+  TV* __restrict__ v = V + (size_t)q * vs;
+  double s[2] = {0.0, 0.0};
+  for (size_t p = (size_t)blockIdx.x * blockDim.x + threadIdx.x; p < n; p += (size_t)gridDim.x * blockDim.x) {
+    const double bp = b[p];
+    const TV r = (TV)(FIRST ? bp : bp - (double)w[p]);
+    v[p] = r;
+    if (FIRST) {
+      X.p[q][p] = 0.0;
+      s[1] += bp * bp;
+    }
+    s[0] += (double)r * (double)r;
+  }
+  double* part = st.part + (size_t)q * 2 * (st.m + 1) * st.G;
+  block_sums<2>(s, 2, red, part + blockIdx.x, st.G);
+  if (!last_block(ist + 6)) return;
+  sum_partials(part, st.G, 2, vals);
+  if (threadIdx.x == 0) {
+    double* d = st.d + (size_t)q * st.sd;
+    const double beta = sqrt(vals[0]);
+    if (FIRST) {
+      ist[0] = 0;
+      ist[4] = maxits;
+      d[st.oScal()] = 0.0;
+      d[st.oScal() + 1] = eps * sqrt(vals[1]);
+    }
+    const int done = beta == 0.0;
+    if (done) d[st.oScal()] = 0.0;
+    ist[1] = done;
+    ist[2] = -1;
+    ist[3] = 1;
+    ist[5] = 0;
+    d[st.oG()] = beta;
+    d[st.oSig()] = done ? 0.0 : 1.0 / beta;
+    if (done) publish(st.pub + q, 0, 1, ist[0], 0.0);
+  }
+}
+
+// Sweep 1 of iteration j: v_i.w and v_i.v_j for every i <= j (eight basis
+// vectors per pass over w and v_j, so that a thread has ten 16-byte loads in
+// flight), then the coefficients h by the triangular solve.
+template <class TV>
+__global__ void __launch_bounds__(kGsT, 1) k_gs_dots(size_t n, int j, const TV* __restrict__ V, size_t vs, size_t ld,
+                                                     const TV* __restrict__ W, size_t ws, GsDev st) {
+  extern __shared__ double sh[];   // vals [2 (m + 1)], a [m + 1], L
+  __shared__ double red[(kGsT / 32) * 16];
+  const int q = blockIdx.y;
+  int* ist = st.i + 8 * q;
+  if (ist[1]) return;
+  using VT = typename Vec16<TV>::T;
+  constexpr int E = Vec16<TV>::W, U = 8;
+  const TV* __restrict__ Vq = V + (size_t)q * vs;
+  const TV* __restrict__ w = W + (size_t)q * ws;
+  const TV* __restrict__ vj = Vq + (size_t)j * ld;
+  double* part = st.part + (size_t)q * 2 * (st.m + 1) * st.G;
+  const size_t nv = n / E, t0 = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const size_t stride = (size_t)gridDim.x * blockDim.x;
+  for (int i0 = 0; i0 <= j; i0 += U) {
+    const int c = min(U, j + 1 - i0);
+    const TV* __restrict__ Vi = Vq + (size_t)i0 * ld;
+    double s[2 * U];
+#pragma unroll
+    for (int u = 0; u < 2 * U; ++u) s[u] = 0.0;
+    for (size_t p = t0; p < nv; p += stride) {
+      const VT wv = reinterpret_cast<const VT*>(w)[p], jv = reinterpret_cast<const VT*>(vj)[p];
+      VT x[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (u < c) x[u] = reinterpret_cast<const VT*>(Vi + (size_t)u * ld)[p];
+      const TV* wp = reinterpret_cast<const TV*>(&wv);
+      const TV* jp = reinterpret_cast<const TV*>(&jv);
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (u < c) {
+          const TV* xp = reinterpret_cast<const TV*>(&x[u]);
+#pragma unroll
+          for (int k = 0; k < E; ++k) {
+            s[2 * u] += (double)wp[k] * (double)xp[k];
+            s[2 * u + 1] += (double)jp[k] * (double)xp[k];
+          }
+        }
+    }
+    for (size_t p = nv * E + t0; p < n; p += stride) {
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (u < c) {
+          const double x = (double)Vi[(size_t)u * ld + p];
+          s[2 * u] += (double)w[p] * x;
+          s[2 * u + 1] += (double)vj[p] * x;
+        }
+    }
+    block_sums<2 * U>(s, 2 * c, red, part + (size_t)2 * i0 * st.G + blockIdx.x, st.G);
+  }
+  if (!last_block(ist + 6)) return;
+  double* vals = sh;
+  double* a = vals + 2 * (st.m + 1);
+  double* sL = a + st.m + 1;
+  double* d = st.d + (size_t)q * st.sd;
+  double* L = d + st.oL();
+  const double* sig = d + st.oSig();
+  const bool cached = j * (j + 1) / 2 <= kGsL;   // rows 1..j, packed
+  sum_partials(part, st.G, 2 * (j + 1), vals);
+  const double sj = sig[j];
+  for (int k = threadIdx.x; k <= j; k += blockDim.x) {
+    const double sk = sig[k];
+    a[k] = sj * sk * vals[2 * k];
+    if (k < j) {
+      const double l = sj * sk * vals[2 * k + 1];
+      L[(size_t)j * st.m + k] = l;
+      if (cached) sL[j * (j - 1) / 2 + k] = l;
+    }
+  }
+  if (cached)
+    for (int i = 1 + (int)(threadIdx.x >> 5); i < j; i += blockDim.x >> 5)
+      for (int k = threadIdx.x & 31; k < i; k += 32) sL[i * (i - 1) / 2 + k] = L[(size_t)i * st.m + k];
+  __threadfence_block();
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    for (int k = 0; k < j; ++k) {
+      const double hk = a[k];
+      for (int i = k + 1 + (int)threadIdx.x; i <= j; i += 32)
+        a[i] -= (cached ? sL[i * (i - 1) / 2 + k] : L[(size_t)i * st.m + k]) * hk;
+      __syncwarp();
+    }
+  }
+  __syncthreads();
+  for (int k = threadIdx.x; k <= j; k += blockDim.x) d[st.oH() + k] = a[k];
+}
+
+// Sweep 2 of iteration j: v_{j+1} = w - sum_i h_i v_i (FP64 per element,
+// rounded once) and its norm; then the Givens update of the Hessenberg
+// column, written with explicitly rounded operations (the host loop's
+// arithmetic), and the step's result for the host.
+template <class TV>
+__global__ void __launch_bounds__(kGsT, 1) k_gs_update(size_t n, int j, TV* __restrict__ V, size_t vs, size_t ld,
+                                                       const TV* __restrict__ W, size_t ws, GsDev st) {
+  extern __shared__ double sh[];   // c [m + 1]: h_i sig_i, then the column
+  __shared__ double red[kGsT / 32];
+  __shared__ double nrm[1];
+  const int q = blockIdx.y;
+  int* ist = st.i + 8 * q;
+  if (ist[1]) return;
+  using VT = typename Vec16<TV>::T;
+  constexpr int E = Vec16<TV>::W, U = 8;
+  double* d = st.d + (size_t)q * st.sd;
+  const double* sig = d + st.oSig();
+  for (int k = threadIdx.x; k <= j; k += blockDim.x) sh[k] = d[st.oH() + k] * sig[k];
+  const double sj = sig[j];
+  __syncthreads();
+  const TV* __restrict__ Vq = V + (size_t)q * vs;
+  const TV* __restrict__ w = W + (size_t)q * ws;
+  TV* __restrict__ vn = V + (size_t)q * vs + (size_t)(j + 1) * ld;
+  const size_t nv = n / E, t0 = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const size_t stride = (size_t)gridDim.x * blockDim.x;
+  double s = 0.0;
+  for (size_t p = t0; p < nv; p += stride) {
+    VT wv = reinterpret_cast<const VT*>(w)[p];
+    TV* wp = reinterpret_cast<TV*>(&wv);
+    double acc[E];
+#pragma unroll
+    for (int k = 0; k < E; ++k) acc[k] = sj * (double)wp[k];
+    for (int i0 = 0; i0 <= j; i0 += U) {
+      const int c = min(U, j + 1 - i0);
+      const TV* __restrict__ Vi = Vq + (size_t)i0 * ld;
+      VT x[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (u < c) x[u] = reinterpret_cast<const VT*>(Vi + (size_t)u * ld)[p];
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (u < c) {
+          const TV* xp = reinterpret_cast<const TV*>(&x[u]);
+          const double h = sh[i0 + u];
+#pragma unroll
+          for (int k = 0; k < E; ++k) acc[k] -= h * (double)xp[k];
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < E; ++k) {
+      wp[k] = (TV)acc[k];
+      s += (double)wp[k] * (double)wp[k];
+    }
+    reinterpret_cast<VT*>(vn)[p] = wv;
+  }
+  for (size_t p = nv * E + t0; p < n; p += stride) {
+    double acc = sj * (double)w[p];
+    for (int i = 0; i <= j; ++i) acc -= sh[i] * (double)Vq[(size_t)i * ld + p];
+    const TV r = (TV)acc;
+    vn[p] = r;
+    s += (double)r * (double)r;
+  }
+  double* part = st.part + (size_t)q * 2 * (st.m + 1) * st.G;
+  block_sums<1>(&s, 1, red, part + blockIdx.x, st.G);
+  if (!last_block(ist + 7)) return;
+  sum_partials(part, st.G, 1, nrm);
+  for (int k = threadIdx.x; k <= j; k += blockDim.x) sh[k] = d[st.oH() + k];
+  __syncthreads();
+  if (threadIdx.x != 0) return;
+  double* hc = sh;
+  double* cs = d + st.oCs();
+  double* g = d + st.oG();
+  double* H = d;
+  const int m = st.m;
+  const double hj1 = __dsqrt_rn(nrm[0]);
+  const bool breakdown = hj1 == 0.0;
+  double cur = hc[0];
+  for (int i = 0; i < j; ++i) {
+    const double c0 = cs[2 * i], c1 = cs[2 * i + 1];
+    const double a = cur, bb = hc[i + 1];
+    H[(size_t)i * m + j] = __dadd_rn(__dmul_rn(c1, a), __dmul_rn(c0, bb));
+    cur = __dadd_rn(__dmul_rn(-c0, a), __dmul_rn(c1, bb));
+  }
+  double c0, c1;
+  if (__dmul_rn(cur, cur) == 0.0) {
+    c1 = 0.0;
+    c0 = 1.0;
+  } else {
+    const double coef = __ddiv_rn(1.0, __dsqrt_rn(__dadd_rn(__dmul_rn(cur, cur), __dmul_rn(hj1, hj1))));
+    c1 = __dmul_rn(__dsqrt_rn(__dmul_rn(cur, cur)), coef);
+    c0 = __ddiv_rn(__dmul_rn(c1, hj1), cur);
+  }
+  H[(size_t)j * m + j] = __dadd_rn(__dmul_rn(c1, cur), __dmul_rn(c0, hj1));
+  H[(size_t)(j + 1) * m + j] = 0.0;
+  const double gj = g[j], gj1 = __dmul_rn(-c0, gj);
+  g[j + 1] = gj1;
+  g[j] = __dmul_rn(c1, gj);
+  cs[2 * j] = c0;
+  cs[2 * j + 1] = c1;
+  d[st.oSig() + j + 1] = breakdown ? 0.0 : 1.0 / hj1;
+  const int iter = ist[0] + 1;
+  double l2res = d[st.oScal()];
+  bool done = breakdown;
+  if (!breakdown) {
+    l2res = fabs(gj1);
+    done = l2res <= d[st.oScal() + 1] || iter >= ist[4];
+  }
+  d[st.oScal()] = l2res;
+  ist[0] = iter;
+  ist[2] = j;
+  ist[5] = breakdown;
+  ist[1] = done;
+  publish(st.pub + q, j + 1, done, iter, l2res);
+}
+
+// back substitution (KspSolver.C:966-982) of the cycle, one thread per
+// system: y from the rotated Hessenberg matrix and g
+__global__ void k_gs_backsolve(GsDev st) {
+  const int q = blockIdx.x;
+  if (threadIdx.x != 0) return;
+  const int* ist = st.i + 8 * q;
+  if (!ist[3]) return;
+  double* d = st.d + (size_t)q * st.sd;
+  double *H = d, *g = d + st.oG(), *y = d + st.oY();
+  const int j = ist[2];
+  for (int i = j; i >= 0; --i) {
+    double yi = g[i];
+    for (int k = j; k >= i + 1; --k) yi = __dsub_rn(yi, __dmul_rn(H[(size_t)i * st.m + k], y[k]));
+    y[i] = __ddiv_rn(yi, H[(size_t)i * st.m + i]);
+  }
+}
+
+// out = sum_i y_i sig_i Z_i over the cycle's columns: stored as TV (ADD
+// false), or added to x (the flexible method's corrections)
+template <class TV, bool ADD>
+__global__ void __launch_bounds__(256) k_gs_combine(size_t n, const TV* __restrict__ Z, size_t zs, size_t ld, GsDev st,
+                                                    TV* __restrict__ out, size_t os, VecOut X) {
+  extern __shared__ double c[];
+  const int q = blockIdx.y;
+  const int* ist = st.i + 8 * q;
+  if (!ist[3]) return;
+  const double* d = st.d + (size_t)q * st.sd;
+  const int k = ist[2] + 1;
+  for (int i = threadIdx.x; i < k; i += blockDim.x) c[i] = d[st.oY() + i] * d[st.oSig() + i];
+  __syncthreads();
+  const size_t p = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (p >= n) return;
+  double s = 0.0;
+#pragma unroll 8
+  for (int i = 0; i < k; ++i) s += c[i] * (double)Z[(size_t)q * zs + (size_t)i * ld + p];
+  if (ADD) X.p[q][p] += s;
+  else out[(size_t)q * os + p] = (TV)s;
+}
+// x += r of the systems active in the cycle
+template <class TV>
+__global__ void k_gs_add(size_t n, const TV* __restrict__ r, size_t rs, GsDev st, VecOut X) {
+  const int q = blockIdx.y;
+  if (!st.i[8 * q + 3]) return;
+  const size_t p = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (p < n) X.p[q][p] += (double)r[(size_t)q * rs + p];
+}
+
+}  // namespace aerof
