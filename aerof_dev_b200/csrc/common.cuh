@@ -9,6 +9,7 @@
 #include <atomic>
 #include <memory>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "../../include/aerof_gpu.h"
@@ -74,6 +75,10 @@ struct DBuf {
   void upload(const T* h, size_t count, cudaStream_t s) {
     alloc(count);
     if (count) AEROF_CUDA(cudaMemcpyAsync(p, h, count * sizeof(T), cudaMemcpyHostToDevice, s));
+  }
+  void swap(DBuf& o) {
+    std::swap(p, o.p);
+    std::swap(n, o.n);
   }
   void zero(cudaStream_t s) {
     if (n) AEROF_CUDA(cudaMemsetAsync(p, 0, n * sizeof(T), s));
@@ -268,6 +273,21 @@ struct KrylovWork {
   }
 };
 
+// State-based products with H1 (h1free.cuh): per-neighbour data (once per
+// mesh geometry), node records of the linearisation state, packed vectors.
+struct H1Free {
+  bool topo = false;               // wptr and the sizes below, for the mesh
+  bool geo32 = false, geo64 = false;  // per-neighbour data current, per precision
+  bool ready = false;              // node records hold the operator's state
+  size_t total = 0;                // neighbour entries, padded per warp
+  DBuf<int> wptr;                  // [warps + 1] steps before each warp
+  DBuf<unsigned short> slot;       // [total] neighbour's staged slot
+  DBuf<float> nrm32, rec32;        // [4][total] unit normal, half length; [N][8]
+  DBuf<double> nrm64, rec64;       // the same in FP64; [N][6]
+  DBuf<double> mrow, idt, z;       // [N][4] (sum n/2, 1/vol); [N] 1/dt; packed vectors
+  void drop_geometry() { geo32 = geo64 = false; }
+};
+
 // Implicit operator: BSR-by-rows of the H1 Jacobian.
 struct Implicit {
   int precision = 0;       // 32 or 64, 0 = not assembled
@@ -275,6 +295,11 @@ struct Implicit {
   DBuf<double> diag64, off64, dinv64;   // [N][25], [2E][25], [N][25]
   DBuf<float> diag32, off32, dinv32;
   bool prec_ready = false;
+  H1Free h1;
+  // operator of a solver of this library: only its diagonal blocks are
+  // assembled, the others on demand from the linearisation point
+  bool lazy = false, lin_dt = false;
+  DBuf<double> linU, lindt;             // [N][5], [N]
   // Krylov workspace
   DBuf<double> basis;      // [(m+1)][5N]
   DBuf<double> w, r, x, b, t;

@@ -103,6 +103,12 @@ __device__ __forceinline__ void store_diag(S* __restrict__ diag, int r, const do
   store_block_vec<S>(diag, sl_dblk(r), r & 31, t);
 }
 
+}  // namespace aerof
+
+#include "h1free.cuh"
+
+namespace aerof {
+
 // One thread per row r; a warp is one slice of the sliced layout, so for
 // each neighbour position k the 32 rows write every block element as one
 // coalesced line.  For the edge e = (r, s) (r first endpoint, sg = +1) or
@@ -356,72 +362,6 @@ __global__ void __launch_bounds__(256) k_spmv(int N, const int* __restrict__ nbr
   for (int k = 0; k < 5; ++k) y[5 * (size_t)r + k] = (TO)acc[k];
 }
 
-// y_q = A p_q (or A^T p_q) for the R vectors of a batch (vector q at p + q ps,
-// y + q ys): every block is read once per group of RB vectors and applied to
-// each in k_spmv's per-row order (diagonal block, then the neighbours
-// ascending).  skip: flags, one per 8 ints; flagged vectors are left out.
-template <class S, bool TRANS, class TV, int RB>
-__global__ void __launch_bounds__(256) k_spmv_batch(int N, int R, const int* __restrict__ nbr_ptr,
-                                                    const int* __restrict__ nbr_tpos, const int* __restrict__ sptr,
-                                                    const int* __restrict__ scol, const S* __restrict__ diag,
-                                                    const S* __restrict__ off, const TV* __restrict__ p, size_t ps,
-                                                    TV* __restrict__ y, size_t ys, const int* __restrict__ skip) {
-  const int r = blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= N) return;
-  const int p0 = nbr_ptr[r], cnt = nbr_ptr[r + 1] - p0;
-  const size_t cb = (size_t)sptr[r >> 5] * 32 + (r & 31);
-  for (int q0 = 0; q0 < R; q0 += RB) {
-    bool on[RB], any = false;
-    double acc[RB][5];
-#pragma unroll
-    for (int q = 0; q < RB; ++q) {
-      on[q] = q0 + q < R && !(skip && skip[8 * (q0 + q)]);
-      any = any || on[q];
-#pragma unroll
-      for (int k = 0; k < 5; ++k) acc[q][k] = 0.0;
-    }
-    if (!any) continue;
-    auto apply = [&](const double* av, int col, bool tr) {
-#pragma unroll
-      for (int q = 0; q < RB; ++q) {
-        if (!on[q]) continue;
-        const TV* x = p + (size_t)(q0 + q) * ps + 5 * (size_t)col;
-        double xv[5];
-#pragma unroll
-        for (int k = 0; k < 5; ++k) xv[k] = (double)x[k];
-#pragma unroll
-        for (int rr = 0; rr < 5; ++rr) {
-          double t = (tr ? av[rr] : av[5 * rr]) * xv[0];
-#pragma unroll
-          for (int k = 1; k < 5; ++k) t += (tr ? av[5 * k + rr] : av[5 * rr + k]) * xv[k];
-          acc[q][rr] += t;
-        }
-      }
-    };
-    double av[25];
-    load_block<S>(diag, sl_dblk(r), r & 31, av);
-    apply(av, r, TRANS);
-    for (int k = 0; k < cnt; ++k) {
-      const int sn = scol[cb + (size_t)32 * k];
-      if (!TRANS) {
-        load_block<S>(off, sl_blk(sptr, r, k), r & 31, av);
-        apply(av, sn, false);
-      } else {
-        const int kt = nbr_tpos[p0 + k] - nbr_ptr[sn];
-        load_block<S>(off, sl_blk(sptr, sn, kt), sn & 31, av);
-        apply(av, sn, true);
-      }
-    }
-#pragma unroll
-    for (int q = 0; q < RB; ++q) {
-      if (!on[q]) continue;
-      TV* yr = y + (size_t)(q0 + q) * ys + 5 * (size_t)r;
-#pragma unroll
-      for (int k = 0; k < 5; ++k) yr[k] = (TV)acc[q][k];
-    }
-  }
-}
-
 // Block-Jacobi set-up (JacobiPrec::setup -> DiagMat::invert, DiagMatrix.C:
 // 44-80): blocks with a zero diagonal entry are left as they are (as the
 // reference does); a zero pivot counts into bad[0].
@@ -465,6 +405,19 @@ __global__ void k_bj_apply(int N, const S* __restrict__ dinv, const TI* __restri
   TO* zi = z + (size_t)q * zs + 5 * (size_t)i;
 #pragma unroll
   for (int k = 0; k < 5; ++k) zi[k] = (TO)acc[k];
+}
+
+// z = D^-1 x (or D^-T x) packed for the state-based product (h1free.cuh):
+// row o2n[i] of the blocked vector, times 1/vol for the transposed product
+template <class S>
+__global__ void k_bj_pack(int N, const S* __restrict__ dinv, const S* __restrict__ x, size_t xs,
+                          const int* __restrict__ o2n, const double* __restrict__ vol, int prodT, S* __restrict__ z,
+                          size_t zs, int trans, const int* __restrict__ skip) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x, q = blockIdx.y;
+  if (i >= N || (skip && skip[8 * q])) return;
+  double acc[5] = {0, 0, 0, 0, 0};
+  gemv_sl(dinv, sl_dblk(i), i & 31, x + (size_t)q * xs + 5 * (size_t)i, acc, trans != 0);
+  h1_put<S>(z + (size_t)q * zs, o2n[i], prodT ? 1.0 / vol[i] : 1.0, acc);
 }
 
 // ------------------------------------------------------------ vector ops
@@ -616,7 +569,82 @@ static void need_jac(aerof_gpu_ctx* c) {
 static size_t sl_diag_size(const DeviceMesh& m) { return (size_t)m.nsl * 800; }
 static size_t sl_off_size(const DeviceMesh& m) { return std::max<size_t>((size_t)m.h_sptr.back() * 800, 1); }
 
-void jacobian_dev(aerof_gpu_ctx* c, const double* dU, const double* ddt, int precision, bool transposed) {
+// shared memory of the state-based product for this mesh
+static size_t h1_smem(const DeviceMesh& m, int precision) {
+  const size_t w = precision == AEROF_PREC_FP32 ? sizeof(float) * H1Rec<float>::SM : sizeof(double) * H1Rec<double>::SM;
+  return w * (m.NB + m.maxH);
+}
+static bool h1_fits(const DeviceMesh& m, int precision) {
+  return kIB % m.NB == 0 && kIB / m.NB <= 32 && h1_smem(m, precision) <= 200 * 1024;
+}
+
+// Per-neighbour data of the state-based product, once per mesh geometry and
+// precision.
+static void h1_geometry(aerof_gpu_ctx* c, int precision) {
+  DeviceMesh& m = c->mesh;
+  H1Free& f = c->imp.h1;
+  cudaStream_t s = c->stream;
+  const int L = kIB / m.NB, wpb = kIB / 32;
+  if (!f.topo) {
+    // steps of each warp: the most neighbours of any of its nodes, by lanes
+    std::vector<int> n2o(m.N), wp((size_t)m.nblk * wpb + 1, 0);
+    for (int o = 0; o < m.N; ++o) n2o[m.h_o2n[o]] = o;
+    for (int b = 0; b < m.nblk; ++b)
+      for (int w = 0; w < wpb; ++w) {
+        int steps = 0;
+        for (int t = w * 32 / L; t < (w + 1) * 32 / L; ++t) {
+          const int n = b * m.NB + t;
+          if (t >= m.NB || n >= m.N) break;
+          const int deg = m.h_nbr_ptr[n2o[n] + 1] - m.h_nbr_ptr[n2o[n]];
+          steps = std::max(steps, (deg + L - 1) / L);
+        }
+        wp[(size_t)b * wpb + w + 1] = wp[(size_t)b * wpb + w] + steps;
+      }
+    f.total = std::max<size_t>((size_t)wp.back() * 32, 32);
+    f.wptr.upload(wp.data(), wp.size(), s);
+    AEROF_CUDA(cudaStreamSynchronize(s));
+    f.slot.alloc(f.total);
+    f.mrow.alloc(4 * (size_t)m.N);
+    f.topo = true;
+  }
+  auto go = [&](auto& nrm, bool& ready) {
+    if (ready) return;
+    using S = std::remove_pointer_t<decltype(nrm.p)>;
+    nrm.alloc(4 * f.total);
+    k_h1_geometry<S><<<m.nblk, kIB, 0, s>>>(m.N, m.NB, m.E, m.n2o.p, m.o2n.p, m.nbr_ptr.p, m.nbr_node.p, m.nbr_edge.p,
+                                            m.en.p, m.hptr.p, m.hnode.p, m.vol.p, f.wptr.p, f.total, nrm.p, f.slot.p,
+                                            f.mrow.p);
+    AEROF_LAUNCH_CHECK();
+    ready = true;
+  };
+  if (precision == AEROF_PREC_FP32) go(f.nrm32, f.geo32);
+  else go(f.nrm64, f.geo64);
+}
+
+// Node records of the state-based product at the state of the primitive
+// records P, in the operator's precision.
+static void h1_records(aerof_gpu_ctx* c, const double* ddt, int precision) {
+  DeviceMesh& m = c->mesh;
+  H1Free& f = c->imp.h1;
+  const Gas g = make_gas(c->cfg.gamma);
+  f.idt.ensure(m.N);
+  auto go = [&](auto& rec) {
+    using S = std::remove_pointer_t<decltype(rec.p)>;
+    rec.ensure((size_t)H1Rec<S>::W * m.N);
+    k_h1_records<S><<<grid_for(m.N, kIB), kIB, 0, c->stream>>>(m.N, g, m.n2o.p, m.P.p, ddt, rec.p, f.idt.p);
+    AEROF_LAUNCH_CHECK();
+  };
+  if (precision == AEROF_PREC_FP32) go(f.rec32);
+  else go(f.rec64);
+}
+
+// H1 at device state dU with device time steps ddt (may be null).  lazy:
+// only what the Krylov solvers with block-Jacobi read, the node records of
+// the state-based product and the diagonal blocks; the off-diagonal blocks
+// are formed by need_blocks if a later call asks for them, from dU and ddt,
+// which the caller keeps in imp.linU / imp.lindt.
+void jacobian_dev(aerof_gpu_ctx* c, const double* dU, const double* ddt, int precision, bool transposed,
+                  bool lazy = false) {
   DeviceMesh& m = c->mesh;
   Implicit& J = c->imp;
   const Gas g = make_gas(c->cfg.gamma);
@@ -636,23 +664,55 @@ void jacobian_dev(aerof_gpu_ctx* c, const double* dU, const double* ddt, int pre
                                                         m.sptr.p, off, diag);
     AEROF_LAUNCH_CHECK();
   };
+  auto diag_only = [&](auto* diag, auto kern) {
+    kern<<<grid_for((size_t)m.N, 128), 128, 0, c->stream>>>(m.N, m.E, g, m.nbr_ptr.p, m.nbr_node.p, m.nbr_edge.p,
+                                                            m.en.p, m.P.p, m.vol.p, m.brow.p, J.fsum.p, ddt, diag);
+    AEROF_LAUNCH_CHECK();
+  };
+  J.h1.ready = h1_fits(m, precision);
+  lazy = lazy && J.h1.ready;
+  if (J.h1.ready) h1_records(c, ddt, precision);
   if (precision == AEROF_PREC_FP32) {
     J.diag64.release(); J.off64.release(); J.dinv64.release();
     J.diag32.alloc(sl_diag_size(m));
-    J.off32.alloc(sl_off_size(m));
-    if (transposed) rows(J.off32.p, J.diag32.p, k_jac_rows<float, true>);
-    else rows(J.off32.p, J.diag32.p, k_jac_rows<float, false>);
+    if (lazy) {
+      if (transposed) diag_only(J.diag32.p, k_h1_diag<float, true>);
+      else diag_only(J.diag32.p, k_h1_diag<float, false>);
+    } else {
+      J.off32.alloc(sl_off_size(m));
+      if (transposed) rows(J.off32.p, J.diag32.p, k_jac_rows<float, true>);
+      else rows(J.off32.p, J.diag32.p, k_jac_rows<float, false>);
+    }
   } else {
     J.diag32.release(); J.off32.release(); J.dinv32.release();
     J.diag64.alloc(sl_diag_size(m));
-    J.off64.alloc(sl_off_size(m));
-    if (transposed) rows(J.off64.p, J.diag64.p, k_jac_rows<double, true>);
-    else rows(J.off64.p, J.diag64.p, k_jac_rows<double, false>);
+    if (lazy) {
+      if (transposed) diag_only(J.diag64.p, k_h1_diag<double, true>);
+      else diag_only(J.diag64.p, k_h1_diag<double, false>);
+    } else {
+      J.off64.alloc(sl_off_size(m));
+      if (transposed) rows(J.off64.p, J.diag64.p, k_jac_rows<double, true>);
+      else rows(J.off64.p, J.diag64.p, k_jac_rows<double, false>);
+    }
   }
+  J.lazy = lazy;
+  J.lin_dt = ddt != nullptr;
   J.precision = precision;
   J.transposed = transposed;
   J.prec_ready = false;
   J.ilu_ready = false;
+}
+
+// the stored blocks of an operator that was assembled lazily (a product, a
+// read-back or an ILU(0) set-up after a Newton or linearised solve); the
+// preconditioner set up from it stays
+static void need_blocks(aerof_gpu_ctx* c) {
+  Implicit& J = c->imp;
+  if (!J.lazy) return;
+  const bool pr = J.prec_ready, il = J.ilu_ready;
+  jacobian_dev(c, J.linU.p, J.lin_dt ? J.lindt.p : nullptr, J.precision, J.transposed);
+  J.prec_ready = pr;
+  J.ilu_ready = il;
 }
 
 // products with H1 (trans = 0) or H1^T (trans = 1); the stored blocks may
@@ -678,7 +738,10 @@ void matvec_t(aerof_gpu_ctx* c, const TI* p, TO* y, int trans, const int* skip =
     else go(k_spmv<double, false, TI, TO>, J.diag64.p, J.off64.p);
   }
 }
-void matvec_dev(aerof_gpu_ctx* c, const double* p, double* y, int trans) { matvec_t<double, double>(c, p, y, trans); }
+void matvec_dev(aerof_gpu_ctx* c, const double* p, double* y, int trans) {
+  need_blocks(c);
+  matvec_t<double, double>(c, p, y, trans);
+}
 
 // ---------------------------------------------------------------------
 // Block ILU(0) (IluPrec, KspPrec.C:138-330; SparseMat::numericILU and
@@ -1023,6 +1086,7 @@ __global__ void k_ilu_bwd_b(int i0, int cnt, int s0, int R, const int* __restric
 // gather + factorisation of the operator read with orientation tr;
 // returns the number of singular diagonal blocks (waits for the stream)
 static int ilu_setup(aerof_gpu_ctx* c, int tr) {
+  need_blocks(c);
   DeviceMesh& m = c->mesh;
   Implicit& J = c->imp;
   cudaStream_t s = c->stream;
@@ -1186,30 +1250,56 @@ static bool gmres_device_loop_enabled() {
   return v != 0;
 }
 
-// y_q = H1 x_q (or H1^T x_q) of the R vectors x + q xs, y + q ys
+// y_q = H1 M^-1 x_q (or H1^T M^-T x_q) of the R vectors x + q xs, y + q ys
+// (M the preconditioner, or the identity when !precond; scratch z, R vectors
+// at stride zs).  Formed from the states (h1free.cuh) whenever the operator
+// was assembled here and the mesh's blocks fit; an operator given by the
+// caller (aerof_gpu_set_jacobian) is read from its stored blocks.  skip:
+// device flags, one per 8 ints.
 template <class TV>
-static void h1_product(aerof_gpu_ctx* c, int R, const TV* x, size_t xs, TV* y, size_t ys, int trans,
-                       const int* skip) {
-  if (R == 1) {
-    matvec_t<TV, TV>(c, x, y, trans, skip);
-    return;
-  }
+static void h1_precond_product(aerof_gpu_ctx* c, int R, const TV* x, size_t xs, TV* y, size_t ys, TV* z, size_t zs,
+                               int trans, bool precond, const int* skip) {
   DeviceMesh& m = c->mesh;
   Implicit& J = c->imp;
-  TimerScope t(c, AEROF_T_KSP_MATVEC);
-  const bool tr = (trans != 0) != J.transposed;
-  auto go = [&](auto kern, auto* diag, auto* off) {
-    kern<<<grid_for(m.N, kIB), kIB, 0, c->stream>>>(m.N, R, m.nbr_ptr.p, m.nbr_tpos.p, m.sptr.p, m.scol.p, diag, off,
-                                                    x, xs, y, ys, skip);
-    AEROF_LAUNCH_CHECK();
-  };
-  if (J.precision == AEROF_PREC_FP32) {
-    if (tr) go(k_spmv_batch<float, true, TV, 4>, J.diag32.p, J.off32.p);
-    else go(k_spmv_batch<float, false, TV, 4>, J.diag32.p, J.off32.p);
-  } else {
-    if (tr) go(k_spmv_batch<double, true, TV, 4>, J.diag64.p, J.off64.p);
-    else go(k_spmv_batch<double, false, TV, 4>, J.diag64.p, J.off64.p);
+  H1Free& f = J.h1;
+  cudaStream_t s = c->stream;
+  const bool f32 = std::is_same<TV, float>::value;
+  // the Krylov vectors are stored in the operator's precision
+  if (!f.ready || (J.precision == AEROF_PREC_FP32) != f32) {
+    if (precond) prec_apply_t<TV, TV>(c, x, z, trans, R, xs, zs, skip);
+    for (int q = 0; q < R; ++q)
+      matvec_t<TV, TV>(c, precond ? z + (size_t)q * zs : x + (size_t)q * xs, y + (size_t)q * ys, trans,
+                       skip ? skip + 8 * q : nullptr);
+    return;
   }
+  h1_geometry(c, J.precision);
+  const size_t pz = (size_t)H1Rec<TV>::W * m.N;
+  f.z.ensure(((size_t)R * pz * sizeof(TV) + 7) / 8);
+  TV* zp = reinterpret_cast<TV*>(f.z.p);
+  TV *rec, *nrm, *dinv;
+  if constexpr (std::is_same<TV, float>::value) { rec = f.rec32.p; nrm = f.nrm32.p; dinv = J.dinv32.p; }
+  else { rec = f.rec64.p; nrm = f.nrm64.p; dinv = J.dinv64.p; }
+  const dim3 gn(grid_for(m.N, kIB), R);
+  {
+    TimerScope t(c, AEROF_T_KSP_OTHER);
+    if (precond && J.pc != AEROF_PC_ILU0) {
+      k_bj_pack<TV><<<gn, kIB, 0, s>>>(m.N, dinv, x, xs, m.o2n.p, m.vol.p, trans, zp, pz,
+                                       (trans != 0) != J.transposed ? 1 : 0, skip);
+    } else {
+      if (precond) prec_apply_t<TV, TV>(c, x, z, trans, R, xs, zs, skip);
+      k_h1_pack<TV, TV><<<gn, kIB, 0, s>>>(m.N, m.o2n.p, m.vol.p, trans, precond ? z : x, precond ? zs : xs, zp, pz,
+                                           skip);
+    }
+    AEROF_LAUNCH_CHECK();
+  }
+  TimerScope t(c, AEROF_T_KSP_MATVEC);
+  const size_t smem = h1_smem(m, J.precision);
+  auto kern = trans ? k_h1_apply<TV, true> : k_h1_apply<TV, false>;
+  AEROF_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  kern<<<dim3(m.nblk, R), kIB, smem, s>>>(m.N, m.NB, make_gas(c->cfg.gamma), m.n2o.p, m.hptr.p, m.hnode.p, f.wptr.p,
+                                         f.total, nrm, f.slot.p, f.mrow.p, rec, f.idt.p, m.brow.p, J.fsum.p, zp, pz,
+                                         y, ys, skip);
+  AEROF_LAUNCH_CHECK();
 }
 
 // Device state of R systems with restart length m over vectors of n
@@ -1334,14 +1424,13 @@ static void gmres_device(aerof_gpu_ctx* c, int R, const double* const* B, double
         k_scale<double, TV><<<grid_for(n, kIB), kIB, 0, s>>>(n, 1.0, X[q], Z + (size_t)q * ld);
         AEROF_LAUNCH_CHECK();
       }
-      h1_product<TV>(c, R, Z, ld, W, ld, trans, done);
+      h1_precond_product<TV>(c, R, Z, ld, W, ld, nullptr, 0, trans, false, done);
       k_gs_start<TV, false><<<gs, kGsT, 0, s>>>(n, b, x, W, ld, V, vs, st, eps, maxits);
     }
     AEROF_LAUNCH_CHECK();
     for (int j = 0; j < numVec; ++j) {
       if (gs_wait(c, kw, R, j - kGsAhead)) break;
-      prec_apply_t<TV, TV>(c, V + (size_t)j * ld, Z, trans, R, vs, ld, done);
-      h1_product<TV>(c, R, Z, ld, W, ld, trans, done);
+      h1_precond_product<TV>(c, R, V + (size_t)j * ld, vs, W, ld, Z, ld, trans, true, done);
       gs_iteration<TV>(c, st, R, n, j, V, vs, ld, W, ld);
     }
     k_gs_backsolve<<<R, 32, 0, s>>>(st);
@@ -1474,7 +1563,11 @@ static int gmres_t(aerof_gpu_ctx* c, const double* b, double* x, int numVec, int
   double* yd = J.hcol.p + numVec + 2;  // [numVec + 1] solution coefficients
   double* part = c->s.red.p;
   auto op = [&](const TV* p, TV* y) {
-    if (!exactU) { matvec_t<TV, TV>(c, p, y, trans); return; }
+    if (!exactU) {
+      need_blocks(c);
+      matvec_t<TV, TV>(c, p, y, trans);
+      return;
+    }
     TimerScope t(c, AEROF_T_KSP_MATVEC);
     exact_product(c, exactU, reinterpret_cast<const double*>(p), reinterpret_cast<double*>(y), trans);
   };
@@ -1605,6 +1698,7 @@ extern "C" int aerof_gpu_get_jacobian(aerof_gpu_ctx* c, double* A) {
   return guard(c, [&]() -> int {
     need_jac(c);
     if (!A) return AEROF_EINVAL;
+    need_blocks(c);
     DeviceMesh& m = c->mesh;
     Implicit& J = c->imp;
     const size_t nd = sl_diag_size(m), no = sl_off_size(m);
@@ -1816,6 +1910,8 @@ extern "C" int aerof_gpu_set_jacobian(aerof_gpu_ctx* c, const double* A, int pre
     }
     J.precision = precision;
     J.transposed = false;
+    J.lazy = false;
+    J.h1.ready = false;
     J.prec_ready = false;
     J.ilu_ready = false;
     return AEROF_OK;
@@ -1939,13 +2035,17 @@ extern "C" int aerof_gpu_newton(aerof_gpu_ctx* c, double* U, const aerof_newton_
       AEROF_CUDA(cudaMemcpyAsync(c->s.Ustage.p, U, n * sizeof(double), cudaMemcpyHostToDevice, s));
       dU = c->s.Ustage.p;
     }
-    c->imp.b.ensure(n); c->imp.x.ensure(n); c->s.dt.ensure(m.N); c->s.k1.ensure(n); c->s.U0.ensure(n);
+    c->imp.b.ensure(n); c->imp.x.ensure(n); c->s.k1.ensure(n);
     c->s.counters.ensure(8);
     double* R = c->s.k1.p;
     double* rhs = c->imp.b.p;
     double* dQ = c->imp.x.p;
-    double* dt = c->s.dt.p;
-    double* Uprev = c->s.U0.p;
+    // the linearisation point of the step: what a redo restores, and what
+    // need_blocks assembles from after the call
+    c->imp.linU.ensure(n);
+    c->imp.lindt.ensure(m.N);
+    double* dt = c->imp.lindt.p;
+    double* Uprev = c->imp.linU.p;
     int* nbad_d = c->s.counters.p + 5;
     const int gv = grid_for(n, kIB);
     cudaEvent_t e0, e1;
@@ -1971,8 +2071,11 @@ extern "C" int aerof_gpu_newton(aerof_gpu_ctx* c, double* U, const aerof_newton_
         rel_prev = rel;
       }
       redo = false;
+      // (not lazily before this point: an operator assembled lazily by the
+      // previous step is replaced as a whole)
+      AEROF_CUDA(cudaMemcpyAsync(Uprev, dU, n * sizeof(double), cudaMemcpyDeviceToDevice, s));
       timestep_dev(c, dU, cfl, dt);
-      jacobian_dev(c, dU, dt, p->precision, false);
+      jacobian_dev(c, dU, dt, p->precision, false, c->imp.pc == AEROF_PC_JACOBI && gmres_device_loop_enabled());
       if (int nb = prec_setup_dev(c)) {
         c->last_error = std::to_string(nb) + " singular diagonal block(s) at Newton step " + std::to_string(k);
         return AEROF_ESINGULAR;
@@ -1980,12 +2083,11 @@ extern "C" int aerof_gpu_newton(aerof_gpu_ctx* c, double* U, const aerof_newton_
       k_scale<double, double><<<gv, kIB, 0, s>>>(n, -1.0, R, rhs);
       AEROF_LAUNCH_CHECK();
       lits += gmres_dev(c, rhs, dQ, p->ksp_krylov, p->ksp_maxits, p->ksp_eps, 0, nullptr, nullptr);
-      // rhs = Q; Q += dQ, then the physical-solution check
+      // Q += dQ, then the physical-solution check
       // (NewtonSolver.h:187-215): on a non-positive density or pressure the
       // state is restored and the step redone with half the CFL number
       // (TsParameters::computeCflNumber, TsParameters.C:187-195), which
       // gives up below cfl0/1000
-      AEROF_CUDA(cudaMemcpyAsync(Uprev, dU, n * sizeof(double), cudaMemcpyDeviceToDevice, s));
       k_add<double><<<gv, kIB, 0, s>>>(n, dQ, dU);
       AEROF_LAUNCH_CHECK();
       AEROF_CUDA(cudaMemsetAsync(nbad_d, 0, sizeof(int), s));
@@ -2054,10 +2156,11 @@ extern "C" int aerof_gpu_linearized_solve(aerof_gpu_ctx* c, const double* U, con
     need_mesh_or_throw(c);
     if (!U || !b || !x || krylov < 1 || maxits < 1 || !(eps >= 0.0) || inner_its < 0) return AEROF_EINVAL;
     const size_t n = 5 * (size_t)c->mesh.N;
+    // the state becomes the operator's linearisation point once assembled
+    // (an earlier operator keeps its own until then)
     c->imp.t.ensure(n);
     const double* dU0 = in_dev(c, U, n, c->s.Ustage);
-    if (dU0 != c->imp.t.p)
-      AEROF_CUDA(cudaMemcpyAsync(c->imp.t.p, dU0, n * sizeof(double), cudaMemcpyDeviceToDevice, c->stream));
+    AEROF_CUDA(cudaMemcpyAsync(c->imp.t.p, dU0, n * sizeof(double), cudaMemcpyDeviceToDevice, c->stream));
     const double* dU = c->imp.t.p;
     const double* db = in_dev(c, b, n, c->s.Vstage);
     double* dx = out_dev(c, x, n, c->s.Rstage);
@@ -2071,7 +2174,11 @@ extern "C" int aerof_gpu_linearized_solve(aerof_gpu_ctx* c, const double* U, con
       h2_evaluate_dev(c, dU);
       c->h2.use = true;
     }
-    jacobian_dev(c, dU, nullptr, inner_its ? AEROF_PREC_FP32 : AEROF_PREC_FP64, inner_its && transpose);
+    // with block-Jacobi only the diagonal blocks are read (the inner products
+    // are formed from the states, and inner_its = 0 has no products with H1)
+    const bool lazy = c->imp.pc == AEROF_PC_JACOBI && gmres_device_loop_enabled();
+    jacobian_dev(c, dU, nullptr, inner_its ? AEROF_PREC_FP32 : AEROF_PREC_FP64, inner_its && transpose, lazy);
+    c->imp.linU.swap(c->imp.t);
     if (int nb = prec_setup_dev(c, transpose)) {
       c->last_error = std::to_string(nb) + " singular diagonal block(s)";
       return AEROF_ESINGULAR;
@@ -2107,10 +2214,11 @@ extern "C" int aerof_gpu_linearized_solve_batch(aerof_gpu_ctx* c, const double* 
       return AEROF_EINVAL;
     if (nrhs == 0) return AEROF_OK;
     const size_t n = 5 * (size_t)c->mesh.N;
+    // the state becomes the operator's linearisation point once assembled
+    // (an earlier operator keeps its own until then)
     c->imp.t.ensure(n);
     const double* dU0 = in_dev(c, U, n, c->s.Ustage);
-    if (dU0 != c->imp.t.p)
-      AEROF_CUDA(cudaMemcpyAsync(c->imp.t.p, dU0, n * sizeof(double), cudaMemcpyDeviceToDevice, c->stream));
+    AEROF_CUDA(cudaMemcpyAsync(c->imp.t.p, dU0, n * sizeof(double), cudaMemcpyDeviceToDevice, c->stream));
     const double* dU = c->imp.t.p;
     struct UseStored {
       H2Op& h;
@@ -2118,7 +2226,11 @@ extern "C" int aerof_gpu_linearized_solve_batch(aerof_gpu_ctx* c, const double* 
     } use_stored{c->h2};
     h2_evaluate_dev(c, dU);
     c->h2.use = true;
-    jacobian_dev(c, dU, nullptr, inner_its ? AEROF_PREC_FP32 : AEROF_PREC_FP64, inner_its && transpose);
+    // with block-Jacobi only the diagonal blocks are read (the inner products
+    // are formed from the states, and inner_its = 0 has no products with H1)
+    const bool lazy = c->imp.pc == AEROF_PC_JACOBI && gmres_device_loop_enabled();
+    jacobian_dev(c, dU, nullptr, inner_its ? AEROF_PREC_FP32 : AEROF_PREC_FP64, inner_its && transpose, lazy);
+    c->imp.linU.swap(c->imp.t);
     if (int nb = prec_setup_dev(c, transpose)) {
       c->last_error = std::to_string(nb) + " singular diagonal block(s)";
       return AEROF_ESINGULAR;

@@ -391,6 +391,7 @@ void compute_blocked_geometry(aerof_gpu_ctx* c) {
 void compute_geometry(aerof_gpu_ctx* c) {
   DeviceMesh& m = c->mesh;
   cudaStream_t s = c->stream;
+  c->imp.h1.drop_geometry();
   m.vol.alloc(m.N);
   m.en.alloc(3 * (size_t)m.E);
   m.fnrm.alloc(3 * (size_t)std::max(m.F, 1));
@@ -483,6 +484,7 @@ extern "C" int aerof_gpu_set_mesh(aerof_gpu_ctx* c, int N, int T, int F, const d
     cudaStream_t s = c->stream;
     m.N = N; m.T = T; m.F = F; m.E = E;
     m.grad_grid = 0;
+    c->imp.h1.topo = false;
     for (int k = 0; k < 5; ++k) m.Ub[k] = Ub[k];
     m.Ubd.upload(Ub, 5, s);
     m.X.upload(X, 3 * (size_t)N, s);
