@@ -116,7 +116,7 @@ __global__ void k_d_edge_flux(int E, Gas g, int rec, double beta, const int2* __
     atomicAdd(&counters[0], 1);
   } else {
     Dual n0 = en[l], n1 = en[(size_t)E + l], n2 = en[2 * (size_t)E + l];
-    if (sqrt(n0.v * n0.v + n1.v * n1.v + n2.v * n2.v) >= 1e-18) roe_flux(g, n0, n1, n2, Vi, Vj, f);
+    if (n0.v * n0.v + n1.v * n1.v + n2.v * n2.v >= 1e-36) roe_flux(g, n0, n1, n2, Vi, Vj, f);
   }
 #pragma unroll
   for (int k = 0; k < 5; ++k) flux[(size_t)k * E + l] = f[k];
@@ -252,7 +252,7 @@ __global__ void k_a_edges(int E, Gas g, int rec, double beta, const int2* __rest
 #pragma unroll
   for (int k = 0; k < 5; ++k) gF[k] = lam[5 * (size_t)ij.x + k] - lam[5 * (size_t)ij.y + k];
   const double n0 = en[l], n1 = en[(size_t)E + l], n2 = en[2 * (size_t)E + l];
-  if (sqrt(n0 * n0 + n1 * n1 + n2 * n2) >= 1e-18) roe_flux_adj(g, n0, n1, n2, Vi, Vj, gF, gL, gR, gn);
+  if (n0 * n0 + n1 * n1 + n2 * n2 >= 1e-36) roe_flux_adj(g, n0, n1, n2, Vi, Vj, gF, gL, gR, gn);
   double* o = out + 32 * (size_t)l;
   double gdx0 = 0.0, gdx1 = 0.0, gdx2 = 0.0;
 #pragma unroll
@@ -462,6 +462,12 @@ __global__ void k_a_lam2(int N, const int* __restrict__ n2o, const double* __res
   lam2[6 * (size_t)n + 5] = 0.0;
 }
 
+// Threads of the reverse sweep.  Its staging leaves one CTA per SM, so the
+// warps in flight are the CTA's: 8 at 256 threads and 234 registers, 16 at
+// 512 and 128 (some spills).  Adjoint products at 101^3: 4.41 ms with 384,
+// 4.24 ms with 512 (4.70 ms with 256 and exact divisions and roots).
+constexpr int kRevThreads = 512;
+
 // One CTA per block.  Phase 0: node records, gradients and lam of the
 // block's nodes and forward halo are staged in shared memory (cp.async).
 // Phase 1, thread per edge: the reconstruction is recomputed, the Roe flux
@@ -474,7 +480,7 @@ __global__ void k_a_lam2(int N, const int* __restrict__ n2o, const double* __res
 // the node's side: g_V += g_Vside, g_grad += dx (x) g_ddside; xor-tree lane
 // sum; written to gVp / gGp.
 template <bool GEO>
-__global__ void __launch_bounds__(256, 1) k_a_fv_blocked(int N, int E, int NB, Gas g, int rec, double beta,
+__global__ void __launch_bounds__(kRevThreads, 1) k_a_fv_blocked(int N, int E, int NB, Gas g, int rec, double beta,
                                                          const ushort2* __restrict__ bl, const double* __restrict__ bn,
                                                          const int* __restrict__ beptr, const int* __restrict__ hfptr,
                                                          const int* __restrict__ hfpad, int maxHf,
@@ -555,7 +561,7 @@ __global__ void __launch_bounds__(256, 1) k_a_fv_blocked(int N, int E, int NB, G
     double gF[5], gL[5] = {0, 0, 0, 0, 0}, gR[5] = {0, 0, 0, 0, 0}, gn[3] = {0, 0, 0};
 #pragma unroll
     for (int k = 0; k < 5; ++k) gF[k] = Ln[6 * lq.x + k] - Ln[6 * lq.y + k];
-    if (sqrt(n0_ * n0_ + n1_ * n1_ + n2_ * n2_) >= 1e-18) roe_flux_adj(g, n0_, n1_, n2_, Vi, Vj, gF, gL, gR, gn);
+    if (n0_ * n0_ + n1_ * n1_ + n2_ * n2_ >= 1e-36) roe_flux_adj(g, n0_, n1_, n2_, Vi, Vj, gF, gL, gR, gn);
     double* es = Es + 10 * (q - e0);
 #pragma unroll
     for (int k = 0; k < 5; ++k) { es[k] = gL[k]; es[5 + k] = gR[k]; }
@@ -988,7 +994,7 @@ static void reverse_sweep_blocked(aerof_gpu_ctx* c, const double* dw, bool geo, 
   const size_t smem = ((size_t)(kPS + kGS + 6) * (m.NB + m.maxHf) + (size_t)10 * m.maxE) * sizeof(double);
   auto go = [&](auto kern) {
     AEROF_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    kern<<<m.nblk, 256, smem, s>>>(m.N, m.E, m.NB, g, rec, c->cfg.beta, m.bl.p, m.bnorm.p, m.beptr.p, m.hfptr.p,
+    kern<<<m.nblk, kRevThreads, smem, s>>>(m.N, m.E, m.NB, g, rec, c->cfg.beta, m.bl.p, m.bnorm.p, m.beptr.p, m.hfptr.p,
                                    m.hfpad.p, m.maxHf, m.P2.p, c->s.G2.p, a.lam2.p, m.lptr.p, m.lidx.p, m.xslot.p,
                                    m.bsrc.p, a.gVp.p, a.gGp.p, a.spill.p, geo ? a.geo.p : nullptr);
     AEROF_LAUNCH_CHECK();
@@ -1513,7 +1519,7 @@ __global__ void __launch_bounds__(128) k_h2_edges(int N, int E, int NB, Gas g, i
         cq1[k] = cq2[k] = beta;
       }
     }
-    const bool live = sqrt(n0_ * n0_ + n1_ * n1_ + n2_ * n2_) >= 1e-18;
+    const bool live = n0_ * n0_ + n1_ * n1_ + n2_ * n2_ >= 1e-36;
 #pragma unroll 1
     for (int r = 0; r < 5; ++r) {
       double gF[5], gL[5] = {0, 0, 0, 0, 0}, gR[5] = {0, 0, 0, 0, 0};
