@@ -237,6 +237,7 @@ struct Scratch {
   DBuf<double> G2;         // [N][16] gradients, blocked numbering
   DBuf<double> part;       // [N][5] block-local flux sums, blocked numbering
   DBuf<double> spill;      // [nX][5] fluxes of block-crossing edges
+  DBuf<double> wpart, wspill;  // [N], [nX] wave-speed sums, blocked numbering
   DBuf<double> Ustage, Rstage, Vstage, Xstage;  // staging for host arrays
   DBuf<double> dt, k1, k2, U0;
   DBuf<int> tag;           // [N] failsafe tags

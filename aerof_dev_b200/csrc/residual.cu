@@ -590,39 +590,17 @@ __global__ void __launch_bounds__(THREADS, MINB)
   }
 }
 
-// BLOCKED organisation, per node in the blocked numbering: block-local sum,
-// minus the spilled fluxes of incoming block-crossing edges, plus the
-// node's boundary subface fluxes (face order), times 1/ctrlVol; written to
-// R in the caller's numbering through n2o.  Partial sums, spills and
-// subface fluxes are read in node order (coalesced); the caller-order
-// variant that gathers them through o2n measured slower.  FACES: the
-// subface fluxes are evaluated here from the node's own state (the
-// operations of k_face_flux: normal n_f / 3, face_flux), instead of being
-// read from fbuf.
+// Node n's flux sum in the blocked numbering: block-local part, minus the
+// spilled fluxes of incoming block-crossing edges, plus the node's boundary
+// subface fluxes (face order; FACES: evaluated here from the node's own
+// state, the operations of k_face_flux, instead of read from fbuf).
 template <bool FACES>
-__global__ void k_fv_nodes_b(int N, Gas g, const int* __restrict__ n2o, const double* __restrict__ part,
-                             const int* __restrict__ xin_ptr, const double* __restrict__ spill,
-                             const int* __restrict__ bnf_ptr, const int* __restrict__ bnf_ent,
-                             const double* __restrict__ fbuf, int F, const double* __restrict__ Ub0,
-                             const int* __restrict__ fcode, const double* __restrict__ fn,
-                             const double* __restrict__ P2, const double* __restrict__ vol2, double* __restrict__ R,
-                             const int* __restrict__ blist, int nlist, int NB, int* __restrict__ cnt,
-                             volatile int* __restrict__ pub) {
-  int n = blockIdx.x * blockDim.x + threadIdx.x;
-  // the edge fluxes are complete: their unphysical count goes to the host's
-  // page-locked word, and the counter back to zero for the next call
-  if (pub && n == 0) {
-    *pub = *cnt;
-    *cnt = 0;
-  }
-  if (blist) {
-    // the nodes of blocks blist[0, nlist)
-    const int i = n / NB;
-    if (i >= nlist) return;
-    n = blist[i] * NB + n % NB;
-  }
-  if (n >= N) return;
-  double acc[5];
+__device__ __forceinline__ void node_sum(int n, const Gas& g, const double* __restrict__ part,
+                                         const int* __restrict__ xin_ptr, const double* __restrict__ spill,
+                                         const int* __restrict__ bnf_ptr, const int* __restrict__ bnf_ent,
+                                         const double* __restrict__ fbuf, int F, const double* __restrict__ Ub0,
+                                         const int* __restrict__ fcode, const double* __restrict__ fn,
+                                         const double* P2, double* acc) {
 #pragma unroll
   for (int c = 0; c < 5; ++c) acc[c] = part[5 * (size_t)n + c];
   for (int k = xin_ptr[n]; k < xin_ptr[n + 1]; ++k) {
@@ -652,6 +630,39 @@ __global__ void k_fv_nodes_b(int N, Gas g, const int* __restrict__ n2o, const do
       for (int c = 0; c < 5; ++c) acc[c] += ff[c];
     }
   }
+}
+
+// BLOCKED organisation, per node in the blocked numbering: block-local sum,
+// minus the spilled fluxes of incoming block-crossing edges, plus the
+// node's boundary subface fluxes (face order), times 1/ctrlVol; written to
+// R in the caller's numbering through n2o.  Partial sums, spills and
+// subface fluxes are read in node order (coalesced); the caller-order
+// variant that gathers them through o2n measured slower.
+template <bool FACES>
+__global__ void k_fv_nodes_b(int N, Gas g, const int* __restrict__ n2o, const double* __restrict__ part,
+                             const int* __restrict__ xin_ptr, const double* __restrict__ spill,
+                             const int* __restrict__ bnf_ptr, const int* __restrict__ bnf_ent,
+                             const double* __restrict__ fbuf, int F, const double* __restrict__ Ub0,
+                             const int* __restrict__ fcode, const double* __restrict__ fn,
+                             const double* __restrict__ P2, const double* __restrict__ vol2, double* __restrict__ R,
+                             const int* __restrict__ blist, int nlist, int NB, int* __restrict__ cnt,
+                             volatile int* __restrict__ pub) {
+  int n = blockIdx.x * blockDim.x + threadIdx.x;
+  // the edge fluxes are complete: their unphysical count goes to the host's
+  // page-locked word, and the counter back to zero for the next call
+  if (pub && n == 0) {
+    *pub = *cnt;
+    *cnt = 0;
+  }
+  if (blist) {
+    // the nodes of blocks blist[0, nlist)
+    const int i = n / NB;
+    if (i >= nlist) return;
+    n = blist[i] * NB + n % NB;
+  }
+  if (n >= N) return;
+  double acc[5];
+  node_sum<FACES>(n, g, part, xin_ptr, spill, bnf_ptr, bnf_ent, fbuf, F, Ub0, fcode, fn, P2, acc);
   const double invcv = 1.0 / vol2[n];
   const size_t o = (size_t)n2o[n];
 #pragma unroll
@@ -876,6 +887,153 @@ __global__ void k_timestep(int N, int E, int F, Gas g, double cfl, const int2* _
   dt[i] = cfl * vol[i] / (-1.0 * idti);
 }
 
+// The same sums in the blocked organisation: every edge is evaluated once
+// (both endpoints' terms min(+-un - a, 0) S of the mean state) by the block
+// of its first endpoint, from staged node states; the two terms stay in
+// shared memory for the gather per node, the second endpoint's goes to
+// wspill for a block-crossing edge.  With un S = u.n and a S =
+// sqrt(gam p/rho n.n) an edge takes one reciprocal and one reciprocal square
+// root.  Bound by the 60 bytes per edge; the thread-per-node form
+// (k_timestep) evaluates each edge twice, three roots and a division each,
+// with its normals gathered one component at a time.
+constexpr int kWS = 6;  // doubles per staged state: 48 bytes, conflict-free 16-byte loads
+__global__ void __launch_bounds__(256) k_wave_blocked(int N, int E, int NB, Gas g, const ushort2* __restrict__ bl,
+                                                      const double* __restrict__ bn, const int* __restrict__ beptr,
+                                                      const int* __restrict__ hfptr, const int* __restrict__ hfpad,
+                                                      int maxHf, const double* __restrict__ P2,
+                                                      const int* __restrict__ lptr, const int* __restrict__ lidx,
+                                                      const int* __restrict__ xslot, double* __restrict__ wpart,
+                                                      double* __restrict__ wspill) {
+  extern __shared__ double sm[];
+  const int blk = blockIdx.x;
+  const int n0 = blk * NB, nn = min(NB, N - n0);
+  const int nh = hfptr[blk + 1] - hfptr[blk], ns = nn + nh;
+  const int e0 = beptr[blk], e1 = beptr[blk + 1];
+  double* Vn = sm;                                               // [ns][kWS]
+  double2* Ws = reinterpret_cast<double2*>(sm + kWS * (size_t)ns);  // [e1 - e0] (first, second)
+  const int* hf = hfpad + (size_t)blk * maxHf;
+  for (int k = threadIdx.x; k < 3 * ns; k += blockDim.x) {
+    const int q = k / 3, c = k - 3 * q;
+    const size_t j = (size_t)(q < nn ? n0 + q : hf[q - nn]);
+    cp_async16(Vn + kWS * q + 2 * c, P2 + 8 * j + 2 * c);
+  }
+  cp_async_wait_all();
+  __syncthreads();
+  for (int q = e0 + threadIdx.x; q < e1; q += blockDim.x) {
+    const ushort2 lq = bl[q];
+    const double nx = bn[q], ny = bn[(size_t)E + q], nz = bn[2 * (size_t)E + q];
+    const int xs = xslot[q];
+    const double2* a = reinterpret_cast<const double2*>(Vn + kWS * lq.x);
+    const double2* b = reinterpret_cast<const double2*>(Vn + kWS * lq.y);
+    const double2 a0 = a[0], a1 = a[1], a2 = a[2], b0 = b[0], b1 = b[1], b2 = b[2];
+    const double rho = 0.5 * (a0.x + b0.x), p = 0.5 * (a2.x + b2.x);
+    const double us = 0.5 * ((a0.y + b0.y) * nx + (a1.x + b1.x) * ny + (a1.y + b1.y) * nz);
+    const double s2 = nx * nx + ny * ny + nz * nz;
+    double2 w = make_double2(0.0, 0.0);
+    if (s2 > 0.0) {
+      const double x = g.gam * p * rcp_(rho) * s2, as = x * rsqrt_(x);
+      w = make_double2(fmin(us - as, 0.0), fmin(-us - as, 0.0));
+    }
+    Ws[q - e0] = w;
+    if (xs >= 0) wspill[xs] = w.y;
+  }
+  __syncthreads();
+  int L = 1;
+  while (2 * L * NB <= (int)blockDim.x) L *= 2;
+  const int t = threadIdx.x / L, r = threadIdx.x % L;
+  const bool act = t < nn && (int)threadIdx.x < L * NB;
+  double s = 0.0;
+  if (act)
+    for (int k = lptr[n0 + t] + r; k < lptr[n0 + t + 1]; k += L) {
+      const int e = lidx[k];
+      const double2 w = Ws[e & 0x7fffffff];
+      s += e < 0 ? w.y : w.x;
+    }
+  for (int o = 1; o < L; o <<= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  if (act && r == 0) wpart[n0 + t] = s;
+}
+
+// Node n's whole sum (block part, spilled terms, boundary faces with a third
+// of their area): the time step is cfl vol / (-sum).
+__device__ __forceinline__ double wave_sum(int n, const Gas& g, const double* __restrict__ wpart,
+                                           const int* __restrict__ xin_ptr, const double* __restrict__ wspill,
+                                           const int* __restrict__ bnf_ptr, const int* __restrict__ bnf_ent, int F,
+                                           const double* __restrict__ fn, const double* P2) {
+  double s = wpart[n];
+  for (int k = xin_ptr[n]; k < xin_ptr[n + 1]; ++k) s += wspill[k];
+  const int q0 = bnf_ptr[n], q1 = bnf_ptr[n + 1];
+  if (q0 < q1) {
+    const double* v = P2 + 8 * (size_t)n;
+    const double a = sqrt(g.gam * v[4] / v[0]);
+    for (int q = q0; q < q1; ++q) {
+      const int f = bnf_ent[q] / 3;
+      const double x = fn[f], y = fn[(size_t)F + f], z = fn[2 * (size_t)F + f];
+      const double S = sqrt(x * x + y * y + z * z), iS = 1.0 / S;
+      const double un = v[1] * (iS * x) + v[2] * (iS * y) + v[3] * (iS * z);
+      s += fmin(un - a, 0.0) * S / 3;
+    }
+  }
+  return s;
+}
+__global__ void k_wave_dt(int N, Gas g, double cfl, const int* __restrict__ n2o, const double* __restrict__ wpart,
+                          const int* __restrict__ xin_ptr, const double* __restrict__ wspill,
+                          const int* __restrict__ bnf_ptr, const int* __restrict__ bnf_ent, int F,
+                          const double* __restrict__ fn, const double* __restrict__ P2,
+                          const double* __restrict__ vol2, double* __restrict__ dt) {
+  const int n = blockIdx.x * blockDim.x + threadIdx.x;
+  if (n >= N) return;
+  dt[n2o[n]] = cfl * vol2[n] / (-1.0 * wave_sum(n, g, wpart, xin_ptr, wspill, bnf_ptr, bnf_ent, F, fn, P2));
+}
+
+// One stage of the explicit RK2 step fused with the node assembly of its
+// residual (k_fv_nodes_b) and the primitive conversion of the state the next
+// residual needs.  STAGE 1: the local time step from the wave sums, k1 = dt R
+// kept, P2 = prim(U - k1).  STAGE 2: U -= (k1 + k2)/2, P2 = prim(U).  The
+// same operations in the same order as the separate kernels, whose five
+// launches and passes over R, U0 and k2 it replaces (on a small mesh the
+// launches are the step: 21^3, first order, 100 us per step before and 61 us
+// with the wave sums, two edge sweeps and two of these).
+template <int STAGE, bool FACES>
+__global__ void __launch_bounds__(256) k_rk_nodes(int N, Gas g, double cfl, const int* __restrict__ n2o,
+                                                  const double* __restrict__ part, const int* __restrict__ xin_ptr,
+                                                  const double* __restrict__ spill, const double* __restrict__ wpart,
+                                                  const double* __restrict__ wspill, const int* __restrict__ bnf_ptr,
+                                                  const int* __restrict__ bnf_ent, const double* __restrict__ fbuf,
+                                                  int F, const double* __restrict__ Ub0,
+                                                  const int* __restrict__ fcode, const double* __restrict__ fn,
+                                                  const double* __restrict__ vol2, double* __restrict__ dt2,
+                                                  double* __restrict__ k1, double* __restrict__ U, double* P2) {
+  const int n = blockIdx.x * blockDim.x + threadIdx.x;
+  if (n >= N) return;
+  const double vol = vol2[n], invcv = 1.0 / vol;
+  double acc[5];
+  node_sum<FACES>(n, g, part, xin_ptr, spill, bnf_ptr, bnf_ent, fbuf, F, Ub0, fcode, fn, P2, acc);
+  double dt;
+  if (STAGE == 1) {
+    dt = cfl * vol / (-1.0 * wave_sum(n, g, wpart, xin_ptr, wspill, bnf_ptr, bnf_ent, F, fn, P2));
+    dt2[n] = dt;
+  } else {
+    dt = dt2[n];
+  }
+  double* u = U + 5 * (size_t)n2o[n];
+  double* kk = k1 + 5 * (size_t)n;
+  double un[5], v[5];
+#pragma unroll
+  for (int c = 0; c < 5; ++c) {
+    const double k = acc[c] * invcv * dt;
+    if (STAGE == 1) {
+      kk[c] = k;
+      un[c] = u[c] - k;
+    } else {
+      un[c] = u[c] - 1.0 / 2.0 * (kk[c] + k);
+      u[c] = un[c];
+    }
+  }
+  cons2prim(g, un, v);
+#pragma unroll
+  for (int c = 0; c < 5; ++c) P2[8 * (size_t)n + c] = v[c];
+}
+
 // RK2 stage helpers (ExplicitTsDesc.C:98-117): k = dt*R; U0 = U - k1;
 // U = U - 1/2 (k1 + k2).
 __global__ void k_rk_stage1(int N, const double* __restrict__ dt, const double* __restrict__ U,
@@ -1022,7 +1180,7 @@ static void launch_grad_pipe(aerof_gpu_ctx* c, const Gas& g, const double* dU, c
 static void launch_grad_staged(const DeviceMesh& m, const Gas& g, const double* dU, const int* tag, double* G2,
                                size_t smem, bool fused, cudaStream_t s) {
   const int L = kBlock / m.NB;
-  if (!fused) {
+  if (!fused && dU) {
     prim_to_P2(m, g, dU, s);
   }
   auto go = [&](auto kern) {
@@ -1042,15 +1200,16 @@ static void launch_grad_staged(const DeviceMesh& m, const Gas& g, const double* 
   }
 }
 
-// P2 = prim(U) in the blocked numbering and, unless the reconstruction is
-// constant, the gradients G2 (zero at tagged nodes when tag is given).
+// P2 = prim(U) in the blocked numbering (dU null: P2 is current) and, unless
+// the reconstruction is constant, the gradients G2 (zero at tagged nodes when
+// tag is given).
 void prim_grad_blocked_dev(aerof_gpu_ctx* c, const double* dU, const int* tag) {
   DeviceMesh& m = c->mesh;
   const Gas g = make_gas(c->cfg.gamma);
   cudaStream_t s = c->stream;
   c->s.G2.ensure(16 * (size_t)m.N);
   if (c->cfg.reconstruction == AEROF_REC_CONSTANT) {
-    prim_to_P2(m, g, dU, s);
+    if (dU) prim_to_P2(m, g, dU, s);
     return;
   }
   const size_t gsmem = ((size_t)8 * kPS * (m.NB + m.maxH) + (size_t)2 * m.maxL + 15) / 16 * 16;
@@ -1062,9 +1221,9 @@ void prim_grad_blocked_dev(aerof_gpu_ctx* c, const double* dU, const int* tag) {
   if (grad_piped(m)) {
     launch_grad_pipe(c, g, dU, tag, c->s.G2.p, s);
   } else if (staged) {
-    launch_grad_staged(m, g, dU, tag, c->s.G2.p, gsmem, gk == 1, s);
+    launch_grad_staged(m, g, dU, tag, c->s.G2.p, gsmem, gk == 1 && dU, s);
   } else {
-    prim_to_P2(m, g, dU, s);
+    if (dU) prim_to_P2(m, g, dU, s);
     k_grad<<<grid_for(4 * (size_t)m.N, kBlock), kBlock, 0, s>>>(m.N, m.P2.p, m.W2.p, m.nb2_ptr.p, m.nb2_node.p, tag,
                                                                 c->s.G2.p);
     AEROF_LAUNCH_CHECK();
@@ -1085,6 +1244,34 @@ void grad_records_blocked_dev(aerof_gpu_ctx* c, const double* P2src, double* G2d
                                                                 G2dst);
     AEROF_LAUNCH_CHECK();
   }
+}
+
+// Edge fluxes of the blocked organisation from P2 and G2 into part and
+// spill; counter: where unphysical states are counted.
+static void fv_blocked_dev(aerof_gpu_ctx* c, int failsafe, int* counter) {
+  DeviceMesh& m = c->mesh;
+  const size_t smem = fv_blocked_smem(m);
+  // register budget from the CTAs per SM that shared memory allows
+  // (228 KB per SM, 1 KB reserved per CTA)
+  const int by_smem = (int)std::min<size_t>(4, (228 * 1024) / (smem + 1024));
+  // 256 threads with the register budget of the CTAs that fit (384
+  // threads at two CTAs per SM measured slower)
+  // tuning knob AEROF_FV_THREADS = 512: two CTAs of 512 threads per SM at
+  // 64 registers (more warps, some spilling) when shared memory allows two
+  static const int fv_env = [] {
+    const char* e = std::getenv("AEROF_FV_THREADS");
+    return e ? std::atoi(e) : 256;
+  }();
+  const bool wide = fv_env == 512 && by_smem >= 2;
+  const int fv_threads = wide ? 512 : 256;
+  auto fvk = wide ? k_fv_blocked<512, 2>
+                  : by_smem >= 4 ? k_fv_blocked<256, 4> : by_smem == 3 ? k_fv_blocked<256, 3> : k_fv_blocked<256, 2>;
+  AEROF_CUDA(cudaFuncSetAttribute(fvk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  fvk<<<m.nblk, fv_threads, smem, c->stream>>>(m.N, m.E, m.NB, make_gas(c->cfg.gamma), c->cfg.reconstruction,
+                                               c->cfg.beta, failsafe, m.bl.p, m.bnorm.p, m.beptr.p, m.hfptr.p,
+                                               m.hfpad.p, m.maxHf, m.P2.p, c->s.G2.p, m.lptr.p, m.lidx.p, m.xslot.p,
+                                               c->s.part.p, c->s.spill.p, c->s.tag.p, counter, nullptr);
+  AEROF_LAUNCH_CHECK();
 }
 
 // BLOCKED organisation of residual_dev (see k_fv_blocked).
@@ -1111,36 +1298,13 @@ static int residual_blocked_dev(aerof_gpu_ctx* c, const double* dU, double* dR, 
     c->s.tag.ensure(m.N);
     c->s.tag.zero(s);
   }
-  const size_t smem = fv_blocked_smem(m);
-  // register budget from the CTAs per SM that shared memory allows
-  // (228 KB per SM, 1 KB reserved per CTA)
-  const int by_smem = (int)std::min<size_t>(4, (228 * 1024) / (smem + 1024));
-  // 256 threads with the register budget of the CTAs that fit (384
-  // threads at two CTAs per SM measured slower)
-  // tuning knob AEROF_FV_THREADS = 512: two CTAs of 512 threads per SM at
-  // 64 registers (more warps, some spilling) when shared memory allows two
-  static const int fv_env = [] {
-    const char* e = std::getenv("AEROF_FV_THREADS");
-    return e ? std::atoi(e) : 256;
-  }();
-  const bool wide = fv_env == 512 && by_smem >= 2;
-  const int fv_threads = wide ? 512 : 256;
-  auto fvk = wide ? k_fv_blocked<512, 2>
-                  : by_smem >= 4 ? k_fv_blocked<256, 4> : by_smem == 3 ? k_fv_blocked<256, 3> : k_fv_blocked<256, 2>;
-  AEROF_CUDA(cudaFuncSetAttribute(fvk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   {
     TimerScope t(c, AEROF_T_NODAL_GRAD);
     prim_grad_blocked_dev(c, dU, nullptr);
   }
-  auto fv = [&](int fs, int* counter) {
-    fvk<<<m.nblk, fv_threads, smem, s>>>(m.N, m.E, m.NB, g, rec, c->cfg.beta, fs, m.bl.p, m.bnorm.p, m.beptr.p,
-                                         m.hfptr.p, m.hfpad.p, m.maxHf, m.P2.p, c->s.G2.p, m.lptr.p, m.lidx.p,
-                                         m.xslot.p, c->s.part.p, c->s.spill.p, c->s.tag.p, counter, nullptr);
-    AEROF_LAUNCH_CHECK();
-  };
   {
     TimerScope t(c, AEROF_T_FV_EDGES);
-    fv(c->cfg.failsafe, ecnt);
+    fv_blocked_dev(c, c->cfg.failsafe, ecnt);
   }
   // only the failsafe needs the count before the assembly (it re-runs the
   // edges); otherwise the whole residual is queued and waited for once, its
@@ -1159,7 +1323,7 @@ static int residual_blocked_dev(aerof_gpu_ctx* c, const double* dU, double* dR, 
     TimerScope t(c, AEROF_T_FV_TERM);
     prim_grad_blocked_dev(c, dU, c->s.tag.p);
     c->s.p2g2_valid = false;
-    fv(0, cnt + 1);
+    fv_blocked_dev(c, 0, cnt + 1);
   }
   {
     TimerScope t(c, AEROF_T_FV_TERM);
@@ -1603,14 +1767,97 @@ static bool residual_host_pipelined(aerof_gpu_ctx* c, const double* U, double* R
   return true;
 }
 
+static size_t wave_smem(const DeviceMesh& m) {
+  return sizeof(double) * ((size_t)kWS * (m.NB + m.maxHf) + (size_t)2 * m.maxE);
+}
+// wave-speed sums of the states in P2 into wpart / wspill
+static void wave_blocked_dev(aerof_gpu_ctx* c) {
+  DeviceMesh& m = c->mesh;
+  c->s.wpart.ensure(m.N);
+  c->s.wspill.ensure(std::max(m.nX, 1));
+  const size_t smem = wave_smem(m);
+  AEROF_CUDA(cudaFuncSetAttribute(k_wave_blocked, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  k_wave_blocked<<<m.nblk, 256, smem, c->stream>>>(m.N, m.E, m.NB, make_gas(c->cfg.gamma), m.bl.p, m.bnorm.p,
+                                                   m.beptr.p, m.hfptr.p, m.hfpad.p, m.maxHf, m.P2.p, m.lptr.p,
+                                                   m.lidx.p, m.xslot.p, c->s.wpart.p, c->s.wspill.p);
+  AEROF_LAUNCH_CHECK();
+}
+
 void timestep_dev(aerof_gpu_ctx* c, const double* dU, double cfl, double* ddt) {
   DeviceMesh& m = c->mesh;
+  const Gas g = make_gas(c->cfg.gamma);
   TimerScope t(c, AEROF_T_TIME_STEP);
+  if (c->cfg.residual_kernel == AEROF_KERNEL_BLOCKED && wave_smem(m) <= 200 * 1024) {
+    c->s.p2g2_valid = false;
+    prim_to_P2(m, g, dU, c->stream);
+    wave_blocked_dev(c);
+    k_wave_dt<<<grid_for(m.N, kBlock), kBlock, 0, c->stream>>>(m.N, g, cfl, m.n2o.p, c->s.wpart.p, m.xin_ptr.p,
+                                                                c->s.wspill.p, m.bnf_ptr.p, m.bnf_ent.p, m.F,
+                                                                m.fnrm.p, m.P2.p, m.vol2.p, ddt);
+    AEROF_LAUNCH_CHECK();
+    return;
+  }
   prim_dev(c, dU);
   k_timestep<<<grid_for(m.N, kBlock), kBlock, 0, c->stream>>>(
-      m.N, m.E, m.F, make_gas(c->cfg.gamma), cfl, m.edges.p, m.en.p, m.nbr_ptr.p, m.nbr_edge.p, m.nf_ptr.p,
+      m.N, m.E, m.F, g, cfl, m.edges.p, m.en.p, m.nbr_ptr.p, m.nbr_edge.p, m.nf_ptr.p,
       m.nf_face.p, m.fnrm.p, m.P.p, m.vol.p, ddt);
   AEROF_LAUNCH_CHECK();
+}
+
+// Up to this many nodes the boundary fluxes are formed inside the node
+// assembly of an RK2 stage: one launch less, where a launch costs more than
+// the few serial faces per boundary node (large meshes: a thread per face is
+// 26 us faster at 101^3).
+constexpr int kFacesInNodes = 1 << 16;
+
+// nsteps of RK2 on dU in the blocked organisation: per step the wave sums,
+// two edge sweeps (with gradients unless first order) and two fused stages.
+// Unphysical states are counted into counter.
+static void rk2_blocked_dev(aerof_gpu_ctx* c, double* dU, double cfl, int nsteps, int* counter) {
+  DeviceMesh& m = c->mesh;
+  const Gas g = make_gas(c->cfg.gamma);
+  cudaStream_t s = c->stream;
+  const size_t n5 = 5 * (size_t)m.N;
+  c->s.G2.ensure(16 * (size_t)m.N);
+  c->s.part.ensure(n5);
+  c->s.spill.ensure(5 * (size_t)std::max(m.nX, 1));
+  c->s.fbuf.ensure(15 * (size_t)std::max(m.F, 1));
+  c->s.dt.ensure(m.N);
+  c->s.k1.ensure(n5);
+  c->s.p2g2_valid = false;
+  const bool faces = m.N <= kFacesInNodes || !m.F;
+  const int gn = grid_for(m.N, kBlock);
+  prim_to_P2(m, g, dU, s);
+  auto stage = [&](auto kern) {
+    if (!faces) {
+      k_face_flux<<<grid_for(m.F, kBlock), kBlock, 0, s>>>(m.F, g, m.Ubd.p, m.faces.p, m.fcode.p, m.fnrm.p, m.P2.p,
+                                                           m.o2n.p, c->s.fbuf.p);
+      AEROF_LAUNCH_CHECK();
+    }
+    kern<<<gn, kBlock, 0, s>>>(m.N, g, cfl, m.n2o.p, c->s.part.p, m.xin_ptr.p, c->s.spill.p, c->s.wpart.p,
+                               c->s.wspill.p, m.bnf_ptr.p, m.bnf_ent.p, c->s.fbuf.p, m.F, m.Ubd.p, m.fcode.p,
+                               m.fnrm.p, m.vol2.p, c->s.dt.p, c->s.k1.p, dU, m.P2.p);
+    AEROF_LAUNCH_CHECK();
+  };
+  for (int k = 0; k < nsteps; ++k) {
+    {
+      TimerScope t(c, AEROF_T_TIME_STEP);
+      wave_blocked_dev(c);
+    }
+    for (int st = 1; st <= 2; ++st) {
+      {
+        TimerScope t(c, AEROF_T_NODAL_GRAD);
+        prim_grad_blocked_dev(c, nullptr, nullptr);
+      }
+      {
+        TimerScope t(c, AEROF_T_FV_EDGES);
+        fv_blocked_dev(c, 0, counter);
+      }
+      TimerScope t(c, AEROF_T_FV_TERM);
+      if (st == 1) stage(faces ? k_rk_nodes<1, true> : k_rk_nodes<1, false>);
+      else stage(faces ? k_rk_nodes<2, true> : k_rk_nodes<2, false>);
+    }
+  }
 }
 
 double dot_dev(aerof_gpu_ctx* c, const double* x, const double* y, size_t n) {
@@ -1754,12 +2001,19 @@ extern "C" int aerof_gpu_rk2(aerof_gpu_ctx* c, double* U, double cfl, int nsteps
       AEROF_CUDA(cudaMemcpyAsync(c->s.Ustage.p, U, n5 * sizeof(double), cudaMemcpyHostToDevice, c->stream));
       dU = c->s.Ustage.p;
     }
-    c->s.dt.ensure(m.N); c->s.k1.ensure(n5); c->s.k2.ensure(n5); c->s.U0.ensure(n5);
     // the unphysical counts of all steps add up on the device (the failsafe
     // counts on the host, per call): one wait at the end
     int bad = 0;
     int* nbad = counters(c) + kCountSum;
     AEROF_CUDA(cudaMemsetAsync(nbad, 0, sizeof(int), c->stream));
+    const bool blocked = c->cfg.residual_kernel == AEROF_KERNEL_BLOCKED && fv_blocked_smem(m) <= 200 * 1024 &&
+                         wave_smem(m) <= 200 * 1024;
+    if (blocked && !c->cfg.failsafe && c->visc.model == 0) {
+      rk2_blocked_dev(c, dU, cfl, nsteps, nbad);
+      nsteps = 0;
+    } else {
+      c->s.dt.ensure(m.N); c->s.k1.ensure(n5); c->s.k2.ensure(n5); c->s.U0.ensure(n5);
+    }
     const int gb = grid_for(n5, kBlock);
     for (int s = 0; s < nsteps; ++s) {
       timestep_dev(c, dU, cfl, c->s.dt.p);
