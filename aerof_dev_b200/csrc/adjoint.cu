@@ -11,6 +11,7 @@
 // Reverse mode (aerof_gpu_vjp, aerof_gpu_dRdX_T): hand-written adjoints of
 // the same kernels, recomputing the primal state per edge instead of
 // storing it, accumulated per node by gathers in a fixed order.
+#include <type_traits>
 #include <vector>
 
 #include "common.cuh"
@@ -163,6 +164,487 @@ __global__ void k_d_node_residual(int N, int E, int F, Gas g, const double* __re
   }
 }
 
+// ---------------------------------------------------------------------
+// Forward mode in the blocked organisation: the primal records and
+// gradients (P2, G2) are the residual's, beside them tangent records D2
+// (dV, dX) and tangent gradients dG2; the edge sweep differentiates the flux
+// of k_fv_blocked in dual arithmetic from staged records.  The gathered form
+// above (dual numbers interleaved in the caller's numbering, geometry
+// recomputed per node and edge) remains for meshes whose blocks do not fit
+// in shared memory: J v and (dR/dX) Xdot at 61^3 2.67 ms there, 1.13 ms here.
+
+// D2[n] = (dV, dX): dV = (dV/dU) v (VarFcnSGEuler.h:307-327; v null: 0), dX =
+// Xdot, or the coordinates when Xdot is null (the records whose gradients
+// are linear in dV).
+__global__ void k_f_seed(int N, Gas g, const int* __restrict__ n2o, const double* __restrict__ P2,
+                         const double* __restrict__ v, const double* __restrict__ Xdot, double* __restrict__ D2) {
+  const int n = blockIdx.x * blockDim.x + threadIdx.x;
+  if (n >= N) return;
+  const size_t o = (size_t)n2o[n];
+  const double* p = P2 + 8 * (size_t)n;
+  double* d = D2 + 8 * (size_t)n;
+  double du[5] = {0, 0, 0, 0, 0};
+  if (v) {
+#pragma unroll
+    for (int k = 0; k < 5; ++k) du[k] = v[5 * o + k];
+  }
+  const double ir = rcp_(p[0]), a = p[1], b = p[2], c = p[3];
+  d[0] = du[0];
+  d[1] = (du[1] - a * du[0]) * ir;
+  d[2] = (du[2] - b * du[0]) * ir;
+  d[3] = (du[3] - c * du[0]) * ir;
+  d[4] = g.gam1 * (0.5 * (a * a + b * b + c * c) * du[0] - a * du[1] - b * du[2] - c * du[3] + du[4]);
+#pragma unroll
+  for (int k = 0; k < 3; ++k) d[5 + k] = Xdot ? Xdot[3 * o + k] : p[5 + k];
+}
+
+// Tangents of a tet's six edge normals (oriented from the lower to the
+// higher node, as tet_edge_normal) and of its volume in the direction Xdot:
+// tn[t][3 l + c], tv[t].  Thread per tet, so that every tet is evaluated
+// once instead of once per edge; rows staged in shared memory (stride 19:
+// conflict-free) and stored contiguously.  Bound: HBM (152 bytes per tet
+// written here and read once by the gathers).
+template <int TB>
+__global__ void __launch_bounds__(TB) k_f_tets(int T, const double* __restrict__ X, const double* __restrict__ Xdot,
+                                               const int* __restrict__ tets, double* __restrict__ tn,
+                                               double* __restrict__ tv) {
+  __shared__ double st[TB * 19];
+  const int t0 = blockIdx.x * TB, t = t0 + threadIdx.x;
+  if (t < T) {
+    const int4 q4 = *reinterpret_cast<const int4*>(tets + 4 * (size_t)t);
+    const int nd[4] = {q4.x, q4.y, q4.z, q4.w};
+    Vec3<double> x[4], d[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      x[k] = node_x(X, nd[k]);
+      d[k] = node_x(Xdot, nd[k]);
+    }
+    const Vec3<double> e1 = x[1] - x[0], e2 = x[2] - x[0], e3 = x[3] - x[0];
+    const Vec3<double> d1 = d[1] - d[0], d2 = d[2] - d[0], d3 = d[3] - d[0];
+    const Vec3<double> c = cross(e1, e2), dc = cross(d1, e2) + cross(e1, d2);
+    tv[t] = (1.0 / 6.0) * (d3.x * c.x + d3.y * c.y + d3.z * c.z + e3.x * dc.x + e3.y * dc.y + e3.z * dc.z);
+    const double third = 1.0 / 3.0;
+    const Vec3<double> xg = scale(0.25, x[0] + x[1] + x[2] + x[3]), dg = scale(0.25, d[0] + d[1] + d[2] + d[3]);
+    Vec3<double> f[4], df[4];
+    f[0] = scale(third, x[0] + x[1] + x[2]) - xg;
+    f[1] = scale(third, x[0] + x[1] + x[3]) - xg;
+    f[2] = scale(third, x[0] + x[2] + x[3]) - xg;
+    f[3] = scale(third, x[1] + x[2] + x[3]) - xg;
+    df[0] = scale(third, d[0] + d[1] + d[2]) - dg;
+    df[1] = scale(third, d[0] + d[1] + d[3]) - dg;
+    df[2] = scale(third, d[0] + d[2] + d[3]) - dg;
+    df[3] = scale(third, d[1] + d[2] + d[3]) - dg;
+#pragma unroll
+    for (int l = 0; l < 6; ++l) {
+      const int F0 = tet_edge_face(l, 0), F1 = tet_edge_face(l, 1);
+      const double sl = nd[tet_edge_end(l, 0)] < nd[tet_edge_end(l, 1)] ? 1.5 : -1.5;
+      const Vec3<double> n = scale(sl, cross(df[F1], f[F0]) + cross(f[F1], df[F0]));
+      st[19 * threadIdx.x + 3 * l] = n.x;
+      st[19 * threadIdx.x + 3 * l + 1] = n.y;
+      st[19 * threadIdx.x + 3 * l + 2] = n.z;
+    }
+  }
+  __syncthreads();
+  const int cnt = 18 * min(TB, T - t0);
+  double* out = tn + 18 * (size_t)t0;
+  for (int k = threadIdx.x; k < cnt; k += TB) __stcs(out + k, st[19 * (k / 18) + k % 18]);
+}
+// tangents of the blocked edges' oriented normals: three lanes per edge
+__global__ void k_f_edge_normals(int E, const int* __restrict__ bsrc, const int* __restrict__ et_ptr,
+                                 const int* __restrict__ et_tet, const double* __restrict__ tn,
+                                 double* __restrict__ dbn) {
+  const long long j = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (j >= 3 * (long long)E) return;
+  const int q = (int)(j / 3), c = (int)(j - 3 * (long long)q);
+  const int src = bsrc[q];
+  const int l = src & 0x7fffffff;
+  double s = 0.0;
+  for (int p = et_ptr[l]; p < et_ptr[l + 1]; ++p) {
+    const int e = et_tet[p];
+    s += tn[18 * (size_t)(e >> 3) + 3 * (e & 7) + c];
+  }
+  dbn[(size_t)c * E + q] = src < 0 ? -s : s;
+}
+// tangents of the control volumes (blocked numbering) and face normals
+__global__ void k_f_volumes(int N, const int* __restrict__ n2o, const int* __restrict__ nt_ptr,
+                            const int* __restrict__ nt_tet, const double* __restrict__ tv, double* __restrict__ dvol) {
+  const int n = blockIdx.x * blockDim.x + threadIdx.x;
+  if (n >= N) return;
+  const int o = n2o[n];
+  double s = 0.0;
+  for (int p = nt_ptr[o]; p < nt_ptr[o + 1]; ++p) s += 0.25 * tv[nt_tet[p] >> 2];
+  dvol[n] = s;
+}
+__global__ void k_f_face_normals(int F, const double* __restrict__ X, const double* __restrict__ Xdot,
+                                 const int* __restrict__ faces, double* __restrict__ dfn) {
+  const int f = blockIdx.x * blockDim.x + threadIdx.x;
+  if (f >= F) return;
+  const int* nd = faces + 3 * (size_t)f;
+  const Vec3<double> x0 = node_x(X, nd[0]), d0 = node_x(Xdot, nd[0]);
+  const Vec3<double> x1 = node_x(X, nd[1]) - x0, x2 = node_x(X, nd[2]) - x0;
+  const Vec3<double> d1 = node_x(Xdot, nd[1]) - d0, d2 = node_x(Xdot, nd[2]) - d0;
+  const Vec3<double> n = scale(0.5, cross(d2, x1) + cross(x2, d1));
+  dfn[f] = n.x; dfn[(size_t)F + f] = n.y; dfn[2 * (size_t)F + f] = n.z;
+}
+
+// Tangent of the least-squares gradients in (dV, dX): CTA per Morton block,
+// the records P2 and D2 of the block's nodes and halo staged; L lanes per
+// node first sum the tangent of the normal equations, from which the
+// tangents of the Cholesky factor and of the node's constants follow, then
+// the gradient's (fixed xor trees).  Latency of the shared-memory gathers.
+constexpr int kFGradThreads = 512;
+template <int L>
+__global__ void __launch_bounds__(kFGradThreads, 1) k_f_grad(int N, int NB, const double* __restrict__ P2,
+                                                             const double* __restrict__ D2,
+                                                             const double* __restrict__ W2, const int* __restrict__ n2o,
+                                                             const double* __restrict__ lsqR,
+                                                             const int* __restrict__ nb2_ptr,
+                                                             const unsigned short* __restrict__ lnb,
+                                                             const int* __restrict__ hptr,
+                                                             const int* __restrict__ hnode, double* __restrict__ dG2) {
+  extern __shared__ double sm[];
+  const int blk = blockIdx.x;
+  const int n0 = blk * NB, nn = min(NB, N - n0);
+  const int h0 = hptr[blk], ns = nn + hptr[blk + 1] - h0;
+  double* Ps = sm;                            // [ns][kPS]
+  double* Ds = sm + kPS * (size_t)ns;         // [ns][kPS]
+  for (int k = threadIdx.x; k < 4 * ns; k += blockDim.x) {
+    const int q = k >> 2, c = k & 3;
+    const size_t j = (size_t)(q < nn ? n0 + q : hnode[h0 + q - nn]);
+    cp_async16(Ps + kPS * q + 2 * c, P2 + 8 * j + 2 * c);
+    cp_async16(Ds + kPS * q + 2 * c, D2 + 8 * j + 2 * c);
+  }
+  const int t = threadIdx.x / L, r = threadIdx.x % L;
+  const bool act = t < nn;
+  double w[6], R[6];
+  int pb = 0, pe = 0;
+  if (act) {
+    const int n = n0 + t, o = n2o[n];
+#pragma unroll
+    for (int k = 0; k < 6; ++k) { w[k] = W2[(size_t)k * N + n]; R[k] = lsqR[(size_t)k * N + o]; }
+    pb = nb2_ptr[n];
+    pe = nb2_ptr[n + 1];
+  }
+  cp_async_wait_all();
+  __syncthreads();
+  const double* pi = Ps + kPS * (act ? t : 0);
+  const double* di = Ds + kPS * (act ? t : 0);
+  double s[6] = {0, 0, 0, 0, 0, 0};
+#pragma unroll 1
+  for (int p = pb + r; p < pe; p += L) {
+    const int q = lnb[p];
+    const double* pj = Ps + kPS * q;
+    const double* dj = Ds + kPS * q;
+    const double x = pj[5] - pi[5], y = pj[6] - pi[6], z = pj[7] - pi[7];
+    const double dx = dj[5] - di[5], dy = dj[6] - di[6], dz = dj[7] - di[7];
+    s[0] += 2.0 * x * dx;
+    s[1] += x * dy + dx * y;
+    s[2] += x * dz + dx * z;
+    s[3] += 2.0 * y * dy;
+    s[4] += y * dz + dy * z;
+    s[5] += 2.0 * z * dz;
+  }
+#pragma unroll
+  for (int o = 1; o < L; o <<= 1)
+#pragma unroll
+    for (int k = 0; k < 6; ++k) s[k] += __shfl_xor_sync(0xffffffffu, s[k], o);
+  double g[15];
+#pragma unroll
+  for (int k = 0; k < 15; ++k) g[k] = 0.0;
+  if (act) {
+    // R = (r11 r12 r13 r22 r23 r33): w0 = 1/r11, w1 = 1/r22, w2 = 1/r33
+    const double r11 = 0.5 * s[0] * w[0];
+    const double r12 = (s[1] - R[1] * r11) * w[0], r13 = (s[2] - R[2] * r11) * w[0];
+    const double r22 = (0.5 * s[3] - R[1] * r12) * w[1];
+    const double r23 = (s[4] - r12 * R[2] - R[1] * r13 - R[4] * r22) * w[1];
+    const double r33 = (0.5 * s[5] - R[2] * r13 - R[4] * r23) * w[2];
+    double dw[6];
+    dw[0] = -w[0] * w[0] * r11;
+    dw[1] = -w[1] * w[1] * r22;
+    dw[2] = -w[2] * w[2] * r33;
+    dw[3] = r12 * w[0] + R[1] * dw[0];
+    dw[4] = r23 * w[1] + R[4] * dw[1];
+    const double psi = R[1] * R[4] - R[2] * R[3];
+    dw[5] = (r12 * R[4] + R[1] * r23 - r13 * R[3] - R[2] * r22) * (w[0] * w[1]) +
+            psi * (dw[0] * w[1] + w[0] * dw[1]);
+    Dual wd[6];
+#pragma unroll
+    for (int k = 0; k < 6; ++k) wd[k] = Dual(w[k], dw[k]);
+#pragma unroll 1
+    for (int p = pb + r; p < pe; p += L) {
+      const int q = lnb[p];
+      const double* pj = Ps + kPS * q;
+      const double* dj = Ds + kPS * q;
+      Dual W0, W1, W2d;
+      lsq_weights(wd, Dual(pj[5] - pi[5], dj[5] - di[5]), Dual(pj[6] - pi[6], dj[6] - di[6]),
+                  Dual(pj[7] - pi[7], dj[7] - di[7]), W0, W1, W2d);
+#pragma unroll
+      for (int k = 0; k < 5; ++k) {
+        const double v = pj[k] - pi[k], dv = dj[k] - di[k];
+        g[k] += W0.v * dv + W0.d * v;
+        g[5 + k] += W1.v * dv + W1.d * v;
+        g[10 + k] += W2d.v * dv + W2d.d * v;
+      }
+    }
+  }
+#pragma unroll
+  for (int o = 1; o < L; o <<= 1)
+#pragma unroll
+    for (int k = 0; k < 15; ++k) g[k] += __shfl_xor_sync(0xffffffffu, g[k], o);
+  if (!act || r != 0) return;
+  double2* out = reinterpret_cast<double2*>(dG2 + 16 * (size_t)(n0 + t));
+#pragma unroll
+  for (int k = 0; k < 7; ++k) out[k] = make_double2(g[2 * k], g[2 * k + 1]);
+  out[7] = make_double2(g[14], 0.0);
+}
+
+// Tangent edge sweep, organised as k_fv_blocked: records, tangents,
+// gradients and tangent gradients of the block's nodes and forward halo
+// staged; thread per edge in dual arithmetic (GEO: the normal and the offset
+// carry tangents too), the tangent flux to shared memory (and spill for a
+// block-crossing edge), then the gather per node.  One CTA of 512 threads
+// per SM (the staging takes ~180 KB); bound by FP64 issue, about 2.5 primal
+// evaluations per edge.
+constexpr int kFwdThreads = 512;
+template <bool GEO>
+__global__ void __launch_bounds__(kFwdThreads, 1)
+    k_f_fv_blocked(int N, int E, int NB, Gas g, int rec, double beta, const ushort2* __restrict__ bl,
+                   const double* __restrict__ bn, const double* __restrict__ dbn, const int* __restrict__ beptr,
+                   const int* __restrict__ hfptr, const int* __restrict__ hfpad, int maxHf,
+                   const double* __restrict__ P2, const double* __restrict__ D2, const double* __restrict__ G2,
+                   const double* __restrict__ dG2, const int* __restrict__ lptr, const int* __restrict__ lidx,
+                   const int* __restrict__ xslot, double* __restrict__ part, double* __restrict__ spill,
+                   int* __restrict__ counter) {
+  extern __shared__ double sm[];
+  const int blk = blockIdx.x;
+  const int n0 = blk * NB, nn = min(NB, N - n0);
+  const int nh = hfptr[blk + 1] - hfptr[blk], ns = nn + nh;
+  const int e0 = beptr[blk], e1 = beptr[blk + 1];
+  const bool grad = rec != AEROF_REC_CONSTANT;
+  double* Ps = sm;                                    // [ns][kPS]
+  double* Ds = Ps + kPS * (size_t)ns;                 // [ns][kPS]
+  double* Gs = Ds + kPS * (size_t)ns;                 // [ns][kGS]
+  double* Ts = Gs + kGS * (size_t)ns;                 // [ns][kGS]
+  double* Fs = Ts + kGS * (size_t)ns;                 // [e1 - e0][5]
+  const int* hf = hfpad + (size_t)blk * maxHf;
+  for (int k = threadIdx.x; k < 4 * ns; k += blockDim.x) {
+    const int q = k >> 2, c = k & 3;
+    const size_t j = (size_t)(q < nn ? n0 + q : hf[q - nn]);
+    cp_async16(Ps + kPS * q + 2 * c, P2 + 8 * j + 2 * c);
+    cp_async16(Ds + kPS * q + 2 * c, D2 + 8 * j + 2 * c);
+  }
+  if (grad)
+    for (int k = threadIdx.x; k < 8 * ns; k += blockDim.x) {
+      const int q = k >> 3, c = k & 7;
+      const size_t j = (size_t)(q < nn ? n0 + q : hf[q - nn]);
+      cp_async16(Gs + kGS * q + 2 * c, G2 + 16 * j + 2 * c);
+      cp_async16(Ts + kGS * q + 2 * c, dG2 + 16 * j + 2 * c);
+    }
+  cp_async_wait_all();
+  __syncthreads();
+  using TN = typename std::conditional<GEO, Dual, double>::type;
+  for (int q = e0 + threadIdx.x; q < e1; q += blockDim.x) {
+    const ushort2 lq = bl[q];
+    TN n[3], dx[3];
+    const double *pi = Ps + kPS * lq.x, *pj = Ps + kPS * lq.y, *di = Ds + kPS * lq.x, *dj = Ds + kPS * lq.y;
+    const double *gi = Gs + kGS * lq.x, *gj = Gs + kGS * lq.y, *ti = Ts + kGS * lq.x, *tj = Ts + kGS * lq.y;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      if constexpr (GEO) {
+        n[a] = Dual(bn[(size_t)a * E + q], dbn[(size_t)a * E + q]);
+        dx[a] = Dual(pj[5 + a] - pi[5 + a], dj[5 + a] - di[5 + a]);
+      } else {
+        n[a] = bn[(size_t)a * E + q];
+        dx[a] = pj[5 + a] - pi[5 + a];
+      }
+    }
+    Dual Vi[5], Vj[5], f[5];
+#pragma unroll
+    for (int k = 0; k < 5; ++k) {
+      const Dual a(pi[k], di[k]), b(pj[k], dj[k]);
+      if (!grad) {
+        Vi[k] = a;
+        Vj[k] = b;
+        continue;
+      }
+      const Dual ij = dx[0] * Dual(gi[k], ti[k]) + dx[1] * Dual(gi[5 + k], ti[5 + k]) + dx[2] * Dual(gi[10 + k], ti[10 + k]);
+      const Dual ji = dx[0] * Dual(gj[k], tj[k]) + dx[1] * Dual(gj[5 + k], tj[5 + k]) + dx[2] * Dual(gj[10 + k], tj[10 + k]);
+      if (rec == AEROF_REC_VANALBADA) vanalbada(beta, a, ij, b, ji, Vi[k], Vj[k]);
+      else linear_rec(beta, a, ij, b, ji, Vi[k], Vj[k]);
+    }
+    const bool bad = Vi[0].v <= 0.0 || Vi[4].v <= 0.0 || Vj[0].v <= 0.0 || Vj[4].v <= 0.0;
+    if (bad) atomicAdd(counter, 1);
+    else if (vof(n[0]) * vof(n[0]) + vof(n[1]) * vof(n[1]) + vof(n[2]) * vof(n[2]) >= 1e-36)
+      roe_flux(g, n[0], n[1], n[2], Vi, Vj, f);
+    double* fs = Fs + 5 * (q - e0);
+    const int xs = xslot[q];
+#pragma unroll
+    for (int k = 0; k < 5; ++k) {
+      fs[k] = f[k].d;
+      if (xs >= 0) spill[5 * (size_t)xs + k] = f[k].d;
+    }
+  }
+  __syncthreads();
+  int L = 1;
+  while (2 * L * NB <= (int)blockDim.x) L *= 2;
+  const int t = threadIdx.x / L, r = threadIdx.x % L;
+  const bool act = t < nn && (int)threadIdx.x < L * NB;
+  double acc[5] = {0, 0, 0, 0, 0};
+  if (act)
+    for (int k = lptr[n0 + t] + r; k < lptr[n0 + t + 1]; k += L) {
+      const int e = lidx[k];
+      const double* fs = Fs + 5 * (e & 0x7fffffff);
+#pragma unroll
+      for (int c = 0; c < 5; ++c) acc[c] += e < 0 ? -fs[c] : fs[c];
+    }
+  for (int o = 1; o < L; o <<= 1)
+#pragma unroll
+    for (int c = 0; c < 5; ++c) acc[c] += __shfl_xor_sync(0xffffffffu, acc[c], o);
+  if (act && r == 0) {
+#pragma unroll
+    for (int c = 0; c < 5; ++c) part[5 * (size_t)(n0 + t) + c] = acc[c];
+  }
+}
+
+// dR of every node: (tangent flux sum + boundary faces in dual arithmetic) /
+// vol, and with GEO - R dvol / vol (R = S / vol), written to the caller's row
+template <bool GEO>
+__global__ void __launch_bounds__(256) k_f_nodes(int N, int F, Gas g, const double* __restrict__ Ub0,
+                                                 const int* __restrict__ n2o, const double* __restrict__ part,
+                                                 const int* __restrict__ xin_ptr, const double* __restrict__ spill,
+                                                 const int* __restrict__ bnf_ptr, const int* __restrict__ bnf_ent,
+                                                 const int* __restrict__ fcode, const double* __restrict__ fn,
+                                                 const double* __restrict__ dfn, const double* __restrict__ P2,
+                                                 const double* __restrict__ D2, const double* __restrict__ vol2,
+                                                 const double* __restrict__ dvol, const double* __restrict__ R,
+                                                 double* __restrict__ dR) {
+  const int n = blockIdx.x * blockDim.x + threadIdx.x;
+  if (n >= N) return;
+  double acc[5];
+#pragma unroll
+  for (int c = 0; c < 5; ++c) acc[c] = part[5 * (size_t)n + c];
+  for (int k = xin_ptr[n]; k < xin_ptr[n + 1]; ++k) {
+#pragma unroll
+    for (int c = 0; c < 5; ++c) acc[c] -= spill[5 * (size_t)k + c];
+  }
+  const int q0 = bnf_ptr[n], q1 = bnf_ptr[n + 1];
+  if (q0 < q1) {
+    const double third = 1.0 / 3.0;
+    Dual V[5];
+    double Ub[5];
+#pragma unroll
+    for (int k = 0; k < 5; ++k) { V[k] = Dual(P2[8 * (size_t)n + k], D2[8 * (size_t)n + k]); Ub[k] = Ub0[k]; }
+    for (int q = q0; q < q1; ++q) {
+      const int f = bnf_ent[q] / 3;
+      Dual nn[3], ff[5];
+#pragma unroll
+      for (int a = 0; a < 3; ++a) nn[a] = third * Dual(fn[(size_t)a * F + f], GEO ? dfn[(size_t)a * F + f] : 0.0);
+      face_flux(g, fcode[f], nn[0], nn[1], nn[2], V, Ub, ff);
+#pragma unroll
+      for (int c = 0; c < 5; ++c) acc[c] += ff[c].d;
+    }
+  }
+  const double iv = 1.0 / vol2[n];
+  const size_t o = (size_t)n2o[n];
+#pragma unroll
+  for (int c = 0; c < 5; ++c) {
+    double d = acc[c];
+    if (GEO) d -= R[5 * o + c] * dvol[n];
+    dR[5 * o + c] = d * iv;
+  }
+}
+
+static size_t fwd_smem(const DeviceMesh& m) {
+  return sizeof(double) * ((size_t)2 * (kPS + kGS) * (m.NB + m.maxHf) + (size_t)5 * m.maxE);
+}
+static size_t fwd_grad_smem(const DeviceMesh& m) { return sizeof(double) * (size_t)2 * kPS * (m.NB + m.maxH); }
+static bool forward_blocked_fits(const DeviceMesh& m) {
+  const int L = kFGradThreads / m.NB;
+  return m.nblk > 0 && fwd_smem(m) <= 220 * 1024 && fwd_grad_smem(m) <= 200 * 1024 && (L == 2 || L == 4 || L == 8);
+}
+
+static void forward_blocked(aerof_gpu_ctx* c, const double* dU, const double* dv, const double* dXdot, double* ddR,
+                            int* cnt) {
+  DeviceMesh& m = c->mesh;
+  cudaStream_t s = c->stream;
+  const Gas g = make_gas(c->cfg.gamma);
+  DualWork& w = c->dual;
+  const int rec = c->cfg.reconstruction;
+  const bool grad = rec != AEROF_REC_CONSTANT;
+  const int gn = grid_for(m.N, kAB);
+  const bool geo = dXdot != nullptr;
+  w.D2.ensure(8 * (size_t)m.N);
+  w.dG2.ensure(16 * (size_t)m.N);
+  const double* R = nullptr;
+  if (geo) {
+    // the residual itself (its volume tangent) leaves P2 and G2 as well
+    c->s.k2.ensure(5 * (size_t)m.N);
+    residual_dev(c, dU, c->s.k2.p, kCountSum);
+    R = c->s.k2.p;
+    if (!c->s.p2g2_valid) prim_grad_blocked_dev(c, dU, nullptr);
+  } else {
+    prim_grad_blocked_dev(c, dU, nullptr);
+  }
+  c->s.p2g2_valid = false;
+  c->s.part.ensure(5 * (size_t)m.N);
+  c->s.spill.ensure(5 * (size_t)std::max(m.nX, 1));
+  k_f_seed<<<gn, kAB, 0, s>>>(m.N, g, m.n2o.p, m.P2.p, dv, dXdot, w.D2.p);
+  AEROF_LAUNCH_CHECK();
+  if (geo) {
+    w.tn.ensure(18 * (size_t)m.T);
+    w.tv.ensure(m.T);
+    w.dbn.ensure(3 * (size_t)m.E);
+    w.dvol.ensure(m.N);
+    w.dfn.ensure(3 * (size_t)std::max(m.F, 1));
+    k_f_tets<128><<<grid_for(m.T, 128), 128, 0, s>>>(m.T, m.X.p, dXdot, m.tets.p, w.tn.p, w.tv.p);
+    AEROF_LAUNCH_CHECK();
+    k_f_edge_normals<<<grid_for(3 * (size_t)m.E, kAB), kAB, 0, s>>>(m.E, m.bsrc.p, m.et_ptr.p, m.et_tet.p, w.tn.p,
+                                                                    w.dbn.p);
+    AEROF_LAUNCH_CHECK();
+    k_f_volumes<<<gn, kAB, 0, s>>>(m.N, m.n2o.p, m.nt_ptr.p, m.nt_tet.p, w.tv.p, w.dvol.p);
+    AEROF_LAUNCH_CHECK();
+    if (m.F) {
+      k_f_face_normals<<<grid_for(m.F, kAB), kAB, 0, s>>>(m.F, m.X.p, dXdot, m.faces.p, w.dfn.p);
+      AEROF_LAUNCH_CHECK();
+    }
+  }
+  if (grad && geo) {
+    const size_t smem = fwd_grad_smem(m);
+    auto go = [&](auto kern) {
+      AEROF_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+      kern<<<m.nblk, kFGradThreads, smem, s>>>(m.N, m.NB, m.P2.p, w.D2.p, m.W2.p, m.n2o.p, m.lsqR.p, m.nb2_ptr.p,
+                                               m.lnb.p, m.hptr.p, m.hnode.p, w.dG2.p);
+      AEROF_LAUNCH_CHECK();
+    };
+    const int L = kFGradThreads / m.NB;
+    if (L == 8) go(k_f_grad<8>);
+    else if (L == 4) go(k_f_grad<4>);
+    else go(k_f_grad<2>);
+  } else if (grad) {
+    grad_records_blocked_dev(c, w.D2.p, w.dG2.p);
+  }
+  const size_t smem = fwd_smem(m);
+  auto edges = [&](auto kern) {
+    AEROF_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    kern<<<m.nblk, kFwdThreads, smem, s>>>(m.N, m.E, m.NB, g, rec, c->cfg.beta, m.bl.p, m.bnorm.p, w.dbn.p, m.beptr.p,
+                                           m.hfptr.p, m.hfpad.p, m.maxHf, m.P2.p, w.D2.p, c->s.G2.p, w.dG2.p,
+                                           m.lptr.p, m.lidx.p, m.xslot.p, c->s.part.p, c->s.spill.p, cnt);
+    AEROF_LAUNCH_CHECK();
+  };
+  auto nodes = [&](auto kern) {
+    kern<<<gn, kAB, 0, s>>>(m.N, m.F, g, m.Ubd.p, m.n2o.p, c->s.part.p, m.xin_ptr.p, c->s.spill.p, m.bnf_ptr.p,
+                            m.bnf_ent.p, m.fcode.p, m.fnrm.p, w.dfn.p, m.P2.p, w.D2.p, m.vol2.p, w.dvol.p, R, ddR);
+    AEROF_LAUNCH_CHECK();
+  };
+  if (geo) {
+    edges(k_f_fv_blocked<true>);
+    nodes(k_f_nodes<true>);
+  } else {
+    edges(k_f_fv_blocked<false>);
+    nodes(k_f_nodes<false>);
+  }
+}
+
 // Forward-mode residual: tangent of R at (U + eps v, X + eps Xdot) into dR.
 int residual_forward(aerof_gpu_ctx* c, const double* dU, const double* dv, const double* dXdot, double* ddR,
                      bool sync) {
@@ -170,6 +652,18 @@ int residual_forward(aerof_gpu_ctx* c, const double* dU, const double* dv, const
   cudaStream_t s = c->stream;
   const Gas g = make_gas(c->cfg.gamma);
   DualWork& w = c->dual;
+  if (forward_blocked_fits(m)) {
+    c->s.counters.ensure(8);
+    int* cnt = c->s.counters.p + 6;
+    AEROF_CUDA(cudaMemsetAsync(cnt, 0, sizeof(int), s));
+    forward_blocked(c, dU, dv, dXdot, ddR, cnt);
+    int bad = 0;
+    if (sync) {
+      AEROF_CUDA(cudaMemcpyAsync(&bad, cnt, sizeof(int), cudaMemcpyDeviceToHost, s));
+      AEROF_CUDA(cudaStreamSynchronize(s));
+    }
+    return bad;
+  }
   w.XD.ensure(3 * (size_t)m.N); w.PD.ensure(8 * (size_t)m.N); w.GD.ensure(15 * (size_t)m.N);
   w.WD.ensure(6 * (size_t)m.N); w.RD.ensure(6 * (size_t)m.N); w.volD.ensure(m.N);
   w.enD.ensure(3 * (size_t)m.E); w.fnD.ensure(3 * (size_t)std::max(m.F, 1)); w.fluxD.ensure(5 * (size_t)m.E);

@@ -328,6 +328,10 @@ struct Implicit {
 // Dual-number work arrays of the forward-mode linearisation.
 struct DualWork {
   DBuf<Dual> XD, PD, GD, WD, RD, volD, enD, fnD, fluxD;
+  // blocked forward mode: tangent records and gradients, tangents of the
+  // tets' edge normals and volumes, of the blocked edges' normals, control
+  // volumes and face normals
+  DBuf<double> D2, dG2, tn, tv, dbn, dvol, dfn;
   bool geom_static = false;  // dual geometry holds the primal with zero tangents
 };
 

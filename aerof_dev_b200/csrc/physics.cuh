@@ -27,6 +27,13 @@ AEROF_HD Dual operator/(Dual a, Dual b) {
   double q = a.v / b.v;
   return Dual(q, (a.d - q * b.d) / b.v);
 }
+// with a constant: its zero tangent is not multiplied out
+AEROF_HD Dual operator+(Dual a, double b) { return Dual(a.v + b, a.d); }
+AEROF_HD Dual operator+(double a, Dual b) { return Dual(a + b.v, b.d); }
+AEROF_HD Dual operator-(Dual a, double b) { return Dual(a.v - b, a.d); }
+AEROF_HD Dual operator-(double a, Dual b) { return Dual(a - b.v, -b.d); }
+AEROF_HD Dual operator*(Dual a, double b) { return Dual(a.v * b, a.d * b); }
+AEROF_HD Dual operator*(double a, Dual b) { return Dual(a * b.v, a * b.d); }
 AEROF_HD Dual& operator+=(Dual& a, Dual b) { a = a + b; return a; }
 AEROF_HD Dual& operator-=(Dual& a, Dual b) { a = a - b; return a; }
 AEROF_HD Dual& operator*=(Dual& a, Dual b) { a = a * b; return a; }
@@ -174,13 +181,14 @@ AEROF_HD void linear_rec(double beta, T Vi, T ddVij, T Vj, T ddVji, T& Vij, T& V
 // ------------------------------------------------------------ fluxes
 // roeflux7.f:1-202 (type 0, pstiff = 0, static mesh vitno = 0): Roe-averaged
 // upwind selection of the physical flux plus the one-wave dissipation term.
-template <class T>
-AEROF_HD void roe_flux(const Gas& g, T n0, T n1, T n2, const T* Ug, const T* Ud, T* phi) {
+// TN: type of the normal (a constant normal beside dual states is a double).
+template <class T, class TN>
+AEROF_HD void roe_flux(const Gas& g, TN n0, TN n1, TN n2, const T* Ug, const T* Ud, T* phi) {
   const double gam1 = g.gam1, invgam1 = g.invgam1, gog1 = g.gam * g.invgam1;
-  T s2 = n0 * n0 + n1 * n1 + n2 * n2;
-  T invnorm = rsqrt_(s2);
-  T rnorm = s2 * invnorm;
-  T nx = n0 * invnorm, ny = n1 * invnorm, nz = n2 * invnorm;
+  TN s2 = n0 * n0 + n1 * n1 + n2 * n2;
+  TN invnorm = rsqrt_(s2);
+  TN rnorm = s2 * invnorm;
+  TN nx = n0 * invnorm, ny = n1 * invnorm, nz = n2 * invnorm;
   T vitg2 = Ug[1] * Ug[1] + Ug[2] * Ug[2] + Ug[3] * Ug[3];
   T vitd2 = Ud[1] * Ud[1] + Ud[2] * Ud[2] + Ud[3] * Ud[3];
   // sqrt(rho) and 1/sqrt(rho) of both sides

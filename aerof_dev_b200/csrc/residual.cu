@@ -669,6 +669,41 @@ __global__ void k_fv_nodes_b(int N, Gas g, const int* __restrict__ n2o, const do
   for (int c = 0; c < 5; ++c) R[5 * o + c] = acc[c] * invcv;
 }
 
+// The assembly of k_fv_nodes_b<false> with five lanes per node, lane c
+// summing component c: a warp's loads of the partial sums, the spilled
+// fluxes and the subface fluxes are contiguous, and four spills are in
+// flight per lane.  Same sums in the same order.
+__global__ void __launch_bounds__(256) k_fv_nodes5(int N, const int* __restrict__ n2o, const double* __restrict__ part,
+                                                   const int* __restrict__ xin_ptr, const double* __restrict__ spill,
+                                                   const int* __restrict__ bnf_ptr, const int* __restrict__ bnf_ent,
+                                                   const double* __restrict__ fbuf, const double* __restrict__ vol2,
+                                                   double* __restrict__ R, int* __restrict__ cnt,
+                                                   volatile int* __restrict__ pub) {
+  const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (pub && t == 0) {
+    *pub = *cnt;
+    *cnt = 0;
+  }
+  const int n = (int)(t / 5), c = (int)(t - 5 * (unsigned)n);
+  if (n >= N) return;
+  int k = xin_ptr[n];
+  const int k1 = xin_ptr[n + 1], q0 = bnf_ptr[n], q1 = bnf_ptr[n + 1];
+  const double iv = 1.0 / vol2[n];
+  const size_t o = (size_t)n2o[n];
+  double acc = part[(size_t)t];
+  for (; k + 4 <= k1; k += 4) {
+    const double* sp = spill + 5 * (size_t)k + c;
+    const double s0 = __ldcs(sp), s1 = __ldcs(sp + 5), s2 = __ldcs(sp + 10), s3 = __ldcs(sp + 15);
+    acc -= s0;
+    acc -= s1;
+    acc -= s2;
+    acc -= s3;
+  }
+  for (; k < k1; ++k) acc -= __ldcs(spill + 5 * (size_t)k + c);
+  for (int q = q0; q < q1; ++q) acc += fbuf[5 * (size_t)bnf_ent[q] + c];
+  R[5 * o + c] = acc * iv;
+}
+
 // U[N][5] (caller numbering) -> blocked node records P2[n].V
 __global__ void k_prim_blocked(int N, Gas g, const int* __restrict__ n2o, const double* __restrict__ U,
                                double* __restrict__ P2) {
@@ -1343,9 +1378,9 @@ static int residual_blocked_dev(aerof_gpu_ctx* c, const double* dU, double* dR, 
                                                              m.P2.p, m.o2n.p, c->s.fbuf.p);
         AEROF_LAUNCH_CHECK();
       }
-      k_fv_nodes_b<false><<<grid_for(m.N, kBlock), kBlock, 0, s>>>(
-          m.N, g, m.n2o.p, c->s.part.p, m.xin_ptr.p, c->s.spill.p, m.bnf_ptr.p, m.bnf_ent.p, c->s.fbuf.p, m.F,
-          m.Ubd.p, m.fcode.p, m.fnrm.p, m.P2.p, m.vol2.p, dR, nullptr, 0, m.NB, cnt, pub);
+      k_fv_nodes5<<<grid_for(5 * (size_t)m.N, kBlock), kBlock, 0, s>>>(m.N, m.n2o.p, c->s.part.p, m.xin_ptr.p,
+                                                                       c->s.spill.p, m.bnf_ptr.p, m.bnf_ent.p,
+                                                                       c->s.fbuf.p, m.vol2.p, dR, cnt, pub);
     }
     AEROF_LAUNCH_CHECK();
     if (pub) c->s.count_clear = true;
