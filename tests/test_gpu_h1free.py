@@ -1,0 +1,81 @@
+"""Products with H1 formed from the states inside the Krylov solvers against
+the stored blocks, and operators of which only the diagonal was assembled.
+
+The mesh sizes put the node count just below, at and above multiples of the
+128-node block (27 to 1331 nodes), with one block, partial last blocks and
+odd neighbour counts.  Both routes run the same GMRES iterations on the same
+preconditioner; in FP64 the products differ by a few 2^-53 per term, so the
+iterates agree far below 1e-9; in FP32 by a few 2^-24 through up to eight
+iterations: 1e-5."""
+import numpy as np
+import pytest
+
+from aerof_dev_b200 import workloads as W
+from conftest import rel_l2
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("prec,tol", [(64, 1e-9), (32, 1e-5)])
+@pytest.mark.parametrize("transpose", [False, True])
+@pytest.mark.parametrize("n,codes,with_dt", [(3, "channel", True), (5, "farfield", True), (6, "channel", False),
+                                             (8, "channel", True), (11, "farfield", True)])
+def test_products_match_the_stored_blocks(gpu_lib, prec, tol, transpose, n, codes, with_dt):
+    A = gpu_lib
+    m = W.make_lattice_mesh(n, jitter=0.2, codes=codes)
+    ctx = A.Context.from_mesh(m, W.freestream(0.7))
+    U = W.perturbed_state(ctx.N, 0.7, amp=0.05)
+    dt = A.SpaceOperator(ctx).computeTimeStep(U, 30.0) if with_dt else None
+    mv, pc = A.MatVecProdH1(ctx, prec), A.JacobiPrec(ctx)
+    b = np.random.default_rng(n).standard_normal((ctx.N, 5))
+    gm = A.GmresSolver(ctx, 8, 8, 0.0)
+    mv.evaluate(U, dt)
+    blocks = mv.blocks()
+    pc.setup()
+    free, its, res = gm.solve(b, transpose=transpose)
+    mv.set_blocks(blocks)   # an operator given by the caller is read as stored
+    pc.setup()
+    stored, its2, res2 = gm.solve(b, transpose=transpose)
+    assert its == its2 == 8
+    assert rel_l2(free, stored) < tol
+    assert abs(res - res2) <= tol * np.linalg.norm(b)
+
+
+@pytest.mark.parametrize("prec", [64, 32])
+def test_newton_operator_is_complete_afterwards(gpu_lib, prec):
+    # Newton assembles the diagonal blocks only; the operator it leaves
+    # behind reads as the one evaluated at its last linearisation point
+    A = gpu_lib
+    m = W.make_lattice_mesh(7, jitter=0.2, codes="channel")
+    ctx = A.Context.from_mesh(m, W.freestream(0.8))
+    U = W.perturbed_state(ctx.N, 0.8)
+    dt = A.SpaceOperator(ctx).computeTimeStep(U, 10.0)
+    A.ImplicitSteadySolver(ctx, precision=prec, max_steps=1).solve(U)
+    left = A.MatVecProdH1(ctx, prec)
+    p = np.random.default_rng(0).standard_normal((ctx.N, 5))
+    y = left.apply(p)
+    yt = left.applyTranspose(p)
+    fresh = A.MatVecProdH1(A.Context.from_mesh(m, W.freestream(0.8)), prec)
+    fresh.evaluate(U, dt)
+    assert np.array_equal(left.blocks(), fresh.blocks())
+    assert np.array_equal(y, fresh.apply(p)) and np.array_equal(yt, fresh.applyTranspose(p))
+    # its preconditioner stays usable, and an ILU(0) can be set up from it
+    z = A.JacobiPrec(ctx).apply(p)
+    A.JacobiPrec(fresh.ctx).setup()
+    assert rel_l2(z, A.JacobiPrec(fresh.ctx).apply(p)) < (1e-12 if prec == 64 else 1e-5)
+    ctx.set_preconditioner(A.PC_ILU0)
+    A.JacobiPrec(ctx).setup()
+    assert A.GmresSolver(ctx, 30, 30, 1e-8).solve(p)[2] <= 1e-6 * np.linalg.norm(p)
+
+
+@pytest.mark.parametrize("transpose", [False, True])
+def test_linearized_solve_leaves_its_operator(gpu_lib, transpose):
+    A = gpu_lib
+    m = W.make_lattice_mesh(6, jitter=0.2, codes="channel")
+    ctx = A.Context.from_mesh(m, W.freestream(0.5))
+    U = W.smooth_state(m["X"], 0.5)
+    b = np.random.default_rng(2).standard_normal((ctx.N, 5))
+    A.Sensitivity(ctx).solve(U, b, transpose=transpose, maxits=20, inner_its=5)
+    fresh = A.MatVecProdH1(A.Context.from_mesh(m, W.freestream(0.5)), 32)
+    fresh.evaluate(U)
+    assert rel_l2(A.MatVecProdH1(ctx, 32).blocks(), fresh.blocks()) < 1e-6

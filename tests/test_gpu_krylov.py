@@ -1,0 +1,81 @@
+"""Device-driven GMRES and flexible GMRES: restart lengths around the eight
+basis vectors that one pass of the Gram-Schmidt sweep takes, more vectors
+than the triangular solve keeps in shared memory, restarts, a zero right-hand
+side, and systems that converge at different times in one batch.
+
+Tolerances: in FP64 the two orthogonalisations (the oracle's and the two
+sweeps) compute the same Krylov minimiser; its relative change is bounded by
+2^-53 times the squared condition of the basis recurrence, far below the
+1e-9 asked for at these sizes and iteration counts."""
+import numpy as np
+import pytest
+
+from aerof_dev_b200 import workloads as W
+from conftest import rel_l2
+
+pytestmark = pytest.mark.gpu
+
+
+def _operator(A, o, m, U, dt, prec):
+    ctx = A.Context.from_mesh(m, W.freestream(0.8))
+    mv = A.MatVecProdH1(ctx, prec)
+    mv.evaluate(U, dt)
+    A.JacobiPrec(ctx).setup()
+    return ctx, mv
+
+
+@pytest.mark.parametrize("n,krylov,maxits", [(4, 1, 3), (4, 7, 7), (6, 8, 20), (6, 9, 9), (6, 17, 40), (5, 70, 75),
+                                             (3, 100, 100)])
+def test_gmres_restart_lengths(gpu_lib, oracle_mod, n, krylov, maxits):
+    A = gpu_lib
+    m = W.make_lattice_mesh(n, jitter=0.2, codes="channel")
+    Ub = W.freestream(0.8)
+    o = oracle_mod.Oracle(m)
+    U = W.perturbed_state(o.N, 0.8)
+    dt = o.timestep(U, 20.0)
+    ctx, mv = _operator(A, o, m, U, dt, 64)
+    blocks = mv.blocks()
+    b = np.random.default_rng(n).standard_normal((o.N, 5))
+    x, its, res = A.GmresSolver(ctx, krylov, maxits, 1e-11).solve(b)
+    # the true residual equals the method's estimate, within the same
+    # relative accuracy of b
+    r = b - o.matvec(blocks, x)
+    assert its <= maxits
+    assert abs(np.linalg.norm(r) - res) <= 1e-9 * np.linalg.norm(b)
+    assert its == maxits or res <= 1e-11 * np.linalg.norm(b)
+    # a zero right-hand side is answered by zero, without iterations
+    x0, it0, r0 = A.GmresSolver(ctx, krylov, maxits, 1e-11).solve(np.zeros_like(b))
+    assert it0 == 0 and r0 == 0.0 and not x0.any()
+
+
+@pytest.mark.parametrize("pc", [0, 1])
+@pytest.mark.parametrize("transpose", [False, True])
+def test_batch_equals_one_by_one(gpu_lib, pc, transpose):
+    # five systems of very different right-hand sides (one of them zero, one
+    # nearly an eigen-direction's multiple), each as its own solve
+    A = gpu_lib
+    m = W.make_lattice_mesh(7, jitter=0.2, codes="channel")
+    ctx = A.Context.from_mesh(m, W.freestream(0.5))
+    ctx.set_preconditioner(pc)
+    U = W.smooth_state(m["X"], 0.5)
+    S = A.Sensitivity(ctx)
+    rng = np.random.default_rng(1)
+    B = rng.standard_normal((5, ctx.N, 5))
+    B[1] = 0.0
+    B[2] *= 1e-6
+    B[3] = S.jvp(U, np.ones((ctx.N, 5)))
+    X, its, res = S.solve_batch(U, B, transpose=transpose, krylov=11, maxits=200, eps=1e-9, inner_its=6)
+    assert its[1] == 0 and not X[1].any()
+    for k in range(5):
+        if k == 1:
+            continue
+        assert res[k] <= 1e-9 * np.linalg.norm(B[k])
+        J = S.vjp if transpose else S.jvp
+        assert np.linalg.norm(J(U, X[k]) - B[k]) <= 1e-8 * np.linalg.norm(B[k])
+        S.set_exact_operator(True)
+        x1, i1, _ = S.solve(U, B[k], transpose=transpose, krylov=11, maxits=200, eps=1e-9, inner_its=6)
+        S.set_exact_operator(False)
+        # both satisfy the system to 1e-9; their difference is that residual
+        # through J^-1 (condition below 1e3 here)
+        assert rel_l2(X[k], x1) <= 1e-6
+        assert abs(int(its[k]) - i1) <= 1
