@@ -117,9 +117,12 @@ namespace aerof {
 // roejac(n, Va, Vb, +1) = dF/dU of the first endpoint a, (.., -1) of the
 // second) give the off-diagonal block A_rs = sg dF/dU_s / vol_r and the
 // contribution sg dF/dU_r to the diagonal block (Edge.C:4503-4523).  Both
-// Jacobians share the Roe dissipation matrix D, formed one column at a
-// time with the convective parts H(V_s), H(V_r), so no 25-element block is
-// held in registers besides the diagonal sum.  Then the row's boundary
+// Jacobians share the Roe dissipation matrix D; it and the convective parts
+// H(V_s), H(V_r) are a multiple of the identity plus two rank-one terms
+// each, so an element takes a few operations and no 25-element block is held
+// in registers besides the diagonal sum (the eigenvector form of roejac6.f,
+// with its divisions per element: 0.44 ms at 81^3 in FP32, this one 0.30 ms,
+// for 0.75 GB of stored blocks).  Then the row's boundary
 // faces (Face.C:814-847), times 1/vol (SubDomain.C:1760-1765), + I/dt
 // (TimeState.C:731-756).  Every edge's Jacobians are evaluated once by each
 // of its two rows.  TR: the transpose H1^T is stored instead (block k of
@@ -221,24 +224,24 @@ __global__ void __launch_bounds__(JacThreads<S>::T, JacThreads<S>::B)
     S VrS[5], VsS[5];
 #pragma unroll
     for (int k = 0; k < 5; ++k) { VrS[k] = (S)Vr[k]; VsS[k] = (S)Vs[k]; }
-    const auto A = roe_avg<S>(g, un, VrS, VsS);
-    const auto hr = h_state<S>(g, un, VrS);
-    const auto hs = h_state<S>(g, un, VsS);
+    // |A| = f1 I + R1 (x) p + R2 (x) t at the Roe average, A(V) = un I + R1
+    // (x) a + R2 (x) b at each state (RankTwo)
+    const RankTwo<S> D = roe_dissipation<S>(g, un, VrS, VsS);
+    const RankTwo<S> hr = flux_jacobian<S>(g, un, VrS), hs = flux_jacobian<S>(g, un, VsS);
 #pragma unroll
     for (int j = 0; j < 5; ++j) {
-      S d[5];
-      D_col<S>(g, A, un, j, d);
 #pragma unroll
       for (int m = 0; m < 5; ++m) {
         const int el = 5 * m + j;
+        const S d = D.elem(un, m, j);
         // diagonal contribution: roejac(n, Vr, Vs, sg)
-        const S jd = (H_elem<S>(g, hr, un, el) + sgS * d[m]) * half_rn;
+        const S jd = (hr.elem(un, m, j) + sgS * d) * half_rn;
         a[T * el] += sg * (double)jd;
         if (TR) {
           so[T * (5 * j + m)] = jd * sco;
         } else {
           // off-diagonal block: roejac(n, Vs, Vr, -sg)
-          const S jo = (H_elem<S>(g, hs, un, el) + (-sgS) * d[m]) * half_rn;
+          const S jo = (hs.elem(un, m, j) + (-sgS) * d) * half_rn;
           so[T * el] = jo * sco;
         }
       }

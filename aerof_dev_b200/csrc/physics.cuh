@@ -322,49 +322,8 @@ AEROF_HD void post_dVdU(const Gas& g, const double* V, const double* mat, double
 
 // roejac6.f:1-316 (type 0, prec 0 -> beta 1, dissipation coefficient 1):
 // approximate Jacobian of the Roe flux w.r.t. the conservative state Ug,
-// sw = +1 adds the dissipation matrix, sw = -1 subtracts it.
-//
-// Convective part of roejac6: the exact flux Jacobian H(U) of state U along
-// the unit normal n (roejac6.f, first block).
-AEROF_HD void roe_jac_H(const Gas& g, const double* n, const double* Ug, double* H) {
-  const double gam = g.gam, gam1 = g.gam1;
-  const double VdotN = Ug[1] * n[0] + Ug[2] * n[1] + Ug[3] * n[2];
-  const double qir = 0.5 * (Ug[1] * Ug[1] + Ug[2] * Ug[2] + Ug[3] * Ug[3]);
-  const double enth = (gam * Ug[4] + gam1 * Ug[0] * qir) / (gam1 * Ug[0]);
-  H[0] = 0.0; H[1] = n[0]; H[2] = n[1]; H[3] = n[2]; H[4] = 0.0;
-  H[5] = gam1 * n[0] * qir - Ug[1] * VdotN;
-  H[6] = (1.0 - gam1) * n[0] * Ug[1] + VdotN;
-  H[7] = -gam1 * n[0] * Ug[2] + Ug[1] * n[1];
-  H[8] = -gam1 * n[0] * Ug[3] + Ug[1] * n[2];
-  H[9] = gam1 * n[0];
-  H[10] = gam1 * n[1] * qir - Ug[2] * VdotN;
-  H[11] = -gam1 * n[1] * Ug[1] + Ug[2] * n[0];
-  H[12] = (1.0 - gam1) * n[1] * Ug[2] + VdotN;
-  H[13] = -gam1 * n[1] * Ug[3] + Ug[2] * n[2];
-  H[14] = gam1 * n[1];
-  H[15] = gam1 * n[2] * qir - Ug[3] * VdotN;
-  H[16] = -gam1 * n[2] * Ug[1] + Ug[3] * n[0];
-  H[17] = -gam1 * n[2] * Ug[2] + Ug[3] * n[1];
-  H[18] = (1.0 - gam1) * n[2] * Ug[3] + VdotN;
-  H[19] = gam1 * n[2];
-  H[20] = (gam1 * qir - enth) * VdotN;
-  H[21] = enth * n[0] - gam1 * Ug[1] * VdotN;
-  H[22] = enth * n[1] - gam1 * Ug[2] * VdotN;
-  H[23] = enth * n[2] - gam1 * Ug[3] * VdotN;
-  H[24] = (1.0 + gam1) * VdotN;
-}
-
-// Dissipation part of roejac6: |A| at the Roe average of the two states,
-// written through its eigenvectors (roejac6.f, second block).  The Roe
-// average is symmetric in (Ug, Ud), bit for bit (every sum of the two sides
-// is a commutative two-term addition), so one D serves both endpoints.
-// RoeAvg holds the scalars of the average; tmw_elem and D_col form the
-// eigenvector matrix and D one column at a time, so a caller can stream
-// the 5x5 blocks without holding 25-element arrays.
-template <class T = double>
-struct RoeAvg {
-  T uar2, uar3, uar4, enth, VdotN, qir, crsq, gc, usc2, rRT, sRT, tRT, vp1, vp4, vp5;
-};
+// (H(Ug) + sw |A|_Roe) |n| / 2, sw = +1, or called with the states swapped w.r.t.
+// the second, sw = -1.
 // a*b + c*d with both products rounded (no fused multiply-add), so the
 // result does not depend on which pair is named first
 AEROF_HD double sym_dot2(double a, double b, double c, double d) {
@@ -382,163 +341,74 @@ AEROF_HD float sym_dot2(float a, float b, float c, float d) {
 #endif
 }
 
-// T = double: the reference arithmetic; T = float: the same formulas in
-// FP32, for the FP32-stored Jacobian of the mixed-precision solver.  The
-// Roe average is formed symmetrically in (Ug, Ud) (sym_dot2), so the two
-// rows of an edge obtain the same dissipation matrix bit for bit.
-template <class T = double>
-AEROF_HD RoeAvg<T> roe_avg(const Gas& g, const T* n, const T* Ug, const T* Ud) {
+// w I + R1 (x) p + R2 (x) t with R1 = (1, u, H), R2 = (0, n, un): the form
+// of the Euler flux Jacobian along n and of any function of it (n unit).
+// With a = (-un, n, 0) and b = (gam - 1)(q, -u, 1), q = |u|^2 / 2: the
+// Jacobian has w = un, p = a, t = b (roejac6.f, first block), |A| has w =
+// |un|, p = S1 b/c^2 + S2 a/c, t = S1 a + S2 b/c, S1 = (|un+c| + |un-c|)/2 -
+// |un|, S2 = (|un+c| - |un-c|)/2 (the projection form of Liu and Vinokur,
+// "Nonequilibrium flow computations", 1989, equal to the eigenvector product
+// of roejac6.f, second block).
+template <class T>
+struct RankTwo {
+  T w, u[3], H, un, p[5], t[5];
+  AEROF_HD T elem(const T* n, int m, int j) const {
+    const T r1 = m == 0 ? T(1.0) : (m == 4 ? H : u[m == 0 || m == 4 ? 0 : m - 1]);
+    const T r2 = m == 4 ? un : n[m == 0 || m == 4 ? 0 : m - 1];
+    T e = m == 0 ? p[j] : r1 * p[j] + r2 * t[j];
+    if (m == j) e += w;
+    return e;
+  }
+};
+template <class T>
+AEROF_HD RankTwo<T> flux_jacobian(const Gas& g, const T* n, const T* V) {
   const T gam1 = (T)g.gam1;
-  RoeAvg<T> A;
-  T squsr1 = sqrt(Ug[0]), squsr2 = sqrt(Ud[0]);
-  T ener1 = Ug[4] / gam1 + T(0.5) * Ug[0] * (Ug[1] * Ug[1] + Ug[2] * Ug[2] + Ug[3] * Ug[3]);
-  T ener2 = Ud[4] / gam1 + T(0.5) * Ud[0] * (Ud[1] * Ud[1] + Ud[2] * Ud[2] + Ud[3] * Ud[3]);
-  T usro = T(1.0) / (squsr1 + squsr2);
-  A.uar2 = sym_dot2(squsr1, Ug[1], squsr2, Ud[1]) * usro;
-  A.uar3 = sym_dot2(squsr1, Ug[2], squsr2, Ud[2]) * usro;
-  A.uar4 = sym_dot2(squsr1, Ug[3], squsr2, Ud[3]) * usro;
-  T uar5 = ((ener1 + Ug[4]) / squsr1 + (ener2 + Ud[4]) / squsr2) * usro;
-  A.enth = uar5;
-  A.VdotN = n[0] * A.uar2 + n[1] * A.uar3 + n[2] * A.uar4;
-  A.qir = T(0.5) * (A.uar2 * A.uar2 + A.uar3 * A.uar3 + A.uar4 * A.uar4);
-  T cr = sqrt(gam1 * (uar5 - A.qir));
-  A.crsq = cr * cr;
-  A.gc = gam1 / A.crsq;
-  A.usc2 = T(0.5) / A.crsq;
-  // beta = 1: vp4,vp5 = VdotN +- cr written as the reference's general form
-  T sq = sqrt(T(0.0) * A.VdotN * (T(0.0) * A.VdotN) + T(4.0) * A.crsq);
-  T vp4 = T(0.5) * (T(2.0) * A.VdotN + sq);
-  T vp5 = T(0.5) * (T(2.0) * A.VdotN - sq);
-  A.rRT = vp4 - A.VdotN;
-  A.sRT = vp5 - A.VdotN;
-  A.tRT = T(0.5) * (vp5 - vp4);
-  A.vp1 = fabs(A.VdotN);
-  A.vp4 = fabs(vp4);
-  A.vp5 = fabs(vp5);
+  RankTwo<T> A;
+  const T q = T(0.5) * (V[1] * V[1] + V[2] * V[2] + V[3] * V[3]);
+  A.un = V[1] * n[0] + V[2] * n[1] + V[3] * n[2];
+  A.w = A.un;
+  A.H = (T)(g.gam * g.invgam1) * V[4] / V[0] + q;
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    A.u[k] = V[1 + k];
+    A.p[1 + k] = n[k];
+    A.t[1 + k] = -gam1 * V[1 + k];
+  }
+  A.p[0] = -A.un; A.p[4] = T(0.0);
+  A.t[0] = gam1 * q; A.t[4] = gam1;
   return A;
 }
-// element e (row-major) of the left eigenvector matrix tmw
-template <class T = double>
-AEROF_HD T tmw_elem(const Gas& g, const RoeAvg<T>& A, const T* n, int e) {
-  const T gam1 = (T)g.gam1;
-  switch (e) {
-    case 0: return n[0] + n[1] * A.uar4 - A.uar3 * n[2] - A.gc * n[0] * A.qir;
-    case 1: return A.gc * n[0] * A.uar2;
-    case 2: return A.gc * n[0] * A.uar3 + n[2];
-    case 3: return A.gc * n[0] * A.uar4 - n[1];
-    case 4: return -A.gc * n[0];
-    case 5: return n[1] + n[2] * A.uar2 - A.uar4 * n[0] - A.gc * n[1] * A.qir;
-    case 6: return A.gc * n[1] * A.uar2 - n[2];
-    case 7: return A.gc * n[1] * A.uar3;
-    case 8: return A.gc * n[1] * A.uar4 + n[0];
-    case 9: return -A.gc * n[1];
-    case 10: return n[2] + n[0] * A.uar3 - A.uar2 * n[1] - A.gc * n[2] * A.qir;
-    case 11: return A.gc * n[2] * A.uar2 + n[1];
-    case 12: return A.gc * n[2] * A.uar3 - n[0];
-    case 13: return A.gc * n[2] * A.uar4;
-    case 14: return -A.gc * n[2];
-    case 15: return gam1 * A.qir * A.sRT / A.tRT + A.VdotN * A.crsq / A.tRT;
-    case 16: return -gam1 * A.uar2 * A.sRT / A.tRT - A.crsq * n[0] / A.tRT;
-    case 17: return -gam1 * A.uar3 * A.sRT / A.tRT - A.crsq * n[1] / A.tRT;
-    case 18: return -gam1 * A.uar4 * A.sRT / A.tRT - A.crsq * n[2] / A.tRT;
-    case 19: return gam1 * A.sRT / A.tRT;
-    case 20: return -gam1 * A.qir * A.rRT / A.tRT - A.VdotN * A.crsq / A.tRT;
-    case 21: return gam1 * A.uar2 * A.rRT / A.tRT + A.crsq * n[0] / A.tRT;
-    case 22: return gam1 * A.uar3 * A.rRT / A.tRT + A.crsq * n[1] / A.tRT;
-    case 23: return gam1 * A.uar4 * A.rRT / A.tRT + A.crsq * n[2] / A.tRT;
-    default: return -gam1 * A.rRT / A.tRT;
-  }
-}
-// column j of D: d[m] = D[5 m + j]
-template <class T = double>
-AEROF_HD void D_col(const Gas& g, const RoeAvg<T>& A, const T* n, int j, T* d) {
-  const T t0 = tmw_elem(g, A, n, j), t1 = tmw_elem(g, A, n, 5 + j), t2 = tmw_elem(g, A, n, 10 + j);
-  const T t3 = tmw_elem(g, A, n, 15 + j), t4 = tmw_elem(g, A, n, 20 + j);
-  const T uar2 = A.uar2, uar3 = A.uar3, uar4 = A.uar4, qir = A.qir, usc2 = A.usc2, rRT = A.rRT, sRT = A.sRT;
-  const T vp1 = A.vp1, vp4 = A.vp4, vp5 = A.vp5, enth = A.enth, VdotN = A.VdotN;
-  d[0] = vp1 * (n[0] * t0 + n[1] * t1 + n[2] * t2) + vp4 * usc2 * t3 + vp5 * usc2 * t4;
-  d[1] = vp1 * (n[0] * uar2 * t0 + (n[1] * uar2 - n[2]) * t1 + (n[2] * uar2 + n[1]) * t2) +
-         vp4 * (usc2 * (uar2 + rRT * n[0])) * t3 + vp5 * (usc2 * (uar2 + sRT * n[0])) * t4;
-  d[2] = vp1 * (n[1] * uar3 * t1 + (n[0] * uar3 + n[2]) * t0 + (n[2] * uar3 - n[0]) * t2) +
-         vp4 * (usc2 * (uar3 + rRT * n[1])) * t3 + vp5 * (usc2 * (uar3 + sRT * n[1])) * t4;
-  d[3] = vp1 * (n[2] * uar4 * t2 + (n[0] * uar4 - n[1]) * t0 + (n[1] * uar4 + n[0]) * t1) +
-         vp4 * (usc2 * (uar4 + rRT * n[2])) * t3 + vp5 * (usc2 * (uar4 + sRT * n[2])) * t4;
-  d[4] = vp1 * ((n[0] * qir + (n[2] * uar3 - n[1] * uar4)) * t0 + (n[1] * qir + (n[0] * uar4 - n[2] * uar2)) * t1 +
-                (n[2] * qir + (n[1] * uar2 - n[0] * uar3)) * t2) +
-         vp4 * (usc2 * (enth + VdotN * rRT)) * t3 + vp5 * (usc2 * (enth + VdotN * sRT)) * t4;
-}
-AEROF_HD void roe_jac_D(const Gas& g, const double* n, const double* Ug, const double* Ud, double* D) {
-  const RoeAvg<double> A = roe_avg(g, n, Ug, Ud);
+// |A| at the Roe average of the two states, which is formed symmetrically in
+// them, bit for bit (sym_dot2), so the two rows of an edge obtain the same
+// dissipation matrix
+template <class T>
+AEROF_HD RankTwo<T> roe_dissipation(const Gas& g, const T* n, const T* Ug, const T* Ud) {
+  const T gam1 = (T)g.gam1, gog1 = (T)(g.gam * g.invgam1);
+  RankTwo<T> A;
+  const T s1 = sqrt(Ug[0]), s2 = sqrt(Ud[0]);
+  const T rw = T(1.0) / (s1 + s2);
+  const T H1 = gog1 * Ug[4] / Ug[0] + T(0.5) * (Ug[1] * Ug[1] + Ug[2] * Ug[2] + Ug[3] * Ug[3]);
+  const T H2 = gog1 * Ud[4] / Ud[0] + T(0.5) * (Ud[1] * Ud[1] + Ud[2] * Ud[2] + Ud[3] * Ud[3]);
 #pragma unroll
-  for (int j = 0; j < 5; ++j) {
-    double d[5];
-    D_col(g, A, n, j, d);
+  for (int k = 0; k < 3; ++k) A.u[k] = sym_dot2(s1, Ug[1 + k], s2, Ud[1 + k]) * rw;
+  A.H = sym_dot2(s1, H1, s2, H2) * rw;
+  A.un = n[0] * A.u[0] + n[1] * A.u[1] + n[2] * A.u[2];
+  const T q = T(0.5) * (A.u[0] * A.u[0] + A.u[1] * A.u[1] + A.u[2] * A.u[2]);
+  const T c2 = gam1 * (A.H - q), c = sqrt(c2), ic = T(1.0) / c;
+  const T f1 = fabs(A.un), fp = fabs(A.un + c), fm = fabs(A.un - c);
+  const T S1 = T(0.5) * (fp + fm) - f1, S2 = T(0.5) * (fp - fm) * ic;
+  const T kb = gam1 * S1 * ic * ic, tb = gam1 * S2;
+  A.w = f1;
+  A.p[0] = kb * q - S2 * A.un;
+  A.t[0] = tb * q - S1 * A.un;
 #pragma unroll
-    for (int m = 0; m < 5; ++m) D[5 * m + j] = d[m];
+  for (int k = 0; k < 3; ++k) {
+    A.p[1 + k] = S2 * n[k] - kb * A.u[k];
+    A.t[1 + k] = S1 * n[k] - tb * A.u[k];
   }
-}
-
-// Scalars of the convective Jacobian H(U) (see roe_jac_H) and its element
-// e (row-major), for streaming use.
-template <class T = double>
-struct HState {
-  T U1, U2, U3, VdotN, qir, enth;
-};
-template <class T = double>
-AEROF_HD HState<T> h_state(const Gas& g, const T* n, const T* Ug) {
-  HState<T> h;
-  h.U1 = Ug[1]; h.U2 = Ug[2]; h.U3 = Ug[3];
-  h.VdotN = Ug[1] * n[0] + Ug[2] * n[1] + Ug[3] * n[2];
-  h.qir = T(0.5) * (Ug[1] * Ug[1] + Ug[2] * Ug[2] + Ug[3] * Ug[3]);
-  h.enth = ((T)g.gam * Ug[4] + (T)g.gam1 * Ug[0] * h.qir) / ((T)g.gam1 * Ug[0]);
-  return h;
-}
-template <class T = double>
-AEROF_HD T H_elem(const Gas& g, const HState<T>& h, const T* n, int e) {
-  const T gam1 = (T)g.gam1;
-  switch (e) {
-    case 0: return T(0.0);
-    case 1: return n[0];
-    case 2: return n[1];
-    case 3: return n[2];
-    case 4: return T(0.0);
-    case 5: return gam1 * n[0] * h.qir - h.U1 * h.VdotN;
-    case 6: return (T(1.0) - gam1) * n[0] * h.U1 + h.VdotN;
-    case 7: return -gam1 * n[0] * h.U2 + h.U1 * n[1];
-    case 8: return -gam1 * n[0] * h.U3 + h.U1 * n[2];
-    case 9: return gam1 * n[0];
-    case 10: return gam1 * n[1] * h.qir - h.U2 * h.VdotN;
-    case 11: return -gam1 * n[1] * h.U1 + h.U2 * n[0];
-    case 12: return (T(1.0) - gam1) * n[1] * h.U2 + h.VdotN;
-    case 13: return -gam1 * n[1] * h.U3 + h.U2 * n[2];
-    case 14: return gam1 * n[1];
-    case 15: return gam1 * n[2] * h.qir - h.U3 * h.VdotN;
-    case 16: return -gam1 * n[2] * h.U1 + h.U3 * n[0];
-    case 17: return -gam1 * n[2] * h.U2 + h.U3 * n[1];
-    case 18: return (T(1.0) - gam1) * n[2] * h.U3 + h.VdotN;
-    case 19: return gam1 * n[2];
-    case 20: return (gam1 * h.qir - h.enth) * h.VdotN;
-    case 21: return h.enth * n[0] - gam1 * h.U1 * h.VdotN;
-    case 22: return h.enth * n[1] - gam1 * h.U2 * h.VdotN;
-    case 23: return h.enth * n[2] - gam1 * h.U3 * h.VdotN;
-    default: return (T(1.0) + gam1) * h.VdotN;
-  }
-}
-
-// jac = (H(Ug) + sw |A|_Roe) |n| / 2: the derivative of the Roe flux with
-// respect to the first state (sw = +1) or, called with the states swapped,
-// the second (sw = -1).
-AEROF_HD void roe_jac(const Gas& g, double n0, double n1, double n2, const double* Ug, const double* Ud,
-                      double sw, double* jac) {
-  double rnorm = sqrt(n0 * n0 + n1 * n1 + n2 * n2);
-  double invnorm = 1.0 / rnorm;
-  double n[3] = {n0 * invnorm, n1 * invnorm, n2 * invnorm};
-  double H[25], D[25];
-  roe_jac_H(g, n, Ug, H);
-  roe_jac_D(g, n, Ug, Ud, D);
-  const double half_rn = 0.5 * rnorm;
-#pragma unroll
-  for (int k = 0; k < 25; ++k) jac[k] = (H[k] + sw * D[k]) * half_rn;
+  A.p[4] = kb;
+  A.t[4] = tb;
+  return A;
 }
 
 // Face blocks: FluxFcnFD<5>::computeJacobian (FluxFcnBase.h:112-159) for the
