@@ -505,6 +505,30 @@ __device__ __forceinline__ void cp_async4(void* sdst, const void* gsrc) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(s), "l"(gsrc) : "memory");
 }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
+// Programmatic dependent launch: a kernel launched with launch_pdl may start
+// while its predecessor in the stream still runs; what it does before
+// pdl_wait() must touch only data that no kernel since the last ordinary
+// launch writes.  pdl_trigger() lets the successor start that early too.
+// What the predecessors write is read after pdl_wait() through pointers
+// without __restrict__: a restricted read-only pointer allows the compiler to
+// move its loads over the wait and to use the non-coherent path.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+template <class... P, class... A>
+void launch_pdl(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  AEROF_CUDA(cudaLaunchKernelEx(&cfg, kern, (P)args...));
+  AEROF_LAUNCH_CHECK();
+}
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait_prev() { asm volatile("cp.async.wait_group 1;\n" ::: "memory"); }
 // Bulk prefetch of a contiguous global range into L2 (no destination, no

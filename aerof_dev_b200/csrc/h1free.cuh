@@ -146,9 +146,10 @@ __device__ __forceinline__ void h1_put(S* __restrict__ z, int n, double sc, cons
 // vectors x (system q: X.p[q], or X0 + q xs) packed without a preconditioner
 template <class S, class TI>
 __global__ void k_h1_pack(int N, const int* __restrict__ o2n, const double* __restrict__ vol, int tr,
-                          const TI* __restrict__ x, size_t xs, S* __restrict__ z, size_t zs,
-                          const int* __restrict__ skip) {
+                          const TI* x, size_t xs, S* z, size_t zs, const int* skip) {
   const int o = blockIdx.x * blockDim.x + threadIdx.x, q = blockIdx.y;
+  pdl_trigger();
+  pdl_wait();
   if (o >= N || (skip && skip[8 * q])) return;
   double v[5];
 #pragma unroll
@@ -171,34 +172,29 @@ __global__ void __launch_bounds__(256, sizeof(S) == 4 ? 3 : 2)
                const int* __restrict__ hnode, const int* __restrict__ wptr, size_t total,
                const S* __restrict__ nrm, const unsigned short* __restrict__ slot, const double* __restrict__ mrow,
                const S* __restrict__ rec, const double* __restrict__ idt, const int* __restrict__ brow,
-               const double* __restrict__ fsum, const S* __restrict__ z, size_t zs, S* __restrict__ y, size_t ys,
-               const int* __restrict__ skip) {
+               const double* __restrict__ fsum, const S* z, size_t zs, S* __restrict__ y, size_t ys, const int* skip) {
   extern __shared__ __align__(16) char raw[];
   const int q = blockIdx.y;
-  if (skip && skip[8 * q]) return;
+  pdl_trigger();
   constexpr int W = H1Rec<S>::W, SM = H1Rec<S>::SM;
   S* sm = reinterpret_cast<S*>(raw);
   const int blk = blockIdx.x, L = blockDim.x / NB;
   const int n0 = blk * NB, nn = min(NB, N - n0);
   const int h0 = hptr[blk], ns = nn + hptr[blk + 1] - h0;
   const S* zq = z + (size_t)q * zs;
+  // the node records and the first step's neighbour data do not depend on
+  // the kernel before (the one that packs z)
   for (int k = threadIdx.x; k < ns; k += blockDim.x) {
     const size_t j = (size_t)W * (k < nn ? n0 + k : hnode[h0 + k - nn]);
     S* d = sm + SM * k;
+    cp_async16(d, rec + j);
     if constexpr (sizeof(S) == 4) {
       // state 0-3 | vector 0-3 | H, vector 4
-      cp_async16(d, rec + j);
-      cp_async16(d + 4, zq + j);
       cp_async4(d + 8, rec + j + 4);
-      cp_async4(d + 9, zq + j + 4);
     } else {
       // state 0-3 | H, vector 4 | vector 0-3
-      cp_async16(d, rec + j);
       cp_async16(d + 2, rec + j + 2);
       cp_async8(d + 4, rec + j + 4);
-      cp_async8(d + 5, zq + j + 4);
-      cp_async16(d + 6, zq + j);
-      cp_async16(d + 8, zq + j + 2);
     }
   }
   auto load = [&](int s, S* st, S* p) {
@@ -227,6 +223,23 @@ __global__ void __launch_bounds__(256, sizeof(S) == 4 ? 3 : 2)
   if (steps > 0) {
     e0 = nrm[at]; e1 = nrm[total + at]; e2 = nrm[2 * total + at]; hl = nrm[3 * total + at];
     sl = slot[at];
+  }
+  pdl_wait();
+  if (skip && skip[8 * q]) {
+    cp_async_wait_all();
+    return;
+  }
+  for (int k = threadIdx.x; k < ns; k += blockDim.x) {
+    const size_t j = (size_t)W * (k < nn ? n0 + k : hnode[h0 + k - nn]);
+    S* d = sm + SM * k;
+    if constexpr (sizeof(S) == 4) {
+      cp_async16(d + 4, zq + j);
+      cp_async4(d + 9, zq + j + 4);
+    } else {
+      cp_async8(d + 5, zq + j + 4);
+      cp_async16(d + 6, zq + j);
+      cp_async16(d + 8, zq + j + 2);
+    }
   }
   cp_async_wait_all();
   __syncthreads();

@@ -413,14 +413,27 @@ __global__ void k_bj_apply(int N, const S* __restrict__ dinv, const TI* __restri
 // z = D^-1 x (or D^-T x) packed for the state-based product (h1free.cuh):
 // row o2n[i] of the blocked vector, times 1/vol for the transposed product
 template <class S>
-__global__ void k_bj_pack(int N, const S* __restrict__ dinv, const S* __restrict__ x, size_t xs,
-                          const int* __restrict__ o2n, const double* __restrict__ vol, int prodT, S* __restrict__ z,
-                          size_t zs, int trans, const int* __restrict__ skip) {
+__global__ void k_bj_pack(int N, const S* __restrict__ dinv, const S* x, size_t xs, const int* __restrict__ o2n,
+                          const double* __restrict__ vol, int prodT, S* z, size_t zs, int trans, const int* skip) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x, q = blockIdx.y;
-  if (i >= N || (skip && skip[8 * q])) return;
-  double acc[5] = {0, 0, 0, 0, 0};
-  gemv_sl(dinv, sl_dblk(i), i & 31, x + (size_t)q * xs + 5 * (size_t)i, acc, trans != 0);
-  h1_put<S>(z + (size_t)q * zs, o2n[i], prodT ? 1.0 / vol[i] : 1.0, acc);
+  pdl_trigger();
+  if (i >= N) return;
+  // the inverted block and the row's place do not depend on the previous
+  // kernel
+  double a[25];
+  load_block<S>(dinv, sl_dblk(i), i & 31, a);
+  const int n = o2n[i];
+  const double sc = prodT ? 1.0 / vol[i] : 1.0;
+  pdl_wait();
+  if (skip && skip[8 * q]) return;
+  double acc[5] = {0, 0, 0, 0, 0}, xv[5];
+#pragma unroll
+  for (int k = 0; k < 5; ++k) xv[k] = (double)x[(size_t)q * xs + 5 * (size_t)i + k];
+#pragma unroll
+  for (int r = 0; r < 5; ++r)
+#pragma unroll
+    for (int k = 0; k < 5; ++k) acc[r] += (trans ? a[5 * k + r] : a[5 * r + k]) * xv[k];
+  h1_put<S>(z + (size_t)q * zs, n, sc, acc);
 }
 
 // ------------------------------------------------------------ vector ops
@@ -618,6 +631,8 @@ static void h1_geometry(aerof_gpu_ctx* c, int precision) {
                                             m.en.p, m.hptr.p, m.hnode.p, m.vol.p, f.wptr.p, f.total, nrm.p, f.slot.p,
                                             f.mrow.p);
     AEROF_LAUNCH_CHECK();
+    // complete before the solvers' overlapping launches, which read it early
+    AEROF_CUDA(cudaStreamSynchronize(s));
     ready = true;
   };
   if (precision == AEROF_PREC_FP32) go(f.nrm32, f.geo32);
@@ -1286,23 +1301,20 @@ static void h1_precond_product(aerof_gpu_ctx* c, int R, const TV* x, size_t xs, 
   {
     TimerScope t(c, AEROF_T_KSP_OTHER);
     if (precond && J.pc != AEROF_PC_ILU0) {
-      k_bj_pack<TV><<<gn, kIB, 0, s>>>(m.N, dinv, x, xs, m.o2n.p, m.vol.p, trans, zp, pz,
-                                       (trans != 0) != J.transposed ? 1 : 0, skip);
+      launch_pdl(k_bj_pack<TV>, gn, kIB, 0, s, m.N, dinv, x, xs, m.o2n.p, m.vol.p, trans, zp, pz,
+                 (trans != 0) != J.transposed ? 1 : 0, skip);
     } else {
       if (precond) prec_apply_t<TV, TV>(c, x, z, trans, R, xs, zs, skip);
-      k_h1_pack<TV, TV><<<gn, kIB, 0, s>>>(m.N, m.o2n.p, m.vol.p, trans, precond ? z : x, precond ? zs : xs, zp, pz,
-                                           skip);
+      launch_pdl(k_h1_pack<TV, TV>, gn, kIB, 0, s, m.N, m.o2n.p, m.vol.p, trans, precond ? z : x,
+                 precond ? zs : xs, zp, pz, skip);
     }
-    AEROF_LAUNCH_CHECK();
   }
   TimerScope t(c, AEROF_T_KSP_MATVEC);
   const size_t smem = h1_smem(m, J.precision);
   auto kern = trans ? k_h1_apply<TV, true> : k_h1_apply<TV, false>;
   AEROF_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  kern<<<dim3(m.nblk, R), kIB, smem, s>>>(m.N, m.NB, make_gas(c->cfg.gamma), m.n2o.p, m.hptr.p, m.hnode.p, f.wptr.p,
-                                         f.total, nrm, f.slot.p, f.mrow.p, rec, f.idt.p, m.brow.p, J.fsum.p, zp, pz,
-                                         y, ys, skip);
-  AEROF_LAUNCH_CHECK();
+  launch_pdl(kern, dim3(m.nblk, R), kIB, smem, s, m.N, m.NB, make_gas(c->cfg.gamma), m.n2o.p, m.hptr.p, m.hnode.p,
+             f.wptr.p, f.total, nrm, f.slot.p, f.mrow.p, rec, f.idt.p, m.brow.p, J.fsum.p, zp, pz, y, ys, skip);
 }
 
 // Device state of R systems with restart length m over vectors of n
@@ -1317,7 +1329,7 @@ static GsDev gs_state(aerof_gpu_ctx* c, KrylovWork& k, int R, int m, size_t n, i
   st.G = (int)std::max<size_t>(1, std::min<size_t>(need, (size_t)sms));
   st.sd = (st.size() + 1) / 2 * 2;
   k.d.ensure((size_t)R * st.sd);
-  k.part.ensure((size_t)R * 2 * (m + 1) * st.G);
+  k.part.ensure((size_t)R * (2 * (m + 1) + 1) * st.G);
   if (k.i.n < (size_t)8 * R) {
     k.i.alloc((size_t)8 * R);
     k.i.zero(c->stream);   // the tickets start at zero and re-arm themselves
@@ -1329,10 +1341,18 @@ static GsDev gs_state(aerof_gpu_ctx* c, KrylovWork& k, int R, int m, size_t n, i
   st.d = k.d.p;
   st.i = k.i.p;
   st.part = k.part.p;
+  st.norm_part = k.part.p + (size_t)R * 2 * (m + 1) * st.G;
   st.pub = (GsPub*)k.dpub;
   return st;
 }
-// dynamic shared memory of the two sweeps
+static void gs_backsolve(aerof_gpu_ctx* c, const GsDev& st, int R) {
+  const size_t smem = sizeof(double) * ((size_t)st.m + kGsL);
+  if (smem > 44 * 1024)
+    AEROF_CUDA(cudaFuncSetAttribute(k_gs_backsolve, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  k_gs_backsolve<<<R, 256, smem, c->stream>>>(st);
+  AEROF_LAUNCH_CHECK();
+}
+// dynamic shared memory of the second sweep
 static size_t gs_smem(int m) { return sizeof(double) * ((size_t)3 * (m + 1) + kGsL); }
 
 // Gram-Schmidt step j of the R systems and the Givens update.  Measured with
@@ -1342,19 +1362,20 @@ static size_t gs_smem(int m) { return sizeof(double) * ((size_t)3 * (m + 1) + kG
 // (8 to 20 iterations each) 28.7 -> 21.5 ms, where also the idle launches
 // after convergence went (kGsAhead); four sensitivities of 41^3 in one batch
 // 171 -> 102 ms, where every system took j + 2 launches per iteration and
-// the host a wait.
+// the host a wait.  On top of that and of the products from the states:
+// without a last block's fences, sums and triangular solve between the sweeps
+// and with overlapping launches, 5.13 -> 4.95 ms, 17.0 -> 15.4 ms and 101 ->
+// 98 ms (neither of the two gives it alone).
 template <class TV>
 static void gs_iteration(aerof_gpu_ctx* c, const GsDev& st, int R, size_t n, int j, TV* V, size_t vs, size_t ld,
                          const TV* W, size_t ws) {
   TimerScope t(c, AEROF_T_KSP_OTHER);
   const size_t smem = gs_smem(st.m);
   if (smem > 44 * 1024)
-    AEROF_CUDA(cudaFuncSetAttribute(k_gs_dots<TV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    AEROF_CUDA(cudaFuncSetAttribute(k_gs_update<TV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const dim3 grid(st.G, R);
-  k_gs_dots<TV><<<grid, kGsT, smem, c->stream>>>(n, j, V, vs, ld, W, ws, st);
-  AEROF_LAUNCH_CHECK();
-  k_gs_update<TV><<<grid, kGsT, sizeof(double) * (st.m + 1), c->stream>>>(n, j, V, vs, ld, W, ws, st);
-  AEROF_LAUNCH_CHECK();
+  launch_pdl(k_gs_dots<TV>, grid, kGsT, 0, c->stream, n, j, V, vs, ld, W, ws, st);
+  launch_pdl(k_gs_update<TV>, grid, kGsT, smem, c->stream, n, j, V, vs, ld, W, ws, st);
 }
 
 // The host's side of a running cycle: before the cycle, and until every
@@ -1436,8 +1457,7 @@ static void gmres_device(aerof_gpu_ctx* c, int R, const double* const* B, double
       h1_precond_product<TV>(c, R, V + (size_t)j * ld, vs, W, ld, Z, ld, trans, true, done);
       gs_iteration<TV>(c, st, R, n, j, V, vs, ld, W, ld);
     }
-    k_gs_backsolve<<<R, 32, 0, s>>>(st);
-    AEROF_LAUNCH_CHECK();
+    gs_backsolve(c, st, R);
     k_gs_combine<TV, false><<<gv, kIB, sizeof(double) * (numVec + 1), s>>>(n, V, vs, ld, st, W, ld, x);
     AEROF_LAUNCH_CHECK();
     prec_apply_t<TV, TV>(c, W, Z, trans, R, ld, ld);
@@ -1513,8 +1533,7 @@ static void fgmres_device(aerof_gpu_ctx* c, int R, const double* const* B, doubl
       for (size_t k = 0; k < rl.size(); ++k) product(xi[k], W + (size_t)rl[k] * ld);
       gs_iteration<double>(c, st, R, n, j, V, vs, ld, W, ld);
     }
-    k_gs_backsolve<<<R, 32, 0, s>>>(st);
-    AEROF_LAUNCH_CHECK();
+    gs_backsolve(c, st, R);
     k_gs_combine<double, true><<<gv, kIB, sizeof(double) * (numVec + 1), s>>>(n, Z, zs, ld, st, nullptr, 0, x);
     AEROF_LAUNCH_CHECK();
     AEROF_CUDA(cudaStreamSynchronize(s));

@@ -17,8 +17,10 @@
 // the factor sig_i = 1/norm beside them (v_i = sig_i * stored), so no pass
 // normalises them.  Dots, norms and the Hessenberg system are FP64 for
 // either storage type; the projected vector is rounded to it once.
-// Reductions run over a fixed grid in a fixed order (no atomics on values);
-// the block that finishes last does the scalar work of the step.
+// Reductions run over a fixed grid in a fixed order (no atomics on values):
+// every block of the second sweep forms the coefficients from the first
+// sweep's partial sums, and its block that finishes last does the Givens
+// update.  The launches of an iteration overlap (launch_pdl).
 #pragma once
 
 #include "common.cuh"
@@ -43,7 +45,8 @@ struct GsDev {
   double* d;
   size_t sd;
   int* i;
-  double* part;                  // [R][2 (m + 1)][G] partial sums
+  double* part;                  // [R][2 (m + 1)][G] partial sums of the dot products
+  double* norm_part;             // [R][G] of the norm
   GsPub* pub;
   int m, G;
   __host__ __device__ size_t oL() const { return (size_t)(m + 1) * m; }
@@ -51,8 +54,7 @@ struct GsDev {
   __host__ __device__ size_t oG() const { return oCs() + 2 * (size_t)m; }
   __host__ __device__ size_t oY() const { return oG() + m + 1; }
   __host__ __device__ size_t oSig() const { return oY() + m; }
-  __host__ __device__ size_t oH() const { return oSig() + m + 1; }
-  __host__ __device__ size_t oScal() const { return oH() + m + 1; }   // l2res, target
+  __host__ __device__ size_t oScal() const { return oSig() + m + 1; }   // l2res, target
   __host__ __device__ size_t size() const { return oScal() + 2; }
 };
 
@@ -100,12 +102,20 @@ __device__ __forceinline__ bool last_block(int* ticket) {
   return last;
 }
 
-// vals[v] = sum of part[v][0, G) for v < nv, one warp per value
+// vals[v] = sum of part[v][0, G) for v < nv, one warp per value (eight loads
+// in flight per lane: G is at most a few hundred)
 __device__ __forceinline__ void sum_partials(const double* part, int G, int nv, double* vals) {
   const int lane = threadIdx.x & 31;
   for (int v = threadIdx.x >> 5; v < nv; v += blockDim.x >> 5) {
+    const double* p = part + (size_t)v * G;
     double t = 0.0;
-    for (int k = lane; k < G; k += 32) t += __ldcg(part + (size_t)v * G + k);
+    for (int k0 = lane; k0 < G; k0 += 256) {
+      double x[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) x[u] = k0 + 32 * u < G ? __ldcg(p + k0 + 32 * u) : 0.0;
+#pragma unroll
+      for (int u = 0; u < 8; ++u) t += x[u];
+    }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
     if (lane == 0) vals[v] = t;
@@ -179,28 +189,30 @@ __global__ void __launch_bounds__(kGsT) k_gs_start(size_t n, VecIn B, VecOut X, 
   }
 }
 
-// Sweep 1 of iteration j: v_i.w and v_i.v_j for every i <= j (eight basis
-// vectors per pass over w and v_j, so that a thread has ten 16-byte loads in
-// flight), then the coefficients h by the triangular solve.
+// Sweep 1 of iteration j: partial sums of v_i.w and v_i.v_j for every i <= j
+// (eight basis vectors per pass over w and v_j, so that a thread has ten
+// 16-byte loads in flight).  Their totals and the coefficients are formed by
+// every block of sweep 2: a last block that did it here put its fences, its
+// reads and the solve in series between the sweeps (~10 us per iteration).
 template <class TV>
-__global__ void __launch_bounds__(kGsT, 1) k_gs_dots(size_t n, int j, const TV* __restrict__ V, size_t vs, size_t ld,
-                                                     const TV* __restrict__ W, size_t ws, GsDev st) {
-  extern __shared__ double sh[];   // vals [2 (m + 1)], a [m + 1], L
+__global__ void __launch_bounds__(kGsT, 1) k_gs_dots(size_t n, int j, const TV* V, size_t vs, size_t ld,
+                                                     const TV* W, size_t ws, GsDev st) {
   __shared__ double red[(kGsT / 32) * 16];
   const int q = blockIdx.y;
-  int* ist = st.i + 8 * q;
-  if (ist[1]) return;
+  pdl_trigger();
+  pdl_wait();
+  if (st.i[8 * q + 1]) return;
   using VT = typename Vec16<TV>::T;
   constexpr int E = Vec16<TV>::W, U = 8;
-  const TV* __restrict__ Vq = V + (size_t)q * vs;
-  const TV* __restrict__ w = W + (size_t)q * ws;
-  const TV* __restrict__ vj = Vq + (size_t)j * ld;
+  const TV* Vq = V + (size_t)q * vs;
+  const TV* w = W + (size_t)q * ws;
+  const TV* vj = Vq + (size_t)j * ld;
   double* part = st.part + (size_t)q * 2 * (st.m + 1) * st.G;
   const size_t nv = n / E, t0 = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   const size_t stride = (size_t)gridDim.x * blockDim.x;
   for (int i0 = 0; i0 <= j; i0 += U) {
     const int c = min(U, j + 1 - i0);
-    const TV* __restrict__ Vi = Vq + (size_t)i0 * ld;
+    const TV* Vi = Vq + (size_t)i0 * ld;
     double s[2 * U];
 #pragma unroll
     for (int u = 0; u < 2 * U; ++u) s[u] = 0.0;
@@ -234,40 +246,45 @@ __global__ void __launch_bounds__(kGsT, 1) k_gs_dots(size_t n, int j, const TV* 
     }
     block_sums<2 * U>(s, 2 * c, red, part + (size_t)2 * i0 * st.G + blockIdx.x, st.G);
   }
-  if (!last_block(ist + 6)) return;
+}
+
+// The coefficients of iteration j in a[0..j] (shared memory), from the
+// partial sums: the block computes them whole, so every block has the same
+// ones without a grid-wide step.  Block 0 keeps row j of L.  sh: vals
+// [2 (m + 1)], a [m + 1], L (packed rows 1..j while they fit).
+__device__ __forceinline__ double* gs_coefficients(const GsDev& st, int q, int j, double* sh) {
   double* vals = sh;
   double* a = vals + 2 * (st.m + 1);
   double* sL = a + st.m + 1;
   double* d = st.d + (size_t)q * st.sd;
   double* L = d + st.oL();
   const double* sig = d + st.oSig();
-  const bool cached = j * (j + 1) / 2 <= kGsL;   // rows 1..j, packed
-  sum_partials(part, st.G, 2 * (j + 1), vals);
+  const bool cached = j * (j + 1) / 2 <= kGsL;
   const double sj = sig[j];
+  if (cached)
+    for (int i = 1 + (int)(threadIdx.x >> 5); i < j; i += blockDim.x >> 5)
+      for (int k = threadIdx.x & 31; k < i; k += 32) sL[i * (i - 1) / 2 + k] = L[(size_t)i * st.m + k];
+  sum_partials(st.part + (size_t)q * 2 * (st.m + 1) * st.G, st.G, 2 * (j + 1), vals);
   for (int k = threadIdx.x; k <= j; k += blockDim.x) {
     const double sk = sig[k];
     a[k] = sj * sk * vals[2 * k];
     if (k < j) {
       const double l = sj * sk * vals[2 * k + 1];
-      L[(size_t)j * st.m + k] = l;
-      if (cached) sL[j * (j - 1) / 2 + k] = l;
+      vals[2 * k + 1] = l;
+      if (blockIdx.x == 0) L[(size_t)j * st.m + k] = l;
     }
   }
-  if (cached)
-    for (int i = 1 + (int)(threadIdx.x >> 5); i < j; i += blockDim.x >> 5)
-      for (int k = threadIdx.x & 31; k < i; k += 32) sL[i * (i - 1) / 2 + k] = L[(size_t)i * st.m + k];
-  __threadfence_block();
   __syncthreads();
   if (threadIdx.x < 32) {
     for (int k = 0; k < j; ++k) {
       const double hk = a[k];
       for (int i = k + 1 + (int)threadIdx.x; i <= j; i += 32)
-        a[i] -= (cached ? sL[i * (i - 1) / 2 + k] : L[(size_t)i * st.m + k]) * hk;
+        a[i] -= (i == j ? vals[2 * k + 1] : (cached ? sL[i * (i - 1) / 2 + k] : L[(size_t)i * st.m + k])) * hk;
       __syncwarp();
     }
   }
   __syncthreads();
-  for (int k = threadIdx.x; k <= j; k += blockDim.x) d[st.oH() + k] = a[k];
+  return a;
 }
 
 // Sweep 2 of iteration j: v_{j+1} = w - sum_i h_i v_i (FP64 per element,
@@ -275,24 +292,28 @@ __global__ void __launch_bounds__(kGsT, 1) k_gs_dots(size_t n, int j, const TV* 
 // column, written with explicitly rounded operations (the host loop's
 // arithmetic), and the step's result for the host.
 template <class TV>
-__global__ void __launch_bounds__(kGsT, 1) k_gs_update(size_t n, int j, TV* __restrict__ V, size_t vs, size_t ld,
-                                                       const TV* __restrict__ W, size_t ws, GsDev st) {
-  extern __shared__ double sh[];   // c [m + 1]: h_i sig_i, then the column
+__global__ void __launch_bounds__(kGsT, 1) k_gs_update(size_t n, int j, TV* V, size_t vs, size_t ld,
+                                                       const TV* W, size_t ws, GsDev st) {
+  extern __shared__ double sh[];   // see gs_coefficients
   __shared__ double red[kGsT / 32];
   __shared__ double nrm[1];
   const int q = blockIdx.y;
   int* ist = st.i + 8 * q;
+  pdl_trigger();
+  pdl_wait();
   if (ist[1]) return;
   using VT = typename Vec16<TV>::T;
   constexpr int E = Vec16<TV>::W, U = 8;
   double* d = st.d + (size_t)q * st.sd;
   const double* sig = d + st.oSig();
-  for (int k = threadIdx.x; k <= j; k += blockDim.x) sh[k] = d[st.oH() + k] * sig[k];
   const double sj = sig[j];
+  const double* hcol = gs_coefficients(st, q, j, sh);
+  double* cf = sh;                 // h_i sig_i, over the finished sums
+  for (int k = threadIdx.x; k <= j; k += blockDim.x) cf[k] = hcol[k] * sig[k];
   __syncthreads();
-  const TV* __restrict__ Vq = V + (size_t)q * vs;
-  const TV* __restrict__ w = W + (size_t)q * ws;
-  TV* __restrict__ vn = V + (size_t)q * vs + (size_t)(j + 1) * ld;
+  const TV* Vq = V + (size_t)q * vs;
+  const TV* w = W + (size_t)q * ws;
+  TV* vn = V + (size_t)q * vs + (size_t)(j + 1) * ld;
   const size_t nv = n / E, t0 = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   const size_t stride = (size_t)gridDim.x * blockDim.x;
   double s = 0.0;
@@ -304,7 +325,7 @@ __global__ void __launch_bounds__(kGsT, 1) k_gs_update(size_t n, int j, TV* __re
     for (int k = 0; k < E; ++k) acc[k] = sj * (double)wp[k];
     for (int i0 = 0; i0 <= j; i0 += U) {
       const int c = min(U, j + 1 - i0);
-      const TV* __restrict__ Vi = Vq + (size_t)i0 * ld;
+      const TV* Vi = Vq + (size_t)i0 * ld;
       VT x[U];
 #pragma unroll
       for (int u = 0; u < U; ++u)
@@ -313,7 +334,7 @@ __global__ void __launch_bounds__(kGsT, 1) k_gs_update(size_t n, int j, TV* __re
       for (int u = 0; u < U; ++u)
         if (u < c) {
           const TV* xp = reinterpret_cast<const TV*>(&x[u]);
-          const double h = sh[i0 + u];
+          const double h = cf[i0 + u];
 #pragma unroll
           for (int k = 0; k < E; ++k) acc[k] -= h * (double)xp[k];
         }
@@ -327,79 +348,112 @@ __global__ void __launch_bounds__(kGsT, 1) k_gs_update(size_t n, int j, TV* __re
   }
   for (size_t p = nv * E + t0; p < n; p += stride) {
     double acc = sj * (double)w[p];
-    for (int i = 0; i <= j; ++i) acc -= sh[i] * (double)Vq[(size_t)i * ld + p];
+    for (int i = 0; i <= j; ++i) acc -= cf[i] * (double)Vq[(size_t)i * ld + p];
     const TV r = (TV)acc;
     vn[p] = r;
     s += (double)r * (double)r;
   }
-  double* part = st.part + (size_t)q * 2 * (st.m + 1) * st.G;
+  // (not over the dot products' partials, which other blocks may still read)
+  double* part = st.norm_part + (size_t)q * st.G;
   block_sums<1>(&s, 1, red, part + blockIdx.x, st.G);
   if (!last_block(ist + 7)) return;
   sum_partials(part, st.G, 1, nrm);
-  for (int k = threadIdx.x; k <= j; k += blockDim.x) sh[k] = d[st.oH() + k];
-  __syncthreads();
-  if (threadIdx.x != 0) return;
-  double* hc = sh;
+  // the rotations and the state in shared memory before the serial part
   double* cs = d + st.oCs();
   double* g = d + st.oG();
   double* H = d;
   const int m = st.m;
-  const double hj1 = __dsqrt_rn(nrm[0]);
-  const bool breakdown = hj1 == 0.0;
-  double cur = hc[0];
-  for (int i = 0; i < j; ++i) {
-    const double c0 = cs[2 * i], c1 = cs[2 * i + 1];
-    const double a = cur, bb = hc[i + 1];
-    H[(size_t)i * m + j] = __dadd_rn(__dmul_rn(c1, a), __dmul_rn(c0, bb));
-    cur = __dadd_rn(__dmul_rn(-c0, a), __dmul_rn(c1, bb));
+  double* scs = sh;                // [2 j], over the coefficients
+  double* col = const_cast<double*>(hcol);
+  for (int k = threadIdx.x; k < 2 * j; k += blockDim.x) scs[k] = cs[k];
+  __shared__ double sg[3];
+  __shared__ int si[2];
+  if (threadIdx.x == 0) {
+    sg[0] = g[j];
+    sg[1] = d[st.oScal()];
+    sg[2] = d[st.oScal() + 1];
+    si[0] = ist[0];
+    si[1] = ist[4];
   }
-  double c0, c1;
-  if (__dmul_rn(cur, cur) == 0.0) {
-    c1 = 0.0;
-    c0 = 1.0;
-  } else {
-    const double coef = __ddiv_rn(1.0, __dsqrt_rn(__dadd_rn(__dmul_rn(cur, cur), __dmul_rn(hj1, hj1))));
-    c1 = __dmul_rn(__dsqrt_rn(__dmul_rn(cur, cur)), coef);
-    c0 = __ddiv_rn(__dmul_rn(c1, hj1), cur);
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    const double hj1 = __dsqrt_rn(nrm[0]);
+    const bool breakdown = hj1 == 0.0;
+    double cur = col[0];
+    for (int i = 0; i < j; ++i) {
+      const double c0 = scs[2 * i], c1 = scs[2 * i + 1];
+      const double a = cur, bb = col[i + 1];
+      col[i] = __dadd_rn(__dmul_rn(c1, a), __dmul_rn(c0, bb));
+      cur = __dadd_rn(__dmul_rn(-c0, a), __dmul_rn(c1, bb));
+    }
+    double c0, c1;
+    if (__dmul_rn(cur, cur) == 0.0) {
+      c1 = 0.0;
+      c0 = 1.0;
+    } else {
+      const double coef = __ddiv_rn(1.0, __dsqrt_rn(__dadd_rn(__dmul_rn(cur, cur), __dmul_rn(hj1, hj1))));
+      c1 = __dmul_rn(__dsqrt_rn(__dmul_rn(cur, cur)), coef);
+      c0 = __ddiv_rn(__dmul_rn(c1, hj1), cur);
+    }
+    col[j] = __dadd_rn(__dmul_rn(c1, cur), __dmul_rn(c0, hj1));
+    H[(size_t)(j + 1) * m + j] = 0.0;
+    const double gj = sg[0], gj1 = __dmul_rn(-c0, gj);
+    g[j + 1] = gj1;
+    g[j] = __dmul_rn(c1, gj);
+    cs[2 * j] = c0;
+    cs[2 * j + 1] = c1;
+    d[st.oSig() + j + 1] = breakdown ? 0.0 : 1.0 / hj1;
+    const int iter = si[0] + 1;
+    double l2res = sg[1];
+    bool done = breakdown;
+    if (!breakdown) {
+      l2res = fabs(gj1);
+      done = l2res <= sg[2] || iter >= si[1];
+    }
+    d[st.oScal()] = l2res;
+    ist[0] = iter;
+    ist[2] = j;
+    ist[5] = breakdown;
+    ist[1] = done;
+    publish(st.pub + q, j + 1, done, iter, l2res);
   }
-  H[(size_t)j * m + j] = __dadd_rn(__dmul_rn(c1, cur), __dmul_rn(c0, hj1));
-  H[(size_t)(j + 1) * m + j] = 0.0;
-  const double gj = g[j], gj1 = __dmul_rn(-c0, gj);
-  g[j + 1] = gj1;
-  g[j] = __dmul_rn(c1, gj);
-  cs[2 * j] = c0;
-  cs[2 * j + 1] = c1;
-  d[st.oSig() + j + 1] = breakdown ? 0.0 : 1.0 / hj1;
-  const int iter = ist[0] + 1;
-  double l2res = d[st.oScal()];
-  bool done = breakdown;
-  if (!breakdown) {
-    l2res = fabs(gj1);
-    done = l2res <= d[st.oScal() + 1] || iter >= ist[4];
-  }
-  d[st.oScal()] = l2res;
-  ist[0] = iter;
-  ist[2] = j;
-  ist[5] = breakdown;
-  ist[1] = done;
-  publish(st.pub + q, j + 1, done, iter, l2res);
+  __syncthreads();
+  for (int i = threadIdx.x; i <= j; i += blockDim.x) H[(size_t)i * m + j] = col[i];
 }
 
-// back substitution (KspSolver.C:966-982) of the cycle, one thread per
-// system: y from the rotated Hessenberg matrix and g
-__global__ void k_gs_backsolve(GsDev st) {
+// back substitution (KspSolver.C:966-982) of the cycle, one block per
+// system: y from the rotated Hessenberg matrix (staged, row by row of the
+// upper triangle) and g; lane i subtracts column k's product as y_k is known
+__global__ void __launch_bounds__(256) k_gs_backsolve(GsDev st) {
+  extern __shared__ double sh[];   // g [m], H (packed columns while they fit)
   const int q = blockIdx.x;
-  if (threadIdx.x != 0) return;
   const int* ist = st.i + 8 * q;
   if (!ist[3]) return;
   double* d = st.d + (size_t)q * st.sd;
-  double *H = d, *g = d + st.oG(), *y = d + st.oY();
-  const int j = ist[2];
-  for (int i = j; i >= 0; --i) {
-    double yi = g[i];
-    for (int k = j; k >= i + 1; --k) yi = __dsub_rn(yi, __dmul_rn(H[(size_t)i * st.m + k], y[k]));
-    y[i] = __ddiv_rn(yi, H[(size_t)i * st.m + i]);
+  const double *H = d, *g = d + st.oG();
+  double* y = d + st.oY();
+  const int j = ist[2], n = j + 1;
+  double *sy = sh, *sH = sh + st.m;
+  const bool cached = n * (n + 1) / 2 <= kGsL;
+  for (int i = threadIdx.x; i < n; i += blockDim.x) sy[i] = g[i];
+  if (cached)
+    for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
+      const int i = e / n, k = e - n * i;
+      if (i <= k) sH[k * (k + 1) / 2 + i] = H[(size_t)i * st.m + k];
+    }
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    auto h = [&](int i, int k) { return cached ? sH[k * (k + 1) / 2 + i] : H[(size_t)i * st.m + k]; };
+    for (int k = j; k >= 0; --k) {
+      if (threadIdx.x == 0) sy[k] = __ddiv_rn(sy[k], h(k, k));
+      __syncwarp();
+      const double yk = sy[k];
+      for (int i = (int)threadIdx.x; i < k; i += 32) sy[i] = __dsub_rn(sy[i], __dmul_rn(h(i, k), yk));
+      __syncwarp();
+    }
   }
+  __syncthreads();
+  for (int i = threadIdx.x; i < n; i += blockDim.x) y[i] = sy[i];
 }
 
 // out = sum_i y_i sig_i Z_i over the cycle's columns: stored as TV (ADD
