@@ -171,7 +171,7 @@ __global__ void k_d_node_residual(int N, int E, int F, Gas g, const double* __re
 // of k_fv_blocked in dual arithmetic from staged records.  The gathered form
 // above (dual numbers interleaved in the caller's numbering, geometry
 // recomputed per node and edge) remains for meshes whose blocks do not fit
-// in shared memory: J v and (dR/dX) Xdot at 61^3 2.67 ms there, 1.13 ms here.
+// in shared memory.
 
 // D2[n] = (dV, dX): dV = (dV/dU) v (VarFcnSGEuler.h:307-327; v null: 0), dX =
 // Xdot, or the coordinates when Xdot is null (the records whose gradients
@@ -813,6 +813,20 @@ __device__ __forceinline__ Dual5 dsqrt(const Dual5& a) {
   return r;
 }
 __device__ __forceinline__ double vof(const Dual5& a) { return a.v; }
+__device__ __forceinline__ Dual5 rcp_(const Dual5& a) {
+  Dual5 r(rcp_(a.v));
+  const double h = -(r.v * r.v);
+#pragma unroll
+  for (int k = 0; k < 5; ++k) r.d[k] = h * a.d[k];
+  return r;
+}
+__device__ __forceinline__ Dual5 rsqrt_(const Dual5& a) {
+  Dual5 r(rsqrt_(a.v));
+  const double h = -0.5 * r.v * (r.v * r.v);
+#pragma unroll
+  for (int k = 0; k < 5; ++k) r.d[k] = h * a.d[k];
+  return r;
+}
 
 // Face flux cotangents, g_V += (d flux / d V)^T lam, the five state
 // directions in one forward-mode evaluation

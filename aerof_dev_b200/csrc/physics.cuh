@@ -95,13 +95,14 @@ template <class T> AEROF_HD T sel(bool c, T a, T b) { return c ? a : b; }
 
 // ------------------------------------------------------------ gas model
 struct Gas {
-  double gam, gam1, invgam1;
+  double gam, gam1, invgam1, invgam;
 };
 AEROF_HD Gas make_gas(double gam) {
   Gas g;
   g.gam = gam;
   g.gam1 = gam - 1.0;
   g.invgam1 = 1.0 / g.gam1;
+  g.invgam = 1.0 / gam;
   return g;
 }
 
@@ -245,31 +246,58 @@ AEROF_HD void roe_flux(const Gas& g, TN n0, TN n1, TN n2, const T* Ug, const T* 
 
 // boundflux5.f:1-111 (type 0, sig = 0): Steger-Warming far-field flux
 // A+(V) U(V) + A-(V) Ub with V primitive and Ub conservative.
-template <class T>
+// One reciprocal and two reciprocal square roots in place of eleven divisions
+// and two roots: a boundary node's faces are a serial chain.  EXACT keeps the
+// divisions and roots, for the forward differences of face_jac: their
+// increment is 1e-6 |V_k|, which for a velocity component near zero turns a
+// changed last bit into a visible change of the block.
+template <bool EXACT = false, class T>
 AEROF_HD void sw_flux(const Gas& g, T vnx, T vny, T vnz, const T* ua, const double* ub, T* flux) {
-  const double gam = g.gam, gam1 = g.gam1;
-  T cap = dsqrt(vnx * vnx + vny * vny + vnz * vnz);
-  T capd1 = vnx / cap, capd2 = vny / cap, capd3 = vnz / cap;
+  const double gam = g.gam, gam1 = g.gam1, ig = g.invgam, ig1 = g.invgam1;
+  T s2 = vnx * vnx + vny * vny + vnz * vnz;
+  T icap, cap, capd1, capd2, capd3;
+  if constexpr (EXACT) {
+    cap = dsqrt(s2);
+    capd1 = vnx / cap; capd2 = vny / cap; capd3 = vnz / cap;
+  } else {
+    icap = rsqrt_(s2);
+    cap = s2 * icap;
+    capd1 = vnx * icap; capd2 = vny * icap; capd3 = vnz * icap;
+  }
   T ro = ua[0];
-  T usro = 1.0 / ro;
+  T usro;
+  if constexpr (EXACT) usro = 1.0 / ro;
+  else usro = rcp_(ro);
   T u = ua[1], v = ua[2], w = ua[3];
   T vit = u * u + v * v + w * w;
   T pm = ua[4];
-  T rhoE = pm / gam1 + 0.5 * ro * vit;
   T c2 = gam * pm * usro;
-  T c = dsqrt(c2);
-  T usc = 1.0 / c;
-  T cc = 0.5 * vit + c2 / gam1;
+  T rhoE, usc, c, cc;
+  if constexpr (EXACT) {
+    rhoE = pm / gam1 + 0.5 * ro * vit;
+    c = dsqrt(c2);
+    usc = 1.0 / c;
+    cc = 0.5 * vit + c2 / gam1;
+  } else {
+    rhoE = ig1 * pm + 0.5 * ro * vit;
+    usc = rsqrt_(c2);
+    c = c2 * usc;
+    cc = 0.5 * vit + ig1 * c2;
+  }
   T unx = capd1 * u + capd2 * v + capd3 * w;
   T l1 = cap * unx, l4 = cap * (unx + c), l5 = cap * (unx - c);
   T vp1 = tmax0(l1), vp4 = tmax0(l4), vp5 = tmax0(l5);
   T vpp = vp4 + vp5;
   T vpm = vp4 - vp5;
-  T fgp0 = (gam1 * ro * vp1 + 0.5 * ro * vpp) / gam;
+  T fgp0 = gam1 * ro * vp1 + 0.5 * ro * vpp;
+  if constexpr (EXACT) fgp0 = fgp0 / gam;
+  else fgp0 = ig * fgp0;
   T fgp1 = fgp0 * u + 0.5 * pm * usc * capd1 * vpm;
   T fgp2 = fgp0 * v + 0.5 * pm * usc * capd2 * vpm;
   T fgp3 = fgp0 * w + 0.5 * pm * usc * capd3 * vpm;
-  T fgp4 = 0.5 * ((gam1 / gam) * ro * vit * (vp1 - 0.5 * vpp) + rhoE * vpp + ro * unx * c * vpm / gam);
+  T fgp4;
+  if constexpr (EXACT) fgp4 = 0.5 * ((gam1 / gam) * ro * vit * (vp1 - 0.5 * vpp) + rhoE * vpp + ro * unx * c * vpm / gam);
+  else fgp4 = 0.5 * ((gam1 * ig) * ro * vit * (vp1 - 0.5 * vpp) + rhoE * vpp + ig * (ro * unx * c * vpm));
   vp1 = tmin0(l1); vp4 = tmin0(l4); vp5 = tmin0(l5);
   vpp = vp1 - 0.5 * (vp4 + vp5);
   vpm = 0.5 * (vp5 - vp4);
@@ -424,14 +452,14 @@ AEROF_HD void face_jac(const Gas& g, int code, double nx, double ny, double nz, 
   } else {
     const double eps0 = 1.e-6;
     double f0[5], fe[5], Ve[5];
-    sw_flux(g, nx, ny, nz, V, Ub, f0);
+    sw_flux<true>(g, nx, ny, nz, V, Ub, f0);
     for (int k = 0; k < 5; ++k) {
 #pragma unroll
       for (int q = 0; q < 5; ++q) Ve[q] = V[q];
       double eps = (fabs(V[k]) < 1.e-10) ? eps0 : eps0 * V[k];
       double inveps = 1.0 / eps;
       Ve[k] += eps;
-      sw_flux(g, nx, ny, nz, Ve, Ub, fe);
+      sw_flux<true>(g, nx, ny, nz, Ve, Ub, fe);
 #pragma unroll
       for (int j = 0; j < 5; ++j) dfdV[5 * j + k] = (fe[j] - f0[j]) * inveps;
     }

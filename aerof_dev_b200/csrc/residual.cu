@@ -447,6 +447,40 @@ __global__ void k_edge_flux(int E, Gas g, int rec, double beta, int failsafe, co
   for (int k = 0; k < 5; ++k) flux[(size_t)k * E + l] = f[k];
 }
 
+// Boundary subface fluxes as extra blocks of the edge sweep's launch: item
+// 3 f + l is node l of face f, its flux with normal n_f / 3
+// (FaceTriaCore.C:288-308) from the blocked records into fbuf[3F][5].  In a
+// launch of their own (thread per face, its three nodes one after the
+// other) they took 8 us of a 47^3 residual and 17 us at 101^3.
+struct FaceArgs {
+  int F;
+  const double* Ub;
+  const int *faces, *fcode;
+  const double* fn;
+  const int* o2n;
+  double* fbuf;
+};
+constexpr int kFaceItems = 4;  // per thread
+__device__ __forceinline__ void face_items(const Gas& g, const FaceArgs& fa, const double* __restrict__ P, int blk) {
+  const double third = 1.0 / 3.0;
+  double Ub[5];
+#pragma unroll
+  for (int k = 0; k < 5; ++k) Ub[k] = fa.Ub[k];
+  for (int i = 0; i < kFaceItems; ++i) {
+    const int e = (blk * kFaceItems + i) * blockDim.x + threadIdx.x;
+    if (e >= 3 * fa.F) return;
+    const int f = e / 3;
+    const double* v = P + 8 * (size_t)fa.o2n[fa.faces[e]];
+    double V[5], ff[5];
+#pragma unroll
+    for (int k = 0; k < 5; ++k) V[k] = v[k];
+    face_flux(g, fa.fcode[f], third * fa.fn[f], third * fa.fn[(size_t)fa.F + f], third * fa.fn[2 * (size_t)fa.F + f],
+              V, Ub, ff);
+#pragma unroll
+    for (int k = 0; k < 5; ++k) fa.fbuf[5 * (size_t)e + k] = ff[k];
+  }
+}
+
 // BLOCKED organisation: one thread block per NB consecutive (Morton
 // ordered) nodes.  Phase 0: the node records (V, X) and gradients of the
 // block's nodes and of its forward halo (second endpoints of the block's
@@ -469,8 +503,12 @@ __global__ void __launch_bounds__(THREADS, MINB)
                                                     const int* __restrict__ lidx, const int* __restrict__ xslot,
                                                     double* __restrict__ part, double* __restrict__ spill,
                                                     int* __restrict__ tag, int* __restrict__ counters,
-                                                    const int* __restrict__ blist) {
+                                                    const int* __restrict__ blist, int nmain, FaceArgs fa) {
   extern __shared__ double sm[];
+  if ((int)blockIdx.x >= nmain) {
+    face_items(g, fa, P, (int)blockIdx.x - nmain);
+    return;
+  }
   const int blk = blist ? blist[blockIdx.x] : blockIdx.x;
   const int n0 = blk * NB;
   const int nn = min(NB, N - n0);
@@ -590,17 +628,23 @@ __global__ void __launch_bounds__(THREADS, MINB)
   }
 }
 
-// Node n's flux sum in the blocked numbering: block-local part, minus the
-// spilled fluxes of incoming block-crossing edges, plus the node's boundary
-// subface fluxes (face order; FACES: evaluated here from the node's own
-// state, the operations of k_face_flux, instead of read from fbuf).
-template <bool FACES>
-__device__ __forceinline__ void node_sum(int n, const Gas& g, const double* __restrict__ part,
-                                         const int* __restrict__ xin_ptr, const double* __restrict__ spill,
-                                         const int* __restrict__ bnf_ptr, const int* __restrict__ bnf_ent,
-                                         const double* __restrict__ fbuf, int F, const double* __restrict__ Ub0,
-                                         const int* __restrict__ fcode, const double* __restrict__ fn,
-                                         const double* P2, double* acc) {
+// Node assembly of the blocks blist[0, nlist) in a stage of the overlapped
+// residual, thread per node: block-local part, minus the spilled fluxes of
+// incoming block-crossing edges, plus the boundary subface fluxes evaluated
+// from the node's own state (face order), times 1/ctrlVol; written to R in
+// the caller's numbering through n2o.
+__global__ void k_fv_nodes_list(int N, Gas g, const int* __restrict__ n2o, const double* __restrict__ part,
+                                const int* __restrict__ xin_ptr, const double* __restrict__ spill,
+                                const int* __restrict__ bnf_ptr, const int* __restrict__ bnf_ent, int F,
+                                const double* __restrict__ Ub0, const int* __restrict__ fcode,
+                                const double* __restrict__ fn, const double* __restrict__ P2,
+                                const double* __restrict__ vol2, double* __restrict__ R,
+                                const int* __restrict__ blist, int nlist, int NB) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t / NB >= nlist) return;
+  const int n = blist[t / NB] * NB + t % NB;
+  if (n >= N) return;
+  double acc[5];
 #pragma unroll
   for (int c = 0; c < 5; ++c) acc[c] = part[5 * (size_t)n + c];
   for (int k = xin_ptr[n]; k < xin_ptr[n + 1]; ++k) {
@@ -609,70 +653,31 @@ __device__ __forceinline__ void node_sum(int n, const Gas& g, const double* __re
     for (int c = 0; c < 5; ++c) acc[c] -= sp[c];
   }
   const int q0 = bnf_ptr[n], q1 = bnf_ptr[n + 1];
-  if (FACES) {
-    if (q0 < q1) {
-      const double third = 1.0 / 3.0;
-      double V[5], Ub[5];
+  if (q0 < q1) {
+    const double third = 1.0 / 3.0;
+    double V[5], Ub[5];
 #pragma unroll
-      for (int k = 0; k < 5; ++k) { V[k] = P2[8 * (size_t)n + k]; Ub[k] = Ub0[k]; }
-      for (int q = q0; q < q1; ++q) {
-        const int f = bnf_ent[q] / 3;
-        double ff[5];
-        face_flux(g, fcode[f], third * fn[f], third * fn[(size_t)F + f], third * fn[2 * (size_t)F + f], V, Ub, ff);
-#pragma unroll
-        for (int c = 0; c < 5; ++c) acc[c] += ff[c];
-      }
-    }
-  } else {
+    for (int k = 0; k < 5; ++k) { V[k] = P2[8 * (size_t)n + k]; Ub[k] = Ub0[k]; }
     for (int q = q0; q < q1; ++q) {
-      const double* ff = fbuf + 5 * (size_t)bnf_ent[q];
+      const int f = bnf_ent[q] / 3;
+      double ff[5];
+      face_flux(g, fcode[f], third * fn[f], third * fn[(size_t)F + f], third * fn[2 * (size_t)F + f], V, Ub, ff);
 #pragma unroll
       for (int c = 0; c < 5; ++c) acc[c] += ff[c];
     }
   }
-}
-
-// BLOCKED organisation, per node in the blocked numbering: block-local sum,
-// minus the spilled fluxes of incoming block-crossing edges, plus the
-// node's boundary subface fluxes (face order), times 1/ctrlVol; written to
-// R in the caller's numbering through n2o.  Partial sums, spills and
-// subface fluxes are read in node order (coalesced); the caller-order
-// variant that gathers them through o2n measured slower.
-template <bool FACES>
-__global__ void k_fv_nodes_b(int N, Gas g, const int* __restrict__ n2o, const double* __restrict__ part,
-                             const int* __restrict__ xin_ptr, const double* __restrict__ spill,
-                             const int* __restrict__ bnf_ptr, const int* __restrict__ bnf_ent,
-                             const double* __restrict__ fbuf, int F, const double* __restrict__ Ub0,
-                             const int* __restrict__ fcode, const double* __restrict__ fn,
-                             const double* __restrict__ P2, const double* __restrict__ vol2, double* __restrict__ R,
-                             const int* __restrict__ blist, int nlist, int NB, int* __restrict__ cnt,
-                             volatile int* __restrict__ pub) {
-  int n = blockIdx.x * blockDim.x + threadIdx.x;
-  // the edge fluxes are complete: their unphysical count goes to the host's
-  // page-locked word, and the counter back to zero for the next call
-  if (pub && n == 0) {
-    *pub = *cnt;
-    *cnt = 0;
-  }
-  if (blist) {
-    // the nodes of blocks blist[0, nlist)
-    const int i = n / NB;
-    if (i >= nlist) return;
-    n = blist[i] * NB + n % NB;
-  }
-  if (n >= N) return;
-  double acc[5];
-  node_sum<FACES>(n, g, part, xin_ptr, spill, bnf_ptr, bnf_ent, fbuf, F, Ub0, fcode, fn, P2, acc);
   const double invcv = 1.0 / vol2[n];
   const size_t o = (size_t)n2o[n];
 #pragma unroll
   for (int c = 0; c < 5; ++c) R[5 * o + c] = acc[c] * invcv;
 }
 
-// The assembly of k_fv_nodes_b<false> with five lanes per node, lane c
-// summing component c: a warp's loads of the partial sums, the spilled
+// Node assembly of the blocked residual: the sums of k_fv_nodes_list in the
+// same order, the subface fluxes read from fbuf, with five lanes per node,
+// lane c summing component c: a warp's loads of the partial sums, the spilled
 // fluxes and the subface fluxes are contiguous, and four spills are in
-// flight per lane.  Same sums in the same order.
+// flight per lane.  The first thread hands the unphysical count to the host
+// (pub) and re-arms the counter: the edge sweep is complete.
 __global__ void __launch_bounds__(256) k_fv_nodes5(int N, const int* __restrict__ n2o, const double* __restrict__ part,
                                                    const int* __restrict__ xin_ptr, const double* __restrict__ spill,
                                                    const int* __restrict__ bnf_ptr, const int* __restrict__ bnf_ent,
@@ -999,13 +1004,11 @@ __device__ __forceinline__ double wave_sum(int n, const Gas& g, const double* __
   const int q0 = bnf_ptr[n], q1 = bnf_ptr[n + 1];
   if (q0 < q1) {
     const double* v = P2 + 8 * (size_t)n;
-    const double a = sqrt(g.gam * v[4] / v[0]);
+    const double a2 = g.gam * v[4] / v[0], third = 1.0 / 3.0;
     for (int q = q0; q < q1; ++q) {
       const int f = bnf_ent[q] / 3;
       const double x = fn[f], y = fn[(size_t)F + f], z = fn[2 * (size_t)F + f];
-      const double S = sqrt(x * x + y * y + z * z), iS = 1.0 / S;
-      const double un = v[1] * (iS * x) + v[2] * (iS * y) + v[3] * (iS * z);
-      s += fmin(un - a, 0.0) * S / 3;
+      s += third * fmin(v[1] * x + v[2] * y + v[3] * z - sqrt(a2 * (x * x + y * y + z * z)), 0.0);
     }
   }
   return s;
@@ -1021,52 +1024,57 @@ __global__ void k_wave_dt(int N, Gas g, double cfl, const int* __restrict__ n2o,
 }
 
 // One stage of the explicit RK2 step fused with the node assembly of its
-// residual (k_fv_nodes_b) and the primitive conversion of the state the next
-// residual needs.  STAGE 1: the local time step from the wave sums, k1 = dt R
-// kept, P2 = prim(U - k1).  STAGE 2: U -= (k1 + k2)/2, P2 = prim(U).  The
-// same operations in the same order as the separate kernels, whose five
-// launches and passes over R, U0 and k2 it replaces (on a small mesh the
-// launches are the step: 21^3, first order, 100 us per step before and 61 us
-// with the wave sums, two edge sweeps and two of these).
-template <int STAGE, bool FACES>
+// residual (the sums of k_fv_nodes5) and the primitive conversion of the
+// state the next residual needs.  STAGE 1: the local time step from the wave
+// sums, k1 = dt R kept, P2 = prim(U - k1).  STAGE 2: U -= (k1 + k2)/2, P2 =
+// prim(U).  The same operations in the same order as separate kernels, whose
+// five launches and passes over R, U0 and k2 it replaces: on a small mesh
+// the launches are the step.  Eight lanes per node, lane c < 5 component c,
+// lane 5 the wave sum, so that the sums of a node run side by side (one
+// thread per node took 13-16 us at 9,261 nodes, most of it the serial loops
+// of boundary nodes).
+template <int STAGE>
 __global__ void __launch_bounds__(256) k_rk_nodes(int N, Gas g, double cfl, const int* __restrict__ n2o,
                                                   const double* __restrict__ part, const int* __restrict__ xin_ptr,
                                                   const double* __restrict__ spill, const double* __restrict__ wpart,
                                                   const double* __restrict__ wspill, const int* __restrict__ bnf_ptr,
                                                   const int* __restrict__ bnf_ent, const double* __restrict__ fbuf,
-                                                  int F, const double* __restrict__ Ub0,
-                                                  const int* __restrict__ fcode, const double* __restrict__ fn,
+                                                  int F, const double* __restrict__ fn,
                                                   const double* __restrict__ vol2, double* __restrict__ dt2,
                                                   double* __restrict__ k1, double* __restrict__ U, double* P2) {
-  const int n = blockIdx.x * blockDim.x + threadIdx.x;
-  if (n >= N) return;
+  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  const bool act = (t >> 3) < N;
+  const int n = act ? (int)(t >> 3) : N - 1, c = (int)(t & 7), lane0 = threadIdx.x & 24;
   const double vol = vol2[n], invcv = 1.0 / vol;
-  double acc[5];
-  node_sum<FACES>(n, g, part, xin_ptr, spill, bnf_ptr, bnf_ent, fbuf, F, Ub0, fcode, fn, P2, acc);
-  double dt;
+  const size_t o = (size_t)n2o[n];
+  double acc = 0.0, u = 0.0;
+  if (c < 5) {
+    u = U[5 * o + c];
+    acc = part[5 * (size_t)n + c];
+    for (int k = xin_ptr[n]; k < xin_ptr[n + 1]; ++k) acc -= spill[5 * (size_t)k + c];
+    for (int q = bnf_ptr[n]; q < bnf_ptr[n + 1]; ++q) acc += fbuf[5 * (size_t)bnf_ent[q] + c];
+  } else if (c == 5) {
+    acc = STAGE == 1 ? cfl * vol / (-1.0 * wave_sum(n, g, wpart, xin_ptr, wspill, bnf_ptr, bnf_ent, F, fn, P2))
+                     : dt2[n];
+  }
+  const double dt = __shfl_sync(0xffffffffu, acc, lane0 + 5);
+  const double k = acc * invcv * dt;
+  double un;
   if (STAGE == 1) {
-    dt = cfl * vol / (-1.0 * wave_sum(n, g, wpart, xin_ptr, wspill, bnf_ptr, bnf_ent, F, fn, P2));
-    dt2[n] = dt;
+    un = u - k;
+    if (act && c < 5) k1[5 * (size_t)n + c] = k;
+    if (act && c == 5) dt2[n] = dt;
   } else {
-    dt = dt2[n];
+    un = c < 5 ? u - 1.0 / 2.0 * (k1[5 * (size_t)n + c] + k) : 0.0;
+    if (act && c < 5) U[5 * o + c] = un;
   }
-  double* u = U + 5 * (size_t)n2o[n];
-  double* kk = k1 + 5 * (size_t)n;
-  double un[5], v[5];
+  double w[5], v[5];
 #pragma unroll
-  for (int c = 0; c < 5; ++c) {
-    const double k = acc[c] * invcv * dt;
-    if (STAGE == 1) {
-      kk[c] = k;
-      un[c] = u[c] - k;
-    } else {
-      un[c] = u[c] - 1.0 / 2.0 * (kk[c] + k);
-      u[c] = un[c];
-    }
-  }
-  cons2prim(g, un, v);
-#pragma unroll
-  for (int c = 0; c < 5; ++c) P2[8 * (size_t)n + c] = v[c];
+  for (int a = 0; a < 5; ++a) w[a] = __shfl_sync(0xffffffffu, un, lane0 + a);
+  cons2prim(g, w, v);
+  // every lane has read P2 of its node (the wave sum's lane before the first
+  // shuffle); lane c writes its component
+  if (act && c < 5) P2[8 * (size_t)n + c] = c == 0 ? v[0] : c == 1 ? v[1] : c == 2 ? v[2] : c == 3 ? v[3] : v[4];
 }
 
 // RK2 stage helpers (ExplicitTsDesc.C:98-117): k = dt*R; U0 = U - k1;
@@ -1282,9 +1290,11 @@ void grad_records_blocked_dev(aerof_gpu_ctx* c, const double* P2src, double* G2d
 }
 
 // Edge fluxes of the blocked organisation from P2 and G2 into part and
-// spill; counter: where unphysical states are counted.
+// spill, and the boundary subface fluxes into fbuf; counter: where
+// unphysical states are counted.
 static void fv_blocked_dev(aerof_gpu_ctx* c, int failsafe, int* counter) {
   DeviceMesh& m = c->mesh;
+  const FaceArgs fa{m.F, m.Ubd.p, m.faces.p, m.fcode.p, m.fnrm.p, m.o2n.p, c->s.fbuf.p};
   const size_t smem = fv_blocked_smem(m);
   // register budget from the CTAs per SM that shared memory allows
   // (228 KB per SM, 1 KB reserved per CTA)
@@ -1302,10 +1312,11 @@ static void fv_blocked_dev(aerof_gpu_ctx* c, int failsafe, int* counter) {
   auto fvk = wide ? k_fv_blocked<512, 2>
                   : by_smem >= 4 ? k_fv_blocked<256, 4> : by_smem == 3 ? k_fv_blocked<256, 3> : k_fv_blocked<256, 2>;
   AEROF_CUDA(cudaFuncSetAttribute(fvk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  fvk<<<m.nblk, fv_threads, smem, c->stream>>>(m.N, m.E, m.NB, make_gas(c->cfg.gamma), c->cfg.reconstruction,
+  const int nface = grid_for(3 * (size_t)m.F, fv_threads * kFaceItems);
+  fvk<<<m.nblk + nface, fv_threads, smem, c->stream>>>(m.N, m.E, m.NB, make_gas(c->cfg.gamma), c->cfg.reconstruction,
                                                c->cfg.beta, failsafe, m.bl.p, m.bnorm.p, m.beptr.p, m.hfptr.p,
                                                m.hfpad.p, m.maxHf, m.P2.p, c->s.G2.p, m.lptr.p, m.lidx.p, m.xslot.p,
-                                               c->s.part.p, c->s.spill.p, c->s.tag.p, counter, nullptr);
+                                               c->s.part.p, c->s.spill.p, c->s.tag.p, counter, nullptr, m.nblk, fa);
   AEROF_LAUNCH_CHECK();
 }
 
@@ -1362,26 +1373,9 @@ static int residual_blocked_dev(aerof_gpu_ctx* c, const double* dU, double* dR, 
   }
   {
     TimerScope t(c, AEROF_T_FV_TERM);
-    // boundary fluxes in their own kernel (thread per face) or inside the
-    // node assembly (tuning knob AEROF_FACES_IN_NODES=1)
-    static const bool faces_in_nodes = [] {
-      const char* e = std::getenv("AEROF_FACES_IN_NODES");
-      return e && std::atoi(e) == 1;
-    }();
-    if (faces_in_nodes) {
-      k_fv_nodes_b<true><<<grid_for(m.N, kBlock), kBlock, 0, s>>>(
-          m.N, g, m.n2o.p, c->s.part.p, m.xin_ptr.p, c->s.spill.p, m.bnf_ptr.p, m.bnf_ent.p, nullptr, m.F, m.Ubd.p,
-          m.fcode.p, m.fnrm.p, m.P2.p, m.vol2.p, dR, nullptr, 0, m.NB, cnt, pub);
-    } else {
-      if (m.F) {
-        k_face_flux<<<grid_for(m.F, kBlock), kBlock, 0, s>>>(m.F, g, m.Ubd.p, m.faces.p, m.fcode.p, m.fnrm.p,
-                                                             m.P2.p, m.o2n.p, c->s.fbuf.p);
-        AEROF_LAUNCH_CHECK();
-      }
-      k_fv_nodes5<<<grid_for(5 * (size_t)m.N, kBlock), kBlock, 0, s>>>(m.N, m.n2o.p, c->s.part.p, m.xin_ptr.p,
-                                                                       c->s.spill.p, m.bnf_ptr.p, m.bnf_ent.p,
-                                                                       c->s.fbuf.p, m.vol2.p, dR, cnt, pub);
-    }
+    k_fv_nodes5<<<grid_for(5 * (size_t)m.N, kBlock), kBlock, 0, s>>>(m.N, m.n2o.p, c->s.part.p, m.xin_ptr.p,
+                                                                     c->s.spill.p, m.bnf_ptr.p, m.bnf_ent.p,
+                                                                     c->s.fbuf.p, m.vol2.p, dR, cnt, pub);
     AEROF_LAUNCH_CHECK();
     if (pub) c->s.count_clear = true;
     galerkin_add(c, dU, dR);
@@ -1636,16 +1630,16 @@ static void stage_kernels(aerof_gpu_ctx* c, ResidualPipe& p, int st, cudaStream_
   if (nl) {
     fvk<<<nl, 256, fsmem, s>>>(m.N, m.E, m.NB, g, rec, c->cfg.beta, 0, m.bl.p, m.bnorm.p, m.beptr.p, m.hfptr.p,
                                m.hfpad.p, m.maxHf, m.P2.p, c->s.G2.p, m.lptr.p, m.lidx.p, m.xslot.p, c->s.part.p,
-                               c->s.spill.p, c->s.tag.p, cnt, lp);
+                               c->s.spill.p, c->s.tag.p, cnt, lp, nl, FaceArgs{});
     AEROF_LAUNCH_CHECK();
   }
   lp = seg(3, nl);
   if (nl) {
-    // the boundary fluxes inside the assembly (one launch instead of a
-    // small face kernel per stage)
-    k_fv_nodes_b<true><<<grid_for((size_t)nl * m.NB, kBlock), kBlock, 0, s>>>(
-        m.N, g, m.n2o.p, c->s.part.p, m.xin_ptr.p, c->s.spill.p, m.bnf_ptr.p, m.bnf_ent.p, nullptr, m.F, m.Ubd.p,
-        m.fcode.p, m.fnrm.p, m.P2.p, m.vol2.p, dR, lp, nl, m.NB, nullptr, nullptr);
+    // the boundary fluxes inside the assembly (the stages' edge sweeps are
+    // lists of blocks, without the face items)
+    k_fv_nodes_list<<<grid_for((size_t)nl * m.NB, kBlock), kBlock, 0, s>>>(
+        m.N, g, m.n2o.p, c->s.part.p, m.xin_ptr.p, c->s.spill.p, m.bnf_ptr.p, m.bnf_ent.p, m.F, m.Ubd.p, m.fcode.p,
+        m.fnrm.p, m.P2.p, m.vol2.p, dR, lp, nl, m.NB);
     AEROF_LAUNCH_CHECK();
   }
 }
@@ -1839,12 +1833,6 @@ void timestep_dev(aerof_gpu_ctx* c, const double* dU, double cfl, double* ddt) {
   AEROF_LAUNCH_CHECK();
 }
 
-// Up to this many nodes the boundary fluxes are formed inside the node
-// assembly of an RK2 stage: one launch less, where a launch costs more than
-// the few serial faces per boundary node (large meshes: a thread per face is
-// 26 us faster at 101^3).
-constexpr int kFacesInNodes = 1 << 16;
-
 // nsteps of RK2 on dU in the blocked organisation: per step the wave sums,
 // two edge sweeps (with gradients unless first order) and two fused stages.
 // Unphysical states are counted into counter.
@@ -1860,18 +1848,12 @@ static void rk2_blocked_dev(aerof_gpu_ctx* c, double* dU, double cfl, int nsteps
   c->s.dt.ensure(m.N);
   c->s.k1.ensure(n5);
   c->s.p2g2_valid = false;
-  const bool faces = m.N <= kFacesInNodes || !m.F;
-  const int gn = grid_for(m.N, kBlock);
+  const int gn = grid_for(8 * (size_t)m.N, kBlock);
   prim_to_P2(m, g, dU, s);
   auto stage = [&](auto kern) {
-    if (!faces) {
-      k_face_flux<<<grid_for(m.F, kBlock), kBlock, 0, s>>>(m.F, g, m.Ubd.p, m.faces.p, m.fcode.p, m.fnrm.p, m.P2.p,
-                                                           m.o2n.p, c->s.fbuf.p);
-      AEROF_LAUNCH_CHECK();
-    }
     kern<<<gn, kBlock, 0, s>>>(m.N, g, cfl, m.n2o.p, c->s.part.p, m.xin_ptr.p, c->s.spill.p, c->s.wpart.p,
-                               c->s.wspill.p, m.bnf_ptr.p, m.bnf_ent.p, c->s.fbuf.p, m.F, m.Ubd.p, m.fcode.p,
-                               m.fnrm.p, m.vol2.p, c->s.dt.p, c->s.k1.p, dU, m.P2.p);
+                               c->s.wspill.p, m.bnf_ptr.p, m.bnf_ent.p, c->s.fbuf.p, m.F, m.fnrm.p, m.vol2.p,
+                               c->s.dt.p, c->s.k1.p, dU, m.P2.p);
     AEROF_LAUNCH_CHECK();
   };
   for (int k = 0; k < nsteps; ++k) {
@@ -1889,8 +1871,8 @@ static void rk2_blocked_dev(aerof_gpu_ctx* c, double* dU, double cfl, int nsteps
         fv_blocked_dev(c, 0, counter);
       }
       TimerScope t(c, AEROF_T_FV_TERM);
-      if (st == 1) stage(faces ? k_rk_nodes<1, true> : k_rk_nodes<1, false>);
-      else stage(faces ? k_rk_nodes<2, true> : k_rk_nodes<2, false>);
+      if (st == 1) stage(k_rk_nodes<1>);
+      else stage(k_rk_nodes<2>);
     }
   }
 }
