@@ -406,6 +406,27 @@ __global__ void __launch_bounds__(kFGradThreads, 1) k_f_grad(int N, int NB, cons
 // per SM (the staging takes ~180 KB); bound by FP64 issue, about 2.5 primal
 // evaluations per edge.
 constexpr int kFwdThreads = 512;
+// tangent subface fluxes (item 3 f + l: node l of face f) as extra blocks of
+// the launch, into dfb[3F][5]
+template <bool GEO>
+__device__ __forceinline__ void f_face_items(const Gas& g, const FaceArgs& fa, const double* __restrict__ dfn,
+                                             const double* __restrict__ P2, const double* __restrict__ D2, int blk) {
+  const int e = blk * blockDim.x + threadIdx.x;
+  if (e >= 3 * fa.F) return;
+  const int f = e / 3;
+  const double third = 1.0 / 3.0;
+  const size_t n = (size_t)fa.o2n[fa.faces[e]];
+  Dual V[5], nn[3], ff[5];
+  double Ub[5];
+#pragma unroll
+  for (int k = 0; k < 5; ++k) { V[k] = Dual(P2[8 * n + k], D2[8 * n + k]); Ub[k] = fa.Ub[k]; }
+#pragma unroll
+  for (int a = 0; a < 3; ++a)
+    nn[a] = third * Dual(fa.fn[(size_t)a * fa.F + f], GEO ? dfn[(size_t)a * fa.F + f] : 0.0);
+  face_flux(g, fa.fcode[f], nn[0], nn[1], nn[2], V, Ub, ff);
+#pragma unroll
+  for (int k = 0; k < 5; ++k) fa.fbuf[5 * (size_t)e + k] = ff[k].d;
+}
 template <bool GEO>
 __global__ void __launch_bounds__(kFwdThreads, 1)
     k_f_fv_blocked(int N, int E, int NB, Gas g, int rec, double beta, const ushort2* __restrict__ bl,
@@ -414,9 +435,13 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
                    const double* __restrict__ P2, const double* __restrict__ D2, const double* __restrict__ G2,
                    const double* __restrict__ dG2, const int* __restrict__ lptr, const int* __restrict__ lidx,
                    const int* __restrict__ xslot, double* __restrict__ part, double* __restrict__ spill,
-                   int* __restrict__ counter) {
+                   int* __restrict__ counter, int nmain, FaceArgs fa, const double* __restrict__ dfn) {
   extern __shared__ double sm[];
   const int blk = blockIdx.x;
+  if (blk >= nmain) {
+    f_face_items<GEO>(g, fa, dfn, P2, D2, blk - nmain);
+    return;
+  }
   const int n0 = blk * NB, nn = min(NB, N - n0);
   const int nh = hfptr[blk + 1] - hfptr[blk], ns = nn + nh;
   const int e0 = beptr[blk], e1 = beptr[blk + 1];
@@ -506,52 +531,25 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
   }
 }
 
-// dR of every node: (tangent flux sum + boundary faces in dual arithmetic) /
-// vol, and with GEO - R dvol / vol (R = S / vol), written to the caller's row
+// dR of every node, five lanes per node (one component each): tangent flux
+// sum, spills and subface fluxes, / vol, and with GEO - R dvol / vol (R = S /
+// vol), written to the caller's row
 template <bool GEO>
-__global__ void __launch_bounds__(256) k_f_nodes(int N, int F, Gas g, const double* __restrict__ Ub0,
-                                                 const int* __restrict__ n2o, const double* __restrict__ part,
+__global__ void __launch_bounds__(256) k_f_nodes(int N, const int* __restrict__ n2o, const double* __restrict__ part,
                                                  const int* __restrict__ xin_ptr, const double* __restrict__ spill,
                                                  const int* __restrict__ bnf_ptr, const int* __restrict__ bnf_ent,
-                                                 const int* __restrict__ fcode, const double* __restrict__ fn,
-                                                 const double* __restrict__ dfn, const double* __restrict__ P2,
-                                                 const double* __restrict__ D2, const double* __restrict__ vol2,
+                                                 const double* __restrict__ dfb, const double* __restrict__ vol2,
                                                  const double* __restrict__ dvol, const double* __restrict__ R,
                                                  double* __restrict__ dR) {
-  const int n = blockIdx.x * blockDim.x + threadIdx.x;
+  const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
+  const int n = (int)(t / 5), c = (int)(t - 5 * (unsigned)n);
   if (n >= N) return;
-  double acc[5];
-#pragma unroll
-  for (int c = 0; c < 5; ++c) acc[c] = part[5 * (size_t)n + c];
-  for (int k = xin_ptr[n]; k < xin_ptr[n + 1]; ++k) {
-#pragma unroll
-    for (int c = 0; c < 5; ++c) acc[c] -= spill[5 * (size_t)k + c];
-  }
-  const int q0 = bnf_ptr[n], q1 = bnf_ptr[n + 1];
-  if (q0 < q1) {
-    const double third = 1.0 / 3.0;
-    Dual V[5];
-    double Ub[5];
-#pragma unroll
-    for (int k = 0; k < 5; ++k) { V[k] = Dual(P2[8 * (size_t)n + k], D2[8 * (size_t)n + k]); Ub[k] = Ub0[k]; }
-    for (int q = q0; q < q1; ++q) {
-      const int f = bnf_ent[q] / 3;
-      Dual nn[3], ff[5];
-#pragma unroll
-      for (int a = 0; a < 3; ++a) nn[a] = third * Dual(fn[(size_t)a * F + f], GEO ? dfn[(size_t)a * F + f] : 0.0);
-      face_flux(g, fcode[f], nn[0], nn[1], nn[2], V, Ub, ff);
-#pragma unroll
-      for (int c = 0; c < 5; ++c) acc[c] += ff[c].d;
-    }
-  }
-  const double iv = 1.0 / vol2[n];
-  const size_t o = (size_t)n2o[n];
-#pragma unroll
-  for (int c = 0; c < 5; ++c) {
-    double d = acc[c];
-    if (GEO) d -= R[5 * o + c] * dvol[n];
-    dR[5 * o + c] = d * iv;
-  }
+  double acc = part[t];
+  for (int k = xin_ptr[n]; k < xin_ptr[n + 1]; ++k) acc -= spill[5 * (size_t)k + c];
+  for (int q = bnf_ptr[n]; q < bnf_ptr[n + 1]; ++q) acc += dfb[5 * (size_t)bnf_ent[q] + c];
+  const size_t o = 5 * (size_t)n2o[n] + c;
+  if (GEO) acc -= R[o] * dvol[n];
+  dR[o] = acc * (1.0 / vol2[n]);
 }
 
 static size_t fwd_smem(const DeviceMesh& m) {
@@ -588,6 +586,7 @@ static void forward_blocked(aerof_gpu_ctx* c, const double* dU, const double* dv
   c->s.p2g2_valid = false;
   c->s.part.ensure(5 * (size_t)m.N);
   c->s.spill.ensure(5 * (size_t)std::max(m.nX, 1));
+  c->s.fbuf.ensure(15 * (size_t)std::max(m.F, 1));
   k_f_seed<<<gn, kAB, 0, s>>>(m.N, g, m.n2o.p, m.P2.p, dv, dXdot, w.D2.p);
   AEROF_LAUNCH_CHECK();
   if (geo) {
@@ -626,14 +625,18 @@ static void forward_blocked(aerof_gpu_ctx* c, const double* dU, const double* dv
   const size_t smem = fwd_smem(m);
   auto edges = [&](auto kern) {
     AEROF_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    kern<<<m.nblk, kFwdThreads, smem, s>>>(m.N, m.E, m.NB, g, rec, c->cfg.beta, m.bl.p, m.bnorm.p, w.dbn.p, m.beptr.p,
-                                           m.hfptr.p, m.hfpad.p, m.maxHf, m.P2.p, w.D2.p, c->s.G2.p, w.dG2.p,
-                                           m.lptr.p, m.lidx.p, m.xslot.p, c->s.part.p, c->s.spill.p, cnt);
+    const FaceArgs fa{m.F, m.Ubd.p, m.faces.p, m.fcode.p, m.fnrm.p, m.o2n.p, c->s.fbuf.p};
+    const int nface = grid_for(3 * (size_t)m.F, kFwdThreads);
+    kern<<<m.nblk + nface, kFwdThreads, smem, s>>>(m.N, m.E, m.NB, g, rec, c->cfg.beta, m.bl.p, m.bnorm.p, w.dbn.p,
+                                                   m.beptr.p, m.hfptr.p, m.hfpad.p, m.maxHf, m.P2.p, w.D2.p,
+                                                   c->s.G2.p, w.dG2.p, m.lptr.p, m.lidx.p, m.xslot.p, c->s.part.p,
+                                                   c->s.spill.p, cnt, m.nblk, fa, w.dfn.p);
     AEROF_LAUNCH_CHECK();
   };
   auto nodes = [&](auto kern) {
-    kern<<<gn, kAB, 0, s>>>(m.N, m.F, g, m.Ubd.p, m.n2o.p, c->s.part.p, m.xin_ptr.p, c->s.spill.p, m.bnf_ptr.p,
-                            m.bnf_ent.p, m.fcode.p, m.fnrm.p, w.dfn.p, m.P2.p, w.D2.p, m.vol2.p, w.dvol.p, R, ddR);
+    kern<<<grid_for(5 * (size_t)m.N, kAB), kAB, 0, s>>>(m.N, m.n2o.p, c->s.part.p, m.xin_ptr.p, c->s.spill.p,
+                                                        m.bnf_ptr.p, m.bnf_ent.p, c->s.fbuf.p, m.vol2.p, w.dvol.p, R,
+                                                        ddR);
     AEROF_LAUNCH_CHECK();
   };
   if (geo) {
@@ -976,17 +979,24 @@ __global__ void k_a_lam2(int N, const int* __restrict__ n2o, const double* __res
 // 4.24 ms with 512 (4.70 ms with 256 and exact divisions and roots).
 constexpr int kRevThreads = 512;
 
+// Edges per chunk (one per thread) and doubles per edge kept in shared memory
+// (21: conflict-free).
+constexpr int kRevEdge = 21;
+
 // One CTA per block.  Phase 0: node records, gradients and lam of the
 // block's nodes and forward halo are staged in shared memory (cp.async).
-// Phase 1, thread per edge: the reconstruction is recomputed, the Roe flux
-// reversed (gF = lam_i - lam_j), and the cotangents (gL, gR) of the two
-// reconstructed states kept in shared memory; for a block-crossing edge the
-// second endpoint's part (g_Vj, g_ddji, dx) goes to spill; with GEO the
-// cotangents of the oriented edge normal and of dx go to geo in the
-// original edge numbering and orientation.  Phase 2, L lanes per node: the
-// node's edges in edge order, each reversed through the reconstruction for
-// the node's side: g_V += g_Vside, g_grad += dx (x) g_ddside; xor-tree lane
-// sum; written to gVp / gGp.
+// Then the block's edges in chunks of one per thread.  Phase 1, thread per
+// edge: the reconstruction is recomputed, the Roe flux reversed (gF = lam_i -
+// lam_j), and the reconstruction reversed once for both endpoints (g_Vi,
+// g_ddij, g_Vj, g_ddji) into shared memory; for a block-crossing edge the
+// second endpoint's part and dx go to spill; with GEO the cotangents of the
+// oriented edge normal and of dx go to geo in the original edge numbering and
+// orientation.  Phase 2, L lanes per node: the entries of the node's list
+// that lie in the chunk, in edge order, g_V += g_Vside, g_grad += dx (x)
+// g_ddside; xor-tree lane sum, added up over the chunks; written to gVp /
+// gGp.  Keeping only the cotangents of the two reconstructed states per
+// edge (ten doubles, no chunks) had the limiter's reverse evaluated again by
+// each endpoint's gather: 1.62 ms per sweep at 101^3.
 template <bool GEO>
 __global__ void __launch_bounds__(kRevThreads, 1) k_a_fv_blocked(int N, int E, int NB, Gas g, int rec, double beta,
                                                          const ushort2* __restrict__ bl, const double* __restrict__ bn,
@@ -1013,7 +1023,7 @@ __global__ void __launch_bounds__(kRevThreads, 1) k_a_fv_blocked(int N, int E, i
   double* Pn = sm;                           // [ns][kPS]
   double* Gn = sm + kPS * ns;                // [ns][kGS]
   double* Ln = sm + (kPS + kGS) * ns;        // [ns][6]
-  double* Es = sm + (kPS + kGS + 6) * ns;    // [e1 - e0][10]: gL, gR
+  double* Es = sm + (kPS + kGS + 6) * ns;    // [blockDim][kRevEdge]
   const bool grad = rec != AEROF_REC_CONSTANT;
   {
     const int* hf = hfpad + (size_t)blk * maxHf;
@@ -1045,47 +1055,49 @@ __global__ void __launch_bounds__(kRevThreads, 1) k_a_fv_blocked(int N, int E, i
   }
   cp_async_wait_all();
   __syncthreads();
-  for (int q = e0 + threadIdx.x; q < e1; q += blockDim.x) {
-    const ushort2 lq = bl[q];
-    const double n0_ = bn[q], n1_ = bn[(size_t)E + q], n2_ = bn[2 * (size_t)E + q];
-    const double* pi = Pn + kPS * lq.x;
-    const double* pj = Pn + kPS * lq.y;
-    const double* gi = Gn + kGS * lq.x;
-    const double* gj = Gn + kGS * lq.y;
-    const double dx0 = pj[5] - pi[5], dx1 = pj[6] - pi[6], dx2 = pj[7] - pi[7];
-    double Vi[5], Vj[5], ddij[5], ddji[5];
+  double* As = Es + kRevEdge * (size_t)blockDim.x;   // [NB][kRevEdge] node sums over the chunks
+  int kp = lb + r2;
+  for (int c0 = e0; c0 < e1; c0 += blockDim.x) {
+    const int q = c0 + threadIdx.x;
+    if (q < e1) {
+      const ushort2 lq = bl[q];
+      const double n0_ = bn[q], n1_ = bn[(size_t)E + q], n2_ = bn[2 * (size_t)E + q];
+      const double* pi = Pn + kPS * lq.x;
+      const double* pj = Pn + kPS * lq.y;
+      const double* gi = Gn + kGS * lq.x;
+      const double* gj = Gn + kGS * lq.y;
+      const double dx0 = pj[5] - pi[5], dx1 = pj[6] - pi[6], dx2 = pj[7] - pi[7];
+      double Vi[5], Vj[5], ddij[5], ddji[5];
 #pragma unroll
-    for (int k = 0; k < 5; ++k) {
-      if (!grad) {
-        ddij[k] = ddji[k] = 0.0;
-        Vi[k] = pi[k]; Vj[k] = pj[k];
-      } else {
-        ddij[k] = dx0 * gi[k] + dx1 * gi[5 + k] + dx2 * gi[10 + k];
-        ddji[k] = dx0 * gj[k] + dx1 * gj[5 + k] + dx2 * gj[10 + k];
-        if (rec == AEROF_REC_VANALBADA) vanalbada(beta, pi[k], ddij[k], pj[k], ddji[k], Vi[k], Vj[k]);
-        else linear_rec(beta, pi[k], ddij[k], pj[k], ddji[k], Vi[k], Vj[k]);
+      for (int k = 0; k < 5; ++k) {
+        if (!grad) {
+          ddij[k] = ddji[k] = 0.0;
+          Vi[k] = pi[k]; Vj[k] = pj[k];
+        } else {
+          ddij[k] = dx0 * gi[k] + dx1 * gi[5 + k] + dx2 * gi[10 + k];
+          ddji[k] = dx0 * gj[k] + dx1 * gj[5 + k] + dx2 * gj[10 + k];
+          if (rec == AEROF_REC_VANALBADA) vanalbada(beta, pi[k], ddij[k], pj[k], ddji[k], Vi[k], Vj[k]);
+          else linear_rec(beta, pi[k], ddij[k], pj[k], ddji[k], Vi[k], Vj[k]);
+        }
       }
-    }
-    double gF[5], gL[5] = {0, 0, 0, 0, 0}, gR[5] = {0, 0, 0, 0, 0}, gn[3] = {0, 0, 0};
+      double gF[5], gL[5] = {0, 0, 0, 0, 0}, gR[5] = {0, 0, 0, 0, 0}, gn[3] = {0, 0, 0};
 #pragma unroll
-    for (int k = 0; k < 5; ++k) gF[k] = Ln[6 * lq.x + k] - Ln[6 * lq.y + k];
-    if (n0_ * n0_ + n1_ * n1_ + n2_ * n2_ >= 1e-36) roe_flux_adj(g, n0_, n1_, n2_, Vi, Vj, gF, gL, gR, gn);
-    double* es = Es + 10 * (q - e0);
-#pragma unroll
-    for (int k = 0; k < 5; ++k) { es[k] = gL[k]; es[5 + k] = gR[k]; }
-    const int xs = xslot[q];
-    if (GEO || xs >= 0) {
-      double gdx0 = 0.0, gdx1 = 0.0, gdx2 = 0.0;
+      for (int k = 0; k < 5; ++k) gF[k] = Ln[6 * lq.x + k] - Ln[6 * lq.y + k];
+      if (n0_ * n0_ + n1_ * n1_ + n2_ * n2_ >= 1e-36) roe_flux_adj(g, n0_, n1_, n2_, Vi, Vj, gF, gL, gR, gn);
+      double* es = Es + kRevEdge * threadIdx.x;
+      const int xs = xslot[q];
       double* sp = xs >= 0 ? spill + kSP * (size_t)xs : nullptr;
+      double gdx0 = 0.0, gdx1 = 0.0, gdx2 = 0.0;
 #pragma unroll
       for (int k = 0; k < 5; ++k) {
         double gvi = 0.0, gvj = 0.0, gdi, gdj;
         reconstruct_adj(rec, beta, pi[k], ddij[k], pj[k], ddji[k], gL[k], gR[k], gvi, gvj, gdi, gdj);
-        if (grad) {
+        if (GEO && grad) {
           gdx0 += gi[k] * gdi + gj[k] * gdj;
           gdx1 += gi[5 + k] * gdi + gj[5 + k] * gdj;
           gdx2 += gi[10 + k] * gdi + gj[10 + k] * gdj;
         }
+        es[k] = gvi; es[5 + k] = gdi; es[10 + k] = gvj; es[15 + k] = gdj;
         if (sp) { sp[k] = gvj; sp[5 + k] = gdj; }
       }
       if (sp) { sp[10] = dx0; sp[11] = dx1; sp[12] = dx2; }
@@ -1099,50 +1111,55 @@ __global__ void __launch_bounds__(kRevThreads, 1) k_a_fv_blocked(int N, int E, i
         ge[2] = make_double2(sg * gdx1, sg * gdx2);
       }
     }
-  }
-  __syncthreads();
-  double av[5] = {0, 0, 0, 0, 0}, ag[15];
+    __syncthreads();
+    double av[5] = {0, 0, 0, 0, 0}, ag[15];
 #pragma unroll
-  for (int k = 0; k < 15; ++k) ag[k] = 0.0;
-  for (int k = lb + r2; k < le; k += L) {
-    const int e = lidx[k];
-    const int slot = e & 0x7fffffff;
-    const bool second = e < 0;
-    const ushort2 lq = bl[e0 + slot];
-    const double* pi = Pn + kPS * lq.x;
-    const double* pj = Pn + kPS * lq.y;
-    const double* gi = Gn + kGS * lq.x;
-    const double* gj = Gn + kGS * lq.y;
-    const double dx0 = pj[5] - pi[5], dx1 = pj[6] - pi[6], dx2 = pj[7] - pi[7];
-    const double* es = Es + 10 * slot;
+    for (int k = 0; k < 15; ++k) ag[k] = 0.0;
+    const int hi = c0 - e0 + (int)blockDim.x;   // slots [hi - blockDim, hi)
+    for (; kp < le; kp += L) {
+      const int e = lidx[kp];
+      const int slot = e & 0x7fffffff;
+      if (slot >= hi) break;
+      const ushort2 lq = bl[e0 + slot];
+      const double* pi = Pn + kPS * lq.x;
+      const double* pj = Pn + kPS * lq.y;
+      const double dx0 = pj[5] - pi[5], dx1 = pj[6] - pi[6], dx2 = pj[7] - pi[7];
+      const double* es = Es + kRevEdge * (slot - (c0 - e0)) + (e < 0 ? 10 : 0);
 #pragma unroll
-    for (int c = 0; c < 5; ++c) {
-      double ddij = 0.0, ddji = 0.0;
-      if (grad) {
-        ddij = dx0 * gi[c] + dx1 * gi[5 + c] + dx2 * gi[10 + c];
-        ddji = dx0 * gj[c] + dx1 * gj[5 + c] + dx2 * gj[10 + c];
+      for (int c = 0; c < 5; ++c) {
+        const double gd = es[5 + c];
+        av[c] += es[c];
+        ag[c] += dx0 * gd;
+        ag[5 + c] += dx1 * gd;
+        ag[10 + c] += dx2 * gd;
       }
-      double gvi = 0.0, gvj = 0.0, gdi, gdj;
-      reconstruct_adj(rec, beta, pi[c], ddij, pj[c], ddji, es[c], es[5 + c], gvi, gvj, gdi, gdj);
-      const double gd = second ? gdj : gdi;
-      av[c] += second ? gvj : gvi;
-      ag[c] += dx0 * gd;
-      ag[5 + c] += dx1 * gd;
-      ag[10 + c] += dx2 * gd;
     }
-  }
-  for (int o = 1; o < L; o <<= 1) {
+    for (int o = 1; o < L; o <<= 1) {
 #pragma unroll
-    for (int c = 0; c < 5; ++c) av[c] += __shfl_xor_sync(0xffffffffu, av[c], o);
+      for (int c = 0; c < 5; ++c) av[c] += __shfl_xor_sync(0xffffffffu, av[c], o);
 #pragma unroll
-    for (int c = 0; c < 15; ++c) ag[c] += __shfl_xor_sync(0xffffffffu, ag[c], o);
+      for (int c = 0; c < 15; ++c) ag[c] += __shfl_xor_sync(0xffffffffu, ag[c], o);
+    }
+    // the sums wait in shared memory, so that they take no registers while
+    // the next chunk's edges are evaluated (1.2 KB of spills otherwise)
+    if (act2 && r2 == 0) {
+      double* as = As + kRevEdge * t2;
+      const bool first = c0 == e0;
+#pragma unroll
+      for (int c = 0; c < 5; ++c) as[c] = first ? av[c] : as[c] + av[c];
+#pragma unroll
+      for (int c = 0; c < 15; ++c) as[5 + c] = first ? ag[c] : as[5 + c] + ag[c];
+    }
+    __syncthreads();
   }
   if (act2 && r2 == 0) {
     const size_t n = (size_t)(n0 + t2);
+    const double* as = As + kRevEdge * t2;
+    const bool any = e1 > e0;   // a block may own no edge
 #pragma unroll
-    for (int c = 0; c < 5; ++c) gVp[5 * n + c] = av[c];
+    for (int c = 0; c < 5; ++c) gVp[5 * n + c] = any ? as[c] : 0.0;
 #pragma unroll
-    for (int c = 0; c < 15; ++c) gGp[16 * n + c] = ag[c];
+    for (int c = 0; c < 15; ++c) gGp[16 * n + c] = any ? as[5 + c] : 0.0;
     gGp[16 * n + 15] = 0.0;
   }
 }
@@ -1499,7 +1516,7 @@ static void reverse_sweep_blocked(aerof_gpu_ctx* c, const double* dw, bool geo, 
   if (geo) a.geo.ensure(6 * (size_t)std::max(m.E, 1));
   k_a_lam2<<<gn, kAB, 0, s>>>(m.N, m.n2o.p, dw, m.vol2.p, a.lam2.p);
   AEROF_LAUNCH_CHECK();
-  const size_t smem = ((size_t)(kPS + kGS + 6) * (m.NB + m.maxHf) + (size_t)10 * m.maxE) * sizeof(double);
+  const size_t smem = ((size_t)(kPS + kGS + 6) * (m.NB + m.maxHf) + (size_t)kRevEdge * (kRevThreads + m.NB)) * sizeof(double);
   auto go = [&](auto kern) {
     AEROF_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     kern<<<m.nblk, kRevThreads, smem, s>>>(m.N, m.E, m.NB, g, rec, c->cfg.beta, m.bl.p, m.bnorm.p, m.beptr.p, m.hfptr.p,
@@ -1522,7 +1539,7 @@ static void reverse_sweep_blocked(aerof_gpu_ctx* c, const double* dw, bool geo, 
 // whether the blocked reverse sweep's shared memory fits
 static bool reverse_blocked_fits(const DeviceMesh& m) {
   return m.nblk > 0 &&
-         ((size_t)(kPS + kGS + 6) * (m.NB + m.maxHf) + (size_t)10 * m.maxE) * sizeof(double) <= 200 * 1024;
+         ((size_t)(kPS + kGS + 6) * (m.NB + m.maxHf) + (size_t)kRevEdge * (kRevThreads + m.NB)) * sizeof(double) <= 224 * 1024;
 }
 
 // J^T w for device state dU and cotangent dw, into dout ([N][5]).

@@ -465,6 +465,16 @@ int guard(aerof_gpu_ctx* c, F&& f) {
   }
 }
 
+// boundary data of the kernels that form subface fluxes (fbuf: [3F][5])
+struct FaceArgs {
+  int F;
+  const double* Ub;
+  const int *faces, *fcode;
+  const double* fn;
+  const int* o2n;
+  double* fbuf;
+};
+
 inline int grid_for(size_t n, int block) { return (int)((n + block - 1) / block); }
 
 // implemented in mesh.cu: geometry of coordinates XD ([N][3]) in dual

@@ -452,14 +452,6 @@ __global__ void k_edge_flux(int E, Gas g, int rec, double beta, int failsafe, co
 // (FaceTriaCore.C:288-308) from the blocked records into fbuf[3F][5].  In a
 // launch of their own (thread per face, its three nodes one after the
 // other) they took 8 us of a 47^3 residual and 17 us at 101^3.
-struct FaceArgs {
-  int F;
-  const double* Ub;
-  const int *faces, *fcode;
-  const double* fn;
-  const int* o2n;
-  double* fbuf;
-};
 constexpr int kFaceItems = 4;  // per thread
 __device__ __forceinline__ void face_items(const Gas& g, const FaceArgs& fa, const double* __restrict__ P, int blk) {
   const double third = 1.0 / 3.0;
