@@ -498,6 +498,31 @@ struct TimerScope {
 constexpr int kPS = 10;
 constexpr int kGS = 18;
 
+// W doubles of a staged record (16-byte aligned), as 16-byte loads
+template <int W>
+__device__ __forceinline__ void lds_rec(const double* rec, double* v) {
+  const double2* q = reinterpret_cast<const double2*>(rec);
+#pragma unroll
+  for (int k = 0; k < W / 2; ++k) {
+    const double2 a = q[k];
+    v[2 * k] = a.x;
+    v[2 * k + 1] = a.y;
+  }
+}
+// dd[k] = dx . grad V_k of a staged gradient record (ddx(5) ddy(5) ddz(5),
+// pad), from 16-byte loads, each used as it arrives (no
+// record in registers)
+__device__ __forceinline__ void lds_project(const double* rec, const double* dx, double* dd) {
+  const double2* q = reinterpret_cast<const double2*>(rec);
+#pragma unroll
+  for (int m = 0; m < 8; ++m) {
+    const double2 a = q[m];
+    const int e = 2 * m, f = 2 * m + 1;
+    dd[e % 5] = e < 5 ? dx[0] * a.x : dd[e % 5] + dx[e / 5] * a.x;
+    if (f < 15) dd[f % 5] = f < 5 ? dx[0] * a.y : dd[f % 5] + dx[f / 5] * a.y;
+  }
+}
+
 // 16-byte global -> shared copy that completes asynchronously (cp.async,
 // cached in L2 only); cp_async_wait_all() waits for this thread's copies.
 __device__ __forceinline__ void cp_async16(void* sdst, const void* gsrc) {

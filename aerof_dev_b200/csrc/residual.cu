@@ -391,23 +391,16 @@ __global__ void __launch_bounds__(256, 2) k_grad_pipe(int N, int NB, int nblk, i
 // checkReconstructedValues, VarFcnSGEuler.h:90-110; on failure the edge is
 // skipped as in Edge.C:414-421, counted, and with failsafe the offending
 // node tagged, EdgeCore.C:137-168), then the Roe flux.
-__device__ __forceinline__ void edge_flux_rec(const Gas& g, int rec, double beta, int failsafe, int i, int j,
-                                              double n0, double n1, double n2, const double* pi, const double* gi,
-                                              const double* pj, const double* gj, int* __restrict__ tag,
-                                              int* __restrict__ counter, double* f) {
+__device__ __forceinline__ void edge_flux_vals(const Gas& g, int rec, double beta, int failsafe, int i, int j,
+                                               double n0, double n1, double n2, const double* pi, const double* pj,
+                                               const double* ddij, const double* ddji, int* __restrict__ tag,
+                                               int* __restrict__ counter, double* f) {
   double Vi[5], Vj[5];
-  if (rec == AEROF_REC_CONSTANT) {
 #pragma unroll
-    for (int k = 0; k < 5; ++k) { Vi[k] = pi[k]; Vj[k] = pj[k]; }
-  } else {
-    const double dx0 = pj[5] - pi[5], dx1 = pj[6] - pi[6], dx2 = pj[7] - pi[7];
-#pragma unroll
-    for (int k = 0; k < 5; ++k) {
-      double ddVij = dx0 * gi[k] + dx1 * gi[5 + k] + dx2 * gi[10 + k];
-      double ddVji = dx0 * gj[k] + dx1 * gj[5 + k] + dx2 * gj[10 + k];
-      if (rec == AEROF_REC_VANALBADA) vanalbada(beta, pi[k], ddVij, pj[k], ddVji, Vi[k], Vj[k]);
-      else linear_rec(beta, pi[k], ddVij, pj[k], ddVji, Vi[k], Vj[k]);
-    }
+  for (int k = 0; k < 5; ++k) {
+    if (rec == AEROF_REC_CONSTANT) { Vi[k] = pi[k]; Vj[k] = pj[k]; }
+    else if (rec == AEROF_REC_VANALBADA) vanalbada(beta, pi[k], ddij[k], pj[k], ddji[k], Vi[k], Vj[k]);
+    else linear_rec(beta, pi[k], ddij[k], pj[k], ddji[k], Vi[k], Vj[k]);
   }
   // written as !(x > 0) so that a non-finite state counts as unphysical too
   const bool bi = !(Vi[0] > 0.0) || !(Vi[4] > 0.0);
@@ -428,8 +421,18 @@ __device__ __forceinline__ void edge_flux_eval(const Gas& g, int rec, double bet
                                                double n0, double n1, double n2, const double* __restrict__ P,
                                                const double* __restrict__ G, int* __restrict__ tag,
                                                int* __restrict__ counter, double* f) {
-  edge_flux_rec(g, rec, beta, failsafe, i, j, n0, n1, n2, P + 8 * (size_t)i, G + 16 * (size_t)i, P + 8 * (size_t)j,
-                G + 16 * (size_t)j, tag, counter, f);
+  const double *pi = P + 8 * (size_t)i, *pj = P + 8 * (size_t)j;
+  double ddij[5], ddji[5];
+  if (rec != AEROF_REC_CONSTANT) {
+    const double *gi = G + 16 * (size_t)i, *gj = G + 16 * (size_t)j;
+    const double dx0 = pj[5] - pi[5], dx1 = pj[6] - pi[6], dx2 = pj[7] - pi[7];
+#pragma unroll
+    for (int k = 0; k < 5; ++k) {
+      ddij[k] = dx0 * gi[k] + dx1 * gi[5 + k] + dx2 * gi[10 + k];
+      ddji[k] = dx0 * gj[k] + dx1 * gj[5 + k] + dx2 * gj[10 + k];
+    }
+  }
+  edge_flux_vals(g, rec, beta, failsafe, i, j, n0, n1, n2, pi, pj, ddij, ddji, tag, counter, f);
 }
 
 // Roe flux of every edge into flux[5][E] (EDGE organisation).
@@ -571,8 +574,17 @@ __global__ void __launch_bounds__(THREADS, MINB)
     double f[5];
     // global node ids are needed only to tag unphysical states
     const int gi = n0 + li, gj = lj < nn ? n0 + lj : hs[lj - nn];
-    edge_flux_rec(g, rec, beta, failsafe, gi, gj, nx, ny, nz, Pn + kPS * li, Gn + kGS * li, Pn + kPS * lj,
-                  Gn + kGS * lj, tag, counters, f);
+    double pi[8], pj[8], ddij[5], ddji[5];
+    // 16-byte loads of the staged records (46 8-byte ones, one gradient
+    // component at a time, before: 618 -> 600 us for the residual of 101^3)
+    lds_rec<8>(Pn + kPS * li, pi);
+    lds_rec<8>(Pn + kPS * lj, pj);
+    if (rec != AEROF_REC_CONSTANT) {
+      const double dx[3] = {pj[5] - pi[5], pj[6] - pi[6], pj[7] - pi[7]};
+      lds_project(Gn + kGS * li, dx, ddij);
+      lds_project(Gn + kGS * lj, dx, ddji);
+    }
+    edge_flux_vals(g, rec, beta, failsafe, gi, gj, nx, ny, nz, pi, pj, ddij, ddji, tag, counters, f);
     double* fs = Fs + 5 * (q - e0);
 #pragma unroll
     for (int k = 0; k < 5; ++k) fs[k] = f[k];
