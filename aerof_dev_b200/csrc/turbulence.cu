@@ -234,6 +234,8 @@ __device__ __forceinline__ double p1_grad6(const double x[4][3], double g[4][3])
 // are staged in shared memory (row stride 21 doubles: conflict-free) and
 // stored contiguously with evict-first stores (each record is read once,
 // by k_tet_gather).  Q: per-node records of k_sa_records
+// Refined reciprocals and the reciprocal cube root of a square root in place
+// of eight divisions and a power: 208 -> 190 us at 81^3 (3.1 M tets).
 template <int TB>
 __global__ void __launch_bounds__(TB) k_galerkin_sa_tets(int T, Gas gs, SADev sp, const int* __restrict__ tets,
                                                          const double* __restrict__ Q, double* __restrict__ C) {
@@ -242,7 +244,7 @@ __global__ void __launch_bounds__(TB) k_galerkin_sa_tets(int T, Gas gs, SADev sp
   const int t0 = blockIdx.x * TB, t = t0 + threadIdx.x;
   if (t < T) {
     const double cp = gs.gam * gs.invgam1;
-    const double twothird = 2.0 / 3.0, sixth = 1.0 / 6.0;
+    const double twothird = 2.0 / 3.0;
     const int4 q4 = *reinterpret_cast<const int4*>(tets + 4 * (size_t)t);
     const int nd[4] = {q4.x, q4.y, q4.z, q4.w};
     double u[4][3], Tn[4], rh[4], nu[4], dw[4], x[4][3];
@@ -274,7 +276,7 @@ __global__ void __launch_bounds__(TB) k_galerkin_sa_tets(int T, Gas gs, SADev sp
     double mul, lambdal;
     if (sp.model == 2) {
       const double Ta = sp.alpha * Tcg;
-      mul = Ta * sqrt(Ta) * (1.0 + sp.Ts) / (Ta + sp.Ts);
+      mul = Ta * sqrt(Ta) * (1.0 + sp.Ts) * rcp_(Ta + sp.Ts);
       lambdal = -twothird * mul;
     } else {
       mul = 1.0;
@@ -283,7 +285,7 @@ __global__ void __launch_bounds__(TB) k_galerkin_sa_tets(int T, Gas gs, SADev sp
     const double kappal = sp.ooprandtl * cp * mul;
     // eddy viscosity (SATerm::computeTurbulentViscosity)
     const double mutilde = 0.25 * (rh[0] * nu[0] + rh[1] * nu[1] + rh[2] * nu[2] + rh[3] * nu[3]);
-    const double chi0 = mutilde / mul;
+    const double chi0 = mutilde * rcp_(mul);
     const double chi03 = chi0 * chi0 * chi0;
     const double mut = mutilde * (chi03 / (chi03 + sp.cv1_pow3));
     const double lambdat = -2.0 * mut / 3.0;
@@ -293,30 +295,31 @@ __global__ void __launch_bounds__(TB) k_galerkin_sa_tets(int T, Gas gs, SADev sp
     double s5 = 0.0;
     const double d2w = 0.25 * (dw[0] + dw[1] + dw[2] + dw[3]);
     if (d2w >= 1.e-15) {
-      const double chi = fmax(mutilde / mul, 0.001);
+      const double chi = fmax(chi0, 0.001);
       const double chi3 = chi * chi * chi;
-      const double fv1 = chi3 / (chi3 + sp.cv1_pow3);
-      double fv2 = 1. - chi / (1. + chi * fv1);
+      const double fv1 = chi3 * rcp_(chi3 + sp.cv1_pow3);
+      double fv2 = 1. - chi * rcp_(1. + chi * fv1);
       double fv3 = 1.0;
       if (sp.fv3) {
         fv2 = 1.0 + sp.oocv2 * chi;
         fv2 = 1.0 / (fv2 * fv2 * fv2);
         fv3 = (1.0 + chi * fv1) * (1.0 - fv2) / chi;
       }
-      const double ood2wall2 = 1.0 / (d2w * d2w);
+      const double ood2wall2 = rcp_(d2w * d2w);
       const double rho = 0.25 * (rh[0] + rh[1] + rh[2] + rh[3]);
-      const double oorho = 1.0 / rho;
+      const double oorho = rcp_(rho);
       const double zz = sp.ooreynolds * sp.oovkcst2 * maxmutilde * oorho * ood2wall2;
       const double s12 = du[0][1] - du[1][0];
       const double s23 = du[1][2] - du[2][1];
       const double s31 = du[2][0] - du[0][2];
       const double sv = sqrt(s12 * s12 + s23 * s23 + s31 * s31);
       const double Stilde = fmax(sv * fv3 + zz * fv2, 1.0e-12);
-      const double rr = fmin(zz / Stilde, 2.0);
+      const double rr = fmin(zz * rcp_(Stilde), 2.0);
       const double rr2 = rr * rr;
       const double gg = rr + sp.cw2 * (rr2 * rr2 * rr2 - rr);
       const double gg2 = gg * gg;
-      const double fw = sp.opcw3_pow * gg * pow(gg2 * gg2 * gg2 + sp.cw3_pow6, -sixth);
+      // (...)^(-1/6) as the reciprocal cube root of the square root
+      const double fw = sp.opcw3_pow * gg * rcbrt(sqrt(gg2 * gg2 * gg2 + sp.cw3_pow6));
       const double AA = sp.oosigma * sp.cb2 * rho * (dnu[0] * dnu[0] + dnu[1] * dnu[1] + dnu[2] * dnu[2]);
       const double BB = sp.cb1 * Stilde * absmutilde;
       const double CC = -sp.cw1 * fw * oorho * maxmutilde * maxmutilde * ood2wall2;
