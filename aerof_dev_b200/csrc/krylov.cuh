@@ -102,25 +102,58 @@ __device__ __forceinline__ bool last_block(int* ticket) {
   return last;
 }
 
-// vals[v] = sum of part[v][0, G) for v < nv, one warp per value (eight loads
-// in flight per lane: G is at most a few hundred)
+// vals[v] = sum of part[v][0, G) for v < nv, LG lanes per value with eight
+// loads in flight each (G is at most a few hundred): a warp for one or two
+// values, eight lanes for the dot products, so that up to 64 of them are
+// summed side by side
+template <int LG>
 __device__ __forceinline__ void sum_partials(const double* part, int G, int nv, double* vals) {
-  const int lane = threadIdx.x & 31;
-  for (int v = threadIdx.x >> 5; v < nv; v += blockDim.x >> 5) {
+  const int lane = threadIdx.x % LG, ng = blockDim.x / LG;
+  for (int v0 = 0; v0 < nv; v0 += ng) {   // the same trips in every thread
+    const int v = v0 + (int)threadIdx.x / LG;
     const double* p = part + (size_t)v * G;
     double t = 0.0;
-    for (int k0 = lane; k0 < G; k0 += 256) {
-      double x[8];
+    if (v < nv) {
+      for (int k0 = lane; k0 < G; k0 += 8 * LG) {
+        double x[8];
 #pragma unroll
-      for (int u = 0; u < 8; ++u) x[u] = k0 + 32 * u < G ? __ldcg(p + k0 + 32 * u) : 0.0;
+        for (int u = 0; u < 8; ++u) x[u] = k0 + LG * u < G ? __ldcg(p + k0 + LG * u) : 0.0;
 #pragma unroll
-      for (int u = 0; u < 8; ++u) t += x[u];
+        for (int u = 0; u < 8; ++u) t += x[u];
+      }
     }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-    if (lane == 0) vals[v] = t;
+    for (int o = LG / 2; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    if (lane == 0 && v < nv) vals[v] = t;
   }
   __syncthreads();
+}
+
+// The sums of 16 values over a warp's lanes: the lanes exchange halves, so
+// that 16 shuffles do what a tree per value does in 80; lane l returns the
+// total of value l / 2.
+__device__ __forceinline__ double warp_sums16(const double* s) {
+  const int lane = threadIdx.x & 31;
+  double a[8], b[4], c[2];
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    const double keep = lane & 16 ? s[8 + k] : s[k], give = lane & 16 ? s[k] : s[8 + k];
+    a[k] = keep + __shfl_xor_sync(0xffffffffu, give, 16);
+  }
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const double keep = lane & 8 ? a[4 + k] : a[k], give = lane & 8 ? a[k] : a[4 + k];
+    b[k] = keep + __shfl_xor_sync(0xffffffffu, give, 8);
+  }
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    const double keep = lane & 4 ? b[2 + k] : b[k], give = lane & 4 ? b[k] : b[2 + k];
+    c[k] = keep + __shfl_xor_sync(0xffffffffu, give, 4);
+  }
+  const double keep = lane & 2 ? c[1] : c[0], give = lane & 2 ? c[0] : c[1];
+  double d = keep + __shfl_xor_sync(0xffffffffu, give, 2);
+  d += __shfl_xor_sync(0xffffffffu, d, 1);
+  return d;
 }
 
 __device__ __forceinline__ void publish(GsPub* pub, int seq, int done, int iter, double l2res) {
@@ -167,7 +200,7 @@ __global__ void __launch_bounds__(kGsT) k_gs_start(size_t n, VecIn B, VecOut X, 
   double* part = st.part + (size_t)q * 2 * (st.m + 1) * st.G;
   block_sums<2>(s, 2, red, part + blockIdx.x, st.G);
   if (!last_block(ist + 6)) return;
-  sum_partials(part, st.G, 2, vals);
+  sum_partials<32>(part, st.G, 2, vals);
   if (threadIdx.x == 0) {
     double* d = st.d + (size_t)q * st.sd;
     const double beta = sqrt(vals[0]);
@@ -197,7 +230,8 @@ __global__ void __launch_bounds__(kGsT) k_gs_start(size_t n, VecIn B, VecOut X, 
 template <class TV>
 __global__ void __launch_bounds__(kGsT, 1) k_gs_dots(size_t n, int j, const TV* V, size_t vs, size_t ld,
                                                      const TV* W, size_t ws, GsDev st) {
-  __shared__ double red[(kGsT / 32) * 16];
+  constexpr int PB = 8;            // passes whose warp sums wait for one addition over the warps
+  __shared__ double red[kGsT / 32][16 * PB];
   const int q = blockIdx.y;
   pdl_trigger();
   pdl_wait();
@@ -244,7 +278,20 @@ __global__ void __launch_bounds__(kGsT, 1) k_gs_dots(size_t n, int j, const TV* 
           s[2 * u + 1] += (double)vj[p] * x;
         }
     }
-    block_sums<2 * U>(s, 2 * c, red, part + (size_t)2 * i0 * st.G + blockIdx.x, st.G);
+    const int at = 2 * (i0 % (U * PB));
+    const double t = warp_sums16(s);
+    if (!(threadIdx.x & 1)) red[threadIdx.x >> 5][at + ((threadIdx.x & 31) >> 1)] = t;
+    if (i0 + U > j || at + 2 * U == 16 * PB) {
+      __syncthreads();
+      const int first = 2 * i0 - at;   // value of the buffer's first column
+      for (int v = threadIdx.x; v < at + 2 * c; v += blockDim.x) {
+        double x = 0.0;
+#pragma unroll
+        for (int w = 0; w < kGsT / 32; ++w) x += red[w][v];
+        part[(size_t)(first + v) * st.G + blockIdx.x] = x;
+      }
+      __syncthreads();
+    }
   }
 }
 
@@ -264,7 +311,7 @@ __device__ __forceinline__ double* gs_coefficients(const GsDev& st, int q, int j
   if (cached)
     for (int i = 1 + (int)(threadIdx.x >> 5); i < j; i += blockDim.x >> 5)
       for (int k = threadIdx.x & 31; k < i; k += 32) sL[i * (i - 1) / 2 + k] = L[(size_t)i * st.m + k];
-  sum_partials(st.part + (size_t)q * 2 * (st.m + 1) * st.G, st.G, 2 * (j + 1), vals);
+  sum_partials<8>(st.part + (size_t)q * 2 * (st.m + 1) * st.G, st.G, 2 * (j + 1), vals);
   for (int k = threadIdx.x; k <= j; k += blockDim.x) {
     const double sk = sig[k];
     a[k] = sj * sk * vals[2 * k];
@@ -357,7 +404,7 @@ __global__ void __launch_bounds__(kGsT, 1) k_gs_update(size_t n, int j, TV* V, s
   double* part = st.norm_part + (size_t)q * st.G;
   block_sums<1>(&s, 1, red, part + blockIdx.x, st.G);
   if (!last_block(ist + 7)) return;
-  sum_partials(part, st.G, 1, nrm);
+  sum_partials<32>(part, st.G, 1, nrm);
   // the rotations and the state in shared memory before the serial part
   double* cs = d + st.oCs();
   double* g = d + st.oG();
