@@ -314,6 +314,7 @@ __global__ void __launch_bounds__(256, 2) k_grad_pipe(int N, int NB, int nblk, i
   if (i >= nblk) return;
   int a0, a1;
   load_ids(bid(i), a0, a1);
+  pdl_wait();
   issue(bid(i), sm, a0, a1);
   cp_async_commit();
   if (i + (int)gridDim.x < nblk) load_ids(bid(i + gridDim.x), a0, a1);
@@ -456,7 +457,7 @@ __global__ void k_edge_flux(int E, Gas g, int rec, double beta, int failsafe, co
 // launch of their own (thread per face, its three nodes one after the
 // other) they took 8 us of a 47^3 residual and 17 us at 101^3.
 constexpr int kFaceItems = 4;  // per thread
-__device__ __forceinline__ void face_items(const Gas& g, const FaceArgs& fa, const double* __restrict__ P, int blk) {
+__device__ __forceinline__ void face_items(const Gas& g, const FaceArgs& fa, const double* P, int blk) {
   const double third = 1.0 / 3.0;
   double Ub[5];
 #pragma unroll
@@ -476,6 +477,70 @@ __device__ __forceinline__ void face_items(const Gas& g, const FaceArgs& fa, con
   }
 }
 
+// The same sums in the blocked organisation: every edge is evaluated once
+// (both endpoints' terms min(+-un - a, 0) S of the mean state) by the block
+// of its first endpoint, from staged node states; the two terms stay in
+// shared memory for the gather per node, the second endpoint's goes to
+// wspill for a block-crossing edge.  With un S = u.n and a S =
+// sqrt(gam p/rho n.n) an edge takes one reciprocal and one reciprocal square
+// root.  Bound by the 60 bytes per edge; the thread-per-node form
+// (k_timestep) evaluates each edge twice, three roots and a division each,
+// with its normals gathered one component at a time.
+constexpr int kWS = 6;  // doubles per staged state: 48 bytes, conflict-free 16-byte loads
+__device__ __forceinline__ void wave_block(int N, int E, int NB, const Gas& g, const ushort2* __restrict__ bl,
+                                           const double* __restrict__ bn, const int* __restrict__ beptr,
+                                           const int* __restrict__ hfptr, const int* __restrict__ hfpad, int maxHf,
+                                           const double* P2, const int* __restrict__ lptr,
+                                           const int* __restrict__ lidx, const int* __restrict__ xslot, double* wpart,
+                                           double* wspill, int blk, double* sm) {
+  const int n0 = blk * NB, nn = min(NB, N - n0);
+  const int nh = hfptr[blk + 1] - hfptr[blk], ns = nn + nh;
+  const int e0 = beptr[blk], e1 = beptr[blk + 1];
+  double* Vn = sm;                                               // [ns][kWS]
+  double2* Ws = reinterpret_cast<double2*>(sm + kWS * (size_t)ns);  // [e1 - e0] (first, second)
+  const int* hf = hfpad + (size_t)blk * maxHf;
+  pdl_wait();
+  for (int k = threadIdx.x; k < 3 * ns; k += blockDim.x) {
+    const int q = k / 3, c = k - 3 * q;
+    const size_t j = (size_t)(q < nn ? n0 + q : hf[q - nn]);
+    cp_async16(Vn + kWS * q + 2 * c, P2 + 8 * j + 2 * c);
+  }
+  cp_async_wait_all();
+  __syncthreads();
+  for (int q = e0 + threadIdx.x; q < e1; q += blockDim.x) {
+    const ushort2 lq = bl[q];
+    const double nx = bn[q], ny = bn[(size_t)E + q], nz = bn[2 * (size_t)E + q];
+    const int xs = xslot[q];
+    const double2* a = reinterpret_cast<const double2*>(Vn + kWS * lq.x);
+    const double2* b = reinterpret_cast<const double2*>(Vn + kWS * lq.y);
+    const double2 a0 = a[0], a1 = a[1], a2 = a[2], b0 = b[0], b1 = b[1], b2 = b[2];
+    const double rho = 0.5 * (a0.x + b0.x), p = 0.5 * (a2.x + b2.x);
+    const double us = 0.5 * ((a0.y + b0.y) * nx + (a1.x + b1.x) * ny + (a1.y + b1.y) * nz);
+    const double s2 = nx * nx + ny * ny + nz * nz;
+    double2 w = make_double2(0.0, 0.0);
+    if (s2 > 0.0) {
+      const double x = g.gam * p * rcp_(rho) * s2, as = x * rsqrt_(x);
+      w = make_double2(fmin(us - as, 0.0), fmin(-us - as, 0.0));
+    }
+    Ws[q - e0] = w;
+    if (xs >= 0) wspill[xs] = w.y;
+  }
+  __syncthreads();
+  int L = 1;
+  while (2 * L * NB <= (int)blockDim.x) L *= 2;
+  const int t = threadIdx.x / L, r = threadIdx.x % L;
+  const bool act = t < nn && (int)threadIdx.x < L * NB;
+  double s = 0.0;
+  if (act)
+    for (int k = lptr[n0 + t] + r; k < lptr[n0 + t + 1]; k += L) {
+      const int e = lidx[k];
+      const double2 w = Ws[e & 0x7fffffff];
+      s += e < 0 ? w.y : w.x;
+    }
+  for (int o = 1; o < L; o <<= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  if (act && r == 0) wpart[n0 + t] = s;
+}
+
 // BLOCKED organisation: one thread block per NB consecutive (Morton
 // ordered) nodes.  Phase 0: the node records (V, X) and gradients of the
 // block's nodes and of its forward halo (second endpoints of the block's
@@ -487,21 +552,33 @@ __device__ __forceinline__ void face_items(const Gas& g, const FaceArgs& fa, con
 // block also go to spill[].  Phase 2: thread t sums, for node blk*NB+t, its
 // edges held in shared memory in ascending edge order (+ as first endpoint,
 // - as second) into part[].
+// The launches of a residual and of an explicit step overlap (launch_pdl):
+// a kernel reads its block's bounds and lists before it waits for the one
+// before.  With the wave sums in the same launch (rk2_blocked_dev) ten steps
+// of 21^3 take 334 instead of 447 us; the residual of 47^3 83.5 instead of 90
+// us; 101^3 is the same.
 template <int THREADS, int MINB>
 __global__ void __launch_bounds__(THREADS, MINB)
     k_fv_blocked(int N, int E, int NB, Gas g, int rec, double beta, int failsafe,
                                                     const ushort2* __restrict__ bl, const double* __restrict__ bn,
                                                     const int* __restrict__ beptr, const int* __restrict__ hfptr,
-                                                    const int* __restrict__ hfpad, int maxHf,
-                                                    const double* __restrict__ P,
-                                                    const double* __restrict__ G, const int* __restrict__ lptr,
+                                                    const int* __restrict__ hfpad, int maxHf, const double* P,
+                                                    const double* G, const int* __restrict__ lptr,
                                                     const int* __restrict__ lidx, const int* __restrict__ xslot,
                                                     double* __restrict__ part, double* __restrict__ spill,
                                                     int* __restrict__ tag, int* __restrict__ counters,
-                                                    const int* __restrict__ blist, int nmain, FaceArgs fa) {
+                                                    const int* __restrict__ blist, int nmain, FaceArgs fa, int nwave,
+                                                    double* __restrict__ wpart, double* __restrict__ wspill) {
   extern __shared__ double sm[];
+  pdl_trigger();
   if ((int)blockIdx.x >= nmain) {
-    face_items(g, fa, P, (int)blockIdx.x - nmain);
+    const int x = (int)blockIdx.x - nmain;
+    if (x < nwave) {
+      wave_block(N, E, NB, g, bl, bn, beptr, hfptr, hfpad, maxHf, P, lptr, lidx, xslot, wpart, wspill, x, sm);
+    } else {
+      pdl_wait();
+      face_items(g, fa, P, x - nwave);
+    }
     return;
   }
   const int blk = blist ? blist[blockIdx.x] : blockIdx.x;
@@ -523,6 +600,7 @@ __global__ void __launch_bounds__(THREADS, MINB)
   int* hs = reinterpret_cast<int*>(Fs + 5 * (e1 - e0));  // [nh] halo node ids
   const int* hf = hfpad + (size_t)blk * maxHf;            // addresses from the block index alone
   for (int k = threadIdx.x; k < nh; k += blockDim.x) hs[k] = hf[k];
+  pdl_wait();
   {
     const bool grad = rec != AEROF_REC_CONSTANT;
     // own nodes: contiguous records
@@ -682,23 +760,23 @@ __global__ void k_fv_nodes_list(int N, Gas g, const int* __restrict__ n2o, const
 // fluxes and the subface fluxes are contiguous, and four spills are in
 // flight per lane.  The first thread hands the unphysical count to the host
 // (pub) and re-arms the counter: the edge sweep is complete.
-__global__ void __launch_bounds__(256) k_fv_nodes5(int N, const int* __restrict__ n2o, const double* __restrict__ part,
-                                                   const int* __restrict__ xin_ptr, const double* __restrict__ spill,
+__global__ void __launch_bounds__(256) k_fv_nodes5(int N, const int* __restrict__ n2o, const double* part,
+                                                   const int* __restrict__ xin_ptr, const double* spill,
                                                    const int* __restrict__ bnf_ptr, const int* __restrict__ bnf_ent,
-                                                   const double* __restrict__ fbuf, const double* __restrict__ vol2,
-                                                   double* __restrict__ R, int* __restrict__ cnt,
-                                                   volatile int* __restrict__ pub) {
+                                                   const double* fbuf, const double* __restrict__ vol2,
+                                                   double* R, int* cnt, volatile int* pub) {
   const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (pub && t == 0) {
-    *pub = *cnt;
-    *cnt = 0;
-  }
   const int n = (int)(t / 5), c = (int)(t - 5 * (unsigned)n);
   if (n >= N) return;
   int k = xin_ptr[n];
   const int k1 = xin_ptr[n + 1], q0 = bnf_ptr[n], q1 = bnf_ptr[n + 1];
   const double iv = 1.0 / vol2[n];
   const size_t o = (size_t)n2o[n];
+  pdl_wait();
+  if (pub && t == 0) {
+    *pub = *cnt;
+    *cnt = 0;
+  }
   double acc = part[(size_t)t];
   for (; k + 4 <= k1; k += 4) {
     const double* sp = spill + 5 * (size_t)k + c;
@@ -931,76 +1009,21 @@ __global__ void k_timestep(int N, int E, int F, Gas g, double cfl, const int2* _
   dt[i] = cfl * vol[i] / (-1.0 * idti);
 }
 
-// The same sums in the blocked organisation: every edge is evaluated once
-// (both endpoints' terms min(+-un - a, 0) S of the mean state) by the block
-// of its first endpoint, from staged node states; the two terms stay in
-// shared memory for the gather per node, the second endpoint's goes to
-// wspill for a block-crossing edge.  With un S = u.n and a S =
-// sqrt(gam p/rho n.n) an edge takes one reciprocal and one reciprocal square
-// root.  Bound by the 60 bytes per edge; the thread-per-node form
-// (k_timestep) evaluates each edge twice, three roots and a division each,
-// with its normals gathered one component at a time.
-constexpr int kWS = 6;  // doubles per staged state: 48 bytes, conflict-free 16-byte loads
 __global__ void __launch_bounds__(256) k_wave_blocked(int N, int E, int NB, Gas g, const ushort2* __restrict__ bl,
                                                       const double* __restrict__ bn, const int* __restrict__ beptr,
                                                       const int* __restrict__ hfptr, const int* __restrict__ hfpad,
-                                                      int maxHf, const double* __restrict__ P2,
-                                                      const int* __restrict__ lptr, const int* __restrict__ lidx,
-                                                      const int* __restrict__ xslot, double* __restrict__ wpart,
-                                                      double* __restrict__ wspill) {
+                                                      int maxHf, const double* P2, const int* __restrict__ lptr,
+                                                      const int* __restrict__ lidx, const int* __restrict__ xslot,
+                                                      double* wpart, double* wspill) {
   extern __shared__ double sm[];
-  const int blk = blockIdx.x;
-  const int n0 = blk * NB, nn = min(NB, N - n0);
-  const int nh = hfptr[blk + 1] - hfptr[blk], ns = nn + nh;
-  const int e0 = beptr[blk], e1 = beptr[blk + 1];
-  double* Vn = sm;                                               // [ns][kWS]
-  double2* Ws = reinterpret_cast<double2*>(sm + kWS * (size_t)ns);  // [e1 - e0] (first, second)
-  const int* hf = hfpad + (size_t)blk * maxHf;
-  for (int k = threadIdx.x; k < 3 * ns; k += blockDim.x) {
-    const int q = k / 3, c = k - 3 * q;
-    const size_t j = (size_t)(q < nn ? n0 + q : hf[q - nn]);
-    cp_async16(Vn + kWS * q + 2 * c, P2 + 8 * j + 2 * c);
-  }
-  cp_async_wait_all();
-  __syncthreads();
-  for (int q = e0 + threadIdx.x; q < e1; q += blockDim.x) {
-    const ushort2 lq = bl[q];
-    const double nx = bn[q], ny = bn[(size_t)E + q], nz = bn[2 * (size_t)E + q];
-    const int xs = xslot[q];
-    const double2* a = reinterpret_cast<const double2*>(Vn + kWS * lq.x);
-    const double2* b = reinterpret_cast<const double2*>(Vn + kWS * lq.y);
-    const double2 a0 = a[0], a1 = a[1], a2 = a[2], b0 = b[0], b1 = b[1], b2 = b[2];
-    const double rho = 0.5 * (a0.x + b0.x), p = 0.5 * (a2.x + b2.x);
-    const double us = 0.5 * ((a0.y + b0.y) * nx + (a1.x + b1.x) * ny + (a1.y + b1.y) * nz);
-    const double s2 = nx * nx + ny * ny + nz * nz;
-    double2 w = make_double2(0.0, 0.0);
-    if (s2 > 0.0) {
-      const double x = g.gam * p * rcp_(rho) * s2, as = x * rsqrt_(x);
-      w = make_double2(fmin(us - as, 0.0), fmin(-us - as, 0.0));
-    }
-    Ws[q - e0] = w;
-    if (xs >= 0) wspill[xs] = w.y;
-  }
-  __syncthreads();
-  int L = 1;
-  while (2 * L * NB <= (int)blockDim.x) L *= 2;
-  const int t = threadIdx.x / L, r = threadIdx.x % L;
-  const bool act = t < nn && (int)threadIdx.x < L * NB;
-  double s = 0.0;
-  if (act)
-    for (int k = lptr[n0 + t] + r; k < lptr[n0 + t + 1]; k += L) {
-      const int e = lidx[k];
-      const double2 w = Ws[e & 0x7fffffff];
-      s += e < 0 ? w.y : w.x;
-    }
-  for (int o = 1; o < L; o <<= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  if (act && r == 0) wpart[n0 + t] = s;
+  pdl_trigger();
+  wave_block(N, E, NB, g, bl, bn, beptr, hfptr, hfpad, maxHf, P2, lptr, lidx, xslot, wpart, wspill, blockIdx.x, sm);
 }
 
 // Node n's whole sum (block part, spilled terms, boundary faces with a third
 // of their area): the time step is cfl vol / (-sum).
-__device__ __forceinline__ double wave_sum(int n, const Gas& g, const double* __restrict__ wpart,
-                                           const int* __restrict__ xin_ptr, const double* __restrict__ wspill,
+__device__ __forceinline__ double wave_sum(int n, const Gas& g, const double* wpart,
+                                           const int* __restrict__ xin_ptr, const double* wspill,
                                            const int* __restrict__ bnf_ptr, const int* __restrict__ bnf_ent, int F,
                                            const double* __restrict__ fn, const double* P2) {
   double s = wpart[n];
@@ -1039,24 +1062,26 @@ __global__ void k_wave_dt(int N, Gas g, double cfl, const int* __restrict__ n2o,
 // of boundary nodes).
 template <int STAGE>
 __global__ void __launch_bounds__(256) k_rk_nodes(int N, Gas g, double cfl, const int* __restrict__ n2o,
-                                                  const double* __restrict__ part, const int* __restrict__ xin_ptr,
-                                                  const double* __restrict__ spill, const double* __restrict__ wpart,
-                                                  const double* __restrict__ wspill, const int* __restrict__ bnf_ptr,
-                                                  const int* __restrict__ bnf_ent, const double* __restrict__ fbuf,
-                                                  int F, const double* __restrict__ fn,
-                                                  const double* __restrict__ vol2, double* __restrict__ dt2,
-                                                  double* __restrict__ k1, double* __restrict__ U, double* P2) {
+                                                  const double* part, const int* __restrict__ xin_ptr,
+                                                  const double* spill, const double* wpart, const double* wspill,
+                                                  const int* __restrict__ bnf_ptr, const int* __restrict__ bnf_ent,
+                                                  const double* fbuf, int F, const double* __restrict__ fn,
+                                                  const double* __restrict__ vol2, double* dt2, double* k1, double* U,
+                                                  double* P2) {
+  pdl_trigger();
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const bool act = (t >> 3) < N;
   const int n = act ? (int)(t >> 3) : N - 1, c = (int)(t & 7), lane0 = threadIdx.x & 24;
   const double vol = vol2[n], invcv = 1.0 / vol;
   const size_t o = (size_t)n2o[n];
+  const int x0 = xin_ptr[n], x1 = xin_ptr[n + 1], q0 = bnf_ptr[n], q1 = bnf_ptr[n + 1];
+  pdl_wait();
   double acc = 0.0, u = 0.0;
   if (c < 5) {
     u = U[5 * o + c];
     acc = part[5 * (size_t)n + c];
-    for (int k = xin_ptr[n]; k < xin_ptr[n + 1]; ++k) acc -= spill[5 * (size_t)k + c];
-    for (int q = bnf_ptr[n]; q < bnf_ptr[n + 1]; ++q) acc += fbuf[5 * (size_t)bnf_ent[q] + c];
+    for (int k = x0; k < x1; ++k) acc -= spill[5 * (size_t)k + c];
+    for (int q = q0; q < q1; ++q) acc += fbuf[5 * (size_t)bnf_ent[q] + c];
   } else if (c == 5) {
     acc = STAGE == 1 ? cfl * vol / (-1.0 * wave_sum(n, g, wpart, xin_ptr, wspill, bnf_ptr, bnf_ent, F, fn, P2))
                      : dt2[n];
@@ -1213,9 +1238,8 @@ static void launch_grad_pipe(aerof_gpu_ctx* c, const Gas& g, const double* dU, c
       m.grad_grid = std::max(per_sm, 1) * sms;
     }
     const int grid = std::max(1, std::min(m.nblk, m.grad_grid));
-    kern<<<grid, kBlock, smem, s>>>(m.N, m.NB, m.nblk, m.maxH, m.maxLp, st, P2src, m.W2.p, m.nb2_ptr.p, m.lpad.p,
-                                    m.hpad.p, tag, G2, nullptr);
-    AEROF_LAUNCH_CHECK();
+    launch_pdl(kern, grid, kBlock, smem, s, m.N, m.NB, m.nblk, m.maxH, m.maxLp, st, P2src, m.W2.p, m.nb2_ptr.p,
+               m.lpad.p, m.hpad.p, tag, G2, nullptr);
   };
   if (L == 4) go(k_grad_pipe<4>);
   else if (L == 2) go(k_grad_pipe<2>);
@@ -1296,7 +1320,7 @@ void grad_records_blocked_dev(aerof_gpu_ctx* c, const double* P2src, double* G2d
 // Edge fluxes of the blocked organisation from P2 and G2 into part and
 // spill, and the boundary subface fluxes into fbuf; counter: where
 // unphysical states are counted.
-static void fv_blocked_dev(aerof_gpu_ctx* c, int failsafe, int* counter) {
+static void fv_blocked_dev(aerof_gpu_ctx* c, int failsafe, int* counter, bool wave = false) {
   DeviceMesh& m = c->mesh;
   const FaceArgs fa{m.F, m.Ubd.p, m.faces.p, m.fcode.p, m.fnrm.p, m.o2n.p, c->s.fbuf.p};
   const size_t smem = fv_blocked_smem(m);
@@ -1316,12 +1340,11 @@ static void fv_blocked_dev(aerof_gpu_ctx* c, int failsafe, int* counter) {
   auto fvk = wide ? k_fv_blocked<512, 2>
                   : by_smem >= 4 ? k_fv_blocked<256, 4> : by_smem == 3 ? k_fv_blocked<256, 3> : k_fv_blocked<256, 2>;
   AEROF_CUDA(cudaFuncSetAttribute(fvk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  const int nface = grid_for(3 * (size_t)m.F, fv_threads * kFaceItems);
-  fvk<<<m.nblk + nface, fv_threads, smem, c->stream>>>(m.N, m.E, m.NB, make_gas(c->cfg.gamma), c->cfg.reconstruction,
-                                               c->cfg.beta, failsafe, m.bl.p, m.bnorm.p, m.beptr.p, m.hfptr.p,
-                                               m.hfpad.p, m.maxHf, m.P2.p, c->s.G2.p, m.lptr.p, m.lidx.p, m.xslot.p,
-                                               c->s.part.p, c->s.spill.p, c->s.tag.p, counter, nullptr, m.nblk, fa);
-  AEROF_LAUNCH_CHECK();
+  const int nface = grid_for(3 * (size_t)m.F, fv_threads * kFaceItems), nwave = wave ? m.nblk : 0;
+  launch_pdl(fvk, m.nblk + nwave + nface, fv_threads, smem, c->stream, m.N, m.E, m.NB, make_gas(c->cfg.gamma),
+             c->cfg.reconstruction, c->cfg.beta, failsafe, m.bl.p, m.bnorm.p, m.beptr.p, m.hfptr.p, m.hfpad.p, m.maxHf,
+             m.P2.p, c->s.G2.p, m.lptr.p, m.lidx.p, m.xslot.p, c->s.part.p, c->s.spill.p, c->s.tag.p, counter, nullptr,
+             m.nblk, fa, nwave, c->s.wpart.p, c->s.wspill.p);
 }
 
 // BLOCKED organisation of residual_dev (see k_fv_blocked).
@@ -1377,10 +1400,8 @@ static int residual_blocked_dev(aerof_gpu_ctx* c, const double* dU, double* dR, 
   }
   {
     TimerScope t(c, AEROF_T_FV_TERM);
-    k_fv_nodes5<<<grid_for(5 * (size_t)m.N, kBlock), kBlock, 0, s>>>(m.N, m.n2o.p, c->s.part.p, m.xin_ptr.p,
-                                                                     c->s.spill.p, m.bnf_ptr.p, m.bnf_ent.p,
-                                                                     c->s.fbuf.p, m.vol2.p, dR, cnt, pub);
-    AEROF_LAUNCH_CHECK();
+    launch_pdl(k_fv_nodes5, grid_for(5 * (size_t)m.N, kBlock), kBlock, 0, s, m.N, m.n2o.p, c->s.part.p, m.xin_ptr.p,
+               c->s.spill.p, m.bnf_ptr.p, m.bnf_ent.p, c->s.fbuf.p, m.vol2.p, dR, cnt, pub);
     if (pub) c->s.count_clear = true;
     galerkin_add(c, dU, dR);
   }
@@ -1474,8 +1495,8 @@ int residual_dev(aerof_gpu_ctx* c, const double* dU, double* dR, int mode) {
 // storing into R through its device address.  The conversion runs per
 // node (k_prim_nodes), the gradients per block (k_grad_pipe) or per node
 // (k_grad_nodes, with the block kernel's lanes and order), the fluxes and
-// assembly per block (k_fv_blocked, k_fv_nodes_b with the boundary fluxes
-// of k_face_flux inside): the same arithmetic as residual_blocked_dev, so
+// assembly per block (k_fv_blocked, k_fv_nodes_list with the boundary fluxes
+// inside): the same arithmetic as residual_blocked_dev, so
 // the same residual bit for bit.  Each stage's kernels are replayed as one
 // CUDA graph.  Used for page-locked host U and R with the blocked kernel,
 // failsafe off, no viscous term and timers off, on meshes of at least
@@ -1634,7 +1655,7 @@ static void stage_kernels(aerof_gpu_ctx* c, ResidualPipe& p, int st, cudaStream_
   if (nl) {
     fvk<<<nl, 256, fsmem, s>>>(m.N, m.E, m.NB, g, rec, c->cfg.beta, 0, m.bl.p, m.bnorm.p, m.beptr.p, m.hfptr.p,
                                m.hfpad.p, m.maxHf, m.P2.p, c->s.G2.p, m.lptr.p, m.lidx.p, m.xslot.p, c->s.part.p,
-                               c->s.spill.p, c->s.tag.p, cnt, lp, nl, FaceArgs{});
+                               c->s.spill.p, c->s.tag.p, cnt, lp, nl, FaceArgs{}, 0, nullptr, nullptr);
     AEROF_LAUNCH_CHECK();
   }
   lp = seg(3, nl);
@@ -1810,10 +1831,9 @@ static void wave_blocked_dev(aerof_gpu_ctx* c) {
   c->s.wspill.ensure(std::max(m.nX, 1));
   const size_t smem = wave_smem(m);
   AEROF_CUDA(cudaFuncSetAttribute(k_wave_blocked, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  k_wave_blocked<<<m.nblk, 256, smem, c->stream>>>(m.N, m.E, m.NB, make_gas(c->cfg.gamma), m.bl.p, m.bnorm.p,
-                                                   m.beptr.p, m.hfptr.p, m.hfpad.p, m.maxHf, m.P2.p, m.lptr.p,
-                                                   m.lidx.p, m.xslot.p, c->s.wpart.p, c->s.wspill.p);
-  AEROF_LAUNCH_CHECK();
+  launch_pdl(k_wave_blocked, m.nblk, 256, smem, c->stream, m.N, m.E, m.NB, make_gas(c->cfg.gamma), m.bl.p, m.bnorm.p,
+             m.beptr.p, m.hfptr.p, m.hfpad.p, m.maxHf, m.P2.p, m.lptr.p, m.lidx.p, m.xslot.p, c->s.wpart.p,
+             c->s.wspill.p);
 }
 
 void timestep_dev(aerof_gpu_ctx* c, const double* dU, double cfl, double* ddt) {
@@ -1855,13 +1875,21 @@ static void rk2_blocked_dev(aerof_gpu_ctx* c, double* dU, double cfl, int nsteps
   const int gn = grid_for(8 * (size_t)m.N, kBlock);
   prim_to_P2(m, g, dU, s);
   auto stage = [&](auto kern) {
-    kern<<<gn, kBlock, 0, s>>>(m.N, g, cfl, m.n2o.p, c->s.part.p, m.xin_ptr.p, c->s.spill.p, c->s.wpart.p,
-                               c->s.wspill.p, m.bnf_ptr.p, m.bnf_ent.p, c->s.fbuf.p, m.F, m.fnrm.p, m.vol2.p,
-                               c->s.dt.p, c->s.k1.p, dU, m.P2.p);
-    AEROF_LAUNCH_CHECK();
+    launch_pdl(kern, gn, kBlock, 0, s, m.N, g, cfl, m.n2o.p, c->s.part.p, m.xin_ptr.p, c->s.spill.p, c->s.wpart.p,
+               c->s.wspill.p, m.bnf_ptr.p, m.bnf_ent.p, c->s.fbuf.p, m.F, m.fnrm.p, m.vol2.p, c->s.dt.p, c->s.k1.p, dU,
+               m.P2.p);
   };
+  // the wave sums as extra blocks of the first stage's edge sweep up to two
+  // rounds of its blocks (296 resident): one launch less per step.  Beyond
+  // that its shared memory holds the wave blocks to two per SM, where their
+  // own launch has six.  Ten first-order steps, own launch against together:
+  // 21^3 (73 blocks) 415 / 342 us, 31^3 (233) 494 / 450, 41^3 (539) 844 / 804,
+  // 61^3 (1,774) 2,502 / 2,693.
+  const bool together = m.nblk <= 592 && wave_smem(m) <= fv_blocked_smem(m);
+  c->s.wpart.ensure(m.N);
+  c->s.wspill.ensure(std::max(m.nX, 1));
   for (int k = 0; k < nsteps; ++k) {
-    {
+    if (!together) {
       TimerScope t(c, AEROF_T_TIME_STEP);
       wave_blocked_dev(c);
     }
@@ -1872,7 +1900,7 @@ static void rk2_blocked_dev(aerof_gpu_ctx* c, double* dU, double cfl, int nsteps
       }
       {
         TimerScope t(c, AEROF_T_FV_EDGES);
-        fv_blocked_dev(c, 0, counter);
+        fv_blocked_dev(c, 0, counter, together && st == 1);
       }
       TimerScope t(c, AEROF_T_FV_TERM);
       if (st == 1) stage(k_rk_nodes<1>);
