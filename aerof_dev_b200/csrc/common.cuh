@@ -282,8 +282,8 @@ struct H1Free {
   bool ready = false;              // node records hold the operator's state
   size_t total = 0;                // neighbour entries, padded per warp
   DBuf<int> wptr;                  // [warps + 1] steps before each warp
-  DBuf<unsigned short> slot;       // [total] neighbour's staged slot
-  DBuf<float> nrm32, rec32;        // [4][total] unit normal, half length; [N][8]
+  DBuf<int> slot;                  // [total] neighbour's staged slot
+  DBuf<float> nrm32, rec32;        // [total][4] unit normal, half length; [N][8]
   DBuf<double> nrm64, rec64;       // the same in FP64; [N][6]
   DBuf<double> mrow, idt, z;       // [N][4] (sum n/2, 1/vol); [N] 1/dt; packed vectors
   void drop_geometry() { geo32 = geo64 = false; }
@@ -565,6 +565,9 @@ void launch_pdl(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStre
   AEROF_LAUNCH_CHECK();
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+template <int N> __device__ __forceinline__ void cp_async_wait_group() {
+  asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
+}
 __device__ __forceinline__ void cp_async_wait_prev() { asm volatile("cp.async.wait_group 1;\n" ::: "memory"); }
 // Bulk prefetch of a contiguous global range into L2 (no destination, no
 // completion to wait for): src 16-byte aligned, bytes a multiple of 16.

@@ -15,7 +15,7 @@
 //   |A| q = |un| q + (S1 b/c^2 + S2 a/c) R1 + (S1 a + S2 b/c) R2,
 // S1 = (|un+c| + |un-c|)/2 - |un|, S2 = (|un+c| - |un-c|)/2 (the projection
 // form of Liu and Vinokur, "Nonequilibrium flow computations", 1989).  So a
-// block-vector product takes ~90 operations on 18 bytes per neighbour (unit
+// block-vector product takes ~90 operations on 20 bytes per neighbour (unit
 // normal, half length, local slot) plus the staged node records, against 25
 // multiplications on a 100-byte FP32 (200-byte FP64) block: the stored
 // product is bound by HBM at ~92 % of the copy rate, this one by issue.
@@ -29,7 +29,12 @@
 // staged in shared memory (48-byte FP32 or 80-byte FP64 records: odd
 // multiples of 16 bytes, conflict-free vector loads); L lanes per node take
 // its neighbours r, r + L, ..., the row sum is FP64 (fixed xor tree).  The
-// per-neighbour data is stored warp by warp, one coalesced line per step.
+// per-neighbour data is stored warp by warp, coalesced per step, and copied
+// to shared memory four steps ahead, before the wait for the packed vector.  Requested one step ahead into registers, its latency was
+// most of the kernel (seven of thirteen warps waited for it per issue; 47 us
+// at 61^3): a pseudo-time step of 81^3 with 20 FP32 iterations 4.91 -> 4.69
+// ms, five Newton steps of 61^3 15.0 -> 14.8 ms with eight steps and three
+// CTAs per SM; four steps and four CTAs (64 registers) 4.43 ms and 14.0 ms.
 #pragma once
 
 #include "common.cuh"
@@ -39,8 +44,9 @@ namespace aerof {
 
 // widths (elements) of a node's record and of a packed vector row
 template <class S> struct H1Rec;
-template <> struct H1Rec<float> { static constexpr int W = 8, SM = 12; };
-template <> struct H1Rec<double> { static constexpr int W = 6, SM = 10; };
+// and the steps of neighbour data in flight per lane of the product kernel
+template <> struct H1Rec<float> { static constexpr int W = 8, SM = 12, D = 4; };
+template <> struct H1Rec<double> { static constexpr int W = 6, SM = 10, D = 4; };
 
 // (sqrt rho, u, v, w, H) of every node, blocked numbering, from the caller's
 // primitive records; and 1/dt (0 without time steps)
@@ -66,7 +72,7 @@ __global__ void k_h1_records(int N, Gas g, const int* __restrict__ n2o, const do
 
 // Per-neighbour data of every node, in the order the product kernel reads
 // it (warp w's step k, lane l at (wptr[w] + k) 32 + l): outward unit normal
-// and half length, SoA [4][total], and the neighbour's staged slot; entries
+// and half length, four values, and the neighbour's staged slot; entries
 // past a node's list have zero length and its own slot.  mrow[n]: (sum of
 // n/2, 1/vol).  Thread per lane of the product kernel.
 template <class S>
@@ -74,8 +80,8 @@ __global__ void k_h1_geometry(int N, int NB, int E, const int* __restrict__ n2o,
                               const int* __restrict__ nbr_ptr, const int* __restrict__ nbr_node,
                               const int* __restrict__ nbr_edge, const double* __restrict__ en,
                               const int* __restrict__ hptr, const int* __restrict__ hnode,
-                              const double* __restrict__ vol, const int* __restrict__ wptr, size_t total,
-                              S* __restrict__ nrm, unsigned short* __restrict__ slot, double* __restrict__ mrow) {
+                              const double* __restrict__ vol, const int* __restrict__ wptr, S* __restrict__ nrm,
+                              int* __restrict__ slot, double* __restrict__ mrow) {
   const int blk = blockIdx.x, L = blockDim.x / NB;
   const int t = threadIdx.x / L, r = threadIdx.x % L;
   const int n0 = blk * NB, nn = min(NB, N - n0);
@@ -111,8 +117,8 @@ __global__ void k_h1_geometry(int N, int NB, int E, const int* __restrict__ n2o,
       }
     }
 #pragma unroll
-    for (int a = 0; a < 4; ++a) nrm[a * total + at] = (S)u[a];
-    slot[at] = (unsigned short)sl;
+    for (int a = 0; a < 4; ++a) nrm[4 * at + a] = (S)u[a];
+    slot[at] = sl;
   }
   if (!act || r != 0) return;
   double m[3] = {0.0, 0.0, 0.0};
@@ -167,23 +173,38 @@ __device__ __forceinline__ double h1_abs(double x) { return fabs(x); }
 // y = H1 z (TR: H1^T with z packed as p/vol), system blockIdx.y; y in the
 // caller's numbering.  skip: flags, one per 8 ints.
 template <class S, bool TR>
-__global__ void __launch_bounds__(256, sizeof(S) == 4 ? 3 : 2)
+__global__ void __launch_bounds__(256, sizeof(S) == 4 ? 4 : 2)
     k_h1_apply(int N, int NB, Gas g, const int* __restrict__ n2o, const int* __restrict__ hptr,
-               const int* __restrict__ hnode, const int* __restrict__ wptr, size_t total,
-               const S* __restrict__ nrm, const unsigned short* __restrict__ slot, const double* __restrict__ mrow,
+               const int* __restrict__ hnode, const int* __restrict__ wptr, const S* __restrict__ nrm,
+               const int* __restrict__ slot, const double* __restrict__ mrow,
                const S* __restrict__ rec, const double* __restrict__ idt, const int* __restrict__ brow,
                const double* __restrict__ fsum, const S* z, size_t zs, S* __restrict__ y, size_t ys, const int* skip) {
   extern __shared__ __align__(16) char raw[];
   const int q = blockIdx.y;
   pdl_trigger();
-  constexpr int W = H1Rec<S>::W, SM = H1Rec<S>::SM;
-  S* sm = reinterpret_cast<S*>(raw);
+  constexpr int W = H1Rec<S>::W, SM = H1Rec<S>::SM, D = H1Rec<S>::D;
+  // a ring of D steps of neighbour data per lane, then the staged nodes
+  S* rn = reinterpret_cast<S*>(raw) + 4 * threadIdx.x;                         // step d: + 4 d blockDim.x
+  int* rs = reinterpret_cast<int*>(raw + (size_t)4 * sizeof(S) * D * blockDim.x) + threadIdx.x;
+  S* sm = reinterpret_cast<S*>(raw + (size_t)(4 * sizeof(S) + sizeof(int)) * D * blockDim.x);
   const int blk = blockIdx.x, L = blockDim.x / NB;
   const int n0 = blk * NB, nn = min(NB, N - n0);
   const int h0 = hptr[blk], ns = nn + hptr[blk + 1] - h0;
   const S* zq = z + (size_t)q * zs;
-  // the node records and the first step's neighbour data do not depend on
-  // the kernel before (the one that packs z)
+  const int t = threadIdx.x / L, r = threadIdx.x % L;
+  const bool act = t < nn;
+  const int gw = blk * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  const int w0 = wptr[gw], steps = wptr[gw + 1] - w0;
+  const size_t at = (size_t)w0 * 32 + (threadIdx.x & 31);
+  auto issue = [&](int k) {
+    const int d = k % D * blockDim.x;
+    cp_async16(rn + 4 * d, nrm + 4 * (at + 32 * (size_t)k));
+    if constexpr (sizeof(S) == 8) cp_async16(rn + 4 * d + 2, nrm + 4 * (at + 32 * (size_t)k) + 2);
+    cp_async4(rs + d, slot + at + 32 * (size_t)k);
+  };
+  // the neighbour data and the node records do not depend on the kernel
+  // before (the one that packs z)
+  for (int k = 0; k < min(D, steps); ++k) issue(k);
   for (int k = threadIdx.x; k < ns; k += blockDim.x) {
     const size_t j = (size_t)W * (k < nn ? n0 + k : hnode[h0 + k - nn]);
     S* d = sm + SM * k;
@@ -212,18 +233,6 @@ __global__ void __launch_bounds__(256, sizeof(S) == 4 ? 3 : 2)
       p[0] = e.x; p[1] = e.y; p[2] = h.x; p[3] = h.y; p[4] = c.y;
     }
   };
-  const int t = threadIdx.x / L, r = threadIdx.x % L;
-  const bool act = t < nn;
-  const int gw = blk * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  const int w0 = wptr[gw], steps = wptr[gw + 1] - w0;
-  size_t at = (size_t)w0 * 32 + (threadIdx.x & 31);
-  // each step's neighbour data is requested one step ahead
-  S e0 = 0, e1 = 0, e2 = 0, hl = 0;
-  int sl = 0;
-  if (steps > 0) {
-    e0 = nrm[at]; e1 = nrm[total + at]; e2 = nrm[2 * total + at]; hl = nrm[3 * total + at];
-    sl = slot[at];
-  }
   pdl_wait();
   if (skip && skip[8 * q]) {
     cp_async_wait_all();
@@ -250,13 +259,23 @@ __global__ void __launch_bounds__(256, sizeof(S) == 4 ? 3 : 2)
   double acc[5] = {0, 0, 0, 0, 0};
 #pragma unroll 1
   for (int k = 0; k < steps; ++k) {
-    const S x0 = e0, x1 = e1, x2 = e2, hk = hl;
-    const int s = sl;
-    if (k + 1 < steps) {
-      at += 32;
-      e0 = nrm[at]; e1 = nrm[total + at]; e2 = nrm[2 * total + at]; hl = nrm[3 * total + at];
-      sl = slot[at];
+    // (a slot of the ring is refilled an iteration after it was read)
+    if (steps > D && k > 0) {
+      if (k - 1 + D < steps) issue(k - 1 + D);
+      cp_async_commit();
+      if (k >= D) cp_async_wait_group<D - 1>();
     }
+    const int d = k % D * blockDim.x;
+    const S* e = rn + 4 * d;
+    S x0, x1, x2, hk;
+    if constexpr (sizeof(S) == 4) {
+      const float4 f = *reinterpret_cast<const float4*>(e);
+      x0 = f.x; x1 = f.y; x2 = f.z; hk = f.w;
+    } else {
+      const double2 f = reinterpret_cast<const double2*>(e)[0], h = reinterpret_cast<const double2*>(e)[1];
+      x0 = f.x; x1 = f.y; x2 = h.x; hk = h.y;
+    }
+    const int s = rs[d];
     S ss[5], ps[5];
     load(s, ss, ps);
     // Roe average

@@ -587,8 +587,11 @@ static size_t sl_off_size(const DeviceMesh& m) { return std::max<size_t>((size_t
 
 // shared memory of the state-based product for this mesh
 static size_t h1_smem(const DeviceMesh& m, int precision) {
-  const size_t w = precision == AEROF_PREC_FP32 ? sizeof(float) * H1Rec<float>::SM : sizeof(double) * H1Rec<double>::SM;
-  return w * (m.NB + m.maxH);
+  const bool f32 = precision == AEROF_PREC_FP32;
+  const size_t w = f32 ? sizeof(float) * H1Rec<float>::SM : sizeof(double) * H1Rec<double>::SM;
+  const size_t ring = f32 ? (4 * sizeof(float) + sizeof(int)) * H1Rec<float>::D
+                          : (4 * sizeof(double) + sizeof(int)) * H1Rec<double>::D;
+  return w * (m.NB + m.maxH) + ring * kIB;
 }
 static bool h1_fits(const DeviceMesh& m, int precision) {
   return kIB % m.NB == 0 && kIB / m.NB <= 32 && h1_smem(m, precision) <= 200 * 1024;
@@ -628,8 +631,7 @@ static void h1_geometry(aerof_gpu_ctx* c, int precision) {
     using S = std::remove_pointer_t<decltype(nrm.p)>;
     nrm.alloc(4 * f.total);
     k_h1_geometry<S><<<m.nblk, kIB, 0, s>>>(m.N, m.NB, m.E, m.n2o.p, m.o2n.p, m.nbr_ptr.p, m.nbr_node.p, m.nbr_edge.p,
-                                            m.en.p, m.hptr.p, m.hnode.p, m.vol.p, f.wptr.p, f.total, nrm.p, f.slot.p,
-                                            f.mrow.p);
+                                            m.en.p, m.hptr.p, m.hnode.p, m.vol.p, f.wptr.p, nrm.p, f.slot.p, f.mrow.p);
     AEROF_LAUNCH_CHECK();
     // complete before the solvers' overlapping launches, which read it early
     AEROF_CUDA(cudaStreamSynchronize(s));
@@ -1272,7 +1274,7 @@ static void h1_precond_product(aerof_gpu_ctx* c, int R, const TV* x, size_t xs, 
   auto kern = trans ? k_h1_apply<TV, true> : k_h1_apply<TV, false>;
   AEROF_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   launch_pdl(kern, dim3(m.nblk, R), kIB, smem, s, m.N, m.NB, make_gas(c->cfg.gamma), m.n2o.p, m.hptr.p, m.hnode.p,
-             f.wptr.p, f.total, nrm, f.slot.p, f.mrow.p, rec, f.idt.p, m.brow.p, J.fsum.p, zp, pz, y, ys, skip);
+             f.wptr.p, nrm, f.slot.p, f.mrow.p, rec, f.idt.p, m.brow.p, J.fsum.p, zp, pz, y, ys, skip);
 }
 
 // Device state of R systems with restart length m over vectors of n
