@@ -873,10 +873,14 @@ __global__ void k_ilu_factor(int i0, int cnt, int s0, const int* __restrict__ rj
 }
 
 // lusol sweeps for one colour and the vectors q0 = RB blockIdx.y, ... of a
-// batch of R (vector q at x + q xs, z + q zs, work vector w + q ldw; skip:
-// flags, one per 8 ints, flagged vectors are left out): L lanes per row
-// (entries r, r + L, ... of the row, fixed xor-tree lane sum), row t of the
-// colour in slice s0 + t / 32 at lane t % 32.
+// batch of R (vector q at x + q xs, z + q zs; skip: flags, one per 8 ints,
+// flagged vectors are left out): eight lanes per row, RB of them side by side
+// for the vectors (lane % RB) and 8 / RB for the row's entries (h, h + 8 / RB,
+// ..., fixed xor-tree sum); row t of the colour in slice s0 + t / 32 at lane
+// t % 32.  The work vectors of a group are interleaved, w[i][5][RB], so that
+// the lanes of an entry read one sector per component: with a vector after
+// the other in one lane, the gathers of w were 20 loads of 32 separate lines
+// per warp and entry, and bound the sweeps.
 //   Forward: w_i = x_(perm i) - sum_{k<i} L_ik w_k.
 //   Backward: w_i = U_ii^-1 (w_i - sum_{j>i} U_ij w_j), also written to z in
 //   the caller's numbering.
@@ -886,42 +890,10 @@ __global__ void k_ilu_factor(int i0, int cnt, int s0, const int* __restrict__ rj
 // backward, its diagonal are requested before the wait for the previous
 // colour, and only w is read after it.  41^3, eight colours, four FP32
 // vectors: a colour took 11.2 us with four lanes per row and ordinary
-// launches, 47 of the 98 ms of four sensitivities; these 8 us (87.6 ms).
+// launches, 47 of the 98 ms of four sensitivities; overlapping launches and
+// eight lanes per row 87.6 ms; the vectors interleaved 80.9 ms.
 constexpr int kIluLanes = 8;
 constexpr int kIluT = 128;
-// the lanes' sums of RB vectors: with four vectors the lanes exchange halves
-// (20 shuffles where a tree over every value takes 60) and lane sub ends with
-// vector ilu_vec(sub); with one vector every lane has it
-template <int RB> __device__ __forceinline__ int ilu_vec(int sub) { return RB == 4 ? 2 * (sub & 1) + (sub >> 1 & 1) : 0; }
-template <int RB>
-__device__ __forceinline__ void ilu_lane_sums(int sub, const double (*acc)[5], double* out) {
-  if constexpr (RB == 4) {
-    double b[2][5];
-#pragma unroll
-    for (int q = 0; q < 2; ++q)
-#pragma unroll
-      for (int c = 0; c < 5; ++c) {
-        const double keep = sub & 1 ? acc[q + 2][c] : acc[q][c], give = sub & 1 ? acc[q][c] : acc[q + 2][c];
-        b[q][c] = keep + __shfl_xor_sync(0xffffffffu, give, 1);
-      }
-#pragma unroll
-    for (int c = 0; c < 5; ++c) {
-      const double keep = sub & 2 ? b[1][c] : b[0][c], give = sub & 2 ? b[0][c] : b[1][c];
-      out[c] = keep + __shfl_xor_sync(0xffffffffu, give, 2);
-    }
-#pragma unroll
-    for (int c = 0; c < 5; ++c) out[c] += __shfl_xor_sync(0xffffffffu, out[c], 4);
-  } else {
-    static_assert(RB == 1, "one or four vectors");
-#pragma unroll
-    for (int c = 0; c < 5; ++c) {
-      double t = acc[0][c];
-#pragma unroll
-      for (int o = 1; o < kIluLanes; o <<= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-      out[c] = t;
-    }
-  }
-}
 // a row's block as stored (load_block without the conversion: FP32 blocks
 // requested ahead take half the registers)
 template <class S>
@@ -938,41 +910,50 @@ __device__ __forceinline__ void ilu_block(const S* __restrict__ b, int lane, S* 
   }
   a[24] = b[768 + lane];
 }
-// acc -= sum of the row's entries k0 + sub, + L, ... < k1 times w; the first
-// entry's block and column were requested by the caller
+// v = sum over the row's lanes of -(entry k) w_(column k), k = k0 + h, + NH,
+// ... < k1; the first entry's block and column were requested by the caller,
+// each further one is while the one before is used
 template <int RB, class S>
-__device__ __forceinline__ void ilu_row(int sub, int k0, int k1, size_t base, int lane, S* a, int col,
+__device__ __forceinline__ void ilu_row(bool on, int k, int k1, size_t base, int lane, S* a, int col,
                                         const int* __restrict__ jc, const S* __restrict__ lu, const double* w,
-                                        size_t ldw, int q0, const bool* on, double (*acc)[5]) {
-  for (int k = k0 + sub; k < k1; k += kIluLanes) {
-    if (k != k0 + sub) {
-      ilu_block(lu + (base + k) * 800, lane, a);
+                                        double* v) {
+  constexpr int NH = kIluLanes / RB;
+#pragma unroll
+  for (int c = 0; c < 5; ++c) v[c] = 0.0;
+  while (k < k1) {
+    double u[5];
+    const double* wk = w + 5 * RB * (size_t)col;
+#pragma unroll
+    for (int c = 0; c < 5; ++c) u[c] = on ? wk[RB * c] : 0.0;
+    k += NH;
+    S b[25];
+    if (k < k1) {
+      ilu_block(lu + (base + k) * 800, lane, b);
       col = jc[(base + k) * 32 + lane];
     }
 #pragma unroll
-    for (int q = 0; q < RB; ++q) {
-      if (!on[q]) continue;
-      const double* wk = w + (size_t)(q0 + q) * ldw + 5 * (size_t)col;
-      double v[5];
+    for (int r = 0; r < 5; ++r)
 #pragma unroll
-      for (int c = 0; c < 5; ++c) v[c] = wk[c];
+      for (int c = 0; c < 5; ++c) v[r] -= (double)a[5 * r + c] * u[c];
 #pragma unroll
-      for (int r = 0; r < 5; ++r)
-#pragma unroll
-        for (int c = 0; c < 5; ++c) acc[q][r] -= (double)a[5 * r + c] * v[c];
-    }
+    for (int e = 0; e < 25; ++e) a[e] = b[e];
   }
+  __syncwarp();
+#pragma unroll
+  for (int o = RB; o < kIluLanes; o <<= 1)
+#pragma unroll
+    for (int c = 0; c < 5; ++c) v[c] += __shfl_xor_sync(0xffffffffu, v[c], o);
 }
 
 template <int RB, class S, class TI>
-__global__ void __launch_bounds__(kIluT, 4) k_ilu_fwd(int i0, int cnt, int s0, int R, const int* __restrict__ cperm,
-                                                      const int* __restrict__ rju, const int* __restrict__ isp,
-                                                      const int* __restrict__ jc, const S* __restrict__ lu,
-                                                      const TI* x, size_t xs, double* w, size_t ldw,
+__global__ void __launch_bounds__(kIluT, 4) k_ilu_fwd(int N, int i0, int cnt, int s0, int R,
+                                                      const int* __restrict__ cperm, const int* __restrict__ rju,
+                                                      const int* __restrict__ isp, const int* __restrict__ jc,
+                                                      const S* __restrict__ lu, const TI* x, size_t xs, double* w,
                                                       const int* skip) {
   pdl_trigger();
-  const int g = blockIdx.x * blockDim.x + threadIdx.x, q0 = RB * blockIdx.y;
-  const int t = g / kIluLanes, sub = g % kIluLanes;
+  const int g = blockIdx.x * blockDim.x + threadIdx.x;
+  const int t = g / kIluLanes, h = g % kIluLanes / RB, q = RB * blockIdx.y + g % RB;
   const bool act = t < cnt;
   const int lane = t & 31;
   const size_t base = act ? (size_t)isp[s0 + (t >> 5)] : 0;
@@ -980,49 +961,36 @@ __global__ void __launch_bounds__(kIluT, 4) k_ilu_fwd(int i0, int cnt, int s0, i
   const size_t r = act ? (size_t)cperm[i0 + t] : 0;
   S a[25];
   int col = 0;
-  if (sub < d) {
-    ilu_block(lu + (base + sub) * 800, lane, a);
-    col = jc[(base + sub) * 32 + lane];
+  if (h < d) {
+    ilu_block(lu + (base + h) * 800, lane, a);
+    col = jc[(base + h) * 32 + lane];
   }
   pdl_wait();
-  bool on[RB], any = false;
-  double acc[RB][5];
-#pragma unroll
-  for (int q = 0; q < RB; ++q) {
-    on[q] = q0 + q < R && !(skip && skip[8 * (q0 + q)]);
-    any = any || on[q];
-#pragma unroll
-    for (int c = 0; c < 5; ++c) acc[q][c] = 0.0;
-  }
-  if (!any) return;
+  const bool on = q < R && !(skip && skip[8 * q]);
   // the lane that writes a vector's row reads its x meanwhile
-  const int mq = ilu_vec<RB>(sub);
-  bool mine = act && sub < RB;
-#pragma unroll
-  for (int q = 0; q < RB; ++q)
-    if (mq == q) mine = mine && on[q];
+  const bool mine = act && on && h == 0;
   double xv[5] = {0, 0, 0, 0, 0}, v[5];
   if (mine) {
 #pragma unroll
-    for (int c = 0; c < 5; ++c) xv[c] = (double)x[(size_t)(q0 + mq) * xs + 5 * r + c];
+    for (int c = 0; c < 5; ++c) xv[c] = (double)x[(size_t)q * xs + 5 * r + c];
   }
-  ilu_row<RB, S>(sub, 0, d, base, lane, a, col, jc, lu, w, ldw, q0, on, acc);
-  ilu_lane_sums<RB>(sub, acc, v);
+  w += (size_t)blockIdx.y * RB * 5 * N + g % RB;
+  ilu_row<RB, S>(on, h, d, base, lane, a, col, jc, lu, w, v);
   if (!mine) return;
-  double* wi = w + (size_t)(q0 + mq) * ldw + 5 * (size_t)(i0 + t);
+  double* wi = w + 5 * RB * (size_t)(i0 + t);
 #pragma unroll
-  for (int c = 0; c < 5; ++c) wi[c] = xv[c] + v[c];
+  for (int c = 0; c < 5; ++c) wi[RB * c] = xv[c] + v[c];
 }
 
 template <int RB, class S, class TO>
-__global__ void __launch_bounds__(kIluT, 4) k_ilu_bwd(int i0, int cnt, int s0, int R, const int* __restrict__ cperm,
-                                                      const int* __restrict__ rlen, const int* __restrict__ rju,
-                                                      const int* __restrict__ isp, const int* __restrict__ jc,
-                                                      const S* __restrict__ lu, double* w, size_t ldw, TO* z,
-                                                      size_t zs, const int* skip) {
+__global__ void __launch_bounds__(kIluT, 4) k_ilu_bwd(int N, int i0, int cnt, int s0, int R,
+                                                      const int* __restrict__ cperm, const int* __restrict__ rlen,
+                                                      const int* __restrict__ rju, const int* __restrict__ isp,
+                                                      const int* __restrict__ jc, const S* __restrict__ lu, double* w,
+                                                      TO* z, size_t zs, const int* skip) {
   pdl_trigger();
-  const int g = blockIdx.x * blockDim.x + threadIdx.x, q0 = RB * blockIdx.y;
-  const int t = g / kIluLanes, sub = g % kIluLanes;
+  const int g = blockIdx.x * blockDim.x + threadIdx.x;
+  const int t = g / kIluLanes, h = g % kIluLanes / RB, q = RB * blockIdx.y + g % RB;
   const bool act = t < cnt;
   const int lane = t & 31;
   const size_t base = act ? (size_t)isp[s0 + (t >> 5)] : 0;
@@ -1030,14 +998,13 @@ __global__ void __launch_bounds__(kIluT, 4) k_ilu_bwd(int i0, int cnt, int s0, i
   const size_t r = act ? (size_t)cperm[i0 + t] : 0;
   S a[25];
   int col = 0;
-  if (d + 1 + sub < len) {
-    ilu_block(lu + (base + d + 1 + sub) * 800, lane, a);
-    col = jc[(base + d + 1 + sub) * 32 + lane];
+  if (d + 1 + h < len) {
+    ilu_block(lu + (base + d + 1 + h) * 800, lane, a);
+    col = jc[(base + d + 1 + h) * 32 + lane];
   }
-  // the inverted diagonal's rows of this lane: row sub of the one vector, or
-  // rows 0..2 (lanes 0..3) and 3, 4 (lanes 4..7) of the lane's own vector
+  // this lane's rows of the inverted diagonal: row h, or rows 0..2 and 3, 4
   constexpr int MR = RB == 4 ? 3 : 1;
-  const int m0 = RB == 4 ? (sub >> 2) * 3 : sub, m1 = min(5, m0 + MR);
+  const int m0 = MR * h, m1 = min(5, m0 + MR);
   S dg[MR][5];
 #pragma unroll
   for (int m = 0; m < MR; ++m)
@@ -1045,41 +1012,27 @@ __global__ void __launch_bounds__(kIluT, 4) k_ilu_bwd(int i0, int cnt, int s0, i
     for (int c = 0; c < 5; ++c)
       dg[m][c] = act && m0 + m < m1 ? lu[(base + d) * 800 + sl_el<S>(5 * (m0 + m) + c, lane)] : S(0.0);
   pdl_wait();
-  bool on[RB], any = false;
-  double acc[RB][5];
-#pragma unroll
-  for (int q = 0; q < RB; ++q) {
-    on[q] = q0 + q < R && !(skip && skip[8 * (q0 + q)]);
-    any = any || on[q];
-#pragma unroll
-    for (int c = 0; c < 5; ++c) acc[q][c] = 0.0;
-  }
-  if (!any) return;
-  const int mq = ilu_vec<RB>(sub);
-  bool mine = act;
-#pragma unroll
-  for (int q = 0; q < RB; ++q)
-    if (mq == q) mine = mine && on[q];
-  double* wi = w + (size_t)(q0 + mq) * ldw + 5 * (size_t)(i0 + t);
+  const bool on = q < R && !(skip && skip[8 * q]), mine = act && on;
+  w += (size_t)blockIdx.y * RB * 5 * N + g % RB;
+  double* wi = w + 5 * RB * (size_t)(i0 + t);
   double wv[5] = {0, 0, 0, 0, 0}, v[5];
   if (mine) {
 #pragma unroll
-    for (int c = 0; c < 5; ++c) wv[c] = wi[c];
+    for (int c = 0; c < 5; ++c) wv[c] = wi[RB * c];
   }
-  ilu_row<RB, S>(sub, d + 1, len, base, lane, a, col, jc, lu, w, ldw, q0, on, acc);
-  ilu_lane_sums<RB>(sub, acc, v);
+  ilu_row<RB, S>(on, d + 1 + h, len, base, lane, a, col, jc, lu, w, v);
   __syncwarp();   // every lane of the row has read its w
   if (!mine) return;
 #pragma unroll
   for (int c = 0; c < 5; ++c) v[c] += wv[c];
-  TO* zi = z + (size_t)(q0 + mq) * zs + 5 * r;
+  TO* zi = z + (size_t)q * zs + 5 * r;
 #pragma unroll
   for (int m = 0; m < MR; ++m) {
     if (m0 + m >= m1) break;
     double o = 0.0;
 #pragma unroll
     for (int c = 0; c < 5; ++c) o += (double)dg[m][c] * v[c];
-    wi[m0 + m] = o;
+    wi[RB * (m0 + m)] = o;
     zi[m0 + m] = (TO)o;
   }
 }
@@ -1131,8 +1084,7 @@ static void ilu_apply(aerof_gpu_ctx* c, int R, const TI* x, size_t xs, TO* z, si
   DeviceMesh& m = c->mesh;
   Implicit& J = c->imp;
   cudaStream_t s = c->stream;
-  const size_t ldw = 5 * (size_t)m.N;
-  J.iluw.ensure((size_t)R * ldw);
+  J.iluw.ensure((size_t)(R == 1 ? 1 : (R + 3) / 4 * 4) * 5 * m.N);
   double* w = J.iluw.p;
   auto sweeps = [&](const auto* lu, auto rb) {
     using S = std::remove_const_t<std::remove_pointer_t<decltype(lu)>>;
@@ -1140,18 +1092,18 @@ static void ilu_apply(aerof_gpu_ctx* c, int R, const TI* x, size_t xs, TO* z, si
     const int ny = (R + RB - 1) / RB;
     for (int col = 0; col < m.ncolor; ++col) {
       const int i0 = m.h_cptr[col], cnt = m.h_cptr[col + 1] - i0;
-      launch_pdl(k_ilu_fwd<RB, S, TI>, dim3(grid_for((size_t)kIluLanes * cnt, kIluT), ny), kIluT, 0, s, i0, cnt,
-                 m.h_cslice[col], R, m.cperm.p, m.rju.p, m.isp.p, m.jc.p, lu, x, xs, w, ldw, skip);
+      launch_pdl(k_ilu_fwd<RB, S, TI>, dim3(grid_for((size_t)kIluLanes * cnt, kIluT), ny), kIluT, 0, s, m.N, i0, cnt,
+                 m.h_cslice[col], R, m.cperm.p, m.rju.p, m.isp.p, m.jc.p, lu, x, xs, w, skip);
     }
     for (int col = m.ncolor - 1; col >= 0; --col) {
       const int i0 = m.h_cptr[col], cnt = m.h_cptr[col + 1] - i0;
-      launch_pdl(k_ilu_bwd<RB, S, TO>, dim3(grid_for((size_t)kIluLanes * cnt, kIluT), ny), kIluT, 0, s, i0, cnt,
-                 m.h_cslice[col], R, m.cperm.p, m.rlen.p, m.rju.p, m.isp.p, m.jc.p, lu, w, ldw, z, zs, skip);
+      launch_pdl(k_ilu_bwd<RB, S, TO>, dim3(grid_for((size_t)kIluLanes * cnt, kIluT), ny), kIluT, 0, s, m.N, i0, cnt,
+                 m.h_cslice[col], R, m.cperm.p, m.rlen.p, m.rju.p, m.isp.p, m.jc.p, lu, w, z, zs, skip);
     }
   };
   // four vectors per pass over a block: one per pass, with four times the
-  // threads, reads the blocks four times (four sensitivities of 41^3: 105 ms
-  // against 87.6 ms)
+  // threads, reads the blocks four times (four sensitivities of 41^3, both
+  // with a vector's gathers in one lane: 105 ms against 87.6 ms)
   auto run = [&](const auto* lu) {
     if (R == 1) sweeps(lu, std::integral_constant<int, 1>{});
     else sweeps(lu, std::integral_constant<int, 4>{});

@@ -1,7 +1,7 @@
-"""The blocked kernels of the time step and the fused RK2 stages, of the
-forward products and of the Spalart-Allmaras residual, at sizes around the
-128-node block (27 nodes: less than one; 125: one, partial; 216: two, the
-last partial; 512: four full ones), against the oracle and against the edge
+"""The blocked kernels of the time step, the fused RK2 stages and the forward
+products, and the Spalart-Allmaras residual, at sizes around the 128-node
+block (27 nodes: less than one; 125: one, partial; 216: two, the last
+partial; 512: four full ones), against the oracle and against the edge
 organisation.
 
 Tolerances: one evaluation is a sum of at most ~26 edge terms per node with

@@ -1,0 +1,65 @@
+"""Launches that overlap their predecessors, and the kernels' rings and extra
+blocks at the sizes where their rules change.
+
+Explicit step: the wave sums are extra blocks of the first edge sweep up to
+592 Morton blocks (42^3 nodes: 579 blocks; 43^3: 622, their own launch).  Same
+tolerance as one evaluation of the residual, a sum of at most ~26 edge terms
+per node with 2^-53 each, magnified below 100 times by their cancellation.
+
+Products with H1 from the states: a lane has four steps of
+neighbour data in flight; blocks of 64, 128 and 256 nodes give a node four,
+two and one lanes, so four to fourteen steps.  FP64 products differ from the
+stored blocks' by a few 2^-53 per term, FP32 ones by a few 2^-24: 1e-9 and
+1e-5 after eight iterations."""
+import numpy as np
+import pytest
+
+from aerof_dev_b200 import workloads as W
+from conftest import rel_l2
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("rec", [1, 2])
+@pytest.mark.parametrize("n", [42, 43])
+def test_rk2_around_the_wave_blocks_rule(gpu_lib, n, rec):
+    import torch
+    A = gpu_lib
+    m = W.make_lattice_mesh(n, jitter=0.2, codes="channel")
+    Ub = W.freestream(0.6)
+    ctx = A.Context.from_mesh(m, Ub, reconstruction=rec)
+    edge = A.Context.from_mesh(m, Ub, reconstruction=rec, residual_kernel=A.KERNEL_EDGE)
+    U = W.perturbed_state(ctx.N, 0.6, amp=0.02)
+    out, bad = A.ExplicitRK2(ctx, 0.8).run(U, 4)
+    ref, bad_e = A.ExplicitRK2(edge, 0.8).run(U, 4)
+    assert bad == bad_e == 0
+    assert rel_l2(out - U, ref - U) < 1e-12
+    # run after run on one stream, and a residual between them
+    Ud = torch.from_numpy(U).cuda()
+    for _ in range(3):
+        V, _ = A.ExplicitRK2(ctx, 0.8).run(Ud.clone(), 4)
+        A.SpaceOperator(ctx).computeResidual(Ud)
+        assert np.array_equal(V.cpu().numpy(), out)
+
+
+@pytest.mark.parametrize("prec,tol", [(64, 1e-9), (32, 1e-5)])
+@pytest.mark.parametrize("transpose", [False, True])
+@pytest.mark.parametrize("nb", ["64", "128", "256"])
+def test_products_over_lanes_per_node(gpu_lib, monkeypatch, nb, transpose, prec, tol):
+    A = gpu_lib
+    monkeypatch.setenv("AEROF_BLOCK_NODES", nb)
+    m = W.make_lattice_mesh(9, jitter=0.2, codes="channel")
+    ctx = A.Context.from_mesh(m, W.freestream(0.7))
+    U = W.perturbed_state(ctx.N, 0.7, amp=0.05)
+    mv, pc = A.MatVecProdH1(ctx, prec), A.JacobiPrec(ctx)
+    b = np.random.default_rng(1).standard_normal((ctx.N, 5))
+    gm = A.GmresSolver(ctx, 8, 8, 0.0)
+    mv.evaluate(U, A.SpaceOperator(ctx).computeTimeStep(U, 30.0))
+    blocks = mv.blocks()
+    pc.setup()
+    free, its, _ = gm.solve(b, transpose=transpose)
+    mv.set_blocks(blocks)
+    pc.setup()
+    stored, its2, _ = gm.solve(b, transpose=transpose)
+    assert its == its2 == 8
+    assert rel_l2(free, stored) < tol
