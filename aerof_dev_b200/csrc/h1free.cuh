@@ -30,11 +30,12 @@
 // multiples of 16 bytes, conflict-free vector loads); L lanes per node take
 // its neighbours r, r + L, ..., the row sum is FP64 (fixed xor tree).  The
 // per-neighbour data is stored warp by warp, coalesced per step, and copied
-// to shared memory four steps ahead, before the wait for the packed vector.  Requested one step ahead into registers, its latency was
-// most of the kernel (seven of thirteen warps waited for it per issue; 47 us
-// at 61^3): a pseudo-time step of 81^3 with 20 FP32 iterations 4.91 -> 4.69
-// ms, five Newton steps of 61^3 15.0 -> 14.8 ms with eight steps and three
-// CTAs per SM; four steps and four CTAs (64 registers) 4.43 ms and 14.0 ms.
+// to shared memory four steps ahead, before the wait for the packed vector.
+// Requested one step ahead into registers, its latency was most of the
+// kernel (seven of thirteen warps waited for it per issue; 47 us at 61^3): a
+// pseudo-time step of 81^3 with 20 FP32 iterations 4.91 -> 4.69 ms, five
+// Newton steps of 61^3 15.0 -> 14.8 ms with eight steps and three CTAs per
+// SM; with four steps and four CTAs (64 registers) 4.43 and 14.0 ms.
 #pragma once
 
 #include "common.cuh"
@@ -42,9 +43,9 @@
 
 namespace aerof {
 
-// widths (elements) of a node's record and of a packed vector row
+// widths (elements) of a node's record, global and staged, and the steps of
+// neighbour data in flight per lane of the product kernel
 template <class S> struct H1Rec;
-// and the steps of neighbour data in flight per lane of the product kernel
 template <> struct H1Rec<float> { static constexpr int W = 8, SM = 12, D = 4; };
 template <> struct H1Rec<double> { static constexpr int W = 6, SM = 10, D = 4; };
 
