@@ -1526,19 +1526,29 @@ static decltype(&k_fv_blocked<256, 2>) pipe_fv_kernel(const DeviceMesh& m) {
   return by_smem >= 4 ? k_fv_blocked<256, 4> : by_smem == 3 ? k_fv_blocked<256, 3> : k_fv_blocked<256, 2>;
 }
 
+// The shared-memory limits of the stages' kernels.  They belong to the
+// function, and another context with a smaller staging may have lowered them
+// since, so every call sets them.
+static size_t pipe_attributes(const DeviceMesh& m) {
+  AEROF_CUDA(cudaFuncSetAttribute(pipe_fv_kernel(m), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)fv_blocked_smem(m)));
+  const int L = kBlock / m.NB;
+  auto gp = L == 4 ? k_grad_pipe<4> : L == 2 ? k_grad_pipe<2> : k_grad_pipe<1>;
+  const size_t gsmem = (size_t)2 * grad_stage(m).size * sizeof(double);
+  AEROF_CUDA(cudaFuncSetAttribute(gp, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gsmem));
+  return gsmem;
+}
+
 static ResidualPipe& pipe_for(aerof_gpu_ctx* c) {
+  const size_t gsmem = pipe_attributes(c->mesh);
   if (c->pipe) return *c->pipe;
   const DeviceMesh& m = c->mesh;
   auto p = std::make_unique<ResidualPipe>();
   const int K = m.pipeK;
   p->K = K;
   {
-    AEROF_CUDA(cudaFuncSetAttribute(pipe_fv_kernel(m), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)fv_blocked_smem(m)));
     const int L = kBlock / m.NB;
     auto gp = L == 4 ? k_grad_pipe<4> : L == 2 ? k_grad_pipe<2> : k_grad_pipe<1>;
-    const size_t gsmem = (size_t)2 * grad_stage(m).size * sizeof(double);
-    AEROF_CUDA(cudaFuncSetAttribute(gp, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gsmem));
     int per_sm = 0, sms = 0;
     AEROF_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, gp, kBlock, gsmem));
     AEROF_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->cfg.device));
@@ -1619,7 +1629,7 @@ static void stage_kernels(aerof_gpu_ctx* c, ResidualPipe& p, int st, cudaStream_
   double* dU = c->s.Ustage.p;
   double* dR = c->s.Rstage.p;
   // the kernels and launch shapes of residual_blocked_dev (attributes set
-  // by pipe_for, outside any capture)
+  // by pipe_attributes, outside any capture)
   const size_t fsmem = fv_blocked_smem(m);
   auto fvk = pipe_fv_kernel(m);
   const int L = kBlock / m.NB;

@@ -63,3 +63,24 @@ def test_products_over_lanes_per_node(gpu_lib, monkeypatch, nb, transpose, prec,
     stored, its2, _ = gm.solve(b, transpose=transpose)
     assert its == its2 == 8
     assert rel_l2(free, stored) < tol
+
+
+@pytest.mark.parametrize("stream", ["default", "own"])
+def test_host_array_residuals_of_two_meshes_in_turn(gpu_lib, stream):
+    # the blocks of the two meshes stage different amounts; each context's
+    # kernels keep their own shared-memory limit whichever ran before
+    import torch
+    A = gpu_lib
+    with torch.cuda.stream(torch.cuda.Stream() if stream == "own" else torch.cuda.default_stream()):
+        runs = []
+        for jitter in (0.2, 0.05, 0.1):
+            m = W.make_lattice_mesh(51, jitter=jitter, codes="channel")
+            ctx = A.Context.from_mesh(m, W.freestream(0.6))
+            U = W.perturbed_state(ctx.N, 0.6, amp=0.02)
+            ref = A.SpaceOperator(ctx).computeResidual(torch.from_numpy(U).cuda())[0].cpu()
+            runs.append((ctx, torch.from_numpy(U).pin_memory(), ref))
+        for k in (0, 1, 2, 0, 2, 1, 0):
+            ctx, Uh, ref = runs[k]
+            R = torch.empty_like(Uh).pin_memory()
+            A.SpaceOperator(ctx).computeResidual(Uh, R)
+            assert torch.equal(R, ref)
