@@ -587,7 +587,9 @@ __device__ __forceinline__ void prefetch_pairs_l2(const double2* h2, size_t E, i
 // number is added to the device counter of the mode's index (returns 0);
 // with the failsafe on every mode is kCountSync.  kCountAsync: the counter
 // of aerof_gpu_status; kCountSum: one that the caller zeroes and reads.
-constexpr int kCountSync = 0, kCountAsync = 2, kCountSum = 3;
+// kCountSA: the Spalart-Allmaras residual's own (the synchronous one is left
+// at zero by its reader, so nothing else may count into it).
+constexpr int kCountSync = 0, kCountAsync = 2, kCountSum = 3, kCountSA = 7;
 int residual_dev(aerof_gpu_ctx* c, const double* dU, double* dR, int mode = kCountSync);
 void prim_dev(aerof_gpu_ctx* c, const double* dU);
 void prim_grad_blocked_dev(aerof_gpu_ctx* c, const double* dU, const int* tag);

@@ -95,3 +95,31 @@ def test_sa_needs_the_model_and_valid_inputs(gpu_lib, case):
     ctx.set_turbulence(None, None)
     with pytest.raises(A.AerofError):
         A.SpaceOperator(ctx).computeResidualSA(np.ones((o.N, 6)))
+
+
+def test_sa_counts_between_five_variable_residuals(gpu_lib, oracle_mod):
+    # the unphysical count of each call is that call's own: a bad state through
+    # the Spalart-Allmaras residual leaves nothing behind for the
+    # five-variable one on the same context, and the other way round
+    import torch
+    A = gpu_lib
+    m = W.make_lattice_mesh(7, jitter=0.2, codes="channel")
+    o = oracle_mod.Oracle(m)
+    Ub6 = np.concatenate([W.freestream(0.8), [1e-3]])
+    good = W.perturbed_state(o.N, 0.8)
+    V = o.prim(good)
+    i = 3 * 49 + 3 * 7 + 3
+    V[i, 4] *= 40.0
+    V[i + 1, 4] *= 0.02
+    bad = W.prim_to_cons(V)
+    k5 = o.residual(bad, Ub6[:5], 3)[1]
+    d2wall = np.abs(m["X"][:, 2]) + 0.02 * m["X"][:, 0]
+    k6 = o.residual_sa(sa_state(m, bad), Ub6, d2wall, order=3, model=0)[1]
+    assert k5 > 0 and k6 > 0
+    sp = A.SpaceOperator(A.Context.from_mesh(m, Ub6[:5], reconstruction=3))
+    sp.ctx.set_turbulence(d2wall, Ub6)
+    g5, b5, g6, b6 = (torch.from_numpy(x).cuda() for x in (good, bad, sa_state(m, good), sa_state(m, bad)))
+    five = lambda x: sp.computeResidual(x)[1]  # noqa: E731
+    six = lambda x: sp.computeResidualSA(x)[1]  # noqa: E731
+    assert [five(g5), six(b6), five(g5), six(g6), five(b5), six(b6), five(b5), six(g6), five(g5)] == \
+        [0, k6, 0, 0, k5, k6, k5, 0, 0]
