@@ -656,8 +656,7 @@ int residual_forward(aerof_gpu_ctx* c, const double* dU, const double* dv, const
   const Gas g = make_gas(c->cfg.gamma);
   DualWork& w = c->dual;
   if (forward_blocked_fits(m)) {
-    c->s.counters.ensure(8);
-    int* cnt = c->s.counters.p + 6;
+    int* cnt = counters(c) + 6;
     AEROF_CUDA(cudaMemsetAsync(cnt, 0, sizeof(int), s));
     forward_blocked(c, dU, dv, dXdot, ddR, cnt);
     int bad = 0;
@@ -685,8 +684,7 @@ int residual_forward(aerof_gpu_ctx* c, const double* dU, const double* dv, const
     k_d_grad<<<gn, kAB, 0, s>>>(m.N, w.PD.p, w.WD.p, m.nbr_ptr.p, m.nbr_node.p, w.GD.p);
     AEROF_LAUNCH_CHECK();
   }
-  c->s.counters.ensure(8);
-  int* cnt = c->s.counters.p + 6;
+  int* cnt = counters(c) + 6;
   AEROF_CUDA(cudaMemsetAsync(cnt, 0, sizeof(int), s));
   k_d_edge_flux<<<ge, kAB, 0, s>>>(m.E, g, rec, c->cfg.beta, m.edges.p, w.enD.p, w.PD.p, w.GD.p, w.fluxD.p, cnt);
   AEROF_LAUNCH_CHECK();

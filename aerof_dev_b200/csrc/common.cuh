@@ -465,6 +465,16 @@ int guard(aerof_gpu_ctx* c, F&& f) {
   }
 }
 
+// the context's eight device counters, all zero when first asked for
+inline int* counters(aerof_gpu_ctx* c) {
+  DBuf<int>& b = c->s.counters;
+  if (b.n == 0) {
+    b.alloc(8);
+    b.zero(c->stream);
+  }
+  return b.p;
+}
+
 // boundary data of the kernels that form subface fluxes (fbuf: [3F][5])
 struct FaceArgs {
   int F;

@@ -1044,8 +1044,7 @@ static int ilu_setup(aerof_gpu_ctx* c, int tr) {
   DeviceMesh& m = c->mesh;
   Implicit& J = c->imp;
   cudaStream_t s = c->stream;
-  c->s.counters.ensure(8);
-  int* bad = c->s.counters.p + 5;
+  int* bad = counters(c) + 5;
   AEROF_CUDA(cudaMemsetAsync(bad, 0, sizeof(int), s));
   const int gn = grid_for(m.N, kIB);
   auto run = [&](auto* lu, auto* diag, auto* off) {
@@ -1121,8 +1120,7 @@ int prec_setup_dev(aerof_gpu_ctx* c, int trans = 0) {
     J.prec_ready = true;
     return h;
   }
-  c->s.counters.ensure(8);
-  int* bad = c->s.counters.p + 4;
+  int* bad = counters(c) + 4;
   AEROF_CUDA(cudaMemsetAsync(bad, 0, sizeof(int), c->stream));
   const int gn = grid_for(m.N, kIB);
   if (J.precision == AEROF_PREC_FP32) {
@@ -1970,7 +1968,6 @@ extern "C" int aerof_gpu_newton(aerof_gpu_ctx* c, double* U, const aerof_newton_
       dU = c->s.Ustage.p;
     }
     c->imp.b.ensure(n); c->imp.x.ensure(n); c->s.k1.ensure(n);
-    c->s.counters.ensure(8);
     double* R = c->s.k1.p;
     double* rhs = c->imp.b.p;
     double* dQ = c->imp.x.p;
@@ -1980,7 +1977,7 @@ extern "C" int aerof_gpu_newton(aerof_gpu_ctx* c, double* U, const aerof_newton_
     c->imp.lindt.ensure(m.N);
     double* dt = c->imp.lindt.p;
     double* Uprev = c->imp.linU.p;
-    int* nbad_d = c->s.counters.p + 5;
+    int* nbad_d = counters(c) + 5;
     const int gv = grid_for(n, kIB);
     cudaEvent_t e0, e1;
     AEROF_CUDA(cudaEventCreate(&e0));
@@ -1988,7 +1985,7 @@ extern "C" int aerof_gpu_newton(aerof_gpu_ctx* c, double* U, const aerof_newton_
     AEROF_CUDA(cudaEventRecord(e0, s));
     double res0 = 0.0, rel = 1.0, rel_prev = 1.0, cfl = p->cfl0;
     int k = 0, lits = 0, bad = 0, redos = 0;
-    int* bad_d = c->s.counters.p + kCountSum;
+    int* bad_d = counters(c) + kCountSum;
     AEROF_CUDA(cudaMemsetAsync(bad_d, 0, sizeof(int), s));
     bool redo = false;
     while (k <= p->max_steps) {

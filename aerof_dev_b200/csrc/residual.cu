@@ -1168,11 +1168,6 @@ void gradients_dev(aerof_gpu_ctx* c) {
   AEROF_LAUNCH_CHECK();
 }
 
-static int* counters(aerof_gpu_ctx* c) {
-  c->s.counters.ensure(8);
-  return c->s.counters.p;
-}
-
 constexpr size_t kMaxStagedSmem = 160 * 1024;
 
 static int grad_kernel_choice() {
@@ -1969,10 +1964,6 @@ extern "C" int aerof_gpu_residual_async(aerof_gpu_ctx* c, const double* U, doubl
       c->last_error = "aerof_gpu_residual_async needs device pointers";
       return AEROF_EINVAL;
     }
-    if (c->s.counters.n == 0) {
-      counters(c);
-      AEROF_CUDA(cudaMemsetAsync(c->s.counters.p, 0, sizeof(int) * 8, c->stream));
-    }
     residual_dev(c, U, R, kCountAsync);
     return AEROF_OK;
   });
@@ -1982,8 +1973,8 @@ extern "C" int aerof_gpu_status(aerof_gpu_ctx* c) {
   return guard(c, [&]() -> int {
     int bad = 0;
     if (c->s.counters.n) {
-      AEROF_CUDA(cudaMemcpyAsync(&bad, c->s.counters.p + 2, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
-      AEROF_CUDA(cudaMemsetAsync(c->s.counters.p + 2, 0, sizeof(int), c->stream));
+      AEROF_CUDA(cudaMemcpyAsync(&bad, c->s.counters.p + kCountAsync, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+      AEROF_CUDA(cudaMemsetAsync(c->s.counters.p + kCountAsync, 0, sizeof(int), c->stream));
     }
     AEROF_CUDA(cudaStreamSynchronize(c->stream));
     return bad;

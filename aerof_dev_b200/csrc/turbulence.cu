@@ -416,8 +416,7 @@ static int residual_sa_dev(aerof_gpu_ctx* c, const double* dU, double* dR) {
   t.G6.ensure(18 * (size_t)m.N);
   t.flux6.ensure(6 * (size_t)std::max(m.E, 1));
   t.fbuf6.ensure(18 * (size_t)std::max(m.F, 1));
-  c->s.counters.ensure(8);
-  int* cnt = c->s.counters.p + kCountSA;
+  int* cnt = counters(c) + kCountSA;
   AEROF_CUDA(cudaMemsetAsync(cnt, 0, sizeof(int), s));
   k_prim6<<<grid_for(m.N, 256), 256, 0, s>>>(m.N, g, dU, t.V6.p);
   AEROF_LAUNCH_CHECK();
