@@ -1230,8 +1230,9 @@ static void h1_precond_product(aerof_gpu_ctx* c, int R, const TV* x, size_t xs, 
 // Device state of R systems with restart length m over vectors of n
 // elements (E per 16 bytes): one CTA of the sweeps per SM and system, fewer
 // for short vectors.
-static GsDev gs_state(aerof_gpu_ctx* c, KrylovWork& k, int R, int m, size_t n, int E) {
+static GsDev gs_state(aerof_gpu_ctx* c, KrylovWork& k, int R, int m, size_t n, int E, bool unit = false) {
   GsDev st;
+  st.unit = unit;
   int sms = 0;
   AEROF_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->cfg.device));
   const size_t need = (n / E + kGsT - 1) / kGsT;
@@ -1352,14 +1353,18 @@ static void gmres_device(aerof_gpu_ctx* c, int R, const double* const* B, double
   for (bool first = true;; first = false) {
     gs_reset(kw, R);
     if (first) {
-      k_gs_start<TV, true><<<gs, kGsT, 0, s>>>(n, b, x, nullptr, 0, V, vs, st, eps, maxits);
+      k_gs_start<TV, true><<<gs, kGsT, 0, s>>>(n, b, x, nullptr, 0, st, eps, maxits);
+      AEROF_LAUNCH_CHECK();
+      k_gs_first<TV, true><<<gv, kIB, 0, s>>>(n, b, nullptr, 0, V, vs, st);
     } else {
       for (int q = 0; q < R; ++q) {
         k_scale<double, TV><<<grid_for(n, kIB), kIB, 0, s>>>(n, 1.0, X[q], Z + (size_t)q * ld);
         AEROF_LAUNCH_CHECK();
       }
       h1_precond_product<TV>(c, R, Z, ld, W, ld, nullptr, 0, trans, false, done);
-      k_gs_start<TV, false><<<gs, kGsT, 0, s>>>(n, b, x, W, ld, V, vs, st, eps, maxits);
+      k_gs_start<TV, false><<<gs, kGsT, 0, s>>>(n, b, x, W, ld, st, eps, maxits);
+      AEROF_LAUNCH_CHECK();
+      k_gs_first<TV, false><<<gv, kIB, 0, s>>>(n, b, W, ld, V, vs, st);
     }
     AEROF_LAUNCH_CHECK();
     for (int j = 0; j < numVec; ++j) {
@@ -1391,6 +1396,8 @@ static void gmres_device(aerof_gpu_ctx* c, int R, const double* const* B, double
 // of the mixed-precision GMRES on the first-order operator of all running
 // systems (FP32 blocks and Krylov vectors).  The corrections are kept (Z)
 // and x = Z y, so the changing inner solve does not spoil the minimisation.
+// The inner solves are given unit vectors: in FP32 they would answer a
+// residual far from 1 with zero or infinity.
 // A system that converges stops, the others go on.
 static void fgmres_device(aerof_gpu_ctx* c, int R, const double* const* B, double* const* X, int numVec, int maxits,
                           double eps, int trans, const double* exactU, int inner_m, int inner_its, double inner_eps,
@@ -1405,7 +1412,7 @@ static void fgmres_device(aerof_gpu_ctx* c, int R, const double* const* B, doubl
   J.bw.ensure((size_t)R * ld);
   double *V = J.bV.p, *Z = J.bZ.p, *W = J.bw.p;
   KrylovWork& kw = J.kout;
-  const GsDev st = gs_state(c, kw, R, numVec, n, Vec16<double>::W);
+  const GsDev st = gs_state(c, kw, R, numVec, n, Vec16<double>::W, true);
   VecIn b{};
   VecOut x{};
   for (int q = 0; q < R; ++q) { b.p[q] = B[q]; x.p[q] = X[q]; }
@@ -1419,11 +1426,15 @@ static void fgmres_device(aerof_gpu_ctx* c, int R, const double* const* B, doubl
   for (bool first = true;; first = false) {
     gs_reset(kw, R);
     if (first) {
-      k_gs_start<double, true><<<gs, kGsT, 0, s>>>(n, b, x, nullptr, 0, V, vs, st, eps, maxits);
+      k_gs_start<double, true><<<gs, kGsT, 0, s>>>(n, b, x, nullptr, 0, st, eps, maxits);
+      AEROF_LAUNCH_CHECK();
+      k_gs_first<double, true><<<gv, kIB, 0, s>>>(n, b, nullptr, 0, V, vs, st);
     } else {
       for (int q = 0; q < R; ++q)
         if (!fin[q]) product(X[q], W + (size_t)q * ld);
-      k_gs_start<double, false><<<gs, kGsT, 0, s>>>(n, b, x, W, ld, V, vs, st, eps, maxits);
+      k_gs_start<double, false><<<gs, kGsT, 0, s>>>(n, b, x, W, ld, st, eps, maxits);
+      AEROF_LAUNCH_CHECK();
+      k_gs_first<double, false><<<gv, kIB, 0, s>>>(n, b, W, ld, V, vs, st);
     }
     AEROF_LAUNCH_CHECK();
     for (int j = 0; j < numVec; ++j) {
@@ -1442,6 +1453,8 @@ static void fgmres_device(aerof_gpu_ctx* c, int R, const double* const* B, doubl
                           nullptr);
       for (size_t k = 0; k < rl.size(); ++k) product(xi[k], W + (size_t)rl[k] * ld);
       gs_iteration<double>(c, st, R, n, j, V, vs, ld, W, ld);
+      k_gs_unit<double><<<gv, kIB, 0, s>>>(n, V + (size_t)(j + 1) * ld, vs, st);
+      AEROF_LAUNCH_CHECK();
     }
     gs_backsolve(c, st, R);
     k_gs_combine<double, true><<<gv, kIB, sizeof(double) * (numVec + 1), s>>>(n, Z, zs, ld, st, nullptr, 0, x);

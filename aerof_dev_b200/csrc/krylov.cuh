@@ -13,10 +13,14 @@
 // reads of the basis, j reads and writes of w and j + 1 grid-wide sums
 // (bound: HBM; figures at gs_iteration).
 //
-// The basis vectors are stored as they come out of the projection, with
-// the factor sig_i = 1/norm beside them (v_i = sig_i * stored), so no pass
-// normalises them.  Dots, norms and the Hessenberg system are FP64 for
-// either storage type; the projected vector is rounded to it once.
+// The first basis vector of a cycle is stored normalised, so that the vectors
+// do not depend on the scale of the right-hand side.  The others are stored
+// as they come out of the projection, of the size of the preconditioned
+// operator, with the factor sig_i = 1/norm beside them (v_i = sig_i *
+// stored), so no pass normalises them.  The flexible method hands its vectors
+// to inner solves and does normalise them (k_gs_unit, sig_i = 1).  Dots, norms
+// and the Hessenberg system are FP64 for either storage type; a vector is
+// rounded to it once.
 // Reductions run over a fixed grid in a fixed order (no atomics on values):
 // every block of the second sweep forms the coefficients from the first
 // sweep's partial sums, and its block that finishes last does the Givens
@@ -49,13 +53,15 @@ struct GsDev {
   double* norm_part;             // [R][G] of the norm
   GsPub* pub;
   int m, G;
+  bool unit;                     // every basis vector is stored normalised (k_gs_unit)
   __host__ __device__ size_t oL() const { return (size_t)(m + 1) * m; }
   __host__ __device__ size_t oCs() const { return oL() + (size_t)m * m; }
   __host__ __device__ size_t oG() const { return oCs() + 2 * (size_t)m; }
   __host__ __device__ size_t oY() const { return oG() + m + 1; }
   __host__ __device__ size_t oSig() const { return oY() + m; }
-  __host__ __device__ size_t oScal() const { return oSig() + m + 1; }   // l2res, target
-  __host__ __device__ size_t size() const { return oScal() + 2; }
+  // l2res, target, 1/norm of the vector to be normalised
+  __host__ __device__ size_t oScal() const { return oSig() + m + 1; }
+  __host__ __device__ size_t size() const { return oScal() + 3; }
 };
 
 struct VecIn { const double* p[kMaxSys]; };
@@ -165,14 +171,15 @@ __device__ __forceinline__ void publish(GsPub* pub, int seq, int done, int iter,
   p->seq = seq;
 }
 
-// First vector of a cycle: v_0 = b (FIRST, which also zeroes x) or b - w,
-// stored unnormalised, with its norm (and b's, for the target) and the
-// cycle's state.
+// Start of a cycle: the norm of b (FIRST, which also zeroes x) or of b - w,
+// b's for the target, and the cycle's state.  The vector itself is left to
+// k_gs_first: rounded to TV before it is normalised, a right-hand side far
+// from 1 would lose its range.
 template <class TV, bool FIRST>
 __global__ void __launch_bounds__(kGsT) k_gs_start(size_t n, VecIn B, VecOut X, const TV* __restrict__ Wv, size_t ws,
-                                                   TV* __restrict__ V, size_t vs, GsDev st, double eps, int maxits) {
-  __shared__ double red[(kGsT / 32) * 2];
-  __shared__ double vals[2];
+                                                   GsDev st, double eps, int maxits) {
+  __shared__ double red[kGsT / 32];
+  __shared__ double vals[1];
   const int q = blockIdx.y;
   int* ist = st.i + 8 * q;
   if (!FIRST && ist[1]) {
@@ -185,22 +192,16 @@ __global__ void __launch_bounds__(kGsT) k_gs_start(size_t n, VecIn B, VecOut X, 
   }
   const double* __restrict__ b = B.p[q];
   const TV* __restrict__ w = Wv + (size_t)q * ws;
-  TV* __restrict__ v = V + (size_t)q * vs;
-  double s[2] = {0.0, 0.0};
+  double s = 0.0;
   for (size_t p = (size_t)blockIdx.x * blockDim.x + threadIdx.x; p < n; p += (size_t)gridDim.x * blockDim.x) {
-    const double bp = b[p];
-    const TV r = (TV)(FIRST ? bp : bp - (double)w[p]);
-    v[p] = r;
-    if (FIRST) {
-      X.p[q][p] = 0.0;
-      s[1] += bp * bp;
-    }
-    s[0] += (double)r * (double)r;
+    const double r = FIRST ? b[p] : b[p] - (double)w[p];
+    if (FIRST) X.p[q][p] = 0.0;
+    s += r * r;
   }
   double* part = st.part + (size_t)q * 2 * (st.m + 1) * st.G;
-  block_sums<2>(s, 2, red, part + blockIdx.x, st.G);
+  block_sums<1>(&s, 1, red, part + blockIdx.x, st.G);
   if (!last_block(ist + 6)) return;
-  sum_partials<32>(part, st.G, 2, vals);
+  sum_partials<32>(part, st.G, 1, vals);
   if (threadIdx.x == 0) {
     double* d = st.d + (size_t)q * st.sd;
     const double beta = sqrt(vals[0]);
@@ -208,7 +209,7 @@ __global__ void __launch_bounds__(kGsT) k_gs_start(size_t n, VecIn B, VecOut X, 
       ist[0] = 0;
       ist[4] = maxits;
       d[st.oScal()] = 0.0;
-      d[st.oScal() + 1] = eps * sqrt(vals[1]);
+      d[st.oScal() + 1] = eps * beta;
     }
     const int done = beta == 0.0;
     if (done) d[st.oScal()] = 0.0;
@@ -217,9 +218,29 @@ __global__ void __launch_bounds__(kGsT) k_gs_start(size_t n, VecIn B, VecOut X, 
     ist[3] = 1;
     ist[5] = 0;
     d[st.oG()] = beta;
-    d[st.oSig()] = done ? 0.0 : 1.0 / beta;
+    d[st.oSig()] = 1.0;
+    d[st.oScal() + 2] = done ? 0.0 : 1.0 / beta;
     if (done) publish(st.pub + q, 0, 1, ist[0], 0.0);
   }
+}
+// v_0 = (b or b - w) / its norm, rounded once
+template <class TV, bool FIRST>
+__global__ void __launch_bounds__(256) k_gs_first(size_t n, VecIn B, const TV* __restrict__ Wv, size_t ws,
+                                                  TV* __restrict__ V, size_t vs, GsDev st) {
+  const int q = blockIdx.y;
+  if (st.i[8 * q + 1]) return;
+  const size_t p = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (p >= n) return;
+  const double b = B.p[q][p], r = FIRST ? b : b - (double)Wv[(size_t)q * ws + p];
+  V[(size_t)q * vs + p] = (TV)(st.d[(size_t)q * st.sd + st.oScal() + 2] * r);
+}
+// basis vector v of the running systems normalised (flexible method)
+template <class TV>
+__global__ void __launch_bounds__(256) k_gs_unit(size_t n, TV* __restrict__ v, size_t vs, GsDev st) {
+  const int q = blockIdx.y;
+  if (st.i[8 * q + 1]) return;
+  const size_t p = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (p < n) v[(size_t)q * vs + p] *= (TV)st.d[(size_t)q * st.sd + st.oScal() + 2];
 }
 
 // Sweep 1 of iteration j: partial sums of v_i.w and v_i.v_j for every i <= j
@@ -449,7 +470,9 @@ __global__ void __launch_bounds__(kGsT, 1) k_gs_update(size_t n, int j, TV* V, s
     g[j] = __dmul_rn(c1, gj);
     cs[2 * j] = c0;
     cs[2 * j + 1] = c1;
-    d[st.oSig() + j + 1] = breakdown ? 0.0 : 1.0 / hj1;
+    const double inv = breakdown ? 0.0 : 1.0 / hj1;
+    d[st.oSig() + j + 1] = st.unit ? 1.0 : inv;
+    d[st.oScal() + 2] = inv;
     const int iter = si[0] + 1;
     double l2res = sg[1];
     bool done = breakdown;

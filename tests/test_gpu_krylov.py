@@ -79,3 +79,33 @@ def test_batch_equals_one_by_one(gpu_lib, pc, transpose):
         # through J^-1 (condition below 1e3 here)
         assert rel_l2(X[k], x1) <= 1e-6
         assert abs(int(its[k]) - i1) <= 1
+
+
+@pytest.mark.parametrize("pc", [0, 1])
+@pytest.mark.parametrize("transpose", [False, True])
+@pytest.mark.parametrize("e", [-332, 332])
+def test_flexible_solves_scale_with_the_right_hand_side(gpu_lib, pc, transpose, e):
+    # 2^332 is about 1e100, far outside the range of the FP32 inner solves.  A
+    # power of two changes no rounding of the FP64 outer method (sums of
+    # squares stay below 2^1023 and above 2^-1022), so the solutions are each
+    # other's multiples to the last bits
+    A = gpu_lib
+    m = W.make_lattice_mesh(6, jitter=0.2, codes="channel")
+    ctx = A.Context.from_mesh(m, W.freestream(0.5))
+    ctx.set_preconditioner(pc)
+    U = W.smooth_state(m["X"], 0.5)
+    S = A.Sensitivity(ctx)
+    s = 2.0 ** e
+    B = np.random.default_rng(7).standard_normal((3, ctx.N, 5))
+    opt = dict(transpose=transpose, krylov=7, maxits=24, eps=1e-9, inner_its=6)
+    X, its, res = S.solve_batch(U, B, **opt)
+    assert its.max() > 7 and (res < 0.1 * np.sqrt(B[0].size)).all()   # restarted, and below |B_k|
+    Xs, its_s, res_s = S.solve_batch(U, s * B, **opt)
+    assert np.array_equal(its, its_s)
+    assert rel_l2(Xs / s, X) <= 1e-14 and rel_l2(res_s / s, res) <= 1e-14
+    # one flexible solve, and systems of different scale in one batch
+    x1, i1, _ = S.solve(U, B[0], **opt)
+    xs, i2, _ = S.solve(U, s * B[0], **opt)
+    assert i1 == i2 and rel_l2(xs / s, x1) <= 1e-14
+    mixed = S.solve_batch(U, B * np.array([1.0, s, 1.0])[:, None, None], **opt)[0]
+    assert rel_l2(mixed[1] / s, X[1]) <= 1e-14 and np.array_equal(mixed[0], X[0]) and np.array_equal(mixed[2], X[2])
