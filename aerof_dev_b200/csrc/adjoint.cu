@@ -610,7 +610,7 @@ static void forward_blocked(aerof_gpu_ctx* c, const double* dU, const double* dv
   if (grad && geo) {
     const size_t smem = fwd_grad_smem(m);
     auto go = [&](auto kern) {
-      AEROF_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+      allow_smem(kern, smem);
       kern<<<m.nblk, kFGradThreads, smem, s>>>(m.N, m.NB, m.P2.p, w.D2.p, m.W2.p, m.n2o.p, m.lsqR.p, m.nb2_ptr.p,
                                                m.lnb.p, m.hptr.p, m.hnode.p, w.dG2.p);
       AEROF_LAUNCH_CHECK();
@@ -624,7 +624,7 @@ static void forward_blocked(aerof_gpu_ctx* c, const double* dU, const double* dv
   }
   const size_t smem = fwd_smem(m);
   auto edges = [&](auto kern) {
-    AEROF_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    allow_smem(kern, smem);
     const FaceArgs fa{m.F, m.Ubd.p, m.faces.p, m.fcode.p, m.fnrm.p, m.o2n.p, c->s.fbuf.p};
     const int nface = grid_for(3 * (size_t)m.F, kFwdThreads);
     kern<<<m.nblk + nface, kFwdThreads, smem, s>>>(m.N, m.E, m.NB, g, rec, c->cfg.beta, m.bl.p, m.bnorm.p, w.dbn.p,
@@ -1472,7 +1472,7 @@ static void lsq_transpose_blocked(aerof_gpu_ctx* c, const double* dU, int rec, d
   const size_t smem = lsq_blocked_smem(m);
   const int L = kLsqThreads / m.NB;
   auto go = [&](auto kern) {
-    AEROF_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    allow_smem(kern, smem);
     kern<<<m.nblk, kLsqThreads, smem, s>>>(m.N, m.NB, g, rec, m.n2o.p, dU, m.P2.p, m.W2.p, m.nb2_ptr.p, m.lnb.p,
                                            m.hptr.p, m.hnode.p, a.gV2.p, a.gG2.p, dout);
     AEROF_LAUNCH_CHECK();
@@ -1516,7 +1516,7 @@ static void reverse_sweep_blocked(aerof_gpu_ctx* c, const double* dw, bool geo, 
   AEROF_LAUNCH_CHECK();
   const size_t smem = ((size_t)(kPS + kGS + 6) * (m.NB + m.maxHf) + (size_t)kRevEdge * (kRevThreads + m.NB)) * sizeof(double);
   auto go = [&](auto kern) {
-    AEROF_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    allow_smem(kern, smem);
     kern<<<m.nblk, kRevThreads, smem, s>>>(m.N, m.E, m.NB, g, rec, c->cfg.beta, m.bl.p, m.bnorm.p, m.beptr.p, m.hfptr.p,
                                    m.hfpad.p, m.maxHf, m.P2.p, c->s.G2.p, a.lam2.p, m.lptr.p, m.lidx.p, m.xslot.p,
                                    m.bsrc.p, a.gVp.p, a.gGp.p, a.spill.p, geo ? a.geo.p : nullptr);
@@ -2618,13 +2618,13 @@ static void h2_vjp_dev(aerof_gpu_ctx* c, const double* dw, double* dout) {
   const bool wide = (!wide_var || std::atoi(wide_var) != 0) && h2t_wide_smem(m) <= 220 * 1024;
   if (wide) {
     const size_t smem = h2t_wide_smem(m);
-    AEROF_CUDA(cudaFuncSetAttribute(k_h2t_wide, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    allow_smem(k_h2t_wide, smem);
     k_h2t_wide<<<m.nblk, kWideThreads, smem, s>>>(m.N, m.E, m.NB, m.bl.p, m.beptr.p, m.hfptr.p, m.hfpad.p, m.maxHf,
                                                   m.P2.p, a.lam2.p, m.lptr.p, m.lidx.p, m.xslot.p, h2pairs(h),
                                                   a.gVp.p, a.gGp.p, a.spill.p);
   } else {
     const size_t smem = h2t_smem(m);
-    AEROF_CUDA(cudaFuncSetAttribute(k_h2t_blocked, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    allow_smem(k_h2t_blocked, smem);
     k_h2t_blocked<<<m.nblk, 256, smem, s>>>(m.N, m.E, m.NB, m.bl.p, m.beptr.p, m.hfptr.p, m.hfpad.p, m.maxHf,
                                             m.P2.p, a.lam2.p, m.lptr.p, m.lidx.p, m.xslot.p, h2pairs(h), a.gVp.p,
                                             a.gGp.p, a.spill.p);
@@ -2663,7 +2663,7 @@ static void h2_jvp_dev(aerof_gpu_ctx* c, const double* dp, double* dout) {
   const char* fvar = std::getenv("AEROF_H2F_THREADS");
   const int fthreads = fvar && std::atoi(fvar) == 512 ? 512 : fvar && std::atoi(fvar) == 256 ? 256 : 1024;
   auto kf = fthreads == 512 ? k_h2_blocked<512, 2> : fthreads == 256 ? k_h2_blocked<256, 2> : k_h2_blocked<1024, 1>;
-  AEROF_CUDA(cudaFuncSetAttribute(kf, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  allow_smem(kf, smem);
   kf<<<m.nblk, fthreads, smem, s>>>(m.N, m.E, m.NB, h.rec, m.bl.p, m.beptr.p, m.hfptr.p, m.hfpad.p, m.maxHf,
                                          h.dP2.p, h.dG2.p, m.lptr.p, m.lidx.p, m.xslot.p, h2pairs(h), h.part.p,
                                          h.spill.p, h2_prefetch());

@@ -1,10 +1,28 @@
 // capi.cu -- context lifetime, stream selection and host/device staging of
 // the C ABI declared in include/aerof_gpu.h.
+#include <algorithm>
 #include <cstring>
+#include <map>
+#include <mutex>
 
 #include "common.cuh"
 
 namespace aerof {
+
+// The largest limit asked for so far, per device and kernel, is set on every
+// call: under the lock, so that two threads' calls cannot leave the lower one
+// behind, and again when it is known already, since a device reset forgets it.
+void raise_smem_limit(const void* kern, size_t smem) {
+  static std::mutex lock;
+  static std::map<std::pair<int, const void*>, size_t> limits;
+  int dev = 0;
+  AEROF_CUDA(cudaGetDevice(&dev));
+  const std::lock_guard<std::mutex> hold(lock);
+  size_t& m = limits[{dev, kern}];
+  const size_t most = std::max(m, smem);
+  AEROF_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
+  m = most;
+}
 
 bool is_device_ptr(const void* p) {
   cudaPointerAttributes a;

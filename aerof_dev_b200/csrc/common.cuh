@@ -475,6 +475,16 @@ inline int* counters(aerof_gpu_ctx* c) {
   return b.p;
 }
 
+// Lets kern take smem bytes of dynamic shared memory on the current device.
+// The limit belongs to the kernel, which contexts of other meshes share, in
+// other threads too: it only ever rises, so that no context's launch can meet
+// another one's lower limit (capi.cu).
+void raise_smem_limit(const void* kern, size_t smem);
+template <class... P>
+void allow_smem(void (*kern)(P...), size_t smem) {
+  raise_smem_limit((const void*)kern, smem);
+}
+
 // boundary data of the kernels that form subface fluxes (fbuf: [3F][5])
 struct FaceArgs {
   int F;

@@ -1222,7 +1222,7 @@ static void h1_precond_product(aerof_gpu_ctx* c, int R, const TV* x, size_t xs, 
   TimerScope t(c, AEROF_T_KSP_MATVEC);
   const size_t smem = h1_smem(m, J.precision);
   auto kern = trans ? k_h1_apply<TV, true> : k_h1_apply<TV, false>;
-  AEROF_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  allow_smem(kern, smem);
   launch_pdl(kern, dim3(m.nblk, R), kIB, smem, s, m.N, m.NB, make_gas(c->cfg.gamma), m.n2o.p, m.hptr.p, m.hnode.p,
              f.wptr.p, nrm, f.slot.p, f.mrow.p, rec, f.idt.p, m.brow.p, J.fsum.p, zp, pz, y, ys, skip);
 }
@@ -1259,7 +1259,7 @@ static GsDev gs_state(aerof_gpu_ctx* c, KrylovWork& k, int R, int m, size_t n, i
 static void gs_backsolve(aerof_gpu_ctx* c, const GsDev& st, int R) {
   const size_t smem = sizeof(double) * ((size_t)st.m + kGsL);
   if (smem > 44 * 1024)
-    AEROF_CUDA(cudaFuncSetAttribute(k_gs_backsolve, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    allow_smem(k_gs_backsolve, smem);
   k_gs_backsolve<<<R, 256, smem, c->stream>>>(st);
   AEROF_LAUNCH_CHECK();
 }
@@ -1283,7 +1283,7 @@ static void gs_iteration(aerof_gpu_ctx* c, const GsDev& st, int R, size_t n, int
   TimerScope t(c, AEROF_T_KSP_OTHER);
   const size_t smem = gs_smem(st.m);
   if (smem > 44 * 1024)
-    AEROF_CUDA(cudaFuncSetAttribute(k_gs_update<TV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    allow_smem(k_gs_update<TV>, smem);
   const dim3 grid(st.G, R);
   launch_pdl(k_gs_dots<TV>, grid, kGsT, 0, c->stream, n, j, V, vs, ld, W, ws, st);
   launch_pdl(k_gs_update<TV>, grid, kGsT, smem, c->stream, n, j, V, vs, ld, W, ws, st);

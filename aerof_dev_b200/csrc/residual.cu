@@ -1225,7 +1225,7 @@ static void launch_grad_pipe(aerof_gpu_ctx* c, const Gas& g, const double* dU, c
   const size_t smem = (size_t)2 * st.size * sizeof(double);
   const int L = kBlock / m.NB;
   auto go = [&](auto kern) {
-    AEROF_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    allow_smem(kern, smem);
     if (!m.grad_grid) {  // resident CTAs of this mesh's staging size
       int per_sm = 0, sms = 0;
       AEROF_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kBlock, smem));
@@ -1250,7 +1250,7 @@ static void launch_grad_staged(const DeviceMesh& m, const Gas& g, const double* 
     prim_to_P2(m, g, dU, s);
   }
   auto go = [&](auto kern) {
-    AEROF_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    allow_smem(kern, smem);
     kern<<<m.nblk, kBlock, smem, s>>>(m.N, m.NB, g, m.n2o.p, dU, m.P2.p, m.W2.p, m.nb2_ptr.p, m.lnb.p, m.hptr.p,
                                       m.hnode.p, tag, G2);
     AEROF_LAUNCH_CHECK();
@@ -1334,7 +1334,7 @@ static void fv_blocked_dev(aerof_gpu_ctx* c, int failsafe, int* counter, bool wa
   const int fv_threads = wide ? 512 : 256;
   auto fvk = wide ? k_fv_blocked<512, 2>
                   : by_smem >= 4 ? k_fv_blocked<256, 4> : by_smem == 3 ? k_fv_blocked<256, 3> : k_fv_blocked<256, 2>;
-  AEROF_CUDA(cudaFuncSetAttribute(fvk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  allow_smem(fvk, smem);
   const int nface = grid_for(3 * (size_t)m.F, fv_threads * kFaceItems), nwave = wave ? m.nblk : 0;
   launch_pdl(fvk, m.nblk + nwave + nface, fv_threads, smem, c->stream, m.N, m.E, m.NB, make_gas(c->cfg.gamma),
              c->cfg.reconstruction, c->cfg.beta, failsafe, m.bl.p, m.bnorm.p, m.beptr.p, m.hfptr.p, m.hfpad.p, m.maxHf,
@@ -1521,16 +1521,13 @@ static decltype(&k_fv_blocked<256, 2>) pipe_fv_kernel(const DeviceMesh& m) {
   return by_smem >= 4 ? k_fv_blocked<256, 4> : by_smem == 3 ? k_fv_blocked<256, 3> : k_fv_blocked<256, 2>;
 }
 
-// The shared-memory limits of the stages' kernels.  They belong to the
-// function, and another context with a smaller staging may have lowered them
-// since, so every call sets them.
+// the shared-memory limits of the stages' kernels
 static size_t pipe_attributes(const DeviceMesh& m) {
-  AEROF_CUDA(cudaFuncSetAttribute(pipe_fv_kernel(m), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)fv_blocked_smem(m)));
+  allow_smem(pipe_fv_kernel(m), fv_blocked_smem(m));
   const int L = kBlock / m.NB;
   auto gp = L == 4 ? k_grad_pipe<4> : L == 2 ? k_grad_pipe<2> : k_grad_pipe<1>;
   const size_t gsmem = (size_t)2 * grad_stage(m).size * sizeof(double);
-  AEROF_CUDA(cudaFuncSetAttribute(gp, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gsmem));
+  allow_smem(gp, gsmem);
   return gsmem;
 }
 
@@ -1835,7 +1832,7 @@ static void wave_blocked_dev(aerof_gpu_ctx* c) {
   c->s.wpart.ensure(m.N);
   c->s.wspill.ensure(std::max(m.nX, 1));
   const size_t smem = wave_smem(m);
-  AEROF_CUDA(cudaFuncSetAttribute(k_wave_blocked, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  allow_smem(k_wave_blocked, smem);
   launch_pdl(k_wave_blocked, m.nblk, 256, smem, c->stream, m.N, m.E, m.NB, make_gas(c->cfg.gamma), m.bl.p, m.bnorm.p,
              m.beptr.p, m.hfptr.p, m.hfpad.p, m.maxHf, m.P2.p, m.lptr.p, m.lidx.p, m.xslot.p, c->s.wpart.p,
              c->s.wspill.p);

@@ -84,3 +84,47 @@ def test_host_array_residuals_of_two_meshes_in_turn(gpu_lib, stream):
             R = torch.empty_like(Uh).pin_memory()
             A.SpaceOperator(ctx).computeResidual(Uh, R)
             assert torch.equal(R, ref)
+
+
+def test_contexts_of_different_meshes_in_threads(gpu_lib):
+    # every thread has a context of its own; the meshes' blocks stage different
+    # amounts, and a kernel's shared-memory limit is shared by all of them
+    import threading
+
+    import torch
+    A = gpu_lib
+    calls = {
+        "residual": lambda c, U: A.SpaceOperator(c).computeResidual(U)[0],
+        "timestep": lambda c, U: A.SpaceOperator(c).computeTimeStep(U, 1.0),
+        "rk2": lambda c, U: A.ExplicitRK2(c, 0.5).run(U.clone(), 1)[0],
+        "jvp": lambda c, U: A.Sensitivity(c).jvp(U, U),
+        "dRdX": lambda c, U: A.Sensitivity(c).dRdX(U, U[:, :3].contiguous()),
+        "vjp": lambda c, U: A.Sensitivity(c).vjp(U, U),
+        "newton": lambda c, U: A.ImplicitSteadySolver(c, max_steps=1).solve(U.clone())[0],
+    }
+    cases = []
+    for n, jitter in ((9, 0.0), (9, 0.2), (17, 0.05), (7, 0.1)):
+        m = W.make_lattice_mesh(n, jitter=jitter, codes="channel")
+        ctx = A.Context.from_mesh(m, W.freestream(0.6))
+        U = torch.from_numpy(W.perturbed_state(ctx.N, 0.6, amp=0.02)).cuda()
+        cases.append((ctx, U, {k: f(ctx, U) for k, f in calls.items()}))
+    torch.cuda.synchronize()
+    wrong = []
+
+    def work(ctx, U, ref):
+        for k, f in calls.items():
+            for _ in range(100 if k != "newton" else 20):
+                try:
+                    same = torch.equal(f(ctx, U), ref[k])
+                except A.AerofError as e:
+                    same = e
+                if same is not True:
+                    wrong.append((ctx.N, k, same))
+                    return
+
+    threads = [threading.Thread(target=work, args=c) for c in cases]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong
