@@ -266,7 +266,7 @@ struct Scratch {
 // and integers, reduction partials, and the page-locked words its kernels
 // report to the host.
 struct KrylovWork {
-  DBuf<double> d, part;
+  DBuf<double> d, part, scratch;
   DBuf<int> i;
   void *pub = nullptr, *dpub = nullptr;   // GsPub [kMaxSys], host and device address
   ~KrylovWork() {

@@ -1254,17 +1254,22 @@ static GsDev gs_state(aerof_gpu_ctx* c, KrylovWork& k, int R, int m, size_t n, i
   st.part = k.part.p;
   st.norm_part = k.part.p + (size_t)R * 2 * (m + 1) * st.G;
   st.pub = (GsPub*)k.dpub;
+  st.scratch = nullptr;
+  if (m > kGsMax) {
+    k.scratch.ensure((size_t)R * st.G * 3 * ((size_t)m + 1));
+    st.scratch = k.scratch.p;
+  }
   return st;
 }
 static void gs_backsolve(aerof_gpu_ctx* c, const GsDev& st, int R) {
-  const size_t smem = sizeof(double) * ((size_t)st.m + kGsL);
+  const size_t smem = sizeof(double) * ((st.scratch ? 0 : (size_t)st.m) + kGsL);
   if (smem > 44 * 1024)
     allow_smem(k_gs_backsolve, smem);
   k_gs_backsolve<<<R, 256, smem, c->stream>>>(st);
   AEROF_LAUNCH_CHECK();
 }
 // dynamic shared memory of the second sweep
-static size_t gs_smem(int m) { return sizeof(double) * ((size_t)3 * (m + 1) + kGsL); }
+static size_t gs_smem(int m) { return sizeof(double) * ((m > kGsMax ? 0 : (size_t)3 * (m + 1)) + kGsL); }
 
 // Gram-Schmidt step j of the R systems and the Givens update.  Measured with
 // everything around it (stored products): a pseudo-time step of 81^3 with 20
@@ -1337,6 +1342,7 @@ static void gmres_device(aerof_gpu_ctx* c, int R, const double* const* B, double
   DeviceMesh& m = c->mesh;
   Implicit& J = c->imp;
   cudaStream_t s = c->stream;
+  numVec = std::min(numVec, maxits);   // a cycle never gets longer
   const size_t n = 5 * (size_t)m.N, ld = (n + 63) / 64 * 64, vs = (size_t)(numVec + 1) * ld;
   auto bytes = [](size_t count) { return (count * sizeof(TV) + 7) / 8; };
   J.basis.ensure(bytes((size_t)R * vs));
@@ -1373,7 +1379,7 @@ static void gmres_device(aerof_gpu_ctx* c, int R, const double* const* B, double
       gs_iteration<TV>(c, st, R, n, j, V, vs, ld, W, ld);
     }
     gs_backsolve(c, st, R);
-    k_gs_combine<TV, false><<<gv, kIB, sizeof(double) * (numVec + 1), s>>>(n, V, vs, ld, st, W, ld, x);
+    k_gs_combine<TV, false><<<gv, kIB, 0, s>>>(n, V, vs, ld, st, W, ld, x);
     AEROF_LAUNCH_CHECK();
     prec_apply_t<TV, TV>(c, W, Z, trans, R, ld, ld);
     k_gs_add<TV><<<gv, kIB, 0, s>>>(n, Z, ld, st, x);
@@ -1405,6 +1411,7 @@ static void fgmres_device(aerof_gpu_ctx* c, int R, const double* const* B, doubl
   DeviceMesh& m = c->mesh;
   Implicit& J = c->imp;
   cudaStream_t s = c->stream;
+  numVec = std::min(numVec, maxits);   // a cycle never gets longer
   const size_t n = 5 * (size_t)m.N, ld = (n + 63) / 64 * 64;
   const size_t vs = (size_t)(numVec + 1) * ld, zs = (size_t)numVec * ld;
   J.bV.ensure((size_t)R * vs);
@@ -1457,7 +1464,7 @@ static void fgmres_device(aerof_gpu_ctx* c, int R, const double* const* B, doubl
       AEROF_LAUNCH_CHECK();
     }
     gs_backsolve(c, st, R);
-    k_gs_combine<double, true><<<gv, kIB, sizeof(double) * (numVec + 1), s>>>(n, Z, zs, ld, st, nullptr, 0, x);
+    k_gs_combine<double, true><<<gv, kIB, 0, s>>>(n, Z, zs, ld, st, nullptr, 0, x);
     AEROF_LAUNCH_CHECK();
     AEROF_CUDA(cudaStreamSynchronize(s));
     bool all = true;
@@ -2190,9 +2197,10 @@ extern "C" int aerof_gpu_linearized_solve_batch(aerof_gpu_ctx* c, const double* 
       const cudaMemcpyKind kb = is_device_ptr(B) ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
       const cudaMemcpyKind kx = is_device_ptr(X) ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost;
       // per right-hand side: the outer FP64 bases and work vectors, the inner
-      // FP32 basis and work vectors and, with ILU(0), the sweeps' FP64 work
-      // vector (5N doubles)
-      const size_t per = ((size_t)2 * krylov + 5 + (c->imp.pc == AEROF_PC_ILU0 ? 1 : 0)) * ld * sizeof(double) +
+      // FP32 basis and work vectors, with ILU(0) the sweeps' FP64 work vector
+      // (5N doubles), and the Hessenberg matrix and the products of the basis
+      const size_t kv = (size_t)std::min(krylov, maxits);
+      const size_t per = ((2 * kv + 5 + (c->imp.pc == AEROF_PC_ILU0 ? 1 : 0)) * ld + 2 * kv * (kv + 1)) * sizeof(double) +
                          ((size_t)inner_its + 5) * ld * sizeof(float);
       size_t freeb = 0, totalb = 0;
       AEROF_CUDA(cudaMemGetInfo(&freeb, &totalb));

@@ -33,6 +33,7 @@ namespace aerof {
 
 constexpr int kGsT = 512;        // threads of the sweeps
 constexpr int kGsL = 4000;       // doubles of L kept in shared memory by the triangular solve
+constexpr int kGsMax = 7199;     // longest restart whose coefficients fit in shared memory (200 KB)
 constexpr int kMaxSys = 64;      // systems per launch
 
 // what the host reads while the cycle runs (page-locked, mapped)
@@ -52,6 +53,7 @@ struct GsDev {
   double* part;                  // [R][2 (m + 1)][G] partial sums of the dot products
   double* norm_part;             // [R][G] of the norm
   GsPub* pub;
+  double* scratch;               // m > kGsMax: [R][G][3 (m + 1)] for the coefficients, else null
   int m, G;
   bool unit;                     // every basis vector is stored normalised (k_gs_unit)
   __host__ __device__ size_t oL() const { return (size_t)(m + 1) * m; }
@@ -318,12 +320,11 @@ __global__ void __launch_bounds__(kGsT, 1) k_gs_dots(size_t n, int j, const TV* 
 
 // The coefficients of iteration j in a[0..j] (shared memory), from the
 // partial sums: the block computes them whole, so every block has the same
-// ones without a grid-wide step.  Block 0 keeps row j of L.  sh: vals
-// [2 (m + 1)], a [m + 1], L (packed rows 1..j while they fit).
-__device__ __forceinline__ double* gs_coefficients(const GsDev& st, int q, int j, double* sh) {
-  double* vals = sh;
+// ones without a grid-wide step.  Block 0 keeps row j of L.  vals
+// [3 (m + 1)]: the sums, then the coefficients; sL: L (packed rows 1..j while
+// they fit).
+__device__ __forceinline__ double* gs_coefficients(const GsDev& st, int q, int j, double* vals, double* sL) {
   double* a = vals + 2 * (st.m + 1);
-  double* sL = a + st.m + 1;
   double* d = st.d + (size_t)q * st.sd;
   double* L = d + st.oL();
   const double* sig = d + st.oSig();
@@ -362,7 +363,7 @@ __device__ __forceinline__ double* gs_coefficients(const GsDev& st, int q, int j
 template <class TV>
 __global__ void __launch_bounds__(kGsT, 1) k_gs_update(size_t n, int j, TV* V, size_t vs, size_t ld,
                                                        const TV* W, size_t ws, GsDev st) {
-  extern __shared__ double sh[];   // see gs_coefficients
+  extern __shared__ double smem[];   // see gs_coefficients
   __shared__ double red[kGsT / 32];
   __shared__ double nrm[1];
   const int q = blockIdx.y;
@@ -375,7 +376,9 @@ __global__ void __launch_bounds__(kGsT, 1) k_gs_update(size_t n, int j, TV* V, s
   double* d = st.d + (size_t)q * st.sd;
   const double* sig = d + st.oSig();
   const double sj = sig[j];
-  const double* hcol = gs_coefficients(st, q, j, sh);
+  const size_t len = 3 * ((size_t)st.m + 1);
+  double* sh = st.scratch ? st.scratch + ((size_t)q * gridDim.x + blockIdx.x) * len : smem;
+  const double* hcol = gs_coefficients(st, q, j, sh, st.scratch ? smem : smem + len);
   double* cf = sh;                 // h_i sig_i, over the finished sums
   for (int k = threadIdx.x; k <= j; k += blockDim.x) cf[k] = hcol[k] * sig[k];
   __syncthreads();
@@ -495,7 +498,7 @@ __global__ void __launch_bounds__(kGsT, 1) k_gs_update(size_t n, int j, TV* V, s
 // system: y from the rotated Hessenberg matrix (staged, row by row of the
 // upper triangle) and g; lane i subtracts column k's product as y_k is known
 __global__ void __launch_bounds__(256) k_gs_backsolve(GsDev st) {
-  extern __shared__ double sh[];   // g [m], H (packed columns while they fit)
+  extern __shared__ double sh[];   // g [m] (in y itself when m > kGsMax), H (packed columns while they fit)
   const int q = blockIdx.x;
   const int* ist = st.i + 8 * q;
   if (!ist[3]) return;
@@ -503,7 +506,7 @@ __global__ void __launch_bounds__(256) k_gs_backsolve(GsDev st) {
   const double *H = d, *g = d + st.oG();
   double* y = d + st.oY();
   const int j = ist[2], n = j + 1;
-  double *sy = sh, *sH = sh + st.m;
+  double *sy = st.scratch ? y : sh, *sH = st.scratch ? sh : sh + st.m;
   const bool cached = n * (n + 1) / 2 <= kGsL;
   for (int i = threadIdx.x; i < n; i += blockDim.x) sy[i] = g[i];
   if (cached)
@@ -523,27 +526,35 @@ __global__ void __launch_bounds__(256) k_gs_backsolve(GsDev st) {
     }
   }
   __syncthreads();
-  for (int i = threadIdx.x; i < n; i += blockDim.x) y[i] = sy[i];
+  if (sy != y)
+    for (int i = threadIdx.x; i < n; i += blockDim.x) y[i] = sy[i];
 }
 
+constexpr int kGsChunk = 512;    // coefficients staged at a time
 // out = sum_i y_i sig_i Z_i over the cycle's columns: stored as TV (ADD
 // false), or added to x (the flexible method's corrections)
 template <class TV, bool ADD>
 __global__ void __launch_bounds__(256) k_gs_combine(size_t n, const TV* __restrict__ Z, size_t zs, size_t ld, GsDev st,
                                                     TV* __restrict__ out, size_t os, VecOut X) {
-  extern __shared__ double c[];
+  __shared__ double c[kGsChunk];
   const int q = blockIdx.y;
   const int* ist = st.i + 8 * q;
   if (!ist[3]) return;
   const double* d = st.d + (size_t)q * st.sd;
   const int k = ist[2] + 1;
-  for (int i = threadIdx.x; i < k; i += blockDim.x) c[i] = d[st.oY() + i] * d[st.oSig() + i];
-  __syncthreads();
   const size_t p = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= n) return;
   double s = 0.0;
+  for (int i0 = 0; i0 < k; i0 += kGsChunk) {
+    const int nc = min(kGsChunk, k - i0);
+    __syncthreads();
+    for (int i = threadIdx.x; i < nc; i += blockDim.x) c[i] = d[st.oY() + i0 + i] * d[st.oSig() + i0 + i];
+    __syncthreads();
+    if (p < n) {
 #pragma unroll 8
-  for (int i = 0; i < k; ++i) s += c[i] * (double)Z[(size_t)q * zs + (size_t)i * ld + p];
+      for (int i = 0; i < nc; ++i) s += c[i] * (double)Z[(size_t)q * zs + (size_t)(i0 + i) * ld + p];
+    }
+  }
+  if (p >= n) return;
   if (ADD) X.p[q][p] += s;
   else out[(size_t)q * os + p] = (TV)s;
 }

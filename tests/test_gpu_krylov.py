@@ -109,3 +109,29 @@ def test_flexible_solves_scale_with_the_right_hand_side(gpu_lib, pc, transpose, 
     assert i1 == i2 and rel_l2(xs / s, x1) <= 1e-14
     mixed = S.solve_batch(U, B * np.array([1.0, s, 1.0])[:, None, None], **opt)[0]
     assert rel_l2(mixed[1] / s, X[1]) <= 1e-14 and np.array_equal(mixed[0], X[0]) and np.array_equal(mixed[2], X[2])
+
+
+@pytest.mark.parametrize("krylov", [100, 513, 6200, 7199, 7200, 9000])
+def test_long_restarts(gpu_lib, krylov):
+    # more vectors than are staged at a time (512), than 48 KB of shared memory
+    # hold (6144) and than 200 KB do (7199), on a system of 135 unknowns that
+    # needs far fewer: the same solution whatever the longest cycle
+    A = gpu_lib
+    m = W.make_lattice_mesh(3, jitter=0.2, codes="channel")
+    ctx = A.Context.from_mesh(m, W.freestream(0.5))
+    U = W.smooth_state(m["X"], 0.5)
+    S = A.Sensitivity(ctx)
+    B = np.random.default_rng(3).standard_normal((2, ctx.N, 5))
+    X, its, res = S.solve_batch(U, B, krylov=krylov, maxits=krylov, eps=1e-9, inner_its=5)
+    for k in range(2):
+        assert its[k] < 136 and res[k] <= 1e-9 * np.linalg.norm(B[k])
+        assert np.linalg.norm(S.jvp(U, X[k]) - B[k]) <= 1e-8 * np.linalg.norm(B[k])
+    # the same cycle length throughout when the iterations bound it
+    Y = S.solve_batch(U, B, krylov=krylov, maxits=60, eps=0.0, inner_its=5)[0]
+    assert np.array_equal(Y, S.solve_batch(U, B, krylov=60, maxits=60, eps=0.0, inner_its=5)[0])
+    mv = A.MatVecProdH1(ctx, 64)
+    mv.evaluate(U, A.SpaceOperator(ctx).computeTimeStep(U, 50.0))
+    A.JacobiPrec(ctx).setup()
+    x, i, r = A.GmresSolver(ctx, krylov, krylov, 1e-9).solve(B[0])
+    assert i < 136 and r <= 1e-9 * np.linalg.norm(B[0])
+    assert np.linalg.norm(mv.apply(x) - B[0]) <= 1e-8 * np.linalg.norm(B[0])
