@@ -974,7 +974,10 @@ __global__ void k_a_lam2(int N, const int* __restrict__ n2o, const double* __res
 // Threads of the reverse sweep.  Its staging leaves one CTA per SM, so the
 // warps in flight are the CTA's: 8 at 256 threads and 234 registers, 16 at
 // 512 and 128 (some spills).  Adjoint products at 101^3: 4.41 ms with 384,
-// 4.24 ms with 512 (4.70 ms with 256 and exact divisions and roots).
+// 4.24 ms with 512 (4.70 ms with 256 and exact divisions and roots).  Their
+// chunk takes 105 KB beside the staged nodes; where 512 do not fit (stretched
+// cells: more than 448 nodes staged for blocks of 128) the sweep runs with 256
+// threads (up to 606), still without the gathers of the general form.
 constexpr int kRevThreads = 512;
 
 // Edges per chunk (one per thread) and doubles per edge kept in shared memory
@@ -1495,6 +1498,17 @@ static bool assemble_lsq_blocked(aerof_gpu_ctx* c, const double* dU, const doubl
   return true;
 }
 
+static size_t rev_smem(const DeviceMesh& m, int threads) {
+  return ((size_t)(kPS + kGS + 6) * (m.NB + m.maxHf) + (size_t)kRevEdge * (threads + m.NB)) * sizeof(double);
+}
+// threads of the blocked reverse sweep, 0 where its shared memory does not fit
+static int rev_threads(const DeviceMesh& m) {
+  for (int t = kRevThreads; m.nblk > 0 && t >= std::max(m.NB, 256); t /= 2)
+    if (rev_smem(m, t) <= 224 * 1024) return t;
+  return 0;
+}
+static bool reverse_blocked_fits(const DeviceMesh& m) { return rev_threads(m) > 0; }
+
 // Blocked reverse sweep over the edges and faces: a.gV, a.gG (caller
 // numbering) from the cotangent dw; with geo, also the cotangents of the
 // edge normals and dx.  Needs P (caller numbering) and P2/G2 current.
@@ -1514,10 +1528,11 @@ static void reverse_sweep_blocked(aerof_gpu_ctx* c, const double* dw, bool geo, 
   if (geo) a.geo.ensure(6 * (size_t)std::max(m.E, 1));
   k_a_lam2<<<gn, kAB, 0, s>>>(m.N, m.n2o.p, dw, m.vol2.p, a.lam2.p);
   AEROF_LAUNCH_CHECK();
-  const size_t smem = ((size_t)(kPS + kGS + 6) * (m.NB + m.maxHf) + (size_t)kRevEdge * (kRevThreads + m.NB)) * sizeof(double);
+  const int threads = rev_threads(m);
+  const size_t smem = rev_smem(m, threads);
   auto go = [&](auto kern) {
     allow_smem(kern, smem);
-    kern<<<m.nblk, kRevThreads, smem, s>>>(m.N, m.E, m.NB, g, rec, c->cfg.beta, m.bl.p, m.bnorm.p, m.beptr.p, m.hfptr.p,
+    kern<<<m.nblk, threads, smem, s>>>(m.N, m.E, m.NB, g, rec, c->cfg.beta, m.bl.p, m.bnorm.p, m.beptr.p, m.hfptr.p,
                                    m.hfpad.p, m.maxHf, m.P2.p, c->s.G2.p, a.lam2.p, m.lptr.p, m.lidx.p, m.xslot.p,
                                    m.bsrc.p, a.gVp.p, a.gGp.p, a.spill.p, geo ? a.geo.p : nullptr);
     AEROF_LAUNCH_CHECK();
@@ -1532,12 +1547,6 @@ static void reverse_sweep_blocked(aerof_gpu_ctx* c, const double* dw, bool geo, 
                                  m.vol.p, a.gV.p);
     AEROF_LAUNCH_CHECK();
   }
-}
-
-// whether the blocked reverse sweep's shared memory fits
-static bool reverse_blocked_fits(const DeviceMesh& m) {
-  return m.nblk > 0 &&
-         ((size_t)(kPS + kGS + 6) * (m.NB + m.maxHf) + (size_t)kRevEdge * (kRevThreads + m.NB)) * sizeof(double) <= 224 * 1024;
 }
 
 // J^T w for device state dU and cotangent dw, into dout ([N][5]).

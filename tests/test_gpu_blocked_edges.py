@@ -91,3 +91,33 @@ def test_spalart_allmaras(gpu_lib, oracle_mod, n, codes, rec, model):
                            alpha=1.3, Ts=0.35)
     for R in out:
         assert rel_l2(R, ref) < 1e-12 and rel_l2(R[:, 5], ref[:, 5]) < 1e-12
+
+
+@pytest.mark.parametrize("rec", [1, 2])
+@pytest.mark.parametrize("n,squash,nodes", [(29, 0.03, 128), (31, 0.04, 128), (33, 0.02, 128), (8, 1.0, 256)])
+def test_reverse_sweep_with_fewer_threads(gpu_lib, monkeypatch, n, squash, nodes, rec):
+    # stretched cells (or blocks of 256 nodes) stage so many nodes that the
+    # reverse sweep's chunk of 512 edges does not fit beside them: it runs
+    # blocked all the same, in chunks of 256.  Against blocks of 64 nodes,
+    # where 512 fit: the same sums of ~26 terms in another order
+    A = gpu_lib
+    m = W.make_lattice_mesh(n, jitter=0.2, codes="channel")
+    m["X"] = m["X"] * np.array([1.0, 1.0, squash])
+    rng = np.random.default_rng(n)
+    N = m["X"].shape[0]
+    U, lam = W.perturbed_state(N, 0.6), rng.standard_normal((N, 5))
+    out = []
+    for nb in (nodes, 64):
+        monkeypatch.setenv("AEROF_BLOCK_NODES", str(nb))
+        S = A.Sensitivity(A.Context.from_mesh(m, W.freestream(0.6), reconstruction=rec))
+        A.launch_count()
+        w = S.vjp(U, lam)
+        launches = A.launch_count()
+        out.append((w, *S.adjoint_products(U, lam), launches))
+    (w, jt, gx, k), (w64, jt64, gx64, k64) = out
+    assert k == k64   # the same organisation
+    assert rel_l2(w, w64) < 1e-12 and rel_l2(jt, jt64) < 1e-12 and rel_l2(gx, gx64) < 1e-11
+    S = A.Sensitivity(A.Context.from_mesh(m, W.freestream(0.6), reconstruction=rec))
+    v = rng.standard_normal((N, 5))
+    Jv = S.jvp(U, v)
+    assert abs((lam * Jv).sum() - (w * v).sum()) < 1e-12 * np.linalg.norm(lam) * np.linalg.norm(Jv)
