@@ -1262,10 +1262,11 @@ static GsDev gs_state(aerof_gpu_ctx* c, KrylovWork& k, int R, int m, size_t n, i
   return st;
 }
 static void gs_backsolve(aerof_gpu_ctx* c, const GsDev& st, int R) {
-  const size_t smem = sizeof(double) * ((st.scratch ? 0 : (size_t)st.m) + kGsL);
-  if (smem > 44 * 1024)
-    allow_smem(k_gs_backsolve, smem);
-  k_gs_backsolve<<<R, 256, smem, c->stream>>>(st);
+  const bool big = st.scratch != nullptr;
+  const size_t smem = sizeof(double) * ((big ? 0 : (size_t)st.m) + kGsL);
+  auto kern = big ? k_gs_backsolve<true> : k_gs_backsolve<false>;
+  if (smem > 44 * 1024) allow_smem(kern, smem);
+  kern<<<R, 256, smem, c->stream>>>(st);
   AEROF_LAUNCH_CHECK();
 }
 // dynamic shared memory of the second sweep
@@ -1287,11 +1288,11 @@ static void gs_iteration(aerof_gpu_ctx* c, const GsDev& st, int R, size_t n, int
                          const TV* W, size_t ws) {
   TimerScope t(c, AEROF_T_KSP_OTHER);
   const size_t smem = gs_smem(st.m);
-  if (smem > 44 * 1024)
-    allow_smem(k_gs_update<TV>, smem);
+  auto update = st.scratch ? k_gs_update<TV, true> : k_gs_update<TV, false>;
+  if (smem > 44 * 1024) allow_smem(update, smem);
   const dim3 grid(st.G, R);
   launch_pdl(k_gs_dots<TV>, grid, kGsT, 0, c->stream, n, j, V, vs, ld, W, ws, st);
-  launch_pdl(k_gs_update<TV>, grid, kGsT, smem, c->stream, n, j, V, vs, ld, W, ws, st);
+  launch_pdl(update, grid, kGsT, smem, c->stream, n, j, V, vs, ld, W, ws, st);
 }
 
 // The host's side of a running cycle: before the cycle, and until every

@@ -360,7 +360,10 @@ __device__ __forceinline__ double* gs_coefficients(const GsDev& st, int q, int j
 // rounded once) and its norm; then the Givens update of the Hessenberg
 // column, written with explicitly rounded operations (the host loop's
 // arithmetic), and the step's result for the host.
-template <class TV>
+// BIG: the coefficients in global memory (m > kGsMax).  A kernel of its own:
+// chosen at run time, the pointer made the inner loop's coefficient loads
+// generic ones, 1.8 us per iteration of 61^3.
+template <class TV, bool BIG>
 __global__ void __launch_bounds__(kGsT, 1) k_gs_update(size_t n, int j, TV* V, size_t vs, size_t ld,
                                                        const TV* W, size_t ws, GsDev st) {
   extern __shared__ double smem[];   // see gs_coefficients
@@ -377,8 +380,8 @@ __global__ void __launch_bounds__(kGsT, 1) k_gs_update(size_t n, int j, TV* V, s
   const double* sig = d + st.oSig();
   const double sj = sig[j];
   const size_t len = 3 * ((size_t)st.m + 1);
-  double* sh = st.scratch ? st.scratch + ((size_t)q * gridDim.x + blockIdx.x) * len : smem;
-  const double* hcol = gs_coefficients(st, q, j, sh, st.scratch ? smem : smem + len);
+  double* sh = BIG ? st.scratch + ((size_t)q * gridDim.x + blockIdx.x) * len : smem;
+  const double* hcol = gs_coefficients(st, q, j, sh, BIG ? smem : smem + len);
   double* cf = sh;                 // h_i sig_i, over the finished sums
   for (int k = threadIdx.x; k <= j; k += blockDim.x) cf[k] = hcol[k] * sig[k];
   __syncthreads();
@@ -497,8 +500,9 @@ __global__ void __launch_bounds__(kGsT, 1) k_gs_update(size_t n, int j, TV* V, s
 // back substitution (KspSolver.C:966-982) of the cycle, one block per
 // system: y from the rotated Hessenberg matrix (staged, row by row of the
 // upper triangle) and g; lane i subtracts column k's product as y_k is known
+template <bool BIG>
 __global__ void __launch_bounds__(256) k_gs_backsolve(GsDev st) {
-  extern __shared__ double sh[];   // g [m] (in y itself when m > kGsMax), H (packed columns while they fit)
+  extern __shared__ double sh[];   // g [m] (BIG: in y itself), H (packed columns while they fit)
   const int q = blockIdx.x;
   const int* ist = st.i + 8 * q;
   if (!ist[3]) return;
@@ -506,7 +510,7 @@ __global__ void __launch_bounds__(256) k_gs_backsolve(GsDev st) {
   const double *H = d, *g = d + st.oG();
   double* y = d + st.oY();
   const int j = ist[2], n = j + 1;
-  double *sy = st.scratch ? y : sh, *sH = st.scratch ? sh : sh + st.m;
+  double *sy = BIG ? y : sh, *sH = BIG ? sh : sh + st.m;
   const bool cached = n * (n + 1) / 2 <= kGsL;
   for (int i = threadIdx.x; i < n; i += blockDim.x) sy[i] = g[i];
   if (cached)
@@ -526,7 +530,7 @@ __global__ void __launch_bounds__(256) k_gs_backsolve(GsDev st) {
     }
   }
   __syncthreads();
-  if (sy != y)
+  if (!BIG)
     for (int i = threadIdx.x; i < n; i += blockDim.x) y[i] = sy[i];
 }
 
