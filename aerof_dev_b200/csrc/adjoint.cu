@@ -829,6 +829,26 @@ __device__ __forceinline__ Dual5 rsqrt_(const Dual5& a) {
   return r;
 }
 
+__device__ __forceinline__ Dual5 sqrt_(const Dual5& x, const Dual5& y) {
+  Dual5 r(sqrt_(x.v, y.v));
+  const double h = 0.5 * y.v;
+#pragma unroll
+  for (int k = 0; k < 5; ++k) r.d[k] = h * x.d[k];
+  return r;
+}
+__device__ __forceinline__ Dual5 quot_(const Dual5& a, const Dual5& b, const Dual5& i) {
+  Dual5 r(quot_(a.v, b.v, i.v));
+#pragma unroll
+  for (int k = 0; k < 5; ++k) r.d[k] = (a.d[k] - r.v * b.d[k]) * i.v;
+  return r;
+}
+__device__ __forceinline__ Dual5 quot_(const Dual5& a, double b, double i) {
+  Dual5 r(quot_(a.v, b, i));
+#pragma unroll
+  for (int k = 0; k < 5; ++k) r.d[k] = a.d[k] * i;
+  return r;
+}
+
 // Face flux cotangents, g_V += (d flux / d V)^T lam, the five state
 // directions in one forward-mode evaluation
 __device__ void face_vjp_V(const Gas& g, int code, double nx, double ny, double nz, const double* V, const double* Ub,

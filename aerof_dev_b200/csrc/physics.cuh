@@ -83,6 +83,34 @@ AEROF_HD double rsqrt_(double x) {
   return 1.0 / sqrt(x);
 #endif
 }
+// sqrt(x) given y = rsqrt_(x), and a / b given r = rcp_(b): the products x y
+// and a r, each with one correction by its own residual (Newton's step for
+// s^2 = x, and for q b = a; Markstein 2000 as above).  Without the correction
+// a product is off by up to 1.5 ulp, with it by 0.5 and a little.
+AEROF_HD double sqrt_(double x, double y) {
+#ifdef __CUDA_ARCH__
+  const double s = x * y;
+  return fma(0.5 * y, fma(-s, s, x), s);
+#else
+  (void)y;
+  return sqrt(x);
+#endif
+}
+AEROF_HD double quot_(double a, double b, double r) {
+#ifdef __CUDA_ARCH__
+  const double q = a * r;
+  return fma(r, fma(-b, q, a), q);
+#else
+  (void)r;
+  return a / b;
+#endif
+}
+AEROF_HD Dual sqrt_(Dual x, Dual y) { return Dual(sqrt_(x.v, y.v), 0.5 * y.v * x.d); }
+AEROF_HD Dual quot_(Dual a, Dual b, Dual r) {
+  const double q = quot_(a.v, b.v, r.v);
+  return Dual(q, (a.d - q * b.d) * r.v);
+}
+AEROF_HD Dual quot_(Dual a, double b, double r) { return Dual(quot_(a.v, b, r), a.d * r); }
 AEROF_HD Dual rcp_(Dual x) {
   const double r = rcp_(x.v);
   return Dual(r, -(r * r) * x.d);
@@ -95,7 +123,7 @@ template <class T> AEROF_HD T sel(bool c, T a, T b) { return c ? a : b; }
 
 // ------------------------------------------------------------ gas model
 struct Gas {
-  double gam, gam1, invgam1, invgam;
+  double gam, gam1, invgam1, invgam, gogam;   // gogam: gam1 / gam
 };
 AEROF_HD Gas make_gas(double gam) {
   Gas g;
@@ -103,6 +131,7 @@ AEROF_HD Gas make_gas(double gam) {
   g.gam1 = gam - 1.0;
   g.invgam1 = 1.0 / g.gam1;
   g.invgam = 1.0 / gam;
+  g.gogam = g.gam1 / gam;
   return g;
 }
 
@@ -249,11 +278,14 @@ AEROF_HD void roe_flux(const Gas& g, TN n0, TN n1, TN n2, const T* Ug, const T* 
 
 // boundflux5.f:1-111 (type 0, sig = 0): Steger-Warming far-field flux
 // A+(V) U(V) + A-(V) Ub with V primitive and Ub conservative.
-// One reciprocal and two reciprocal square roots in place of eleven divisions
-// and two roots: a boundary node's faces are a serial chain.  EXACT keeps the
-// divisions and roots, for the forward differences of face_jac: their
-// increment is 1e-6 |V_k|, which for a velocity component near zero turns a
-// changed last bit into a visible change of the block.
+// A boundary node's faces are a serial chain, so the divisions and roots come
+// from one reciprocal and two reciprocal square roots with corrected products
+// (ten steps of 21^3 take 336 us, with divisions and roots 382 us).  Plain
+// products were no faster, and rounded 11 % worse
+// (tests/test_gpu_flux_rounding.py).  EXACT keeps the divisions and roots, for
+// the forward differences of face_jac: their increment is 1e-6 |V_k|, which
+// for a velocity component near zero turns a changed last bit into a visible
+// change of the block.
 template <bool EXACT = false, class T>
 AEROF_HD void sw_flux(const Gas& g, T vnx, T vny, T vnz, const T* ua, const double* ub, T* flux) {
   const double gam = g.gam, gam1 = g.gam1, ig = g.invgam, ig1 = g.invgam1;
@@ -264,8 +296,8 @@ AEROF_HD void sw_flux(const Gas& g, T vnx, T vny, T vnz, const T* ua, const doub
     capd1 = vnx / cap; capd2 = vny / cap; capd3 = vnz / cap;
   } else {
     icap = rsqrt_(s2);
-    cap = s2 * icap;
-    capd1 = vnx * icap; capd2 = vny * icap; capd3 = vnz * icap;
+    cap = sqrt_(s2, icap);
+    capd1 = quot_(vnx, cap, icap); capd2 = quot_(vny, cap, icap); capd3 = quot_(vnz, cap, icap);
   }
   T ro = ua[0];
   T usro;
@@ -282,10 +314,11 @@ AEROF_HD void sw_flux(const Gas& g, T vnx, T vny, T vnz, const T* ua, const doub
     usc = 1.0 / c;
     cc = 0.5 * vit + c2 / gam1;
   } else {
-    rhoE = ig1 * pm + 0.5 * ro * vit;
-    usc = rsqrt_(c2);
-    c = c2 * usc;
-    cc = 0.5 * vit + ig1 * c2;
+    rhoE = quot_(pm, gam1, ig1) + 0.5 * ro * vit;
+    const T yc = rsqrt_(c2);
+    c = sqrt_(c2, yc);
+    usc = quot_(T(1.0), c, yc);
+    cc = 0.5 * vit + quot_(c2, gam1, ig1);
   }
   T unx = capd1 * u + capd2 * v + capd3 * w;
   T l1 = cap * unx, l4 = cap * (unx + c), l5 = cap * (unx - c);
@@ -294,13 +327,13 @@ AEROF_HD void sw_flux(const Gas& g, T vnx, T vny, T vnz, const T* ua, const doub
   T vpm = vp4 - vp5;
   T fgp0 = gam1 * ro * vp1 + 0.5 * ro * vpp;
   if constexpr (EXACT) fgp0 = fgp0 / gam;
-  else fgp0 = ig * fgp0;
+  else fgp0 = quot_(fgp0, gam, ig);
   T fgp1 = fgp0 * u + 0.5 * pm * usc * capd1 * vpm;
   T fgp2 = fgp0 * v + 0.5 * pm * usc * capd2 * vpm;
   T fgp3 = fgp0 * w + 0.5 * pm * usc * capd3 * vpm;
   T fgp4;
   if constexpr (EXACT) fgp4 = 0.5 * ((gam1 / gam) * ro * vit * (vp1 - 0.5 * vpp) + rhoE * vpp + ro * unx * c * vpm / gam);
-  else fgp4 = 0.5 * ((gam1 * ig) * ro * vit * (vp1 - 0.5 * vpp) + rhoE * vpp + ig * (ro * unx * c * vpm));
+  else fgp4 = 0.5 * (g.gogam * ro * vit * (vp1 - 0.5 * vpp) + rhoE * vpp + quot_(ro * unx * c * vpm, gam, ig));
   vp1 = tmin0(l1); vp4 = tmin0(l4); vp5 = tmin0(l5);
   vpp = vp1 - 0.5 * (vp4 + vp5);
   vpm = 0.5 * (vp5 - vp4);
