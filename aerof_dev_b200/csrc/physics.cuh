@@ -582,40 +582,38 @@ namespace aerof {
 __device__ __forceinline__ void roe_flux_adj(const Gas& g, double n0, double n1, double n2, const double* Ug,
                                              const double* Ud, const double* gphi, double* gUg, double* gUd,
                                              double* gn) {
-  const double gam1 = g.gam1, invgam1 = g.invgam1, gog1 = g.gam * g.invgam1;
+  const double gam = g.gam, gam1 = g.gam1, invgam1 = g.invgam1;
   // ---- forward
   const double s2 = n0 * n0 + n1 * n1 + n2 * n2;
-  const double invnorm = rsqrt_(s2);
-  const double rnorm = s2 * invnorm;
+  const double yn = rsqrt_(s2), rnorm = sqrt_(s2, yn), invnorm = quot_(1.0, rnorm, yn);
   const double nx = n0 * invnorm, ny = n1 * invnorm, nz = n2 * invnorm;
   const double vitg2 = Ug[1] * Ug[1] + Ug[2] * Ug[2] + Ug[3] * Ug[3];
   const double vitd2 = Ud[1] * Ud[1] + Ud[2] * Ud[2] + Ud[3] * Ud[3];
   // sqrt(rho) and 1/sqrt(rho) of both sides
   const double rs1 = rsqrt_(Ug[0]), rs2 = rsqrt_(Ud[0]);
-  const double sq1 = Ug[0] * rs1, sq2 = Ud[0] * rs2;
+  const double sq1 = sqrt_(Ug[0], rs1), sq2 = sqrt_(Ud[0], rs2);
   const double ener1 = Ug[4] * invgam1 + 0.5 * Ug[0] * vitg2;
   const double ener2 = Ud[4] * invgam1 + 0.5 * Ud[0] * vitd2;
   const double usro = rcp_(sq1 + sq2);
   const double m2 = sq1 * Ug[1] + sq2 * Ud[1], m3 = sq1 * Ug[2] + sq2 * Ud[2], m4 = sq1 * Ug[3] + sq2 * Ud[3];
   const double uar2 = m2 * usro, uar3 = m3 * usro, uar4 = m4 * usro;
-  const double a1 = (ener1 + Ug[4]) * rs1, a2 = (ener2 + Ud[4]) * rs2;
+  const double a1 = quot_(ener1 + Ug[4], sq1, rs1), a2 = quot_(ener2 + Ud[4], sq2, rs2);
   const double uar5 = (a1 + a2) * usro;
   const double VdotN = nx * uar2 + ny * uar3 + nz * uar4;
   const bool left = VdotN > 0.0;
   const double* Us = left ? Ug : Ud;
   const double vits2 = left ? vitg2 : vitd2;
   const double vn = Us[1] * nx + Us[2] * ny + Us[3] * nz;
-  const double rss = left ? rs1 : rs2;
-  const double irs = rss * rss;  // 1/rho of the upwind side
-  const double H = gog1 * Us[4] * irs + 0.5 * vits2;
+  const double gr = gam1 * Us[0], igr = rcp_(gr);
+  const double H = quot_(gam * Us[4] + 0.5 * gr * vits2, gr, igr);
   const double f0 = Us[0] * vn;
   const double f1 = f0 * Us[1] + Us[4] * nx, f2 = f0 * Us[2] + Us[4] * ny, f3 = f0 * Us[3] + Us[4] * nz;
   const double f4 = f0 * H;
   const double qir = 0.5 * (uar2 * uar2 + uar3 * uar3 + uar4 * uar4);
   const double c2 = gam1 * (uar5 - qir);
   const double rc = rsqrt_(c2);
-  const double cr = c2 * rc;
-  const double cr2 = rc * rc;
+  const double cr = sqrt_(c2, rc);
+  const double cr2 = rcp_(c2);
   const double dif1 = Ud[0] - Ug[0];
   const double dif2 = Ud[0] * Ud[1] - Ug[0] * Ug[1];
   const double dif3 = Ud[0] * Ud[2] - Ug[0] * Ug[2];
@@ -672,7 +670,7 @@ __device__ __forceinline__ void roe_flux_adj(const Gas& g, double n0, double n1,
   double g_qir = dif1 * g_B;
   g_uar2 -= dif2 * g_B; g_uar3 -= dif3 * g_B; g_uar4 -= dif4 * g_B;
   // cr2 = 1/c2 ; cr = sqrt(c2) ; c2 = gam1 (uar5 - qir)
-  double g_c2 = -cr2 * cr2 * g_cr2 + 0.5 * rc * g_cr;
+  double g_c2 = -cr2 * cr2 * g_cr2 + quot_(0.5, cr, rc) * g_cr;
   g_uar5 += gam1 * g_c2;
   g_qir -= gam1 * g_c2;
   g_uar2 += uar2 * g_qir; g_uar3 += uar3 * g_qir; g_uar4 += uar4 * g_qir;
@@ -693,8 +691,8 @@ __device__ __forceinline__ void roe_flux_adj(const Gas& g, double n0, double n1,
     const double g_H = f0 * g_f4;
     gs[0] += vn * g_f0t;
     const double g_vn = Us[0] * g_f0t;
-    gs[4] += gog1 * irs * g_H;
-    gs[0] += -gog1 * Us[4] * (irs * irs) * g_H;
+    gs[4] += quot_(gam, gr, igr) * g_H;
+    gs[0] -= quot_(gam * Us[4], gr * Us[0], gam1 * (igr * igr)) * g_H;
     const double g_vits2 = 0.5 * g_H;
     gs[1] += 2.0 * Us[1] * g_vits2 + nx * g_vn;
     gs[2] += 2.0 * Us[2] * g_vits2 + ny * g_vn;
@@ -710,9 +708,10 @@ __device__ __forceinline__ void roe_flux_adj(const Gas& g, double n0, double n1,
   // Roe averages
   const double g_S = usro * g_uar5;
   double g_usro = (a1 + a2) * g_uar5;
-  g_ener1 += g_S * rs1; gL[4] += g_S * rs1;
-  g_ener2 += g_S * rs2; gR[4] += g_S * rs2;
-  double g_sq1 = -a1 * rs1 * g_S, g_sq2 = -a2 * rs2 * g_S;
+  const double gS1 = quot_(g_S, sq1, rs1), gS2 = quot_(g_S, sq2, rs2);
+  g_ener1 += gS1; gL[4] += gS1;
+  g_ener2 += gS2; gR[4] += gS2;
+  double g_sq1 = -a1 * gS1, g_sq2 = -a2 * gS2;
   const double gm2 = usro * g_uar2, gm3 = usro * g_uar3, gm4 = usro * g_uar4;
   g_usro += m2 * g_uar2 + m3 * g_uar3 + m4 * g_uar4;
   g_sq1 += Ug[1] * gm2 + Ug[2] * gm3 + Ug[3] * gm4;
@@ -728,8 +727,8 @@ __device__ __forceinline__ void roe_flux_adj(const Gas& g, double n0, double n1,
   const double g_vitd2 = 0.5 * Ud[0] * g_ener2;
   gL[1] += 2.0 * Ug[1] * g_vitg2; gL[2] += 2.0 * Ug[2] * g_vitg2; gL[3] += 2.0 * Ug[3] * g_vitg2;
   gR[1] += 2.0 * Ud[1] * g_vitd2; gR[2] += 2.0 * Ud[2] * g_vitd2; gR[3] += 2.0 * Ud[3] * g_vitd2;
-  gL[0] += 0.5 * rs1 * g_sq1;
-  gR[0] += 0.5 * rs2 * g_sq2;
+  gL[0] += quot_(0.5, sq1, rs1) * g_sq1;
+  gR[0] += quot_(0.5, sq2, rs2) * g_sq2;
 #pragma unroll
   for (int k = 0; k < 5; ++k) { gUg[k] += gL[k]; gUd[k] += gR[k]; }
   if (gn) {

@@ -97,6 +97,48 @@ def test_far_field_flux(probe):
     assert refined <= 1.02 * divided
 
 
+def roe(n, Vi, Vj):
+    """The physical flux of the upwind side and the acoustic wave against it."""
+    S = np.sqrt((n * n).sum(1))
+    e = n / S[:, None]
+    wi, wj = np.sqrt(Vi[:, 0]), np.sqrt(Vj[:, 0])
+    u = (wi[:, None] * Vi[:, 1:4] + wj[:, None] * Vj[:, 1:4]) / (wi + wj)[:, None]
+    Hi, Hj = ((cons(V)[:, 4] + V[:, 4]) / V[:, 0] for V in (Vi, Vj))
+    H = (wi * Hi + wj * Hj) / (wi + wj)
+    c = np.sqrt((G - 1) * (H - (u * u).sum(1) / 2))
+    un = (u * e).sum(1)
+    left = un.real > 0
+    Vs = np.where(left[:, None], Vi, Vj)
+    Us = cons(Vs)
+    m = Vs[:, 0] * (Vs[:, 1:4] * e).sum(1)
+    f = np.concatenate([m[:, None], m[:, None] * Vs[:, 1:4] + Vs[:, 4:5] * e,
+                        (m / Vs[:, 0] * (Us[:, 4] + Vs[:, 4]))[:, None]], 1)
+    z, lam = 0 * un, np.where(left, neg(un - c), pos(un + c))
+    add = apply(z, np.where(left, z, lam), np.where(left, lam, z), e, u, H, c, cons(Vj) - cons(Vi))
+    return (f + np.where(left[:, None], add, -add)) * S[:, None]
+
+
+def test_adjoint_of_the_roe_flux(probe):
+    rng = np.random.default_rng(2)
+    Vi = states(rng, N)
+    Vj = Vi * (1.0 + 0.2 * rng.uniform(-1, 1, (N, 5)))
+    n, w = normals(rng, N), rng.standard_normal((N, 5))
+    out = probe(1, np.column_stack([Vi, Vj, n, w]), 13)
+    # derivative of w . flux in every direction by a complex step
+    x = np.column_stack([Vi, Vj, n]).astype(L)
+    ref, h = np.empty((N, 13)), L(1e-40)
+    for k in range(13):
+        y = x.astype(CL)
+        s = np.where(k < 10, L(1.0), np.abs(x[:, 10:]).max(1))   # step relative to the normal's size
+        y[:, k] += 1j * h * s
+        ref[:, k] = ((roe(y[:, 10:], y[:, :5], y[:, 5:10]) * w).sum(1).imag / (h * s)).astype(np.float64)
+    e = [rms_error(out[:, a:b], ref[:, a:b]) for a, b in ((0, 10), (10, 13))]
+    print("adjoint of the Roe flux: states %.4g, normal %.4g" % tuple(e))
+    # with divisions and roots: 2.850e-16 and 2.647e-16
+    assert e[0] <= 1.02 * 2.850e-16
+    assert e[1] <= 1.02 * 2.647e-16
+
+
 def test_corrected_products(probe):
     # sqrt_ and quot_: half a unit in the last place, and what the correction's
     # own rounding adds (a few 2^-20 of it, from the seed's 23 bits)
