@@ -174,33 +174,30 @@ AEROF_HD void lsq_weights(const T* w, T dx0, T dx1, T dx2, T& W0, T& W1, T& W2) 
 }
 
 // ------------------------------------------------------------ reconstruction
-// RecFcn::vanalbada (RecFcn.h:432-446) with RecFcn::computeVanAlbadaFcn
-// (RecFcn.h:268-281); beta2 = 1-2 beta.  For a*b > 0 the limiter's numerator
-// a(b^2+eps) + b(a^2+eps) equals (a+b)(ab+eps); for a*b == 0 the reference's
-// 0.5 eps (a+b) is the same expression with ab+eps replaced by eps/2;
-// otherwise the result is 0 (branch-free selection).  The two sides' limiters
-// share b, and one reciprocal of the product of their denominators serves
-// both (1/d1 = d2/(d1 d2): denominators of squared state differences, at
-// least 2 eps, so the product stays a normal number).
+// RecFcn::computeVanAlbadaFcn (RecFcn.h:268-281).  For a*b > 0 the
+// numerator a(b^2+eps) + b(a^2+eps) equals (a+b)(ab+eps); for a*b == 0 the
+// reference's 0.5 eps (a+b) is the same expression with ab+eps replaced by
+// eps/2; otherwise the result is 0.  One reciprocal of the denominator,
+// branch-free selection.
 template <class T>
-AEROF_HD T vanalbada_num(T a, T b) {
+AEROF_HD T vanalbada_fcn(T a, T b) {
   const double eps = 1.e-16;
   T ab = a * b;
   const double abv = vof(ab);
-  return (a + b) * sel(abv > 0.0, ab + eps, sel(abv == 0.0, T(0.5 * eps), T(0.0)));
+  T den = a * a + (b * b + 2.0 * eps);
+  T t = sel(abv > 0.0, ab + eps, sel(abv == 0.0, T(0.5 * eps), T(0.0)));
+  return (a + b) * t * rcp_(den);
 }
+// RecFcn::vanalbada (RecFcn.h:432-446); beta2 = 1-2 beta
 template <class T>
 AEROF_HD void vanalbada(double beta, T Vi, T ddVij, T Vj, T ddVji, T& Vij, T& Vji) {
-  const double beta2 = 1.0 - 2.0 * beta, eps = 1.e-16;
+  const double beta2 = 1.0 - 2.0 * beta;
   T dVji = Vj - Vi;
   T dV = beta2 * dVji;
   T dVi = dV + 2.0 * beta * ddVij;
   T dVj = dV + 2.0 * beta * ddVji;
-  T b2 = dVji * dVji + 2.0 * eps;
-  T d1 = dVi * dVi + b2, d2 = dVj * dVj + b2;
-  T r = 0.5 * rcp_(d1 * d2);
-  Vij = Vi + vanalbada_num(dVi, dVji) * (r * d2);
-  Vji = Vj - vanalbada_num(dVj, dVji) * (r * d1);
+  Vij = Vi + 0.5 * vanalbada_fcn(dVi, dVji);
+  Vji = Vj - 0.5 * vanalbada_fcn(dVj, dVji);
 }
 // RecFcn::linear (RecFcn.h:240-249); beta1 = 1/2 - beta
 template <class T>

@@ -139,6 +139,37 @@ def test_adjoint_of_the_roe_flux(probe):
     assert e[1] <= 1.02 * 2.647e-16
 
 
+def limited(a, b):
+    eps, ab = L(1e-16), a * b
+    num = np.where(ab > 0, a * (b * b + eps) + b * (a * a + eps), np.where(ab == 0, eps * (a + b) / 2, 0 * a))
+    return num / (a * a + b * b + 2 * eps)
+
+
+def reconstructed(x):
+    Vi, di, Vj, dj = x.astype(L).T
+    beta = L(1.0 / 3.0)
+    d = Vj - Vi
+    b2 = (1 - 2 * beta) * d
+    return np.column_stack([Vi + limited(b2 + 2 * beta * di, d) / 2, Vj - limited(b2 + 2 * beta * dj, d) / 2])
+
+
+def test_limiter_rounding_and_range(probe):
+    rng = np.random.default_rng(3)
+    # the limited increments themselves: V_i = 0 leaves them bare
+    d = 10.0 ** rng.uniform(-6, 1, N)
+    x = np.column_stack([np.zeros(N), d * rng.uniform(0.2, 2.0, N), d, d * rng.uniform(0.2, 2.0, N)])
+    out, ref = probe(2, x, 2), reconstructed(x)
+    e = rms_error(out[:, :1], ref[:, :1])
+    print(f"limited increment: {e:.4g}")
+    # with a reciprocal per side: 1.353e-16
+    assert e <= 1.02 * 1.353e-16
+    # differences up to 1e100: the numerator's third powers still fit
+    big = np.column_stack([np.ones(64), np.ones(64), np.ones(64), np.ones(64)])
+    big *= rng.uniform(0.5, 2.0, big.shape) * 10.0 ** rng.uniform(70, 100, (64, 1))
+    out, ref = probe(2, big, 2), reconstructed(big)
+    assert np.isfinite(out).all() and rms_error(out, ref.astype(np.float64)) < 1e-14
+
+
 def test_corrected_products(probe):
     # sqrt_ and quot_: half a unit in the last place, and what the correction's
     # own rounding adds (a few 2^-20 of it, from the seed's 23 bits)
