@@ -171,7 +171,7 @@ __global__ void k_d_node_residual(int N, int E, int F, Gas g, const double* __re
 // of k_fv_blocked in dual arithmetic from staged records.  The gathered form
 // above (dual numbers interleaved in the caller's numbering, geometry
 // recomputed per node and edge) remains for meshes whose blocks do not fit
-// in shared memory: J v and (dR/dX) Xdot at 61^3 2.67 ms there, 1.13 ms here.
+// in shared memory: J v and (dR/dX) Xdot at 61^3 2.53 ms there, 1.00 ms here.
 
 // D2[n] = (dV, dX): dV = (dV/dU) v (VarFcnSGEuler.h:307-327; v null: 0), dX =
 // Xdot, or the coordinates when Xdot is null (the records whose gradients
@@ -993,11 +993,11 @@ __global__ void k_a_lam2(int N, const int* __restrict__ n2o, const double* __res
 
 // Threads of the reverse sweep.  Its staging leaves one CTA per SM, so the
 // warps in flight are the CTA's: 8 at 256 threads and 234 registers, 16 at
-// 512 and 128 (some spills).  Adjoint products at 101^3: 4.41 ms with 384,
-// 4.24 ms with 512 (4.70 ms with 256 and exact divisions and roots).  Their
-// chunk takes 105 KB beside the staged nodes; where 512 do not fit (stretched
-// cells: more than 448 nodes staged for blocks of 128) the sweep runs with 256
-// threads (up to 606), still without the gathers of the general form.
+// 512 and 128 (some spills).  Adjoint products at 101^3: 4.05 ms with 512,
+// 4.43 ms with 256.  Their chunk takes 105 KB beside the staged nodes; where
+// 512 do not fit (stretched cells: more than 448 nodes staged for blocks of
+// 128) the sweep runs with 256 threads (up to 606 nodes), still without the
+// gathers of the general form.
 constexpr int kRevThreads = 512;
 
 // Edges per chunk (one per thread) and doubles per edge kept in shared memory
@@ -1016,8 +1016,8 @@ constexpr int kRevEdge = 21;
 // that lie in the chunk, in edge order, g_V += g_Vside, g_grad += dx (x)
 // g_ddside; xor-tree lane sum, added up over the chunks; written to gVp /
 // gGp.  Keeping only the cotangents of the two reconstructed states per
-// edge (ten doubles, no chunks) had the limiter's reverse evaluated again by
-// each endpoint's gather: 1.62 ms per sweep at 101^3.
+// edge (ten doubles, no chunks) has the limiter's reverse evaluated again by
+// each endpoint's gather: 1.62 ms per sweep at 101^3, 1.50 with the chunks.
 template <bool GEO>
 __global__ void __launch_bounds__(kRevThreads, 1) k_a_fv_blocked(int N, int E, int NB, Gas g, int rec, double beta,
                                                          const ushort2* __restrict__ bl, const double* __restrict__ bn,

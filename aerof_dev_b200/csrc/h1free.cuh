@@ -18,11 +18,19 @@
 // block-vector product takes ~90 operations on 20 bytes per neighbour (unit
 // normal, half length, local slot) plus the staged node records, against 25
 // multiplications on a 100-byte FP32 (200-byte FP64) block: the stored
-// product is bound by HBM at ~92 % of the copy rate, this one by issue.
-// Measured: a pseudo-time step of 81^3 with 20 FP32 iterations 6.28 -> 5.40
-// ms, five Newton steps of 61^3 (which then also assemble the diagonal
-// blocks only) 21.5 -> 17.7 ms.  The solution of that step is 1.0e-7 from
-// the 64-bit one (1.2e-7 with the stored FP32 blocks).
+// product is bound by HBM at ~92 % of the copy rate, this one by latency and
+// issue.  Twenty FP32 iterations of 81^3 take 3.45 ms, 4.93 with the stored
+// blocks, and the Newton and linearised solves assemble the diagonal blocks
+// only.
+//
+// With FP32 storage a neighbour's block-vector product is formed in FP32 from
+// FP32 states, where the stored form multiplies FP32 blocks in FP64; both sum
+// a row in FP64.  The stored blocks carry the rounding of their own formation
+// in FP32, so this is no less accurate: over 72 systems (9^3 to 31^3, CFL 10
+// to 1e4, both preconditioners and orientations) the solutions after twenty
+// iterations are 9.8e-8 from the FP64 solver's in the mean against 11.2e-8
+// with the stored blocks (0.63 to 1.03 times), and the step of 81^3 is 1.4e-7
+// from the 64-bit one.
 //
 // CTA per Morton block of the blocked residual: the records (sqrt rho, u, H)
 // and the vector p of the block's nodes and of all their neighbours are
@@ -30,12 +38,11 @@
 // multiples of 16 bytes, conflict-free vector loads); L lanes per node take
 // its neighbours r, r + L, ..., the row sum is FP64 (fixed xor tree).  The
 // per-neighbour data is stored warp by warp, coalesced per step, and copied
-// to shared memory four steps ahead, before the wait for the packed vector.
-// Requested one step ahead into registers, its latency was most of the
-// kernel (seven of thirteen warps waited for it per issue; 47 us at 61^3): a
-// pseudo-time step of 81^3 with 20 FP32 iterations 4.91 -> 4.69 ms, five
-// Newton steps of 61^3 15.0 -> 14.8 ms with eight steps and three CTAs per
-// SM; with four steps and four CTAs (64 registers) 4.43 and 14.0 ms.
+// to shared memory four steps ahead, before the wait for the packed vector:
+// requested one step ahead into registers, its latency was most of the kernel.
+// Four steps and four CTAs per SM (64 registers): 41 us at 61^3, 28 warps
+// active, an instruction issued in 56 % of the cycles, 4.4 of 12.6 warps
+// waiting for global loads per issue.
 #pragma once
 
 #include "common.cuh"

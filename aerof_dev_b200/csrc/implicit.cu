@@ -109,25 +109,6 @@ __device__ __forceinline__ void store_diag(S* __restrict__ diag, int r, const do
 
 namespace aerof {
 
-// One thread per row r; a warp is one slice of the sliced layout, so for
-// each neighbour position k the 32 rows write every block element as one
-// coalesced line.  For the edge e = (r, s) (r first endpoint, sg = +1) or
-// (s, r) (r second, sg = -1) the approximate Roe Jacobians at the
-// un-reconstructed states (roejacappr3Dgas, FluxFcnDescSG.C:155-262;
-// roejac(n, Va, Vb, +1) = dF/dU of the first endpoint a, (.., -1) of the
-// second) give the off-diagonal block A_rs = sg dF/dU_s / vol_r and the
-// contribution sg dF/dU_r to the diagonal block (Edge.C:4503-4523).  Both
-// Jacobians share the Roe dissipation matrix D; it and the convective parts
-// H(V_s), H(V_r) are a multiple of the identity plus two rank-one terms
-// each, so an element takes a few operations and no 25-element block is held
-// in registers besides the diagonal sum (the eigenvector form of roejac6.f,
-// with its divisions per element: 0.44 ms at 81^3 in FP32, this one 0.30 ms,
-// for 0.75 GB of stored blocks).  Then the row's boundary
-// faces (Face.C:814-847), times 1/vol (SubDomain.C:1760-1765), + I/dt
-// (TimeState.C:731-756).  Every edge's Jacobians are evaluated once by each
-// of its two rows.  TR: the transpose H1^T is stored instead (block k of
-// row r = A_sr^T with A_sr = -sg dF/dU_r / vol_s, the Jacobian formed for
-// the diagonal), for products with the transpose that read coalesced.
 // Boundary-face blocks of the boundary rows (Face.C:814-847: FD flux
 // Jacobians for far field, the analytic wall block, in face order), summed
 // per row into fsum; k_jac_rows adds them to the diagonal.  Kept apart so
@@ -164,6 +145,25 @@ template <class S> struct JacThreads {
   static constexpr int B = sizeof(S) == 4 ? 4 : 1;
 };
 
+// One thread per row r; a warp is one slice of the sliced layout, so for
+// each neighbour position k the 32 rows write every block element as one
+// coalesced line.  For the edge e = (r, s) (r first endpoint, sg = +1) or
+// (s, r) (r second, sg = -1) the approximate Roe Jacobians at the
+// un-reconstructed states (roejacappr3Dgas, FluxFcnDescSG.C:155-262;
+// roejac(n, Va, Vb, +1) = dF/dU of the first endpoint a, (.., -1) of the
+// second) give the off-diagonal block A_rs = sg dF/dU_s / vol_r and the
+// contribution sg dF/dU_r to the diagonal block (Edge.C:4503-4523).  Both
+// Jacobians share the Roe dissipation matrix D; it and the convective parts
+// H(V_s), H(V_r) are a multiple of the identity plus two rank-one terms
+// each, so an element takes a few operations and no 25-element block is held
+// in registers besides the diagonal sum (the eigenvector form of roejac6.f,
+// with its divisions per element: 0.44 ms at 81^3 in FP32, this one 0.30 ms,
+// for 0.75 GB of stored blocks).  Then the row's boundary
+// faces (Face.C:814-847), times 1/vol (SubDomain.C:1760-1765), + I/dt
+// (TimeState.C:731-756).  Every edge's Jacobians are evaluated once by each
+// of its two rows.  TR: the transpose H1^T is stored instead (block k of
+// row r = A_sr^T with A_sr = -sg dF/dU_r / vol_s, the Jacobian formed for
+// the diagonal), for products with the transpose that read coalesced.
 template <class S, bool TR>
 __global__ void __launch_bounds__(JacThreads<S>::T, JacThreads<S>::B)
     k_jac_rows(int N, int E, int F, Gas g, const double* __restrict__ Ub0,
@@ -437,11 +437,6 @@ __global__ void k_bj_pack(int N, const S* __restrict__ dinv, const S* x, size_t 
 }
 
 // ------------------------------------------------------------ vector ops
-__global__ void k_axpby(size_t n, double a, const double* __restrict__ x, double b, const double* __restrict__ y,
-                        double* __restrict__ z) {
-  size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (q < n) z[q] = a * x[q] + b * y[q];
-}
 template <class TI, class TO>
 __global__ void k_scale(size_t n, double a, const TI* __restrict__ x, TO* __restrict__ z) {
   size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -888,10 +883,9 @@ __global__ void k_ilu_factor(int i0, int cnt, int s0, const int* __restrict__ rj
 // bound by the latency of that chain, not by the blocks' bytes.  So the
 // launches overlap (launch_pdl): the list, the row's first block and, going
 // backward, its diagonal are requested before the wait for the previous
-// colour, and only w is read after it.  41^3, eight colours, four FP32
-// vectors: a colour took 11.2 us with four lanes per row and ordinary
-// launches, 47 of the 98 ms of four sensitivities; overlapping launches and
-// eight lanes per row 87.6 ms; the vectors interleaved 80.9 ms.
+// colour, and only w is read after it.  Four sensitivities of 41^3 (eight
+// colours, four FP32 vectors) in the same solver: 98 ms with ordinary
+// launches, four lanes per row and a vector after the other, 81 ms with this.
 constexpr int kIluLanes = 8;
 constexpr int kIluT = 128;
 // a row's block as stored (load_block without the conversion: FP32 blocks
@@ -1101,8 +1095,7 @@ static void ilu_apply(aerof_gpu_ctx* c, int R, const TI* x, size_t xs, TO* z, si
     }
   };
   // four vectors per pass over a block: one per pass, with four times the
-  // threads, reads the blocks four times (four sensitivities of 41^3, both
-  // with a vector's gathers in one lane: 105 ms against 87.6 ms)
+  // threads, reads the blocks four times and was a fifth slower
   auto run = [&](const auto* lu) {
     if (R == 1) sweeps(lu, std::integral_constant<int, 1>{});
     else sweeps(lu, std::integral_constant<int, 4>{});
@@ -1272,17 +1265,13 @@ static void gs_backsolve(aerof_gpu_ctx* c, const GsDev& st, int R) {
 // dynamic shared memory of the second sweep
 static size_t gs_smem(int m) { return sizeof(double) * ((m > kGsMax ? 0 : (size_t)3 * (m + 1)) + kGsL); }
 
-// Gram-Schmidt step j of the R systems and the Givens update.  Measured with
-// everything around it (stored products): a pseudo-time step of 81^3 with 20
-// FP32 iterations 7.21 -> 6.28 ms against one cooperative launch per
-// iteration with a grid barrier per dot product; five Newton steps of 61^3
-// (8 to 20 iterations each) 28.7 -> 21.5 ms, where also the idle launches
-// after convergence went (kGsAhead); four sensitivities of 41^3 in one batch
-// 171 -> 102 ms, where every system took j + 2 launches per iteration and
-// the host a wait.  On top of that and of the products from the states:
-// without a last block's fences, sums and triangular solve between the sweeps
-// and with overlapping launches, 5.13 -> 4.95 ms, 17.0 -> 15.4 ms and 101 ->
-// 98 ms (neither of the two gives it alone).
+// Gram-Schmidt step j of the R systems and the Givens update: two launches
+// and two reads of the basis.  Modified Gram-Schmidt in one cooperative launch
+// with a grid barrier per dot product took, with the stored products beside
+// either, 7.2 ms instead of 6.3 for a pseudo-time step of 81^3 with 20 FP32
+// iterations.  In the solver as it is, an iteration of 61^3 takes 110 us of
+// overlapping kernels: product 38, first sweep 26, second 32, preconditioner
+// 17 (each with its wait for the one before).
 template <class TV>
 static void gs_iteration(aerof_gpu_ctx* c, const GsDev& st, int R, size_t n, int j, TV* V, size_t vs, size_t ld,
                          const TV* W, size_t ws) {

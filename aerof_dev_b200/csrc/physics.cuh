@@ -381,10 +381,10 @@ AEROF_HD void post_dVdU(const Gas& g, const double* V, const double* mat, double
   }
 }
 
-// roejac6.f:1-316 (type 0, prec 0 -> beta 1, dissipation coefficient 1):
-// approximate Jacobian of the Roe flux w.r.t. the conservative state Ug,
-// (H(Ug) + sw |A|_Roe) |n| / 2, sw = +1, or called with the states swapped w.r.t.
-// the second, sw = -1.
+// Approximate Jacobian of the Roe flux w.r.t. either state (roejac6.f:1-316,
+// type 0, prec 0 -> beta 1, dissipation coefficient 1): (A(V) +- |A|_Roe)
+// |n| / 2, from the forms below.
+
 // a*b + c*d with both products rounded (no fused multiply-add), so the
 // result does not depend on which pair is named first
 AEROF_HD double sym_dot2(double a, double b, double c, double d) {

@@ -477,8 +477,8 @@ __device__ __forceinline__ void face_items(const Gas& g, const FaceArgs& fa, con
   }
 }
 
-// The same sums in the blocked organisation: every edge is evaluated once
-// (both endpoints' terms min(+-un - a, 0) S of the mean state) by the block
+// The sums of k_timestep in the blocked organisation: every edge is evaluated
+// once (both endpoints' terms min(+-un - a, 0) S of the mean state) by the block
 // of its first endpoint, from staged node states; the two terms stay in
 // shared memory for the gather per node, the second endpoint's goes to
 // wspill for a block-crossing edge.  With un S = u.n and a S =
@@ -555,8 +555,8 @@ __device__ __forceinline__ void wave_block(int N, int E, int NB, const Gas& g, c
 // The launches of a residual and of an explicit step overlap (launch_pdl):
 // a kernel reads its block's bounds and lists before it waits for the one
 // before.  With the wave sums in the same launch (rk2_blocked_dev) ten steps
-// of 21^3 take 334 instead of 447 us; the residual of 47^3 83.5 instead of 90
-// us; 101^3 is the same.
+// of 21^3 take 336 us, 447 with ordinary launches; the residual of 47^3 83 and
+// 90 us; 101^3 is the same.
 template <int THREADS, int MINB>
 __global__ void __launch_bounds__(THREADS, MINB)
     k_fv_blocked(int N, int E, int NB, Gas g, int rec, double beta, int failsafe,
@@ -653,8 +653,8 @@ __global__ void __launch_bounds__(THREADS, MINB)
     // global node ids are needed only to tag unphysical states
     const int gi = n0 + li, gj = lj < nn ? n0 + lj : hs[lj - nn];
     double pi[8], pj[8], ddij[5], ddji[5];
-    // 16-byte loads of the staged records (46 8-byte ones, one gradient
-    // component at a time, before: 618 -> 600 us for the residual of 101^3)
+    // 16-byte loads of the staged records (with 8-byte ones, one gradient
+    // component at a time, the residual of 101^3 takes 3 % longer)
     lds_rec<8>(Pn + kPS * li, pi);
     lds_rec<8>(Pn + kPS * lj, pj);
     if (rec != AEROF_REC_CONSTANT) {
@@ -1377,9 +1377,7 @@ static int residual_blocked_dev(aerof_gpu_ctx* c, const double* dU, double* dR, 
   // only the failsafe needs the count before the assembly (it re-runs the
   // edges); otherwise the whole residual is queued and waited for once, its
   // count written to the host by the assembly.  Copying the count back and
-  // waiting for it before the assembly left the GPU idle for 12 us per call
-  // (641 -> 629 us per call at 101^3, 121 -> 103 us at 47^3; ten RK2 steps
-  // of 21^3, which now wait once: 1.32 -> 1.00 ms)
+  // waiting for it before the assembly leaves the GPU idle for 12 us per call
   int bad = 0;
   if (mode == kCountSync && failsafe) {
     AEROF_CUDA(cudaMemcpyAsync(&bad, cnt, sizeof(int), cudaMemcpyDeviceToHost, s));

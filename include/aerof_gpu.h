@@ -61,9 +61,16 @@ extern "C" {
 #define AEROF_PC_JACOBI 0
 #define AEROF_PC_ILU0 1
 
-/* Precision of the assembled H1 Jacobian and block-Jacobi preconditioner. */
+/* Precision of the assembled H1 Jacobian and of its preconditioner.  FP32:
+ * blocks, factors and the Krylov vectors of aerof_gpu_gmres, aerof_gpu_newton
+ * and of the inner solves are stored in FP32.  Products with stored blocks
+ * (aerof_gpu_matvec, an operator given by aerof_gpu_set_jacobian) multiply
+ * and sum in FP64; the products of the solvers with an operator assembled
+ * here are formed from FP32 node states, each neighbour's in FP32, summed per
+ * row in FP64.  Dot products, norms, the Hessenberg system, right-hand sides
+ * and solutions are FP64 either way.                                       */
 #define AEROF_PREC_FP64 64
-#define AEROF_PREC_FP32 32 /* FP32 blocks, FP64 vectors and accumulation */
+#define AEROF_PREC_FP32 32
 
 typedef struct aerof_gpu_ctx aerof_gpu_ctx;
 
