@@ -291,7 +291,9 @@ __global__ void __launch_bounds__(256, sizeof(S) == 4 ? 4 : 2)
     const S u0 = wr * sr[1] + ws * ss[1], u1 = wr * sr[2] + ws * ss[2], u2 = wr * sr[3] + ws * ss[3];
     const S H = wr * sr[4] + ws * ss[4];
     const S qq = half * (u0 * u0 + u1 * u1 + u2 * u2);
-    const S c2 = gam1 * (H - qq), ic = h1_rsqrt(c2), c = c2 * ic;
+    // an entry past the node's list averages the node with itself: its zero
+    // length must not meet the infinity of a node without pressure
+    const S c2 = hk == S(0) ? S(1) : gam1 * (H - qq), ic = h1_rsqrt(c2), c = c2 * ic;
     const S un = u0 * x0 + u1 * x1 + u2 * x2;
     const S f1 = h1_abs(un), fp = h1_abs(un + c), fm = h1_abs(un - c);
     const S S1 = half * (fp + fm) - f1, S2 = half * (fp - fm);

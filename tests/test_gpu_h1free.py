@@ -79,3 +79,33 @@ def test_linearized_solve_leaves_its_operator(gpu_lib, transpose):
     fresh = A.MatVecProdH1(A.Context.from_mesh(m, W.freestream(0.5)), 32)
     fresh.evaluate(U)
     assert rel_l2(A.MatVecProdH1(ctx, 32).blocks(), fresh.blocks()) < 1e-6
+
+
+@pytest.mark.parametrize("prec,tol", [(64, 1e-9), (32, 1e-4)])
+@pytest.mark.parametrize("nb", ["64", "128", "256"])
+def test_node_without_pressure(gpu_lib, monkeypatch, nb, prec, tol):
+    # the lanes of a node take its neighbours in whole steps; what fills the
+    # last step up must not contribute, also where the node's own speed of
+    # sound is zero (its averages with its neighbours are regular)
+    A = gpu_lib
+    monkeypatch.setenv("AEROF_BLOCK_NODES", nb)
+    m = W.make_lattice_mesh(6, jitter=0.2, codes="channel")
+    ctx = A.Context.from_mesh(m, W.freestream(0.6), reconstruction=1)
+    U = W.perturbed_state(ctx.N, 0.6, amp=0.02)
+    for i in (86, 93, 122):   # inner nodes, no neighbours of each other
+        U[i, 4] = 0.5 * (U[i, 1:4] ** 2).sum() / U[i, 0]
+    sp = A.SpaceOperator(ctx)
+    dt = sp.computeTimeStep(U, 10.0)
+    b = np.random.default_rng(0).standard_normal((ctx.N, 5))
+    mv, pc = A.MatVecProdH1(ctx, prec), A.JacobiPrec(ctx)
+    for transpose in (False, True):
+        mv.evaluate(U, dt)
+        blocks = mv.blocks()
+        assert np.isfinite(blocks).all()
+        pc.setup()
+        free, its, _ = A.GmresSolver(ctx, 8, 8, 0.0).solve(b, transpose=transpose)
+        mv.set_blocks(blocks)
+        pc.setup()
+        stored, its2, _ = A.GmresSolver(ctx, 8, 8, 0.0).solve(b, transpose=transpose)
+        assert its == its2 == 8
+        assert np.isfinite(free).all() and rel_l2(free, stored) < tol
