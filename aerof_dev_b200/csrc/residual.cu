@@ -519,7 +519,10 @@ __device__ __forceinline__ void wave_block(int N, int E, int NB, const Gas& g, c
     const double s2 = nx * nx + ny * ny + nz * nz;
     double2 w = make_double2(0.0, 0.0);
     if (s2 > 0.0) {
-      const double x = g.gam * p * rcp_(rho) * s2, as = x * rsqrt_(x);
+      const double x = g.gam * p * rcp_(rho) * s2;
+      double as = x * rsqrt_(x);
+      // zero, negative and infinite states as the divisions and roots take them
+      if (!(x > 1e-290 && x < 1e290)) as = sqrt(g.gam * p / rho) * sqrt(s2);
       w = make_double2(fmin(us - as, 0.0), fmin(-us - as, 0.0));
     }
     Ws[q - e0] = w;

@@ -121,3 +121,30 @@ def test_reverse_sweep_with_fewer_threads(gpu_lib, monkeypatch, n, squash, nodes
     v = rng.standard_normal((N, 5))
     Jv = S.jvp(U, v)
     assert abs((lam * Jv).sum() - (w * v).sum()) < 1e-12 * np.linalg.norm(lam) * np.linalg.norm(Jv)
+
+
+@pytest.mark.parametrize("what", ["no pressure", "negative pressure", "infinite density", "infinite energy"])
+def test_time_step_at_degenerate_states(gpu_lib, what):
+    # the blocked sums take the reciprocals' special values as the divisions
+    # and roots of the edge organisation do
+    A = gpu_lib
+    m = W.make_lattice_mesh(6, jitter=0.2, codes="channel")
+    Ub = W.freestream(0.6)
+    ctx = A.Context.from_mesh(m, Ub)
+    edge = A.Context.from_mesh(m, Ub, residual_kernel=A.KERNEL_EDGE)
+    U = W.perturbed_state(ctx.N, 0.6, amp=0.02)
+    for i in (86, 87, 122):   # two neighbours, and one alone
+        if what == "no pressure":
+            U[i] = [1.0, 0.0, 0.0, 0.0, 0.0]
+        elif what == "negative pressure":
+            U[i, 4] = -3.0
+        elif what == "infinite density":
+            U[i, 0] = np.inf
+        else:
+            U[i, 4] = np.inf
+    a = A.SpaceOperator(ctx).computeTimeStep(U, 0.8)
+    b = A.SpaceOperator(edge).computeTimeStep(U, 0.8)
+    ok = np.isfinite(b)
+    assert np.array_equal(np.isfinite(a), ok) and ok.sum() > 100
+    assert rel_l2(a[ok], b[ok]) < 1e-13
+    assert np.array_equal(np.isnan(a), np.isnan(b))
