@@ -234,7 +234,10 @@ __global__ void __launch_bounds__(256) k_gs_first(size_t n, VecIn B, const TV* _
   const size_t p = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= n) return;
   const double b = B.p[q][p], r = FIRST ? b : b - (double)Wv[(size_t)q * ws + p];
-  V[(size_t)q * vs + p] = (TV)(st.d[(size_t)q * st.sd + st.oScal() + 2] * r);
+  // (a norm beyond FP64 has the reciprocal 0: FP32 vectors are then not a
+  // number, as the right-hand side is infinite in FP32, and so is the result)
+  const double sc = st.d[(size_t)q * st.sd + st.oScal() + 2];
+  V[(size_t)q * vs + p] = sc != 0.0 ? (TV)(sc * r) : (TV)r * TV(0);
 }
 // basis vector v of the running systems normalised (flexible method)
 template <class TV>

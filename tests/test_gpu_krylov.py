@@ -135,3 +135,21 @@ def test_long_restarts(gpu_lib, krylov):
     x, i, r = A.GmresSolver(ctx, krylov, krylov, 1e-9).solve(B[0])
     assert i < 136 and r <= 1e-9 * np.linalg.norm(B[0])
     assert np.linalg.norm(mv.apply(x) - B[0]) <= 1e-8 * np.linalg.norm(B[0])
+
+
+def test_right_hand_side_beyond_the_range_is_not_reported_as_solved(gpu_lib):
+    # the squared norm of 1e200 overflows FP64: the FP32 solver's residual is
+    # not a number, and no small one
+    A = gpu_lib
+    m = W.make_lattice_mesh(4, jitter=0.2, codes="channel")
+    ctx = A.Context.from_mesh(m, W.freestream(0.5))
+    U = W.smooth_state(m["X"], 0.5)
+    A.MatVecProdH1(ctx, 32).evaluate(U, A.SpaceOperator(ctx).computeTimeStep(U, 10.0))
+    A.JacobiPrec(ctx).setup()
+    b = np.random.default_rng(0).standard_normal((ctx.N, 5))
+    x, its, res = A.GmresSolver(ctx, 5, 10, 1e-6).solve(1e200 * b)
+    assert np.isnan(res) and not np.isfinite(x).all()
+    # far smaller ones are solved at any scale that FP32 can hold the answer of
+    for s in (1e-25, 1.0, 1e25):
+        xs, i, r = A.GmresSolver(ctx, 30, 30, 1e-4).solve(s * b)
+        assert r <= 1e-4 * s * np.linalg.norm(b) and np.isfinite(xs).all()
