@@ -385,6 +385,19 @@ __device__ __forceinline__ void load5(const double* __restrict__ P, int j, doubl
   v[4] = P[8 * (size_t)j + 4];
 }
 
+// Diagonal entries that cancelled to exactly zero, of contributions whose
+// identity parts add up to size: round-off of that size instead.  The
+// reference's eigenvector products leave some there (the first entry of |A| on
+// supersonic edges), and block-Jacobi leaves a block with a zero on its
+// diagonal uninverted (DiagMatrix.C:44-80); a fluid at rest has no such
+// contributions and keeps its zero.  T: stride of the block's elements.
+template <int T>
+__device__ __forceinline__ void keep_nonzero(double* a, double size) {
+#pragma unroll
+  for (int k = 0; k < 5; ++k)
+    if (a[T * 6 * k] == 0.0 && size > 0.0) a[T * 6 * k] = 0x1p-54 * size;
+}
+
 // Diagonal blocks of H1 alone (what block-Jacobi needs), in FP64 from the
 // caller's records: thread per row, sum over its edges of |A||n|/2 (the two
 // rank-one terms and |un| I), A(V_r, m_r), the face blocks, 1/vol, I/dt.
@@ -402,7 +415,9 @@ __global__ void __launch_bounds__(128) k_h1_diag(int N, int E, Gas g, const int*
 #pragma unroll
   for (int k = 0; k < 25; ++k) a[k] = 0.0;
   // + w I + R1 (x) p + R2 (x) t with R1 = (1, u, H), R2 = (0, n, un)
+  double size = 0.0;   // sum of |w|, see keep_nonzero
   auto rank = [&](double w, const double* u, double H, const double* n, double un, const double* p, const double* t) {
+    size += fabs(w);
 #pragma unroll
     for (int c = 0; c < 5; ++c) {
       a[c] += p[c];
@@ -461,6 +476,7 @@ __global__ void __launch_bounds__(128) k_h1_diag(int N, int E, Gas g, const int*
     for (int k = 0; k < 25; ++k) a[k] += fsum[25 * (size_t)br + k];
   }
   const double iv = 1.0 / vol[r], it = dt ? 1.0 / dt[r] : 0.0;
+  keep_nonzero<1>(a, size);
 #pragma unroll
   for (int k = 0; k < 25; ++k) a[k] = a[k] * iv + (k % 6 == 0 ? it : 0.0);
   store_diag<S, TR>(diag, r, a);

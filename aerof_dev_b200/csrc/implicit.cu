@@ -188,6 +188,7 @@ __global__ void __launch_bounds__(JacThreads<S>::T, JacThreads<S>::B)
   double Vr[5];
 #pragma unroll
   for (int k = 0; k < 5; ++k) Vr[k] = P[8 * (size_t)r + k];
+  double size = 0.0;   // see keep_nonzero
   const double volr = 1.0 / vol[r];
   const int p0 = nbr_ptr[r], p1 = nbr_ptr[r + 1];
   for (int p = p0; p < p1; ++p) {
@@ -228,6 +229,7 @@ __global__ void __launch_bounds__(JacThreads<S>::T, JacThreads<S>::B)
     // (x) a + R2 (x) b at each state (RankTwo)
     const RankTwo<S> D = roe_dissipation<S>(g, un, VrS, VsS);
     const RankTwo<S> hr = flux_jacobian<S>(g, un, VrS), hs = flux_jacobian<S>(g, un, VsS);
+    size += fabs((double)(D.w * half_rn));
 #pragma unroll
     for (int j = 0; j < 5; ++j) {
 #pragma unroll
@@ -253,6 +255,7 @@ __global__ void __launch_bounds__(JacThreads<S>::T, JacThreads<S>::B)
 #pragma unroll
     for (int k = 0; k < 25; ++k) a[T * k] += fsum[25 * (size_t)br + k];
   }
+  keep_nonzero<T>(a, size);
   double v[25];
 #pragma unroll
   for (int k = 0; k < 25; ++k) v[k] = a[T * k] * volr;
