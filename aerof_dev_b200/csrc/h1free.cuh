@@ -81,8 +81,10 @@ __global__ void k_h1_records(int N, Gas g, const int* __restrict__ n2o, const do
 // Per-neighbour data of every node, in the order the product kernel reads
 // it (warp w's step k, lane l at (wptr[w] + k) 32 + l): outward unit normal
 // and half length, four values, and the neighbour's staged slot; entries
-// past a node's list have zero length and its own slot.  mrow[n]: (sum of
-// n/2, 1/vol).  Thread per lane of the product kernel.
+// past a node's list have zero length and its first neighbour's slot (with its
+// own, the average at a node without pressure would be no number, and no
+// length cancels that).  mrow[n]: (sum of n/2, 1/vol).  Thread per lane of the
+// product kernel.
 template <class S>
 __global__ void k_h1_geometry(int N, int NB, int E, const int* __restrict__ n2o, const int* __restrict__ o2n,
                               const int* __restrict__ nbr_ptr, const int* __restrict__ nbr_node,
@@ -98,23 +100,23 @@ __global__ void k_h1_geometry(int N, int NB, int E, const int* __restrict__ n2o,
   const bool act = t < nn;
   const int o = act ? n2o[n0 + t] : 0;
   const int p0 = act ? nbr_ptr[o] : 0, deg = act ? nbr_ptr[o + 1] - p0 : 0;
+  auto staged = [&](int e) {   // slot of neighbour e
+    const int j = o2n[nbr_node[p0 + e]];
+    if (j >= n0 && j < n0 + nn) return j - n0;
+    int lo = hptr[blk], hi = hptr[blk + 1] - 1;   // ascending halo ids
+    while (lo < hi) {
+      const int mid = (lo + hi) >> 1;
+      if (hnode[mid] < j) lo = mid + 1;
+      else hi = mid;
+    }
+    return nn + lo - hptr[blk];
+  };
   for (int k = 0; k < steps; ++k) {
     const size_t at = ((size_t)w0 + k) * 32 + lane;
     const int e = r + k * L;
     double u[4] = {0.0, 0.0, 0.0, 0.0};
-    int sl = act ? t : 0;
+    const int sl = deg ? staged(e < deg ? e : 0) : (act ? t : 0);
     if (e < deg) {
-      const int j = o2n[nbr_node[p0 + e]];
-      if (j >= n0 && j < n0 + nn) sl = j - n0;
-      else {
-        int lo = hptr[blk], hi = hptr[blk + 1] - 1;   // ascending halo ids
-        while (lo < hi) {
-          const int mid = (lo + hi) >> 1;
-          if (hnode[mid] < j) lo = mid + 1;
-          else hi = mid;
-        }
-        sl = nn + lo - hptr[blk];
-      }
       const int er = nbr_edge[p0 + e];
       const size_t l = (size_t)(er & 0x7fffffff);
       const double sg = er < 0 ? -1.0 : 1.0;
@@ -291,9 +293,7 @@ __global__ void __launch_bounds__(256, sizeof(S) == 4 ? 4 : 2)
     const S u0 = wr * sr[1] + ws * ss[1], u1 = wr * sr[2] + ws * ss[2], u2 = wr * sr[3] + ws * ss[3];
     const S H = wr * sr[4] + ws * ss[4];
     const S qq = half * (u0 * u0 + u1 * u1 + u2 * u2);
-    // an entry past the node's list averages the node with itself: its zero
-    // length must not meet the infinity of a node without pressure
-    const S c2 = hk == S(0) ? S(1) : gam1 * (H - qq), ic = h1_rsqrt(c2), c = c2 * ic;
+    const S c2 = gam1 * (H - qq), ic = h1_rsqrt(c2), c = c2 * ic;
     const S un = u0 * x0 + u1 * x1 + u2 * x2;
     const S f1 = h1_abs(un), fp = h1_abs(un + c), fm = h1_abs(un - c);
     const S S1 = half * (fp + fm) - f1, S2 = half * (fp - fm);
